@@ -88,6 +88,7 @@ struct ProfScope {   // brackets the launches issued during its lifetime when pr
 struct RuntimeFlags {
     bool pdl = true;                 // B200ATTN_PDL=0: ordinary stream order instead of programmatic dependent launch
     bool decode_gemm_tc = false;     // B200ATTN_DECODE_GEMM=tc: the fused decode step on the tcgen05 skinny GEMMs (default: library GEMMs + norm / SwiGLU kernels)
+    bool decode_gemm_rows = true;    // B200ATTN_DECODE_GEMM=cublas: library GEMMs for few rows too
     bool lm_head_cublas = false;     // B200ATTN_LM_HEAD=cublas: library GEMM + argmax kernel instead of the fused epilogue
     bool la_prefill_serial = false;  // B200ATTN_LA_PREFILL=serial: token-serial fp32 recurrence instead of the chunked tensor-core kernels
     unsigned la_stagger_ns = 2750;   // B200ATTN_LA_DECODE_STAGGER_NS
@@ -114,19 +115,34 @@ void per_device_once_end(PerDeviceOnce& o, int dev);
 // Launch with the programmatic-stream-serialization attribute: the kernel may become resident while the previous
 // kernel of the stream drains; it must call pdl_wait() before touching anything that kernel produced or still reads.
 // `on` = false (or B200ATTN_PDL=0) gives the ordinary stream order.
+//
+// `share_sm`: the launch asks for the largest shared-memory part of the L1 store.  An SM keeps the split that it was given until it is
+// empty, so with one split for a chain of kernels the next one can become resident, and fetch its weights, beside the one that still
+// runs: a decode step of 8 rows took 196 us with the splits that the driver chose and 149 us with one.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+inline cudaError_t launch_pdl_split(bool on, bool share_sm, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (on && g_flags.pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (share_sm) {
+        attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[n++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = (on && g_flags.pdl) ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+    return launch_pdl_split(on, false, kernel, grid, block, smem, s, static_cast<Args&&>(args)...);
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {

@@ -26,6 +26,7 @@ void refresh_runtime_flags() {
     RuntimeFlags f;
     f.pdl = env("B200ATTN_PDL")[0] != '0';
     f.decode_gemm_tc = env("B200ATTN_DECODE_GEMM")[0] == 't';
+    f.decode_gemm_rows = env("B200ATTN_DECODE_GEMM")[0] != 'c';
     f.lm_head_cublas = env("B200ATTN_LM_HEAD")[0] == 'c';
     f.la_prefill_serial = env("B200ATTN_LA_PREFILL")[0] == 's';
     f.la_stagger_ns = env_uint("B200ATTN_LA_DECODE_STAGGER_NS", 2750u, 20000u);

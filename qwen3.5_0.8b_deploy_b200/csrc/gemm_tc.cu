@@ -532,6 +532,12 @@ int gemm_tc_residual(cudaStream_t s, const __half* X, const __half* W, float* h,
     return 0;
 }
 
+int launch_argmax_unpack(unsigned long long* d_packed, int M, int* tokens, cudaStream_t s) {
+    launch_pdl_split(true, M <= kRowsGemmMax, argmax_unpack_kernel, dim3(ceil_div(M, 128)), dim3(128), 0, s, d_packed, M, tokens);
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+
 // tokens[m] = argmax_n X[m] . W[n]   (d_packed: M zeroed 64-bit words, left zeroed again).
 int gemm_tc_argmax(cudaStream_t s, const __half* X, const __half* W, unsigned long long* d_packed, int* tokens,
                    int M, int N, int K, int* d_error) {
@@ -540,9 +546,7 @@ int gemm_tc_argmax(cudaStream_t s, const __half* X, const __half* W, unsigned lo
     B2_TRY(fp16_map(X, M, K, 128, &mx));
     B2_TRY(fp16_map(W, N, K, 256, &mw));
     B2_TRY((launch_one<256, kEpiArgmax>(mx, mw, M, N, K, 1, nullptr, 0, 0, nullptr, d_packed, nullptr, 0.f, d_error, s)));
-    launch_pdl(argmax_unpack_kernel, dim3(ceil_div(M, 128)), dim3(128), 0, s, d_packed, M, tokens);
-    B2_LAUNCH_CHECK();
-    return 0;
+    return launch_argmax_unpack(d_packed, M, tokens, s);
 }
 
 }  // namespace b200

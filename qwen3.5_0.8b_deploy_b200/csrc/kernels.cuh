@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "gemm_rows.cuh"
 
 #include <vector>
 
@@ -92,16 +93,31 @@ int gemm_tc_residual(cudaStream_t s, const __half* X, const __half* W, float* h,
                      int* d_error);
 int gemm_tc_argmax(cudaStream_t s, const __half* X, const __half* W, unsigned long long* d_packed, int* tokens,
                    int M, int N, int K, int* d_error);
+int launch_argmax_unpack(unsigned long long* d_packed, int M, int* tokens, cudaStream_t s);   // packed argmax words -> tokens, words back to zero
 void gemm_tc_forget(const void* ptr);
 int gemm_tc_map(const void* ptr, int rows, int cols, int box_rows, void* tensor_map_out);   // cached CUtensorMap of a fp16 matrix
-// The fused form of a decode step (tcgen05 projections): the operator's input is the UN-normalised residual stream as
+// The fused forms of a decode step.  On tcgen05 (gemm_tc.cu): the operator's input is the UN-normalised residual stream as
 // fp16 (`d_x`), whose RMSNorm scale the input projection applies in its epilogue from `rowsq`; the output projection
 // adds into the residual stream `d_y` and refreshes `xh` and `rowsq` for the next projection.
 struct DecodeOut {
     __half* xh;        // [rows, hidden] fp16 copy of the residual stream (read as d_x, rewritten by the output projection)
     float* rowsq;      // [128][kRowsqParts] partial sums of squares of the residual rows
     float eps;         // RMSNorm epsilon
+    bool rows = false; // few rows (gemm_rows.cu): d_x is the fp32 residual stream, normalised by the projection itself, or already normalised
+                       // fp16 rows; xh and rowsq are not used
 };
+
+// The same over few rows: Y = norm(X) W^T or X W^T, and h += X W^T.
+inline int rows_project(cudaStream_t s, const void* x, bool normed, float eps, const __half* w, float* y, int M, int N, int K, int* error) {
+    RowsGemm a;
+    a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.eps = eps; a.y = y; a.ldy = N; a.error = error;
+    return gemm_rows(s, a, ELEM_F16, kRowsStore, !normed, ELEM_F32);
+}
+inline int rows_residual(cudaStream_t s, const __half* x, const __half* w, float* h, int M, int N, int K, int* error) {
+    RowsGemm a;
+    a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.y = h; a.ldy = N; a.error = error;
+    return gemm_rows(s, a, ELEM_F16, kRowsResidual, false, ELEM_F32);
+}
 
 // ---- operator internals shared with the stack ------------------------------------------------------------------------
 size_t fa_scratch_bytes(const b200attn_fa_config& c);

@@ -345,11 +345,12 @@ int launch_kv_append(const KvView& kv, int layer, const AppendTile* d_tiles, int
 
 int launch_fa_decode_pre(const KvView& kv, int layer, const int* d_slots, int n_seqs, const float* qkv_raw, const float* q_norm_w,
                          const float* k_norm_w, const float* inv_freq, __half* q_out, __half* gate_out, cudaStream_t s) {
+    const bool few = n_seqs <= kRowsGemmMax;
     if (kv.is_fp16)
-        launch_pdl(fa_decode_pre_kernel<true>, dim3(n_seqs), dim3(384), 0, s, kv, layer, d_slots, qkv_raw, q_norm_w, k_norm_w, inv_freq,
+        launch_pdl_split(true, few, fa_decode_pre_kernel<true>, dim3(n_seqs), dim3(384), 0, s, kv, layer, d_slots, qkv_raw, q_norm_w, k_norm_w, inv_freq,
                    q_out, gate_out);
     else
-        launch_pdl(fa_decode_pre_kernel<false>, dim3(n_seqs), dim3(384), 0, s, kv, layer, d_slots, qkv_raw, q_norm_w, k_norm_w, inv_freq,
+        launch_pdl_split(true, few, fa_decode_pre_kernel<false>, dim3(n_seqs), dim3(384), 0, s, kv, layer, d_slots, qkv_raw, q_norm_w, k_norm_w, inv_freq,
                    q_out, gate_out);
     B2_LAUNCH_CHECK();
     return 0;

@@ -464,7 +464,7 @@ int launch_la_decode(const float* mixed, const int* d_slots, int n_seqs, int max
     // The kernel requests its state before the programmatic-launch wait.  That is only sound when another kernel that
     // executes the wait runs between two writers of the same state (the decode step of a stack).  A caller that may
     // launch this kernel twice in a row on one layer (the core entry) takes the ordinary stream order instead.
-#define LA_DEC(T) launch_pdl_if(early_state_loads, la_decode_kernel<T, 3, 16>, grid, dim3(256), 0, s, mixed, d_slots, max_seqs, rec_layer, \
+#define LA_DEC(T) launch_pdl_split(early_state_loads, n_seqs <= kRowsGemmMax, la_decode_kernel<T, 3, 16>, grid, dim3(256), 0, s, mixed, d_slots, max_seqs, rec_layer, \
                                 rec_stride, conv_layer, conv_stride, conv_w, a_log, dt_bias, norm_w, (T*)out, stagger_ns, (unsigned)n_sm, l2_ahead, stamp)
     if (out_fp16) LA_DEC(__half); else LA_DEC(float);
 #undef LA_DEC

@@ -312,6 +312,8 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
     float* conv_layer = st->d_conv + (size_t)layer * st->cfg.max_seqs * st->conv_stride_slot();
     auto project_in = [&](int rows) -> int {
         if (fp16) {
+            if (decode && dout && dout->rows)
+                return rows_project(s, d_x, x_is_fp16, dout->eps, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, la->d_error);
             if (decode && dout)   // decode step of a stack: d_x is the un-normalised residual stream, its RMSNorm scale is applied in the epilogue
                 return gemm_tc_store(s, (const __half*)d_x, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, kLaProjCols, dout->rowsq,
                                      dout->eps, la->d_error);
@@ -322,6 +324,8 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
         return gemm_xwT(s, d_x, false, la->d_win_f32, false, la->d_mixed, false, rows, kLaProjCols, kHidden);
     };
     auto project_out = [&](int rows) -> int {
+        if (decode && dout && dout->rows)
+            return rows_residual(s, (const __half*)la->d_gated, la->d_wout_fp16, d_y, rows, kHidden, kLaHeads * kLaVd, la->d_error);
         if (decode && dout)   // residual stream += gated W_out^T, with the fp16 copy and the sums of squares for the next projection
             return gemm_tc_residual(s, (const __half*)la->d_gated, la->d_wout_fp16, d_y, dout->xh, dout->rowsq, rows, kHidden, kLaHeads * kLaVd,
                                     la->d_error);

@@ -487,6 +487,11 @@ static int stack_ready(b200attn_stack st) {
     return 0;
 }
 
+// Whether a decode step of `rows` rows runs on the few-row projections (gemm_rows.cu).
+static bool rows_step(b200attn_stack st, int rows) {
+    return rows <= kRowsGemmMax && st->cfg.intermediate_size <= 4096 && g_flags.decode_gemm_rows && !gemm_tc_enabled();
+}
+
 // All layers over `rows` rows already embedded in d_h (and, for the fused decode step, in d_xh / d_rowsq).
 static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const int* h_counts, int n_seqs, const int* d_slots,
                         bool decode, cudaStream_t s) {
@@ -505,6 +510,30 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
                                        st->d_xh, true, st->d_h, 1.0f, &f, s));
             B2_TRY(gemm_tc_swiglu(s, st->d_xh, st->d_wgu[i], st->d_act, rows, 2 * inter, kHidden, st->d_rowsq, st->cfg.rms_eps, st->d_error));
             B2_TRY(gemm_tc_residual(s, st->d_act, st->d_wdown[i], st->d_h, st->d_xh, st->d_rowsq, rows, kHidden, inter, st->d_error));
+        }
+        return 0;
+    }
+    if (decode && rows_step(st, rows)) {
+        // Few rows, five launches per DeltaNet layer: the projections normalise the fp32 residual rows as they load them, the output
+        // projections add to them.
+        DecodeOut f{nullptr, nullptr, st->cfg.rms_eps, true};
+        for (int i = 0; i < st->cfg.num_layers; ++i) {
+            if (st->layer_kind[i])
+                B2_TRY(fa_forward_rows(st->fa[st->layer_sub[i]], st->pool, st->layer_sub[i], h_slots, h_counts, n_seqs, d_slots, true, st->d_h, false,
+                                       st->d_h, 1.0f, &f, s));
+            else
+                B2_TRY(la_forward_rows(st->la[st->layer_sub[i]], st->state, st->layer_sub[i], h_slots, h_counts, n_seqs, d_slots, true, st->d_h, false,
+                                       st->d_h, 1.0f, &f, s));
+            RowsGemm g;
+            g.x = st->d_h;
+            g.ldx = g.K = kHidden;
+            g.w = st->d_wgu[i];
+            g.M = rows; g.N = 2 * inter; g.group = 32;
+            g.eps = st->cfg.rms_eps;
+            g.y = st->d_act; g.ldy = inter;
+            g.error = st->d_error;
+            B2_TRY(gemm_rows(s, g, ELEM_F16, kRowsSwiglu, true, ELEM_F16));
+            B2_TRY(rows_residual(s, st->d_act, st->d_wdown[i], st->d_h, rows, kHidden, inter, st->d_error));
         }
         return 0;
     }
@@ -535,6 +564,20 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
     return 0;
 }
 
+// The LM head over the selected rows of d_h, or over the normalised rows in d_xb.
+static RowsGemm head_product(b200attn_stack st, int n, const int* d_row_index, bool norm_on_load) {
+    RowsGemm a;
+    a.x = norm_on_load ? (const void*)st->d_h : (const void*)st->d_xb;
+    a.row_index = norm_on_load ? d_row_index : nullptr;
+    a.norm_w = st->d_final_norm;
+    a.norm_base = 1.0f;
+    a.eps = st->cfg.rms_eps;
+    a.w = st->d_embed;
+    a.M = n; a.N = st->cfg.vocab_size; a.K = a.ldx = kHidden;
+    a.error = st->d_error;
+    return a;
+}
+
 // Final norm of the selected rows, tied LM head, greedy argmax.
 static int stack_head(b200attn_stack st, int n_seqs, const int* d_row_index, int* d_next, float* d_hidden_out, cudaStream_t s) {
     if (st->blocks) {
@@ -542,9 +585,19 @@ static int stack_head(b200attn_stack st, int n_seqs, const int* d_row_index, int
         B2_TRY(block_logits(*st->blocks, n_seqs, d_row_index, st->d_logits, s));
         return launch_argmax_rows(st->d_logits, n_seqs, st->cfg.vocab_size, d_next, s);
     }
-    launch_pdl(rmsnorm_kernel, dim3(n_seqs), dim3(256), 0, s, st->d_h, d_row_index, st->d_final_norm, st->cfg.rms_eps, n_seqs, st->d_xb,
-               d_hidden_out);
-    B2_LAUNCH_CHECK();
+    const bool few = n_seqs <= kRowsGemmMax && g_flags.decode_gemm_rows && !g_flags.lm_head_cublas;
+    const bool norm_on_load = few && !d_hidden_out;
+    if (!norm_on_load) {
+        launch_pdl(rmsnorm_kernel, dim3(n_seqs), dim3(256), 0, s, st->d_h, d_row_index, st->d_final_norm, st->cfg.rms_eps, n_seqs, st->d_xb,
+                   d_hidden_out);
+        B2_LAUNCH_CHECK();
+    }
+    if (few) {
+        RowsGemm a = head_product(st, n_seqs, d_row_index, norm_on_load);
+        a.packed = st->d_packed;
+        B2_TRY(gemm_rows(s, a, ELEM_F16, kRowsArgmax, norm_on_load, ELEM_F32));
+        return launch_argmax_unpack(st->d_packed, n_seqs, d_next, s);
+    }
     // LM head with the argmax in the GEMM epilogue (the logits never reach memory): 103 us per step against 112 + 31 us for
     // the cuBLAS GEMM and the argmax kernel.  B200ATTN_LM_HEAD=cublas (read at create time) selects the latter.
     if (n_seqs <= 128 && !g_flags.lm_head_cublas)
@@ -565,7 +618,7 @@ static int stack_decode_layers(b200attn_stack st, int n_seqs, const int* d_token
         launch_pdl(embed_gather_fused_kernel, dim3(n_seqs), dim3(256), 0, s, d_tokens_in, st->d_embed, st->cfg.vocab_size, st->d_h, st->d_xh,
                    st->d_rowsq);
     else
-        launch_pdl(embed_gather_kernel, dim3(n_seqs), dim3(256), 0, s, d_tokens_in, st->d_embed, st->cfg.vocab_size, st->d_h);
+        launch_pdl_split(true, n_seqs <= kRowsGemmMax, embed_gather_kernel, dim3(n_seqs), dim3(256), 0, s, d_tokens_in, st->d_embed, st->cfg.vocab_size, st->d_h);
     B2_LAUNCH_CHECK();
     if (st->pool) st->pool->lens_dirty = true;
     return stack_layers(st, n_seqs, nullptr, nullptr, n_seqs, d_slots, true, s);
@@ -579,6 +632,12 @@ static int stack_decode_step(b200attn_stack st, int n_seqs, const int* d_tokens_
 // Logits (fp32 [n, vocab]) of selected rows of the last pass.
 static int stack_logits(b200attn_stack st, int n, const int* d_row_index, float* d_logits, cudaStream_t s) {
     if (st->blocks) return block_logits(*st->blocks, n, d_row_index, d_logits, s);
+    if (n <= kRowsGemmMax && g_flags.decode_gemm_rows) {
+        RowsGemm a = head_product(st, n, d_row_index, true);
+        a.y = d_logits;
+        a.ldy = st->cfg.vocab_size;
+        return gemm_rows(s, a, ELEM_F16, kRowsStore, true, ELEM_F32);
+    }
     launch_pdl(rmsnorm_kernel, dim3(n), dim3(256), 0, s, st->d_h, d_row_index, st->d_final_norm, st->cfg.rms_eps, n, st->d_xb, nullptr);
     B2_LAUNCH_CHECK();
     return gemm_xwT(s, st->d_xb, true, st->d_embed, true, d_logits, false, n, st->cfg.vocab_size, kHidden);

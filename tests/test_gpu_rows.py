@@ -1,0 +1,68 @@
+"""GPU: the few-row projections of a decode step against the library GEMMs, at the edges of their row tiles (8 / 9, 16 / 17, 32 / 33 rows) and
+of their column tiles (feed-forward widths of one gate / up group and of a ragged last batch, vocabularies below and above a wave)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+L, T, STEPS = 4, 6, 3
+
+
+def _weights(synth, seed, inter, vocab):
+    from oracle import cpu_stack
+    return cpu_stack.make_stack_weights(synth, seed, L, inter, vocab, int8=False, norm_std=0.1)
+
+
+def _stack(ops, weights, inter, vocab, rows):
+    st = ops.HybridStack(num_layers=L, intermediate_size=inter, vocab_size=vocab, max_seqs=rows, max_seq_len=64, prefill_chunk_seqs=rows, kv_dtype=1,
+                         int8_weights=False)
+    for i, lw in enumerate(weights["layers"]):
+        st.set_layer_weights(i, lw, lw["ffn"], fa=lw.get("fa"), la=lw.get("la"))
+    st.set_embedding(weights["embed"], weights["final_norm"])
+    return st
+
+
+def _decode(torch, ops, weights, inter, vocab, rows, tokens):
+    """Tokens of every step, and the normed hidden rows of a second prompt behind the steps: they see every step's cache and state."""
+    st = _stack(ops, weights, inter, vocab, rows)
+    picks = [st.forward_batch_prefill(tokens[:, :T].contiguous()).clone()]
+    for d in range(STEPS):
+        picks.append(st.forward_batch_decode(tokens[:, T + d].contiguous()).clone())
+    hidden = st.forward_batch_prefill(tokens[:, :4].contiguous(), want_hidden=True)[1].clone()
+    torch.cuda.synchronize()
+    assert st.device_status() == 0
+    return torch.stack(picks), hidden
+
+
+def _logits(torch, ops, weights, inter, vocab, tokens):
+    """The trace path: logits of single tokens behind a prompt."""
+    st = _stack(ops, weights, inter, vocab, 2)
+    st.begin_batching()
+    row = st.open(T + STEPS)
+    out = [st.extend(row, tokens[0, :T].contiguous(), [T - 1]).clone()]
+    for d in range(STEPS):
+        out.append(st.extend(row, tokens[0, T + d:T + d + 1].contiguous(), [0]).clone())
+    return torch.cat([x.reshape(1, -1) for x in out])
+
+
+# The two sides round the same values to fp16 at the same places; their sums differ in order only, so a rounding differs now and then by one
+# unit, 2^-10 of a value.  Over 4 layers of about 8 rounded vectors each that stays under sqrt(32) * 2^-10 = 6e-3 of the result.
+REL = 6e-3
+
+
+@pytest.mark.parametrize("rows,inter,vocab", [(1, 64, 41), (8, 256, 1003), (9, 1088, 512), (16, 3584, 512), (17, 192, 6000), (32, 4096, 2051), (33, 256, 512)])
+def test_decode_rows_against_library_gemms(ops, cuda, synth, monkeypatch, rows, inter, vocab):
+    torch = cuda
+    weights = _weights(synth, 70 + rows, inter, vocab)
+    tokens = torch.from_numpy(synth.rng(70 + rows, "tokens").integers(0, vocab, (rows, T + STEPS)).astype(np.int32)).cuda()
+    monkeypatch.setenv("B200ATTN_DECODE_GEMM", "cublas")
+    want_t, want_h = _decode(torch, ops, weights, inter, vocab, rows, tokens)
+    want_l = _logits(torch, ops, weights, inter, vocab, tokens)
+    monkeypatch.delenv("B200ATTN_DECODE_GEMM")
+    got_t, got_h = _decode(torch, ops, weights, inter, vocab, rows, tokens)
+    got_l = _logits(torch, ops, weights, inter, vocab, tokens)
+    assert (got_h - want_h).norm() <= REL * want_h.norm()
+    assert (got_l - want_l).norm() <= REL * want_l.norm()
+    # a pick may differ where two logits are closer than the error: a few per cent at these vocabularies
+    assert (got_t == want_t).float().mean() >= 0.9
+    assert ((got_t >= 0) & (got_t < vocab)).all()
