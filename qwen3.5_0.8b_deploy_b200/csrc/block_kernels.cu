@@ -37,7 +37,7 @@ rot_table_kernel(const int* __restrict__ row_pos, const double* __restrict__ fre
 }
 
 int launch_rot_table(const int* row_pos, const double* freq, int half, int rows, float2* table, cudaStream_t s) {
-    launch_pdl(rot_table_kernel, dim3(rows), dim3(64), 0, s, row_pos, freq, half, table);
+    launch_pdl_split(true, rows <= kRowsGemmMax, rot_table_kernel, dim3(rows), dim3(64), 0, s, row_pos, freq, half, table);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -75,7 +75,7 @@ int launch_embed_scaled(ElemType t, const int* tokens, const void* embed, int vo
                         const int* lens, int max_seqs, int* row_slot, int* row_pos, float* x, void* xt, cudaStream_t s) {
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
-        launch_pdl(embed_scaled_kernel<T>, dim3(rows), dim3(128), 0, s, tokens, (const T*)embed, vocab, width, scale, d_slots, lens, max_seqs,
+        launch_pdl_split(true, rows <= kRowsGemmMax, embed_scaled_kernel<T>, dim3(rows), dim3(128), 0, s, tokens, (const T*)embed, vocab, width, scale, d_slots, lens, max_seqs,
                    row_slot, row_pos, x, (T*)xt);
     });
     B2_LAUNCH_CHECK();
@@ -136,7 +136,7 @@ norm_rows_kernel(const float* __restrict__ y, const int* __restrict__ row_index,
 int launch_post_norm_residual(ElemType t, const float* y, const float* w, float eps, int rows, int width, float* x, void* xt, cudaStream_t s) {
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
-        launch_pdl(norm_rows_kernel<T, true>, dim3(rows), dim3(128), 0, s, y, nullptr, w, eps, width, x, (T*)xt);
+        launch_pdl_split(true, rows <= kRowsGemmMax, norm_rows_kernel<T, true>, dim3(rows), dim3(128), 0, s, y, nullptr, w, eps, width, x, (T*)xt);
     });
     B2_LAUNCH_CHECK();
     return 0;
@@ -196,7 +196,7 @@ pre_norm_kernel(float* __restrict__ x, const float* __restrict__ add, const floa
 int launch_pre_norm(ElemType t, float* x, const float* add, const float* w, float eps, int rows, int width, void* out, cudaStream_t s) {
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
-        launch_pdl(add ? pre_norm_kernel<T, true> : pre_norm_kernel<T, false>, dim3(rows), dim3(128), 0, s, x, add, w, eps, width, (T*)out);
+        launch_pdl_split(true, rows <= kRowsGemmMax, add ? pre_norm_kernel<T, true> : pre_norm_kernel<T, false>, dim3(rows), dim3(128), 0, s, x, add, w, eps, width, (T*)out);
     });
     B2_LAUNCH_CHECK();
     return 0;
@@ -264,7 +264,7 @@ __global__ void lens_advance_kernel(int* __restrict__ lens, int n_layers, int ma
 }
 
 int launch_lens_advance(int* lens, int n_layers, int max_seqs, const int* d_slots, const LaSeqMeta* d_seqs, int n, cudaStream_t s) {
-    launch_pdl(lens_advance_kernel, dim3(ceil_div(n, 128)), dim3(128), 0, s, lens, n_layers, max_seqs, d_slots, d_seqs, n);
+    launch_pdl_split(true, n <= kRowsGemmMax, lens_advance_kernel, dim3(ceil_div(n, 128)), dim3(128), 0, s, lens, n_layers, max_seqs, d_slots, d_seqs, n);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -70,7 +70,7 @@ int lightning_forward(BlockModel& m, MlstmOp& op, const LayerRun& run, const Pas
         }
         return launch_row_norm_gate(op.elem, sh, m.core.f(), m.proj.p, false, sh.cols(), op.norm_w.f(), p.rows, m.mixed.p, s);
     }
-    B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.pitch(), op.elem, ELEM_F32, p.rows, sh.pitch(), W));
+    B2_TRY(block_project(m, p, op.w_in.p, sh.pitch(), m.proj.p, ELEM_F32, s));
     MlstmStepArgs a{sh, m.proj.f(), op.bias.f(), op.norm_w.f(), state, p.decode ? p.d_slots : nullptr, p.decode ? nullptr : p.d_seqs, m.cfg.max_seqs,
                     m.core.f(), m.mixed.p};
     B2_TRY(launch_mlstm_step(op.elem, a, p.n_seqs, s));
@@ -158,7 +158,7 @@ int delta_forward(BlockModel& m, DeltaOp& op, const LayerRun& run, const PassRow
     const DeltaShape& sh = op.sh;
     const int W = m.cfg.width;
     float* state = m.state->d_recurrent + m.state->block_offset[run.state_layer];
-    B2_TRY(gemm_typed(s, m.xt.p, W, op.w_low.p, m.low.p, sh.low(), op.elem, op.elem, p.rows, sh.low(), W));
+    B2_TRY(block_project(m, p, op.w_low.p, sh.low(), m.low.p, op.elem, s));
     if (!p.decode && op.chunk && p.max_count >= 16) {
         // q | k | v in bf16; decay and beta pre-activations in fp32, those of the output gate in bf16 behind them
         const int acols = sh.heads * sh.dp, gcols = sh.heads * sh.vp, qkv = sh.off_b();
@@ -176,8 +176,14 @@ int delta_forward(BlockModel& m, DeltaOp& op, const LayerRun& run, const PassRow
         }
         return launch_delta_head_norm(op.elem, sh, m.core.f(), g, false, gcols, op.norm_w.f(), p.rows, m.mixed.p, s);
     }
-    B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.pitch(), op.elem, ELEM_F32, p.rows, sh.pitch(), W));
-    B2_TRY(gemm_typed(s, m.low.p, sh.low(), op.w_gate.p, m.gates.p, sh.gate_cols(), op.elem, ELEM_F32, p.rows, sh.gate_cols(), sh.low()));
+    B2_TRY(block_project(m, p, op.w_in.p, sh.pitch(), m.proj.p, ELEM_F32, s));
+    RowsGemm gate;
+    gate.x = m.low.p; gate.w = op.w_gate.p;
+    gate.M = p.rows; gate.N = sh.gate_cols(); gate.K = gate.ldx = sh.low();
+    gate.y = m.gates.p; gate.ldy = sh.gate_cols();
+    gate.error = m.error.i();
+    if (p.in && gemm_rows_takes(gate, kRowsStore)) B2_TRY(gemm_rows(s, gate, op.elem, kRowsStore, false, ELEM_F32));
+    else B2_TRY(gemm_typed(s, m.low.p, sh.low(), op.w_gate.p, m.gates.p, sh.gate_cols(), op.elem, ELEM_F32, p.rows, sh.gate_cols(), sh.low()));
     DeltaStepArgs a{sh, m.proj.f(), m.gates.f(), op.conv.f(), sh.taps <= 4 ? op.conv4.f() : nullptr, op.a_log.f(), op.dt_bias.f(), op.norm_w.f(), state, p.decode ? p.d_slots : nullptr,
                     p.decode ? nullptr : p.d_seqs, m.cfg.max_seqs, m.core.f(), m.mixed.p};
     B2_TRY(launch_delta_step(op.elem, a, p.n_seqs, s));
@@ -245,9 +251,8 @@ int set_diff(DiffOp& op, const std::string& n, const char* name, const Source& t
 
 int diff_forward(BlockModel& m, DiffOp& op, const LayerRun& run, const PassRows& p, cudaStream_t s) {
     const DiffShape& sh = op.sh;
-    const int W = m.cfg.width;
     const LatentView cache = m.pool->latent_view(run.pool_layer);
-    B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.pitch(), op.elem, ELEM_F32, p.rows, sh.pitch(), W));
+    B2_TRY(block_project(m, p, op.w_in.p, sh.pitch(), m.proj.p, ELEM_F32, s));
     const bool split = p.decode && op.tc_decode;
     DiffPreArgs a{sh, m.proj.f(), (const float2*)m.rot[op.rot_table].cs.p, op.q_norm.f(), op.k_norm.f(), p.row_slot, p.row_pos, cache, m.q.p,
                   split ? m.qa.p : nullptr};

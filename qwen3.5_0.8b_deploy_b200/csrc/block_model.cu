@@ -202,6 +202,7 @@ int block_model_create(const b200attn_model_config* cfg, const b200attn_layer_de
     B2_TRY(m.x.alloc(R * W * 4));
     if (times > 1) B2_TRY(m.x0.alloc(R * W * 4));
     B2_TRY(m.xt.alloc(R * W * e));
+    if (!cfg->pre_norm) B2_TRY(m.x_alt.alloc((size_t)kRowsGemmMax * W * 4));
     if (!cfg->pre_norm) B2_TRY(m.y.alloc(R * W * 4));
     B2_TRY(m.proj.alloc(R * z.proj * 4));
     B2_TRY(m.gates.alloc(R * z.gates * 4));
@@ -388,7 +389,7 @@ static int mlstm_forward(BlockModel& m, MlstmOp& op, const LayerRun& run, const 
         }
         B2_TRY(launch_mlstm_head_norm(op.elem, sh, m.core.f(), m.proj.p, false, sh.cols(), op.norm_w.f(), p.rows, m.mixed.p, s));
     } else {
-        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.pitch(), op.elem, ELEM_F32, p.rows, sh.pitch(), W));
+        B2_TRY(block_project(m, p, op.w_in.p, sh.pitch(), m.proj.p, ELEM_F32, s));
         MlstmStepArgs a{sh, m.proj.f(), op.bias.f(), op.norm_w.f(), state, p.decode ? p.d_slots : nullptr, p.decode ? nullptr : p.d_seqs,
                         m.cfg.max_seqs, m.core.f(), m.mixed.p};
         B2_TRY(launch_mlstm_step(op.elem, a, p.n_seqs, s));
@@ -472,31 +473,101 @@ static int latent_expanded(BlockModel& m, LatentOp& op, const LayerRun& run, con
 
 static int latent_forward(BlockModel& m, LatentOp& op, const LayerRun& run, const PassRows& p, cudaStream_t s) {
     const LatentShape& sh = op.sh;
-    const int W = m.cfg.width;
     const LatentView cache = m.pool->latent_view(run.pool_layer);
-    B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.pitch(), op.elem, ELEM_F32, p.rows, sh.pitch(), W));
+    B2_TRY(block_project(m, p, op.w_in.p, sh.pitch(), m.proj.p, ELEM_F32, s));
     return !p.decode && op.tc_prefill ? latent_expanded(m, op, run, p, cache, s) : latent_absorbed(m, op, p, cache, s);
 }
 
-static int run_layers(BlockModel& m, const PassRows& p, cudaStream_t s) {
+// Decode steps that run on the few-row products.
+static bool rows_step(const BlockModel& m, int rows) {
+    return m.elem == ELEM_BF16 && rows <= kRowsGemmMax && m.cfg.width % 32 == 0 && m.cfg.width <= 1024 && g_flags.decode_gemm_rows;
+}
+
+int block_project(BlockModel& m, const PassRows& p, const void* w, int cols, void* out, ElemType out_type, cudaStream_t s) {
+    const int W = m.cfg.width;
+    if (!p.in) return gemm_typed(s, m.xt.p, W, w, out, cols, m.elem, out_type, p.rows, cols, W);
+    RowsGemm a = *p.in;
+    a.w = w; a.N = cols;
+    a.y = out; a.ldy = cols;
+    return gemm_rows(s, a, m.elem, kRowsStore, a.x != m.xt.p, out_type);
+}
+
+static int run_layers(BlockModel& m, const PassRows& pass, cudaStream_t s) {
+    PassRows p = pass;
     const int W = m.cfg.width, R = p.rows;
     const float eps = (float)m.cfg.norm_eps;
-    const bool pre = m.cfg.pre_norm != 0;
+    const bool pre = m.cfg.pre_norm != 0, few = p.decode && rows_step(m, R);
     m.staged_layer = -1;
     for (RotTable& t : m.rot)
         if (t.half > 0) B2_TRY(launch_rot_table(p.row_pos, (const double*)t.freq.p, t.half, R, (float2*)t.cs.p, s));
     if (m.x0.bytes) B2_CUDA(cudaMemcpyAsync(m.x0.p, m.x.p, (size_t)R * W * 4, cudaMemcpyDeviceToDevice, s));
+
+    // Few rows: the next product normalises x itself (norms on the inputs), or adds the normalised output of the sublayer before to x and
+    // leaves the sum in the other of two buffers, since every CTA of it reads x (norms on the outputs).
+    float *x = m.x.f(), *other = m.x_alt.f();
+    const DevBuf* pending = nullptr;       // norm of the sublayer output in y that has not been added yet
+    int joins = 0;                         // how many products may do that: an even number, so that x ends in its own buffer
+    if (few && !pre && m.stop_after < 0) {
+        for (const LayerRun& run : m.runs) {
+            const BlockLayer& L = m.layers[run.layer];
+            joins += (L.delta == nullptr) + (L.ff > 0);
+        }
+        joins = (joins - (m.layers[m.runs[0].layer].delta == nullptr)) / 2 * 2;
+    }
+    auto add_pending = [&]() -> int {
+        const DevBuf* norm = pending;
+        pending = nullptr;
+        return norm ? launch_post_norm_residual(m.elem, m.y.f(), norm->f(), eps, R, W, x, m.xt.p, s) : 0;
+    };
+    RowsGemm in;
+    in.M = R; in.K = in.ldx = W;
+    in.eps = eps;
+    in.error = m.error.i();
+    // Sets up what the next sublayer's products read.  `norm`: the norm on its input, `once`: one product reads it.
+    auto enter = [&](const DevBuf& norm, bool once, const float* add) -> int {
+        if (!few) return pre ? launch_pre_norm(m.elem, x, add, norm.f(), eps, R, W, m.xt.p, s) : 0;
+        in.x = m.xt.p;
+        in.add = nullptr;
+        in.norm_w = nullptr;
+        if (pre && !add) {
+            in.x = x;
+            in.norm_w = norm.f();
+        } else if (pre) {
+            B2_TRY(launch_pre_norm(m.elem, x, add, norm.f(), eps, R, W, m.xt.p, s));
+        } else if (pending && once && joins > 0) {
+            --joins;
+            in.x = x;
+            in.norm_w = pending->f();
+            in.add = m.y.f();
+            in.x_out = other;
+            pending = nullptr;
+            std::swap(x, other);
+        } else {
+            B2_TRY(add_pending());
+        }
+        p.in = &in;
+        return 0;
+    };
     // A sublayer's last product: into y, whose norm is added to x, or straight onto x.
-    auto out = [&](const void* in, int cols, const DevBuf& w, const DevBuf& norm) -> int {
-        if (pre) return gemm_typed(s, in, cols, w.p, m.x.p, W, m.elem, ELEM_F32, R, W, cols, 1.0f);
-        B2_TRY(gemm_typed(s, in, cols, w.p, m.y.p, W, m.elem, ELEM_F32, R, W, cols));
-        return launch_post_norm_residual(m.elem, m.y.f(), norm.f(), eps, R, W, m.x.f(), m.xt.p, s);
+    auto out = [&](const void* from, int cols, const DevBuf& w, const DevBuf& norm) -> int {
+        RowsGemm a;
+        a.x = from; a.w = w.p;
+        a.M = R; a.N = W; a.K = a.ldx = cols;
+        a.y = pre ? x : m.y.f();
+        a.ldy = W;
+        a.error = m.error.i();
+        const int epi = pre ? kRowsResidual : kRowsDeepStore;
+        if (few && gemm_rows_takes(a, epi)) B2_TRY(gemm_rows(s, a, m.elem, epi, false, ELEM_F32));
+        else B2_TRY(gemm_typed(s, from, cols, w.p, a.y, W, m.elem, ELEM_F32, R, W, cols, pre ? 1.0f : 0.0f));
+        if (pre) return 0;
+        pending = &norm;
+        return few ? 0 : add_pending();
     };
     for (size_t i = 0; i < m.runs.size(); ++i) {
         if (m.stop_after >= 0 && (int)i >= m.stop_after) break;
         const LayerRun& run = m.runs[i];
         BlockLayer& L = m.layers[run.layer];
-        if (pre) B2_TRY(launch_pre_norm(m.elem, m.x.f(), run.add_embedding ? m.x0.f() : nullptr, L.norm1.f(), eps, R, W, m.xt.p, s));
+        B2_TRY(enter(L.norm1, !L.delta, run.add_embedding ? m.x0.f() : nullptr));
         if (L.mlstm) {
             const MlstmShape& sh = L.mlstm->sh;
             B2_TRY(sh.gated ? mlstm_forward(m, *L.mlstm, run, p, s) : lightning_forward(m, *L.mlstm, run, p, s));
@@ -512,11 +583,21 @@ static int run_layers(BlockModel& m, const PassRows& p, cudaStream_t s) {
             B2_TRY(out(m.mixed.p, L.diff->sh.heads * L.diff->sh.vp, L.diff->w_out, L.norm1));
         }
         if (L.ff == 0) continue;
-        if (pre) B2_TRY(launch_pre_norm(m.elem, m.x.f(), nullptr, L.norm2.f(), eps, R, W, m.xt.p, s));
-        B2_TRY(gemm_typed(s, m.xt.p, W, L.w_gu.p, m.gu.p, 2 * L.ff, m.elem, m.elem, R, 2 * L.ff, W));
-        B2_TRY(launch_act_mul(m.elem, L.act, m.gu.p, R, L.ff, m.act.p, s));
+        B2_TRY(enter(L.norm2, true, nullptr));
+        if (few) {
+            RowsGemm a = in;
+            a.w = L.w_gu.p;
+            a.N = 2 * L.ff;
+            a.group = L.ff;
+            a.y = m.act.p; a.ldy = L.ff;
+            B2_TRY(gemm_rows(s, a, m.elem, L.act == B200ATTN_ACT_SILU ? kRowsSwiglu : kRowsGeglu, a.x != m.xt.p, m.elem));
+        } else {
+            B2_TRY(gemm_typed(s, m.xt.p, W, L.w_gu.p, m.gu.p, 2 * L.ff, m.elem, m.elem, R, 2 * L.ff, W));
+            B2_TRY(launch_act_mul(m.elem, L.act, m.gu.p, R, L.ff, m.act.p, s));
+        }
         B2_TRY(out(m.act.p, L.ff, L.w_down, L.norm2));
     }
+    B2_TRY(add_pending());
     if (m.pool)
         B2_TRY(launch_lens_advance(m.pool->d_lens, m.pool->cfg.num_layers, m.cfg.max_seqs, p.d_slots, p.decode ? nullptr : p.d_seqs, p.n_seqs, s));
     return 0;
@@ -597,6 +678,20 @@ int block_prefill_rows(BlockModel& m, int n_seqs, const int* h_slots, const int*
 
 int block_logits(BlockModel& m, int n, const int* d_row_index, float* d_logits, cudaStream_t s) {
     const int W = m.cfg.width;
+    if (rows_step(m, n)) {
+        RowsGemm a;
+        a.x = m.x.p;
+        a.row_index = d_row_index;
+        a.norm_w = m.final_norm.f();
+        a.eps = (float)m.cfg.norm_eps;
+        a.w = m.cfg.own_head ? m.head.p : m.embed.p;
+        a.M = n; a.N = m.cfg.vocab_size; a.K = a.ldx = W;
+        a.scale = (float)m.cfg.logit_scale;
+        a.cap = (float)m.cfg.logit_softcap;
+        a.y = d_logits; a.ldy = m.cfg.vocab_size;
+        a.error = m.error.i();
+        return gemm_rows(s, a, m.elem, kRowsStore, true, ELEM_F32);
+    }
     B2_TRY(launch_rms_norm_rows(m.elem, m.x.f(), d_row_index, m.final_norm.f(), (float)m.cfg.norm_eps, n, W, m.xt.p, s));
     B2_TRY(gemm_typed(s, m.xt.p, W, m.cfg.own_head ? m.head.p : m.embed.p, d_logits, m.cfg.vocab_size, m.elem, ELEM_F32, n, m.cfg.vocab_size, W, 0.f,
                       (float)m.cfg.logit_scale));

@@ -49,6 +49,7 @@ struct PassRows {
     const int* row_slot = nullptr;
     const int* row_pos = nullptr;
     int max_count = 0;
+    const RowsGemm* in = nullptr;      // decode steps of few rows: what the next product over the width reads and how (gemm_rows.cu)
 };
 
 // ---- block_kernels.cu: element-wise steps around the mixers -----------------------------------------------------------
@@ -324,7 +325,7 @@ struct BlockModel {
     int max_rows = 0, abs_rows = 0, ctx_rows = 0, max_spans = 0;
     b200attn_kv_pool pool = nullptr;   // owned by the stack
     b200attn_la_state state = nullptr;
-    DevBuf x, x0, xt, low, proj, gates, core, mixed, y, gu, act, q, qa, olat, c_stage, r_stage, k_up, v_up, part, counters, chunk, meta, error;
+    DevBuf x, x_alt, x0, xt, low, proj, gates, core, mixed, y, gu, act, q, qa, olat, c_stage, r_stage, k_up, v_up, part, counters, chunk, meta, error;
     int* row_slot() const { return meta.i(); }
     int* row_pos() const { return meta.i() + max_rows; }
     LaSeqMeta* seqs() const { return reinterpret_cast<LaSeqMeta*>(meta.i() + 2 * (size_t)max_rows); }
@@ -334,6 +335,9 @@ struct BlockModel {
     int staged_layer = -1;
     std::vector<LatentSpan> staged;
 };
+
+// out[rows, cols] = in W^T over the width, `in` being m.xt or, for few rows, what p.in says.
+int block_project(BlockModel& m, const PassRows& p, const void* w, int cols, void* out, ElemType out_type, cudaStream_t s);
 
 // block_mixers.cu: the mixers of layers with norms on their inputs.
 int make_lightning(const b200attn_layer_desc& d, const b200attn_model_config& c, ElemType elem, MlstmOp& op, BlockSizes& z);

@@ -271,7 +271,7 @@ int launch_delta_step(ElemType t, const DeltaStepArgs& a, int n, cudaStream_t s)
         using T = decltype(tag);
         auto go = [&](auto kernel) -> int {
             if (smem > 48 * 1024) B2_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            launch_pdl(kernel, grid, dim3(256), smem, s, a, stamp);
+            launch_pdl_split(true, n <= kRowsGemmMax, kernel, grid, dim3(256), smem, s, a, stamp);
             return 0;
         };
         auto pick = [&](auto fuse) -> int {

@@ -164,7 +164,7 @@ diff_pre_vec_kernel(const DiffPreArgs a) {
 int launch_diff_pre(ElemType t, const DiffPreArgs& a, int rows, cudaStream_t s) {
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
-        launch_pdl(a.sh.dp == 64 ? diff_pre_vec_kernel<T, 16> : a.sh.dp == 128 ? diff_pre_vec_kernel<T, 32> : diff_pre_kernel<T>, dim3(rows), dim3(256), 0, s, a);
+        launch_pdl_split(true, rows <= kRowsGemmMax, a.sh.dp == 64 ? diff_pre_vec_kernel<T, 16> : a.sh.dp == 128 ? diff_pre_vec_kernel<T, 32> : diff_pre_kernel<T>, dim3(rows), dim3(256), 0, s, a);
     });
     B2_LAUNCH_CHECK();
     return 0;

@@ -16,20 +16,18 @@
 // tcgen05 would pad the rows to 64 or 128 and pay for a TMEM round trip (the kernels of gemm_tc.cu: 9.0, 10.8 and 10.5 us).  From 33 rows on X no
 // longer fits beside the slabs, and the library GEMMs serve the step.
 #include "gemm_rows.cuh"
+#include "elem.cuh"
 #include "kernels.cuh"
 #include "ptx_utils.cuh"
 
-#include <cuda_bf16.h>
+#include <type_traits>
 
 namespace b200 {
 namespace {
 
 template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
 template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) { return pack_half2(lo, hi); }
-template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) { return pack_bf16x2(lo, hi); }
 template <typename T> __device__ __forceinline__ void mma_rows(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1);
 template <> __device__ __forceinline__ void mma_rows<__half>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     mma_16816(d, a0, a1, a2, a3, b0, b1);
@@ -69,16 +67,26 @@ __device__ __forceinline__ void store_part(unsigned char* slice, int pitch, int 
     }
 }
 
+// The gate's activation: library functions in fp16 stacks (swiglu_kernel), the forms of act_mul_kernel where the result is rounded to bf16.
+template <typename T, int EPI>
+__device__ __forceinline__ float rows_act(float g) {
+    using A = std::conditional_t<std::is_same_v<T, __nv_bfloat16>, __nv_bfloat16, float>;
+    if constexpr (EPI == kRowsGeglu) return times_sigmoid<A>(g, 1.5957691216057308f * (g + 0.044715f * g * g * g));
+    else return times_sigmoid<A>(g, g);
+}
+
 constexpr int kRowsThreads = 512, kRowsWarps = 16;
 
 // Many columns, K <= 1024: X in shared memory as 16-bit rows, `tiles` column tiles at a time.  A warp multiplies four tiles (two groups
 // of eight warps when there are more than four) over its part of K.  grid: CTAs walk batches of `tiles` tiles; `buffers` slabs of
-// weights in a ring.  LOAD: how X comes in, kLoad* below.
-enum { kLoadAsIs = 0, kLoadF32, kLoadNorm };
+// weights in a ring.  LOAD: X comes in as 16-bit rows, as fp32 rows to normalise, or as
+// fp32 rows to which normalised rows `add` are added first; the sums then also go to x_out, row m from CTA m.
+enum { kLoadAsIs = 0, kLoadNorm, kLoadAddNorm };
 template <typename T, int MT, int LOAD, int EPI, typename YT>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
     constexpr int kRows = 16 * MT;
+    constexpr bool kGated = EPI == kRowsSwiglu || EPI == kRowsGeglu;
     extern __shared__ __align__(128) unsigned char smem[];
     const int pitch = rows_pitch(a.K), batch_rows = 8 * a.tiles;
     const uint32_t slab = (uint32_t)(batch_rows * pitch);
@@ -91,7 +99,7 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
 
     // Weight row behind row j of a batch.  SwiGLU: pairs of tiles, 8 gate rows then the 8 matching up rows.
     auto weight_row = [&](int batch, int j) {
-        if constexpr (EPI == kRowsSwiglu) {
+        if constexpr (kGated) {
             const int ch = batch * (batch_rows / 2) + (j >> 4) * 8 + (j & 7);
             return 2 * ch < a.N ? (ch / a.group) * 2 * a.group + ch % a.group + ((j & 8) ? a.group : 0) : -1;
         } else {
@@ -139,31 +147,36 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
                 if (k < a.K) *reinterpret_cast<uint4*>(dst + 2 * k) = __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.x) + at + k));
             }
         } else {
+            const float* xr = static_cast<const float*>(a.x) + at;
+            const float* src = LOAD == kLoadAddNorm ? a.add + (size_t)m * a.K : xr;
             float4 v[8];
             float ss = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int k = 4 * (32 * i + lane);
-                v[i] = k < a.K ? __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + at + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[i] = k < a.K ? __ldcg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            float rs = 1.f;
-            if constexpr (LOAD == kLoadNorm) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+            for (int i = 0; i < 8; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                rs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
-            }
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            const float rs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int k = 4 * (32 * i + lane);
                 if (k < a.K) {
                     float4 w = make_float4(rs, rs, rs, rs);
-                    if (LOAD == kLoadNorm && a.norm_w) {
+                    if (a.norm_w) {
                         const float4 f = __ldg(reinterpret_cast<const float4*>(a.norm_w + k));
                         w = make_float4(rs * (a.norm_base + f.x), rs * (a.norm_base + f.y), rs * (a.norm_base + f.z), rs * (a.norm_base + f.w));
                     }
-                    *reinterpret_cast<uint2*>(dst + 2 * k) = make_uint2(pack2<T>(v[i].x * w.x, v[i].y * w.y), pack2<T>(v[i].z * w.z, v[i].w * w.w));
+                    float4 n = make_float4(v[i].x * w.x, v[i].y * w.y, v[i].z * w.z, v[i].w * w.w);
+                    if constexpr (LOAD == kLoadAddNorm) {
+                        const float4 h = __ldcg(reinterpret_cast<const float4*>(xr + k));
+                        n = make_float4(h.x + n.x, h.y + n.y, h.z + n.z, h.w + n.w);
+                        if (blockIdx.x == m % gridDim.x) *reinterpret_cast<float4*>(a.x_out + (size_t)m * a.K + k) = n;
+                    }
+                    *reinterpret_cast<uint2*>(dst + 2 * k) = make_uint2(pack2<T>(n.x, n.y), pack2<T>(n.z, n.w));
                 }
             }
         }
@@ -220,18 +233,20 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
         };
         const int n8 = tid & 7, em = (tid >> 3) % kRows;
         if (em < a.M) {
-            if constexpr (EPI == kRowsSwiglu) {
+            if constexpr (kGated) {
                 for (int p = tid / (8 * kRows); p < a.tiles / 2; p += kRowsThreads / (8 * kRows)) {
                     const int ch = batch * (batch_rows / 2) + 8 * p + n8;
                     if (2 * ch >= a.N) break;
                     const float g = total(2 * p, em, n8), u = total(2 * p + 1, em, n8);
-                    static_cast<YT*>(a.y)[(size_t)em * a.ldy + ch] = to_out<YT>(g / (1.0f + expf(-g)) * u);
+                    static_cast<YT*>(a.y)[(size_t)em * a.ldy + ch] = to_out<YT>(rows_act<T, EPI>(g) * u);
                 }
             } else {
                 for (int t = tid / (8 * kRows); t < a.tiles; t += kRowsThreads / (8 * kRows)) {
                     const int n = batch * batch_rows + 8 * t + n8;
                     if (n >= a.N) break;
-                    const float v = total(t, em, n8);
+                    float v = total(t, em, n8);
+                    if (a.scale != 1.0f) v *= a.scale;
+                    if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
                     if constexpr (EPI == kRowsStore) static_cast<YT*>(a.y)[(size_t)em * a.ldy + n] = to_out<YT>(v);
                     else if (v > -INFINITY) best = max(best, pack_max(v, n));
                 }
@@ -257,9 +272,9 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (tid == 0 && *abort_flag && a.error) atomicExch(a.error, 7);
 }
 
-// Few columns, deep K <= 4096: Y[M, N] += X W^T for fp32 Y.  One column tile per CTA, the 16 warps split K, X goes from L2 straight into the
+// Few columns, deep K <= 4096: fp32 Y[M, N] = X W^T, added to what is there with ADD.  One column tile per CTA, the 16 warps split K, X goes from L2 straight into the
 // registers of the warp that multiplies it, kAhead chunks at a time.
-template <typename T, int MT>
+template <typename T, int MT, bool ADD>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     constexpr int kRows = 16 * MT, kAhead = MT == 1 ? 4 : 2;
@@ -287,7 +302,7 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     const int active = (chunks + per - 1) / per;
     const bool writes = tid < 8 * kRows && em < a.M && n < a.N;
     float res = 0.f;
-    if (writes) res = __ldcg(static_cast<const float*>(a.y) + (size_t)em * a.ldy + n);
+    if (ADD && writes) res = __ldcg(static_cast<const float*>(a.y) + (size_t)em * a.ldy + n);
     const T* xp = static_cast<const T*>(a.x) + (size_t)r * a.ldx + 8 * c;
     auto load = [&](int i, int ch) {             // rows 8 i + r, chunk ch
         return 8 * i + r < a.M && ch < c1 ? __ldcg(reinterpret_cast<const uint4*>(xp + (size_t)8 * i * a.ldx + 32 * ch)) : make_uint4(0u, 0u, 0u, 0u);
@@ -356,7 +371,7 @@ int launch_wide(RowsGemm a, cudaStream_t s, ProfKind kind) {
     B2_TRY(prepare(once, rows_wide_kernel<T, MT, LOAD, EPI, YT>));
     int sms = 0;
     B2_TRY(device_sm_count(&sms));
-    const int unit = EPI == kRowsSwiglu ? 2 : 1, n_tiles = ceil_div(a.N, 8), tile = 8 * host_pitch(a.K);
+    const int unit = EPI == kRowsSwiglu || EPI == kRowsGeglu ? 2 : 1, n_tiles = ceil_div(a.N, 8), tile = 8 * host_pitch(a.K);
     const int room = kSharedMost - 16 * MT * host_pitch(a.K) - 128;
     a.tiles = ceil_div(ceil_div(n_tiles, unit), sms) * unit;      // one batch per CTA, one CTA per SM ...
     a.buffers = 1;
@@ -372,38 +387,55 @@ int launch_wide(RowsGemm a, cudaStream_t s, ProfKind kind) {
     return 0;
 }
 
-template <typename T, int MT>
+template <typename T, int MT, bool ADD>
 int launch_deep(const RowsGemm& a, cudaStream_t s) {
     static PerDeviceOnce once;
-    B2_TRY(prepare(once, rows_deep_kernel<T, MT>));
+    B2_TRY(prepare(once, rows_deep_kernel<T, MT, ADD>));
     unsigned long long* stamp = prof_stamp_slot(PROF_GEMM_RES);
-    launch_pdl_split(true, true, rows_deep_kernel<T, MT>, dim3(ceil_div(a.N, 8)), dim3(kRowsThreads), (size_t)8 * host_pitch(a.K) + 16, s, a, stamp);
+    launch_pdl_split(true, true, rows_deep_kernel<T, MT, ADD>, dim3(ceil_div(a.N, 8)), dim3(kRowsThreads), (size_t)8 * host_pitch(a.K) + 16, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
-template <typename T, int EPI, typename YT>
-int dispatch(const RowsGemm& a, int load, cudaStream_t s, ProfKind kind) {
-    const bool small = a.M <= 16;
-    if (load == kLoadNorm) return small ? launch_wide<T, 1, kLoadNorm, EPI, YT>(a, s, kind) : launch_wide<T, 2, kLoadNorm, EPI, YT>(a, s, kind);
-    return small ? launch_wide<T, 1, kLoadAsIs, EPI, YT>(a, s, kind) : launch_wide<T, 2, kLoadAsIs, EPI, YT>(a, s, kind);
+template <typename T, int LOAD, int EPI, typename YT>
+int wide(const RowsGemm& a, cudaStream_t s, ProfKind kind) {
+    return a.M <= 16 ? launch_wide<T, 1, LOAD, EPI, YT>(a, s, kind) : launch_wide<T, 2, LOAD, EPI, YT>(a, s, kind);
+}
+template <typename T, bool ADD>
+int deep(const RowsGemm& a, cudaStream_t s) {
+    return a.M <= 16 ? launch_deep<T, 1, ADD>(a, s) : launch_deep<T, 2, ADD>(a, s);
 }
 
 }  // namespace
 
 bool gemm_rows_takes(const RowsGemm& a, int epi) {
-    return a.M > 0 && a.M <= kRowsGemmMax && a.N > 0 && a.K > 0 && a.K % 32 == 0 && a.K <= (epi == kRowsResidual ? 4096 : 1024) && a.ldx % 8 == 0 &&
+    const bool deep = epi == kRowsResidual || epi == kRowsDeepStore;
+    return a.M > 0 && a.M <= kRowsGemmMax && a.N > 0 && a.K > 0 && a.K % 32 == 0 && a.K <= (deep ? 4096 : 1024) && a.ldx % 8 == 0 &&
            (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
 }
 
-int gemm_rows(cudaStream_t s, RowsGemm a, ElemType type, int epi, bool norm, ElemType out) {
+int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, bool norm, ElemType out) {
     if (!gemm_rows_takes(a, epi)) B2_FAIL(B200ATTN_ERR_UNSUPPORTED, "gemm_rows: unsupported shape %d x %d x %d", a.M, a.N, a.K);
-    const int load = norm ? kLoadNorm : kLoadAsIs;
+    using B = __nv_bfloat16;
     if (type == ELEM_F16) {
-        if (epi == kRowsStore && out == ELEM_F32) return dispatch<__half, kRowsStore, float>(a, load, s, PROF_GEMM_IN);
-        if (epi == kRowsSwiglu && out == ELEM_F16) return dispatch<__half, kRowsSwiglu, __half>(a, load, s, PROF_GEMM_FFN);
-        if (epi == kRowsResidual && out == ELEM_F32) return a.M <= 16 ? launch_deep<__half, 1>(a, s) : launch_deep<__half, 2>(a, s);
-        if (epi == kRowsArgmax) return dispatch<__half, kRowsArgmax, float>(a, load, s, PROF_LM_HEAD);
+        if (epi == kRowsStore && out == ELEM_F32)
+            return norm ? wide<__half, kLoadNorm, kRowsStore, float>(a, s, PROF_GEMM_IN) : wide<__half, kLoadAsIs, kRowsStore, float>(a, s, PROF_GEMM_IN);
+        if (epi == kRowsSwiglu && out == ELEM_F16 && norm) return wide<__half, kLoadNorm, kRowsSwiglu, __half>(a, s, PROF_GEMM_FFN);
+        if (epi == kRowsResidual) return deep<__half, true>(a, s);
+        if (epi == kRowsArgmax)
+            return norm ? wide<__half, kLoadNorm, kRowsArgmax, float>(a, s, PROF_LM_HEAD) : wide<__half, kLoadAsIs, kRowsArgmax, float>(a, s, PROF_LM_HEAD);
+    }
+    if (type == ELEM_BF16) {
+#define ROWS_LOADS(EPI, YT, PROF)                                                                                                     \
+    return a.add ? wide<B, kLoadAddNorm, EPI, YT>(a, s, PROF) : norm ? wide<B, kLoadNorm, EPI, YT>(a, s, PROF) : wide<B, kLoadAsIs, EPI, YT>(a, s, PROF)
+        if (epi == kRowsStore && out == ELEM_F32) ROWS_LOADS(kRowsStore, float, PROF_GEMM_IN);
+        if (epi == kRowsSwiglu) ROWS_LOADS(kRowsSwiglu, B, PROF_GEMM_FFN);
+        if (epi == kRowsGeglu) ROWS_LOADS(kRowsGeglu, B, PROF_GEMM_FFN);
+#undef ROWS_LOADS
+        if (epi == kRowsStore && out == ELEM_BF16 && !a.add)
+            return norm ? wide<B, kLoadNorm, kRowsStore, B>(a, s, PROF_GEMM_IN) : wide<B, kLoadAsIs, kRowsStore, B>(a, s, PROF_GEMM_IN);
+        if (epi == kRowsResidual) return deep<B, true>(a, s);
+        if (epi == kRowsDeepStore) return deep<B, false>(a, s);
     }
     B2_FAIL(B200ATTN_ERR_UNSUPPORTED, "gemm_rows: unsupported types");
 }

@@ -6,18 +6,21 @@
 namespace b200 {
 
 constexpr int kRowsGemmMax = 32;        // rows a launch takes
-enum { kRowsStore = 0, kRowsSwiglu, kRowsResidual, kRowsArgmax };
+enum { kRowsStore = 0, kRowsSwiglu, kRowsGeglu, kRowsArgmax, kRowsResidual, kRowsDeepStore };    // the last two: deep K, fp32 Y
 
 struct RowsGemm {
     const void* x = nullptr;            // [M, K] 16-bit, or fp32 rows to normalise on the way in
     int ldx = 0;
     const int* row_index = nullptr;     // row m of X is x + row_index[m] * ldx
-    const void* w = nullptr;            // [N, K]; SwiGLU: gate and up rows in alternating groups of `group` rows
+    const void* w = nullptr;            // [N, K]; gated: gate and up rows in alternating groups of `group` rows
     int M = 0, N = 0, K = 0;
     const float* norm_w = nullptr;      // the normalised columns are multiplied by norm_base + norm_w, null: by one
     float norm_base = 0.f;
     float eps = 0.f;
-    void* y = nullptr;                  // store: [M, N]; SwiGLU: [M, N / 2]; residual: fp32 [M, N], added to
+    const float* add = nullptr;         // [M, K] fp32: X = x + norm(add), kept in x_out (another buffer than x)
+    float* x_out = nullptr;
+    float scale = 1.f, cap = 0.f;       // store: y = cap tanh(scale v / cap), no cap at 0
+    void* y = nullptr;                  // store: [M, N]; gated: [M, N / 2]; residual: fp32 [M, N], added to
     int ldy = 0;
     int group = 0;
     unsigned long long* packed = nullptr;   // argmax words of M rows (see gemm_tc_argmax)
@@ -26,6 +29,6 @@ struct RowsGemm {
 };
 
 bool gemm_rows_takes(const RowsGemm& a, int epi);
-int gemm_rows(cudaStream_t s, RowsGemm a, ElemType type, int epi, bool norm, ElemType out);
+int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, bool norm, ElemType out);
 
 }  // namespace b200

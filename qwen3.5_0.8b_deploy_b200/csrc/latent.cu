@@ -114,7 +114,7 @@ int launch_latent_pre(ElemType t, const LatentPreArgs& a, int rows, cudaStream_t
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
 const bool small = a.sh.dp <= 128 && a.sh.rot <= 64;
-        launch_pdl(small ? latent_pre_kernel<T, true> : latent_pre_kernel<T, false>, dim3(rows, a.sh.own ? 2 : 1), dim3(256), 0, s, a);
+        launch_pdl_split(true, rows <= kRowsGemmMax, small ? latent_pre_kernel<T, true> : latent_pre_kernel<T, false>, dim3(rows, a.sh.own ? 2 : 1), dim3(256), 0, s, a);
     });
     B2_LAUNCH_CHECK();
     return 0;

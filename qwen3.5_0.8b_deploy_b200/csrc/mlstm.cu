@@ -172,7 +172,7 @@ int launch_mlstm_step(ElemType t, const MlstmStepArgs& a, int n, cudaStream_t s)
     unsigned long long* stamp = a.seqs ? nullptr : prof_stamp_slot(PROF_LA_DECODE);
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
-        auto go = [&](auto kernel) { launch_pdl(kernel, grid, dim3(256), smem, s, a, stamp); };
+        auto go = [&](auto kernel) { launch_pdl_split(true, n <= kRowsGemmMax, kernel, grid, dim3(256), smem, s, a, stamp); };
         auto pick = [&](auto gated, auto fuse) {
             constexpr bool kGated = decltype(gated)::value, kFuse = decltype(fuse)::value;
             if (sh.dim <= 32) go(mlstm_step_kernel<4, T, kGated, kFuse>);
@@ -314,7 +314,7 @@ int launch_row_norm_gate(ElemType t, const MlstmShape& sh, const float* core, co
     dispatch_elem(t, [&](auto tag) {
         using T = decltype(tag);
         if (g_f32)
-            launch_pdl(row_norm_gate_kernel<T, float>, dim3(rows), dim3(256), 0, s, core, (const float*)g, g_pitch, sh.off_g(), norm_w, sh.eps, cols, n,
+            launch_pdl_split(true, rows <= kRowsGemmMax, row_norm_gate_kernel<T, float>, dim3(rows), dim3(256), 0, s, core, (const float*)g, g_pitch, sh.off_g(), norm_w, sh.eps, cols, n,
                        (T*)gated);
         else
             launch_pdl(row_norm_gate_kernel<T, T>, dim3(rows), dim3(256), 0, s, core, (const T*)g, g_pitch, sh.off_g(), norm_w, sh.eps, cols, n, (T*)gated);

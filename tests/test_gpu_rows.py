@@ -1,7 +1,15 @@
 """GPU: the few-row projections of a decode step against the library GEMMs, at the edges of their row tiles (8 / 9, 16 / 17, 32 / 33 rows) and
 of their column tiles (feed-forward widths of one gate / up group and of a ragged last batch, vocabularies below and above a wave)."""
+import os
+import sys
+
 import numpy as np
 import pytest
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+import test_gpu_gutenex as gutenex  # noqa: E402
+import test_gpu_nuzopel as nuzopel  # noqa: E402
+from test_gpu_nuzopel import models, wts  # noqa: E402,F401
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +74,52 @@ def test_decode_rows_against_library_gemms(ops, cuda, synth, monkeypatch, rows, 
     # a pick may differ where two logits are closer than the error: a few per cent at these vocabularies
     assert (got_t == want_t).float().mean() >= 0.9
     assert ((got_t >= 0) & (got_t < vocab)).all()
+
+
+# ---- layer-described stacks (bf16) -------------------------------------------------------------------------------------------------
+def _gutenex_layers():
+    return [gutenex.lightning(2, 32, 48, ff=96), gutenex.delta(4, 2, 32, 32, conv=4, a_rank=20, g_rank=12, ff=70), gutenex.diff(4, 2, 32, 64, 16, 30, 5, ff=64),
+            gutenex.delta(2, 2, 16, 24, ff=None)]
+
+
+def _designs():
+    return [(nuzopel, nuzopel.make, nuzopel.whole_layers(), {}), (gutenex, gutenex.make, _gutenex_layers(), {}),
+            (gutenex, gutenex.make, _gutenex_layers(), dict(loop=(0, 2, 3)))]
+
+
+@pytest.mark.parametrize("width", [32, 96, 1024])
+@pytest.mark.parametrize("design", [0, 1, 2])
+def test_block_rows_against_the_plain_implementation(cuda, models, wts, design, width):
+    """Single tokens behind a portion: every product over the width on the few-row kernels, and behind them what their K does not fit."""
+    mod, make, layers, more = _designs()[design]
+    c = mod.Case(models, wts, *make(layers, width=width, seed=40 + width, **more), "bfloat16")
+    toks = c.tokens(60)
+    want = c.expect(toks)
+    with nuzopel.on_stream(cuda):
+        c.stack.begin_batching()
+        for cuts in ([1], [20, 1]):
+            row = c.stack.open()
+            c.judge(c.run(cuda, row, toks, cuts), want, f"cuts {cuts}")
+            c.stack.retire(row)
+
+
+@pytest.mark.parametrize("rows", [9, 17, 32, 33])
+@pytest.mark.parametrize("design", [0, 1])
+def test_block_rows_of_a_batch(cuda, models, wts, design, rows):
+    """Residual rows of batched steps against the plain implementation, some rows of the batch."""
+    mod, make, layers, more = _designs()[design]
+    c = mod.Case(models, wts, *make(layers, width=256, seed=60, **more), "bfloat16", max_seqs=rows, max_seq_len=64)
+    tokens = np.stack([c.tokens(24, 5 + k) for k in range(rows)])
+    t = cuda.tensor(tokens, dtype=cuda.int32, device="cuda")
+    with nuzopel.on_stream(cuda):
+        c.stack.forward_batch_prefill(t[:, :20].contiguous())
+        got = []
+        for d in range(20, 24):
+            c.stack.forward_batch_decode(t[:, d].contiguous())
+            got.append(c.stack.residual(rows).clone())
+        assert c.stack.device_status() == 0
+    got = cuda.stack(got, 1).cpu().numpy()
+    for k in (0, 8, rows - 1):
+        _, residual, limit = c.expect(tokens[k])
+        off = np.sqrt(np.mean(((got[k] - residual[20:]) / c.residual_unit(residual)) ** 2, axis=-1))
+        assert (off <= limit[1][20:]).all(), f"row {k}: {off / limit[1][20:]} of the limits"
