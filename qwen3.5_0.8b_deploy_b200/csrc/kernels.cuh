@@ -63,8 +63,12 @@ struct LaSeqMeta {  // per sequence, device array
 };
 // A state pool whose layers hold blocks of block_floats[layer] floats per slot (zeroed by b200attn_la_state_clear).
 int state_pool_create_blocks(const std::vector<size_t>& block_floats, int max_seqs, b200attn_la_state* out);
-int launch_la_conv_seq(const float* mixed, const int* d_row_seq, const LaSeqMeta* d_seqs, const float* conv_layer,
-                       size_t conv_stride, const float* conv_w, const float* a_log, const float* dt_bias, int rows,
+constexpr int kConvRun = 16;
+struct LaRun {  // up to kConvRun consecutive rows of one sequence
+    int row, seq;
+};
+int launch_la_conv_seq(const float* mixed, const LaRun* d_runs, int n_runs, const LaSeqMeta* d_seqs, const float* conv_layer,
+                       size_t conv_stride, const float* conv_w, const float* a_log, const float* dt_bias,
                        float* q, float* k, __half* qh, __half* kh, float* v, __half* vh, float* g, float* beta, cudaStream_t s);
 int launch_la_chunk_tc(const __half* q_h, const __half* k_h, const __half* v_h, const float* g, const float* beta,
                        const LaSeqMeta* d_seqs, int n_seqs, int rows, float* rec_layer, size_t rec_stride, float* out,

@@ -29,45 +29,43 @@ __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : logf(1.0f + expf(x)); }
 
 // ---- C1, sequence form -------------------------------------------------------------------------------
-// One warp per (run of kConvRun consecutive rows, head, part) with part = q, k or v channels of the head: conv +
+// One warp per (run of up to kConvRun consecutive rows of one sequence, head, part) with part = q, k or v channels of the head: conv +
 // SiLU, L2 norm of q and k (eps inside the sqrt), q * 1/sqrt(128); the v warps also produce beta and the log-decay g.
 // A warp requests its whole input window (the run's rows plus three rows of history, 16 bytes per lane and row) before
-// it computes anything, so every input row leaves HBM once and enough loads are in flight to cover the latency.
+// it computes anything, so every input row leaves HBM once and enough loads are in flight to cover the latency.  What is left is bound by
+// issue slots: the joint row norms took 65536 rows from 577 to 499 us (2.4 GB, 362 us at the memory rate), and runs that keep to one sequence
+// took a ragged batch of 4200 rows from 57 to 43 us (with the norms), where runs across two sequences went row by row.
 // q, k and v are written as fp32 (q_out, k_out, v_out) and / or fp16 (qh_out, kh_out, vh_out, the operand format of the
 // tensor-core recurrence); null pointers are skipped.
-constexpr int kConvRun = 16;
 __global__ void __launch_bounds__(128)
-la_conv_seq_kernel(const float* __restrict__ mixed, const int* __restrict__ row_seq,
+la_conv_seq_kernel(const float* __restrict__ mixed, const LaRun* __restrict__ runs, int n_runs,
                    const LaSeqMeta* __restrict__ seqs, const float* __restrict__ conv_state_layer,
                    size_t conv_stride_slot, const float* __restrict__ conv_w, const float* __restrict__ a_log,
-                   const float* __restrict__ dt_bias, int rows, float* __restrict__ q_out,
+                   const float* __restrict__ dt_bias, float* __restrict__ q_out,
                    float* __restrict__ k_out, __half* __restrict__ qh_out, __half* __restrict__ kh_out,
                    float* __restrict__ v_out, __half* __restrict__ vh_out, float* __restrict__ g_out,
                    float* __restrict__ beta_out) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    const int n_runs = (rows + kConvRun - 1) / kConvRun;
     if (gw >= n_runs * kLaHeads * 3) return;
-    const int part = gw % 3, h = (gw / 3) % kLaHeads, run = gw / (3 * kLaHeads);
-    const int row_begin = run * kConvRun, n = min(rows - row_begin, kConvRun);
+    const int part = gw % 3, h = (gw / 3) % kLaHeads;
+    const LaRun run = runs[gw / (3 * kLaHeads)];
+    const LaSeqMeta sm = seqs[run.seq];
+    const int row_begin = run.row, n = min(sm.row0 + sm.count - row_begin, kConvRun);
     const int ch = part * (kLaHeads * kLaKd) + h * kLaKd + 4 * lane;   // kd == vd == 128
     float4 w[4];             // tap weights of this lane's four channels
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(conv_w + (size_t)(ch + i) * kLaConvK);
     const float q_scale = 1.0f / sqrtf((float)kLaKd);
-    const int s_first = row_seq[row_begin], s_last = row_seq[row_begin + n - 1];
     float4 x[kConvRun + 3];  // the window: x[i] = input at (first row of the run) - 3 + i
-    LaSeqMeta sm = seqs[s_first];
-    if (s_first == s_last && n == kConvRun) {
-        const int t0 = row_begin - sm.row0;             // index of the run's first row inside this call's chunk of the sequence
-        const float* st = conv_state_layer + (size_t)sm.slot * conv_stride_slot;
+    const int t0 = row_begin - sm.row0;                 // index of the run's first row inside this call's chunk of the sequence
+    const float* st = conv_state_layer + (size_t)sm.slot * conv_stride_slot;
 #pragma unroll
-        for (int i = 0; i < kConvRun + 3; ++i) {
-            const int tt = t0 - 3 + i;
-            const float* src = (tt >= 0) ? mixed + (size_t)(sm.row0 + tt) * kLaProjCols + ch
-                                         : st + (size_t)(tt + 3) * kLaConvDim + ch;
-            x[i] = *reinterpret_cast<const float4*>(src);
-        }
+    for (int i = 0; i < kConvRun + 3; ++i) {
+        const int tt = t0 - 3 + i;
+        const float* src = (tt >= 0) ? mixed + (size_t)(sm.row0 + tt) * kLaProjCols + ch
+                                     : st + (size_t)(tt + 3) * kLaConvDim + ch;
+        x[i] = i < n + 3 ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     // conv + SiLU of this lane's four channels for one row, from the four taps oldest .. newest
     auto conv_row = [&](const float4& x0, const float4& x1, const float4& x2, const float4& x3, float (&res)[4]) {
@@ -82,7 +80,7 @@ la_conv_seq_kernel(const float* __restrict__ mixed, const int* __restrict__ row_
             res[i] = silu_fast(s2);
         }
     };
-    auto store_row = [&](int row, const float (&res)[4], float ss_total) {
+    auto store_row = [&](int row, const float (&res)[4], float inv) {
         const size_t o = ((size_t)row * kLaHeads + h) * kLaKd + 4 * lane;
         if (part == 2) {
             if (v_out) *reinterpret_cast<float4*>(v_out + o) = make_float4(res[0], res[1], res[2], res[3]);
@@ -92,7 +90,6 @@ la_conv_seq_kernel(const float* __restrict__ mixed, const int* __restrict__ row_
             }
             return;
         }
-        const float inv = ((part == 0) ? q_scale : 1.0f) / sqrtf(ss_total + 1e-6f);     // one division per row, not per channel
         const float4 r4 = make_float4(res[0] * inv, res[1] * inv, res[2] * inv, res[3] * inv);
         float* o32 = (part == 0) ? q_out : k_out;
         __half* o16 = (part == 0) ? qh_out : kh_out;
@@ -102,47 +99,36 @@ la_conv_seq_kernel(const float* __restrict__ mixed, const int* __restrict__ row_
             *reinterpret_cast<uint2*>(o16 + o) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
         }
     };
-    if (s_first == s_last && n == kConvRun) {
-        // whole run inside one sequence: straight-line code, eight rows at a time so that the eight row-norm reductions
-        // (five shuffle steps each) interleave instead of forming eight serial chains
+    // Straight-line code, eight rows at a time.  Their sums of squares are reduced together: every step halves the rows that a lane still
+    // carries, nine shuffles in place of forty, and leaves a row's sum in four lanes, so that a root and a division serve the eight rows.
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float res[8][4], ss[8];
+    for (int half = 0; half < kConvRun / 8; ++half) {
+        if (half * 8 >= n) break;
+        float res[8][4], ss[8], scale = 1.f;
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
-                const int j = half * 8 + jj;
-                conv_row(x[j], x[j + 1], x[j + 2], x[j + 3], res[jj]);
-                ss[jj] = res[jj][0] * res[jj][0] + res[jj][1] * res[jj][1] + res[jj][2] * res[jj][2] + res[jj][3] * res[jj][3];
-            }
-            if (part != 2) {
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-                    for (int jj = 0; jj < 8; ++jj) ss[jj] += __shfl_xor_sync(0xffffffffu, ss[jj], off);
-            }
-#pragma unroll
-            for (int jj = 0; jj < 8; ++jj) store_row(row_begin + half * 8 + jj, res[jj], ss[jj]);
+        for (int jj = 0; jj < 8; ++jj) {
+            const int j = half * 8 + jj;
+            conv_row(x[j], x[j + 1], x[j + 2], x[j + 3], res[jj]);
+            ss[jj] = res[jj][0] * res[jj][0] + res[jj][1] * res[jj][1] + res[jj][2] * res[jj][2] + res[jj][3] * res[jj][3];
         }
-    } else {
-        for (int j = 0; j < n; ++j) {
-            // short run or a run that crosses into another sequence (a length that is not a multiple of the run): four taps per row
-            const int row = row_begin + j;
-            sm = seqs[row_seq[row]];
-            const int t = row - sm.row0;
-            const float* st = conv_state_layer + (size_t)sm.slot * conv_stride_slot;
-            float4 xs[4];
+        if (part != 2) {
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int tt = t - 3 + b;
-                const float* src = (tt >= 0) ? mixed + (size_t)(sm.row0 + tt) * kLaProjCols + ch
-                                             : st + (size_t)(tt + 3) * kLaConvDim + ch;
-                xs[b] = *reinterpret_cast<const float4*>(src);
+            for (int w2 = 4; w2 > 0; w2 >>= 1) {
+                const bool up = lane & (4 * w2);
+#pragma unroll
+                for (int jj = 0; jj < w2; ++jj) {
+                    const float keep = up ? ss[jj + w2] : ss[jj], give = up ? ss[jj] : ss[jj + w2];
+                    ss[jj] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * w2);
+                }
             }
-            float res[4];
-            conv_row(xs[0], xs[1], xs[2], xs[3], res);
-            float ss = res[0] * res[0] + res[1] * res[1] + res[2] * res[2] + res[3] * res[3];
-            if (part != 2) ss = warp_sum_f(ss);
-            store_row(row, res, ss);
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 2);
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+            scale = ((part == 0) ? q_scale : 1.0f) / sqrtf(ss[0] + 1e-6f);      // of row (lane / 4) of the eight
+        }
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+            const float inv = __shfl_sync(0xffffffffu, scale, 4 * jj);
+            if (half * 8 + jj < n) store_row(row_begin + half * 8 + jj, res[jj], inv);
         }
     }
     if (part == 2 && lane < n) {      // beta and log-decay of the run's rows, one row per lane
@@ -411,11 +397,11 @@ __global__ void la_conv_export_kernel(const float* __restrict__ mine, float* __r
 }
 
 // ---- launchers ------------------------------------------------------------------------------------------
-int launch_la_conv_seq(const float* mixed, const int* d_row_seq, const LaSeqMeta* d_seqs, const float* conv_layer,
-                       size_t conv_stride, const float* conv_w, const float* a_log, const float* dt_bias, int rows,
+int launch_la_conv_seq(const float* mixed, const LaRun* d_runs, int n_runs, const LaSeqMeta* d_seqs, const float* conv_layer,
+                       size_t conv_stride, const float* conv_w, const float* a_log, const float* dt_bias,
                        float* q, float* k, __half* qh, __half* kh, float* v, __half* vh, float* g, float* beta, cudaStream_t s) {
-    la_conv_seq_kernel<<<ceil_div(ceil_div(rows, kConvRun) * kLaHeads * 3, 4), 128, 0, s>>>(mixed, d_row_seq, d_seqs, conv_layer, conv_stride,
-                                                                  conv_w, a_log, dt_bias, rows, q, k, qh, kh, v, vh, g, beta);
+    la_conv_seq_kernel<<<ceil_div(n_runs * kLaHeads * 3, 4), 128, 0, s>>>(mixed, d_runs, n_runs, d_seqs, conv_layer, conv_stride,
+                                                                          conv_w, a_log, dt_bias, q, k, qh, kh, v, vh, g, beta);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -45,7 +45,7 @@ void la_carve_scratch(b200attn_la la) {
     la->d_core = (float*)take(R * kLaHeads * kLaVd * 4);
     la->d_xb = (__half*)take(R * kHidden * 2);
     la->d_gated = take(R * kLaHeads * kLaVd * 4);
-    la->meta_cap = (int)(2 * R + 65536);
+    la->meta_cap = (int)(4 * R + 65536);
     la->d_meta = (int*)take((size_t)la->meta_cap * 4);
 }
 
@@ -260,7 +260,7 @@ namespace b200 {
 static bool la_use_tensor_cores() { return !g_flags.la_prefill_serial; }
 
 static int la_build_meta(b200attn_la la, b200attn_la_state st, const int* h_slots, const int* h_counts, int n_seqs,
-                         int* rows_out, std::vector<LaSeqMeta>& seqs, LaSeqMeta** d_seqs, int** d_row_seq, bool need_row_seq,
+                         int* rows_out, std::vector<LaSeqMeta>& seqs, LaSeqMeta** d_seqs, LaRun** d_runs, int* n_runs,
                          cudaStream_t s) {
     B2_CHECK_ARG(h_slots && h_counts && n_seqs > 0, "linear attention: bad batch description");
     seqs.resize(n_seqs);
@@ -274,16 +274,18 @@ static int la_build_meta(b200attn_la la, b200attn_la_state st, const int* h_slot
     }
     *rows_out = rows;
     B2_CHECK_ARG(rows <= la->max_rows, "linear attention: %d rows exceed scratch capacity %d", rows, la->max_rows);
-    const int need = 3 * n_seqs + (need_row_seq ? rows : 0);
+    std::vector<LaRun> runs;
+    if (d_runs)
+        for (int i = 0; i < n_seqs; ++i)
+            for (int j = 0; j < h_counts[i]; j += kConvRun) runs.push_back(LaRun{seqs[i].row0 + j, i});
+    const int need = 3 * n_seqs + 1 + 2 * (int)runs.size();
     B2_CHECK_ARG(need <= la->meta_cap, "linear attention: metadata exceeds scratch");
     *d_seqs = reinterpret_cast<LaSeqMeta*>(la->d_meta);
-    *d_row_seq = la->d_meta + 3 * n_seqs;
     B2_CUDA(cudaMemcpyAsync(*d_seqs, seqs.data(), (size_t)n_seqs * sizeof(LaSeqMeta), cudaMemcpyHostToDevice, s));
-    if (need_row_seq && rows > 0) {
-        std::vector<int> row_seq(rows);
-        for (int i = 0, r = 0; i < n_seqs; ++i)
-            for (int j = 0; j < h_counts[i]; ++j) row_seq[r++] = i;
-        B2_CUDA(cudaMemcpyAsync(*d_row_seq, row_seq.data(), (size_t)rows * 4, cudaMemcpyHostToDevice, s));
+    if (d_runs) {
+        *d_runs = reinterpret_cast<LaRun*>(la->d_meta + 3 * n_seqs + (n_seqs & 1));
+        *n_runs = (int)runs.size();
+        if (!runs.empty()) B2_CUDA(cudaMemcpyAsync(*d_runs, runs.data(), runs.size() * sizeof(LaRun), cudaMemcpyHostToDevice, s));
     }
     return 0;
 }
@@ -344,14 +346,15 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
     int rows = 0;
     std::vector<LaSeqMeta> seqs;
     LaSeqMeta* d_seqs = nullptr;
-    int* d_row_seq = nullptr;
-    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, &d_row_seq, true, s));
+    LaRun* d_runs = nullptr;
+    int n_runs = 0;
+    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, &d_runs, &n_runs, s));
     if (rows == 0) return 0;
     B2_CHECK_ARG(rows <= la->cfg.max_prefill_rows, "la_prefill: %d rows exceed max_prefill_rows %d", rows, la->cfg.max_prefill_rows);
     const bool tc = la_use_tensor_cores();
     B2_TRY(project_in(rows));
-    B2_TRY(launch_la_conv_seq(la->d_mixed, d_row_seq, d_seqs, conv_layer, st->conv_stride_slot(), la->d_conv_w, la->d_a_log,
-                              la->d_dt_bias, rows, tc ? nullptr : la->d_q, tc ? nullptr : la->d_k, tc ? la->d_qh : nullptr,
+    B2_TRY(launch_la_conv_seq(la->d_mixed, d_runs, n_runs, d_seqs, conv_layer, st->conv_stride_slot(), la->d_conv_w, la->d_a_log,
+                              la->d_dt_bias, tc ? nullptr : la->d_q, tc ? nullptr : la->d_k, tc ? la->d_qh : nullptr,
                               tc ? la->d_kh : nullptr, tc ? nullptr : la->d_v, tc ? la->d_vh : nullptr, la->d_g, la->d_beta, s));
     B2_TRY(la_recurrence(la, st, layer, la->d_q, la->d_k, la->d_v, la->d_g, la->d_beta, d_seqs, n_seqs, rows, la->d_core, tc, s));
     B2_TRY(launch_la_conv_state_update(la->d_mixed, d_seqs, n_seqs, conv_layer, st->conv_stride_slot(), s));
@@ -381,8 +384,7 @@ extern "C" int b200attn_la_prefill_core(b200attn_la la, b200attn_la_state st, in
     int rows = 0;
     std::vector<LaSeqMeta> seqs;
     LaSeqMeta* d_seqs = nullptr;
-    int* d_row_seq = nullptr;
-    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, &d_row_seq, false, s));
+    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, nullptr, nullptr, s));
     if (rows == 0) return 0;
     if (use_tensor_cores) {
         B2_TRY(f32_to_f16(s, d_q, la->d_qh, (size_t)rows * kLaHeads * kLaKd));

@@ -328,3 +328,23 @@ def test_errors(ops, cuda, synth):
         la.forward_batch(x, st, 2, [0], [4])         # layer out of range
     with pytest.raises(ops.InvalidArgument):
         st.export_state(0, 9)
+
+
+@pytest.mark.parametrize("counts", [[1, 15, 16, 17], [2, 3, 33, 48, 5], [31, 1, 1, 64]])
+def test_prefill_runs_of_ragged_batches(ops, cuda, oracle, synth, counts):
+    """Lengths around the run of rows that a warp of the convolution takes, each sequence continued once, against the oracle."""
+    torch = cuda
+    w = synth.la_weights(91)
+    la = ops.LinearAttention(ops.PROJ_FP32, max_batch=8, max_prefill_rows=256)
+    la.set_weights(w)
+    st = ops.LinearAttnState(1, 8)
+    slots = [7 - i for i in range(len(counts))]
+    xs = [synth.hidden_states(91, f"run{i}", 2 * c) for i, c in enumerate(counts)]
+    first = la.forward_batch(torch.from_numpy(np.concatenate([x[:c] for x, c in zip(xs, counts)])).cuda(), st, 0, slots, counts).cpu().numpy()
+    then = la.forward_batch(torch.from_numpy(np.concatenate([x[c:] for x, c in zip(xs, counts)])).cuda(), st, 0, slots, counts).cpu().numpy()
+    at = 0
+    for i, (x, c) in enumerate(zip(xs, counts)):
+        want = oracle.OracleLinearAttention(w).forward_sequence(x)
+        ok, msg = allclose_report(np.concatenate([first[at:at + c], then[at:at + c]]), want, ATOL, RTOL)
+        assert ok, f"sequence {i} of {c} tokens: {msg}"
+        at += c
