@@ -182,7 +182,7 @@ int delta_forward(BlockModel& m, DeltaOp& op, const LayerRun& run, const PassRow
     gate.M = p.rows; gate.N = sh.gate_cols(); gate.K = gate.ldx = sh.low();
     gate.y = m.gates.p; gate.ldy = sh.gate_cols();
     gate.error = m.error.i();
-    if (p.in && gemm_rows_takes(gate, kRowsStore)) B2_TRY(gemm_rows(s, gate, op.elem, kRowsStore, false, ELEM_F32));
+    if (p.in && gemm_rows_takes(gate, kRowsStore)) B2_TRY(gemm_rows(s, gate, op.elem, kRowsStore, kLoadAsIs, ELEM_F32));
     else B2_TRY(gemm_typed(s, m.low.p, sh.low(), op.w_gate.p, m.gates.p, sh.gate_cols(), op.elem, ELEM_F32, p.rows, sh.gate_cols(), sh.low()));
     DeltaStepArgs a{sh, m.proj.f(), m.gates.f(), op.conv.f(), sh.taps <= 4 ? op.conv4.f() : nullptr, op.a_log.f(), op.dt_bias.f(), op.norm_w.f(), state, p.decode ? p.d_slots : nullptr,
                     p.decode ? nullptr : p.d_seqs, m.cfg.max_seqs, m.core.f(), m.mixed.p};

@@ -489,7 +489,7 @@ int block_project(BlockModel& m, const PassRows& p, const void* w, int cols, voi
     RowsGemm a = *p.in;
     a.w = w; a.N = cols;
     a.y = out; a.ldy = cols;
-    return gemm_rows(s, a, m.elem, kRowsStore, a.x != m.xt.p, out_type);
+    return gemm_rows(s, a, m.elem, kRowsStore, a.x != m.xt.p ? kLoadNorm : kLoadAsIs, out_type);
 }
 
 static int run_layers(BlockModel& m, const PassRows& pass, cudaStream_t s) {
@@ -557,7 +557,7 @@ static int run_layers(BlockModel& m, const PassRows& pass, cudaStream_t s) {
         a.ldy = W;
         a.error = m.error.i();
         const int epi = pre ? kRowsResidual : kRowsDeepStore;
-        if (few && gemm_rows_takes(a, epi)) B2_TRY(gemm_rows(s, a, m.elem, epi, false, ELEM_F32));
+        if (few && gemm_rows_takes(a, epi)) B2_TRY(gemm_rows(s, a, m.elem, epi, kLoadAsIs, ELEM_F32));
         else B2_TRY(gemm_typed(s, from, cols, w.p, a.y, W, m.elem, ELEM_F32, R, W, cols, pre ? 1.0f : 0.0f));
         if (pre) return 0;
         pending = &norm;
@@ -590,7 +590,7 @@ static int run_layers(BlockModel& m, const PassRows& pass, cudaStream_t s) {
             a.N = 2 * L.ff;
             a.group = L.ff;
             a.y = m.act.p; a.ldy = L.ff;
-            B2_TRY(gemm_rows(s, a, m.elem, L.act == B200ATTN_ACT_SILU ? kRowsSwiglu : kRowsGeglu, a.x != m.xt.p, m.elem));
+            B2_TRY(gemm_rows(s, a, m.elem, L.act == B200ATTN_ACT_SILU ? kRowsSwiglu : kRowsGeglu, a.x != m.xt.p ? kLoadNorm : kLoadAsIs, m.elem));
         } else {
             B2_TRY(gemm_typed(s, m.xt.p, W, L.w_gu.p, m.gu.p, 2 * L.ff, m.elem, m.elem, R, 2 * L.ff, W));
             B2_TRY(launch_act_mul(m.elem, L.act, m.gu.p, R, L.ff, m.act.p, s));
@@ -690,7 +690,7 @@ int block_logits(BlockModel& m, int n, const int* d_row_index, float* d_logits, 
         a.cap = (float)m.cfg.logit_softcap;
         a.y = d_logits; a.ldy = m.cfg.vocab_size;
         a.error = m.error.i();
-        return gemm_rows(s, a, m.elem, kRowsStore, true, ELEM_F32);
+        return gemm_rows(s, a, m.elem, kRowsStore, kLoadNorm, ELEM_F32);
     }
     B2_TRY(launch_rms_norm_rows(m.elem, m.x.f(), d_row_index, m.final_norm.f(), (float)m.cfg.norm_eps, n, W, m.xt.p, s));
     B2_TRY(gemm_typed(s, m.xt.p, W, m.cfg.own_head ? m.head.p : m.embed.p, d_logits, m.cfg.vocab_size, m.elem, ELEM_F32, n, m.cfg.vocab_size, W, 0.f,

@@ -10,9 +10,10 @@
 //     reduction over warps needs no shared memory of its own, and its order is fixed;
 //   * the fp32 residual rows are normalised on the way in (the rounding point is the norm kernel's: one rounding of the normalised value), and
 //     SwiGLU and the residual addition sit in the epilogue.  A layer of a step is five launches in place of eight or nine.
-// Measured in a captured step of 8 rows, from the dependency wait on: input projection (8224 x 1024) 5.4 us, gate / up with SwiGLU (7168 x 1024)
-// 4.6 us, output projections (1024 x 2048 and 1024 x 3584) 3.8 us; the step of four layers and the head 237 -> 149 us.  The first form, with X
-// in registers and one column tile at a time, ran eight warps through 2000 instructions each and took 8.6, 9.5 and 4.1 us.
+// Measured in a captured step of 8 rows, from the dependency wait on: input projection (8224 x 1024) 5.3 us, gate / up with SwiGLU (7168 x 1024)
+// 5.2 us, output projections (1024 x 2048 and 1024 x 3584) 3.1 us; the step of four layers and the head 237 -> 134 us.
+// Taken back: X in registers with one column tile at a time (eight warps through 2000 instructions each: 8.6, 9.5 and 4.1 us); asking L2 for the
+// weights of the launch after next (no change: the copies are not what a launch waits for).
 // tcgen05 would pad the rows to 64 or 128 and pay for a TMEM round trip (the kernels of gemm_tc.cu: 9.0, 10.8 and 10.5 us).  From 33 rows on X no
 // longer fits beside the slabs, and the library GEMMs serve the step.
 #include "gemm_rows.cuh"
@@ -50,22 +51,42 @@ __device__ __forceinline__ unsigned long long pack_max(float v, int idx) {
 }
 
 // k is assigned to lanes in runs of eight (lane % 4), the same for both operands of a product, so every load is 16 bytes.  Rows of
-// operands in shared memory are 64 bytes modulo 128 apart: the two rows that eight lanes read together fill the 32 banks.
-__device__ __forceinline__ int rows_pitch(int k) { return (k * 2 + 127) / 128 * 128 + 64; }
+// operands in shared memory are 64 bytes modulo 128 apart: the two rows that eight lanes read together fill the 32 banks.  A weight row is a bulk
+// copy of its own: few large ones (8 rows each, unpadded) arrived later, 158 us a step in place of 149.
+__device__ __host__ __forceinline__ int rows_pitch(int k) { return (k * 2 + 127) / 128 * 128 + 64; }
 
-// A tile's partial sums of one warp, 16 MT x 8 floats, lie in the eight weight rows they came from, in the slice [64 k0, 64 (k0 + chunks))
-// that this warp alone has read: row m % 8, with the halves m / 8 swapped in every other pair of rows against bank conflicts.
-__device__ __forceinline__ uint32_t part_at(int m, int pitch) {
-    return (uint32_t)((m & 7) * pitch + (((m >> 3) ^ ((m >> 1) & 1)) * 32));
-}
+// The items of a launch, cut evenly: part i of n gets [i items / n, (i + 1) items / n).  A launch has one CTA per SM: with fewer, the next
+// launch put two CTAs on each idle SM and left no registers there for the one behind it, which then came late.
+__device__ __forceinline__ int part_begin(int i, int n, int items) { return (int)((long long)i * items / n); }
+
+// K in slices of `per` chunks of 32, one per warp.  A tile's partial sums of one warp, 16 MT x 8 floats, lie in the eight weight rows they came
+// from, in the slice that this warp alone has read (the last one may reach into the padding): row m % 8, with the halves m / 8 swapped in every
+// other pair of rows against bank conflicts.
 template <int MT>
-__device__ __forceinline__ void store_part(unsigned char* slice, int pitch, int r, int c, const float (&acc)[MT][4]) {
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        *reinterpret_cast<float2*>(slice + part_at(16 * mt + r, pitch) + 8 * c) = make_float2(acc[mt][0], acc[mt][1]);
-        *reinterpret_cast<float2*>(slice + part_at(16 * mt + 8 + r, pitch) + 8 * c) = make_float2(acc[mt][2], acc[mt][3]);
+struct Slices {
+    int chunks, per, active;      // active slices
+    __device__ __forceinline__ Slices(int k, int warps) : chunks(k / 32) {
+        per = max(MT, (chunks + warps - 1) / warps);
+        active = (chunks + per - 1) / per;
     }
-}
+    __device__ __forceinline__ int begin(int w) const { return min(chunks, w * per); }
+    __device__ __forceinline__ static int at(int m, int pitch) { return (m & 7) * pitch + (((m >> 3) ^ ((m >> 1) & 1)) * 32); }
+    __device__ __forceinline__ void store(unsigned char* tile, int pitch, int w, int r, int c, const float (&acc)[MT][4]) const {
+        unsigned char* slice = tile + w * per * 64 + 8 * c;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            *reinterpret_cast<float2*>(slice + at(16 * mt + r, pitch)) = make_float2(acc[mt][0], acc[mt][1]);
+            *reinterpret_cast<float2*>(slice + at(16 * mt + 8 + r, pitch)) = make_float2(acc[mt][2], acc[mt][3]);
+        }
+    }
+    __device__ __forceinline__ float total(const unsigned char* tile, int pitch, int m, int n) const {
+        const unsigned char* p = tile + at(m, pitch) + 4 * n;
+        float v = 0.f;
+#pragma unroll 8
+        for (int w = 0; w < active; ++w) v += *reinterpret_cast<const float*>(p + w * per * 64);
+        return v;
+    }
+};
 
 // The gate's activation: library functions in fp16 stacks (swiglu_kernel), the forms of act_mul_kernel where the result is rounded to bf16.
 template <typename T, int EPI>
@@ -77,67 +98,11 @@ __device__ __forceinline__ float rows_act(float g) {
 
 constexpr int kRowsThreads = 512, kRowsWarps = 16;
 
-// Many columns, K <= 1024: X in shared memory as 16-bit rows, `tiles` column tiles at a time.  A warp multiplies four tiles (two groups
-// of eight warps when there are more than four) over its part of K.  grid: CTAs walk batches of `tiles` tiles; `buffers` slabs of
-// weights in a ring.  LOAD: X comes in as 16-bit rows, as fp32 rows to normalise, or as
-// fp32 rows to which normalised rows `add` are added first; the sums then also go to x_out, row m from CTA m.
-enum { kLoadAsIs = 0, kLoadNorm, kLoadAddNorm };
-template <typename T, int MT, int LOAD, int EPI, typename YT>
-__global__ void __launch_bounds__(kRowsThreads, 2)
-rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
-    constexpr int kRows = 16 * MT;
-    constexpr bool kGated = EPI == kRowsSwiglu || EPI == kRowsGeglu;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int pitch = rows_pitch(a.K), batch_rows = 8 * a.tiles;
-    const uint32_t slab = (uint32_t)(batch_rows * pitch);
-    unsigned char* sx = smem + a.buffers * slab;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sx + kRows * pitch);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + a.buffers);
-    const uint32_t base = smem_u32(smem), bar0 = smem_u32(bars);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
-    const int batches = (a.N + batch_rows - 1) / batch_rows;
-
-    // Weight row behind row j of a batch.  SwiGLU: pairs of tiles, 8 gate rows then the 8 matching up rows.
-    auto weight_row = [&](int batch, int j) {
-        if constexpr (kGated) {
-            const int ch = batch * (batch_rows / 2) + (j >> 4) * 8 + (j & 7);
-            return 2 * ch < a.N ? (ch / a.group) * 2 * a.group + ch % a.group + ((j & 8) ? a.group : 0) : -1;
-        } else {
-            const int n = batch * batch_rows + j;
-            return n < a.N ? n : -1;
-        }
-    };
-    auto fetch = [&](int batch, int buf) {      // warp 0: one bulk copy per row; the barrier first learns the number of bytes
-        const uint32_t bytes = (uint32_t)a.K * 2;
-        int have = 0;
-        for (int j = lane; j < batch_rows; j += 32) have += weight_row(batch, j) >= 0;
-        have = __reduce_add_sync(0xffffffffu, have);
-        if (lane == 0) mbar_arrive_expect_tx(bar0 + 8u * buf, (uint32_t)have * bytes);
-        __syncwarp();
-        for (int j = lane; j < batch_rows; j += 32) {
-            const int n = weight_row(batch, j);
-            if (n >= 0) bulk_g2s(base + buf * slab + j * pitch, static_cast<const T*>(a.w) + (size_t)n * a.K, bytes, bar0 + 8u * buf);
-        }
-    };
-    int next = blockIdx.x;                       // warp 0's next batch to fetch
-    if (warp == 0) {
-        if (lane == 0) {
-            for (int i = 0; i < a.buffers; ++i) mbar_init(bar0 + 8u * i, 1);
-            *abort_flag = 0;
-            mbar_fence_init();
-        }
-        __syncwarp();
-        for (int i = 0; i < a.buffers && next < batches; ++i, next += gridDim.x) fetch(next, i);
-    }
-    // The next kernel of the stream may take its place now.  If it is one of these it fetches weights and waits; any other waits before
-    // it touches what a step writes, or reads recurrent state that a kernel writes only after a wait of its own (la_decode_kernel).
-    pdl_launch_dependents();
-    pdl_wait();
-    stamp_begin(stamp);
-
-    // ---- X: a warp per row ---------------------------------------------------------------------------------------------
+// X into shared memory as 16-bit rows, a warp per row.
+template <typename T, int LOAD, int WARPS>
+__device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, int pitch, int warp, int lane) {
 #pragma unroll 1
-    for (int m = warp; m < a.M; m += kRowsWarps) {
+    for (int m = warp; m < a.M; m += WARPS) {
         const size_t at = (size_t)(a.row_index ? a.row_index[m] : m) * a.ldx;
         unsigned char* dst = sx + m * pitch;
         if constexpr (LOAD == kLoadAsIs) {
@@ -156,17 +121,20 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
                 const int k = 4 * (32 * i + lane);
                 v[i] = k < a.K ? __ldcg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
+            float rs = 1.0f;
+            if constexpr (LOAD != kLoadF32) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+                for (int i = 0; i < 8; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            const float rs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
+                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                rs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int k = 4 * (32 * i + lane);
                 if (k < a.K) {
                     float4 w = make_float4(rs, rs, rs, rs);
-                    if (a.norm_w) {
+                    if (LOAD != kLoadF32 && a.norm_w) {
                         const float4 f = __ldg(reinterpret_cast<const float4*>(a.norm_w + k));
                         w = make_float4(rs * (a.norm_base + f.x), rs * (a.norm_base + f.y), rs * (a.norm_base + f.z), rs * (a.norm_base + f.w));
                     }
@@ -181,89 +149,111 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
             }
         }
     }
+}
+
+// Many columns, K <= 1024: X in shared memory, up to eight column tiles per CTA.  A warp multiplies four tiles (two groups of eight warps when a
+// launch has CTAs with more than four) over its slice of K.  Gated: units of two tiles, 8 gate rows of the weights and the 8 up rows that
+// belong to them; the slab holds all gate rows, then all up rows.
+template <typename T, int MT, int LOAD, int EPI, typename YT>
+__global__ void __launch_bounds__(kRowsThreads, 2)
+rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
+    constexpr int kRows = 16 * MT;
+    constexpr bool kGated = EPI == kRowsSwiglu || EPI == kRowsGeglu;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int pitch = rows_pitch(a.K), row_bytes = a.K * 2;
+    unsigned char* sx = smem + 8 * a.tiles * pitch;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sx + kRows * pitch);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
+    const int cols = kGated ? a.N / 2 : a.N, units = (cols + 7) / 8;                         // output columns, and eights of them
+    const int u0 = part_begin(blockIdx.x, gridDim.x, units), u1 = part_begin(blockIdx.x + 1, gridDim.x, units);
+    const int col0 = 8 * u0, n_cols = min(cols, 8 * u1) - col0, half = 8 * (u1 - u0) * pitch;      // gated: the up rows' place
+    const int tiles = (kGated ? 2 : 1) * (u1 - u0);
+
+    if (warp == 0 && n_cols > 0) {
+        if (lane == 0) {
+            mbar_init(smem_u32(bar), 1);
+            *abort_flag = 0;
+            mbar_fence_init();
+            mbar_arrive_expect_tx(smem_u32(bar), (uint32_t)((kGated ? 2 : 1) * n_cols * row_bytes));
+        }
+        __syncwarp();
+        for (int i = lane; i < n_cols; i += 32) {
+            const int n = col0 + i, from = kGated ? n + n / a.group * a.group : n;
+            bulk_g2s(smem_u32(smem) + i * pitch, static_cast<const T*>(a.w) + (size_t)from * a.K, (uint32_t)row_bytes, smem_u32(bar));
+            if (kGated)
+                bulk_g2s(smem_u32(smem) + half + i * pitch, static_cast<const T*>(a.w) + (size_t)(from + a.group) * a.K, (uint32_t)row_bytes, smem_u32(bar));
+        }
+    }
+    // The next kernel of the stream may take its place now.  If it is one of these it fetches weights and waits; any other waits before
+    // it touches what a step writes, or reads recurrent state that a kernel writes only after a wait of its own (la_decode_kernel).
+    if (!a.late) pdl_launch_dependents();
+    pdl_wait();
+    if (a.late) pdl_launch_dependents();
+    stamp_begin(stamp);
+    load_rows<T, LOAD, kRowsWarps>(a, sx, pitch, warp, lane);
     __syncthreads();
+    if (n_cols <= 0) return;
 
     // ---- products --------------------------------------------------------------------------------------------------------
     const int groups = a.tiles > 4 ? 2 : 1, splits = kRowsWarps / groups, split = warp % splits, tile0 = (warp / splits) * 4;
-    const int chunks = a.K / 32, per = max(MT, (chunks + splits - 1) / splits), c0 = split * per, c1 = min(c0 + per, chunks);
-    const int active = (chunks + per - 1) / per;
+    const Slices<MT> sl(a.K, splits);
+    const int c0 = sl.begin(split), c1 = sl.begin(split + 1);
     const bool high = a.M > 8;
-    unsigned long long best = pack_max(-INFINITY, 0);      // a row without a number above -inf gives token 0
-    int buf = 0;
-    uint32_t parity = 0;
-    for (int batch = blockIdx.x; batch < batches; batch += gridDim.x) {
-        if (!mbar_wait(bar0 + 8u * buf, parity, abort_flag)) break;
-        unsigned char* sw = smem + buf * slab;
-        float acc[4][MT][4] = {};
-        const unsigned char* xp = sx + r * pitch + c * 16;
-        const unsigned char* wp = sw + (8 * tile0 + r) * pitch + c * 16;
+    auto tile_at = [&](int t) { return smem + (kGated ? (t & 1) * half + 8 * (t >> 1) * pitch : 8 * t * pitch); };
+    const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
+    float acc[4][MT][4] = {};
+    const unsigned char* xp = sx + r * pitch + c * 16;
+    auto x_frag = [&](int mt, int ch, uint4& lo, uint4& hi) {
+        lo = *reinterpret_cast<const uint4*>(xp + 16 * mt * pitch + ch * 64);
+        hi = make_uint4(0u, 0u, 0u, 0u);
+        if (high) hi = *reinterpret_cast<const uint4*>(xp + (16 * mt + 8) * pitch + ch * 64);
+    };
+    auto multiply = [&](float (&d)[4], const uint4& lo, const uint4& hi, const uint4& b) {
+        mma_rows<T>(d, lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+        mma_rows<T>(d, lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+    };
 #pragma unroll(MT == 1 ? 2 : 1)
-        for (int ch = c0; ch < c1; ++ch) {
-            uint4 lo[MT], hi[MT];
+    for (int ch = c0; ch < c1; ++ch) {
+        uint4 lo[MT], hi[MT];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                lo[mt] = *reinterpret_cast<const uint4*>(xp + 16 * mt * pitch + ch * 64);
-                hi[mt] = make_uint4(0u, 0u, 0u, 0u);
-                if (high) hi[mt] = *reinterpret_cast<const uint4*>(xp + (16 * mt + 8) * pitch + ch * 64);
+        for (int mt = 0; mt < MT; ++mt) x_frag(mt, ch, lo[mt], hi[mt]);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (tile0 + t < tiles) {
+                const uint4 b = *reinterpret_cast<const uint4*>(tile_at(tile0 + t) + r * pitch + c * 16 + ch * 64);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) multiply(acc[t][mt], lo[mt], hi[mt], b);
             }
+    }
+    __syncwarp();                                // every lane has read the slice: it may be overwritten
+    if (c0 < c1) {
 #pragma unroll
-            for (int t = 0; t < 4; ++t)
-                if (tile0 + t < a.tiles) {
-                    const uint4 b = *reinterpret_cast<const uint4*>(wp + 8 * t * pitch + ch * 64);
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        mma_rows<T>(acc[t][mt], lo[mt].x, hi[mt].x, lo[mt].y, hi[mt].y, b.x, b.y);
-                        mma_rows<T>(acc[t][mt], lo[mt].z, hi[mt].z, lo[mt].w, hi[mt].w, b.z, b.w);
-                    }
-                }
-        }
-        __syncwarp();                            // every lane has read the slice: it may be overwritten
-        if (c0 < chunks) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                if (tile0 + t < a.tiles) store_part<MT>(sw + 8 * (tile0 + t) * pitch + c0 * 64, pitch, r, c, acc[t]);
-        }
-        __syncthreads();
-        auto total = [&](int t, int m, int n) {
-            const unsigned char* p = sw + 8 * t * pitch + part_at(m, pitch) + 4 * n;
-            float v = 0.f;
-#pragma unroll 8
-            for (int w = 0; w < active; ++w) v += *reinterpret_cast<const float*>(p + w * per * 64);
-            return v;
-        };
-        const int n8 = tid & 7, em = (tid >> 3) % kRows;
-        if (em < a.M) {
+        for (int t = 0; t < 4; ++t)
+            if (tile0 + t < tiles) sl.store(tile_at(tile0 + t), pitch, split, r, c, acc[t]);
+    }
+    __syncthreads();
+    const int n8 = tid & 7, em = (tid >> 3) % kRows;
+    unsigned long long best = pack_max(-INFINITY, 0);      // a row without a number above -inf gives token 0
+    if (em < a.M && ok) {
+        for (int u = tid / (8 * kRows); u < u1 - u0; u += kRowsThreads / (8 * kRows)) {
+            const int n = col0 + 8 * u + n8;
+            if (n >= cols) break;
             if constexpr (kGated) {
-                for (int p = tid / (8 * kRows); p < a.tiles / 2; p += kRowsThreads / (8 * kRows)) {
-                    const int ch = batch * (batch_rows / 2) + 8 * p + n8;
-                    if (2 * ch >= a.N) break;
-                    const float g = total(2 * p, em, n8), u = total(2 * p + 1, em, n8);
-                    static_cast<YT*>(a.y)[(size_t)em * a.ldy + ch] = to_out<YT>(rows_act<T, EPI>(g) * u);
-                }
+                const float g = sl.total(tile_at(2 * u), pitch, em, n8), up = sl.total(tile_at(2 * u + 1), pitch, em, n8);
+                static_cast<YT*>(a.y)[(size_t)em * a.ldy + n] = to_out<YT>(rows_act<T, EPI>(g) * up);
             } else {
-                for (int t = tid / (8 * kRows); t < a.tiles; t += kRowsThreads / (8 * kRows)) {
-                    const int n = batch * batch_rows + 8 * t + n8;
-                    if (n >= a.N) break;
-                    float v = total(t, em, n8);
-                    if (a.scale != 1.0f) v *= a.scale;
-                    if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
-                    if constexpr (EPI == kRowsStore) static_cast<YT*>(a.y)[(size_t)em * a.ldy + n] = to_out<YT>(v);
-                    else if (v > -INFINITY) best = max(best, pack_max(v, n));
-                }
+                float v = sl.total(tile_at(u), pitch, em, n8) * a.scale;
+                if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
+                if constexpr (EPI == kRowsStore) static_cast<YT*>(a.y)[(size_t)em * a.ldy + n] = to_out<YT>(v);
+                else if (v > -INFINITY) best = max(best, pack_max(v, n));
             }
         }
-        if (batch + (int)gridDim.x < batches) {
-            fence_proxy_async_smem();            // the slab was read and written by ordinary accesses, the next copy into it is not one
-            __syncthreads();
-            if (warp == 0 && next < batches) { fetch(next, buf); next += gridDim.x; }
-        }
-        if (++buf == a.buffers) { buf = 0; parity ^= 1u; }
     }
     if constexpr (EPI == kRowsArgmax) {
-        const int em = (tid >> 3) % kRows;
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-        if ((tid & 7) == 0 && em < a.M) atomicMax(a.packed + em, best);
+        if (n8 == 0 && em < a.M) atomicMax(a.packed + em, best);
     }
     if (stamp) {
         __syncthreads();
@@ -272,8 +262,114 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (tid == 0 && *abort_flag && a.error) atomicExch(a.error, 7);
 }
 
-// Few columns, deep K <= 4096: fp32 Y[M, N] = X W^T, added to what is there with ADD.  One column tile per CTA, the 16 warps split K, X goes from L2 straight into the
-// registers of the warp that multiplies it, kAhead chunks at a time.
+// More columns than a wave of CTAs holds at eight tiles each (the LM head), K <= 1024: the warps work on tiles of their own.  A warp streams
+// its tiles' weights through one slab in two halves of K, each refilled as soon as it has been multiplied, so that most of the 135 KB are
+// in flight all the time, and no barrier of the CTA and no reduction stands between two tiles.
+// 32768 columns at 8 rows: 15.5 us from the dependency wait on, 67 MB; a ring at whose batches of tiles all warps met took 19.4 us, gemm_tc.cu's 20.9 us.
+constexpr int kStreamWarps = 8;
+template <typename T, int MT, int LOAD, int EPI>
+__global__ void __launch_bounds__(kStreamWarps * 32)
+rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int pitch = rows_pitch(a.K), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
+    unsigned char* sw = smem + warp * 8 * pitch;
+    unsigned char* sx = smem + kStreamWarps * 8 * pitch;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sx + 16 * MT * pitch);              // two per warp
+    unsigned long long* s_best = reinterpret_cast<unsigned long long*>(bars + 2 * kStreamWarps);     // [16 MT]
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(s_best + 16 * MT);
+    const uint32_t bar = smem_u32(bars + 2 * warp);
+    const int chunks = a.K / 32, mid = (chunks + 1) / 2, n_tiles = (a.N + 7) / 8, step = gridDim.x * kStreamWarps;
+    const int first = blockIdx.x + gridDim.x * warp;
+    auto fetch = [&](int tile, int half) {
+        const int k0 = half ? mid * 32 : 0, n = (half ? chunks - mid : mid) * 32, rows = min(8, a.N - 8 * tile);
+        if (n == 0) return;
+        if (lane == 0) mbar_arrive_expect_tx(bar + 8 * half, (uint32_t)(rows * n * 2));
+        __syncwarp();
+        if (lane < rows)
+            bulk_g2s(smem_u32(sw) + lane * pitch + 2 * k0, static_cast<const T*>(a.w) + (size_t)(8 * tile + lane) * a.K + k0, (uint32_t)n * 2, bar + 8 * half);
+    };
+    if (lane == 0) {
+        mbar_init(bar, 1);
+        mbar_init(bar + 8, 1);
+        if (warp == 0) *abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (tid < 16 * MT) s_best[tid] = 0ull;
+    __syncwarp();
+    if (first < n_tiles) { fetch(first, 0); fetch(first, 1); }
+    pdl_launch_dependents();                     // see rows_wide_kernel
+    pdl_wait();
+    stamp_begin(stamp);
+    load_rows<T, LOAD, kStreamWarps>(a, sx, pitch, warp, lane);
+    __syncthreads();
+
+    const bool high = a.M > 8;
+    unsigned long long best[2 * MT];
+#pragma unroll
+    for (int i = 0; i < 2 * MT; ++i) best[i] = pack_max(-INFINITY, 0);       // a row without a number above -inf gives token 0
+    const unsigned char* xp = sx + r * pitch + c * 16;
+    const unsigned char* wp = sw + r * pitch + c * 16;
+    uint32_t parity = 0;
+    bool ok = true;
+    for (int tile = first; ok && tile < n_tiles; tile += step, parity ^= 1u) {
+        float acc[2][MT][4] = {};                // two chains
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            const int c0 = half ? mid : 0, c1 = half ? chunks : mid;
+            if (c0 == c1) continue;
+            ok = mbar_wait_warp(bar + 8 * half, parity, abort_flag);
+            if (!ok) break;
+#pragma unroll 4
+            for (int ch = c0; ch < c1; ++ch) {
+                const uint4 b = *reinterpret_cast<const uint4*>(wp + ch * 64);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    const uint4 lo = *reinterpret_cast<const uint4*>(xp + 16 * mt * pitch + ch * 64);
+                    uint4 hi = make_uint4(0u, 0u, 0u, 0u);
+                    if (high) hi = *reinterpret_cast<const uint4*>(xp + (16 * mt + 8) * pitch + ch * 64);
+                    mma_rows<T>(acc[0][mt], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+                    mma_rows<T>(acc[1][mt], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+                }
+            }
+            __syncwarp();                        // every lane has read the half
+            if (tile + step < n_tiles) {
+                fence_proxy_async_smem();        // it was read by ordinary loads, the next copy into it is not one
+                fetch(tile + step, half);
+            }
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int m = 16 * mt + 8 * (i >> 1) + r, n = 8 * tile + 2 * c + (i & 1);
+                float v = (acc[0][mt][i] + acc[1][mt][i]) * a.scale;
+                if (m >= a.M || n >= a.N) continue;
+                if constexpr (EPI == kRowsStore) {
+                    if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
+                    static_cast<float*>(a.y)[(size_t)m * a.ldy + n] = v;
+                } else if (v > -INFINITY) {
+                    best[2 * mt + (i >> 1)] = max(best[2 * mt + (i >> 1)], pack_max(v, n));
+                }
+            }
+    }
+    if constexpr (EPI == kRowsArgmax) {
+#pragma unroll
+        for (int i = 0; i < 2 * MT; ++i) {
+            best[i] = max(best[i], __shfl_xor_sync(0xffffffffu, best[i], 1));
+            best[i] = max(best[i], __shfl_xor_sync(0xffffffffu, best[i], 2));
+            if (c == 0) atomicMax(s_best + 8 * i + r, best[i]);
+        }
+        __syncthreads();
+        if (tid < 16 * MT && tid < a.M) atomicMax(a.packed + tid, s_best[tid]);
+    }
+    __syncthreads();
+    stamp_end(stamp);
+    if (tid == 0 && *abort_flag && a.error) atomicExch(a.error, 7);
+}
+
+// Few columns, deep K <= 4096: fp32 Y[M, N] = X W^T, added to what is there with ADD.  Up to eight columns per CTA (six or seven of 1024 on 148
+// SMs), the 16 warps split K, X goes from L2 straight into the registers of the warp that multiplies it, kAhead chunks at a time.
 template <typename T, int MT, bool ADD>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
@@ -283,26 +379,27 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 8 * pitch);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
-    const int n0 = blockIdx.x * 8, n = n0 + (tid & 7), em = (tid >> 3) % kRows;
+    const int n0 = part_begin(blockIdx.x, gridDim.x, a.N), cols = part_begin(blockIdx.x + 1, gridDim.x, a.N) - n0;
+    const int n8 = tid & 7, em = (tid >> 3) % kRows;
     if (warp == 0) {
         if (lane == 0) {
             mbar_init(smem_u32(bar), 1);
             *abort_flag = 0;
             mbar_fence_init();
-            mbar_arrive_expect_tx(smem_u32(bar), (uint32_t)(min(8, a.N - n0) * a.K * 2));
+            mbar_arrive_expect_tx(smem_u32(bar), (uint32_t)(cols * a.K * 2));
         }
         __syncwarp();
-        if (lane < 8 && n0 + lane < a.N)
+        if (lane < cols)
             bulk_g2s(smem_u32(smem) + lane * pitch, static_cast<const T*>(a.w) + (size_t)(n0 + lane) * a.K, (uint32_t)a.K * 2, smem_u32(bar));
     }
     pdl_launch_dependents();                     // see rows_wide_kernel
     pdl_wait();
     stamp_begin(stamp);
-    const int chunks = a.K / 32, per = max(MT, (chunks + kRowsWarps - 1) / kRowsWarps), c0 = warp * per, c1 = min(c0 + per, chunks);
-    const int active = (chunks + per - 1) / per;
-    const bool writes = tid < 8 * kRows && em < a.M && n < a.N;
+    const Slices<MT> sl(a.K, kRowsWarps);
+    const int c0 = sl.begin(warp), c1 = sl.begin(warp + 1);
+    const bool writes = tid < 8 * kRows && em < a.M && n8 < cols;
     float res = 0.f;
-    if (ADD && writes) res = __ldcg(static_cast<const float*>(a.y) + (size_t)em * a.ldy + n);
+    if (ADD && writes) res = __ldcg(static_cast<const float*>(a.y) + (size_t)em * a.ldy + n0 + n8);
     const T* xp = static_cast<const T*>(a.x) + (size_t)r * a.ldx + 8 * c;
     auto load = [&](int i, int ch) {             // rows 8 i + r, chunk ch
         return 8 * i + r < a.M && ch < c1 ? __ldcg(reinterpret_cast<const uint4*>(xp + (size_t)8 * i * a.ldx + 32 * ch)) : make_uint4(0u, 0u, 0u, 0u);
@@ -313,24 +410,23 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
 #pragma unroll
         for (int i = 0; i < 2 * MT; ++i) x[j][i] = load(i, c0 + j);
     __syncthreads();                             // the barrier is initialised
-    bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
+    const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
     float acc[2][MT][4] = {};                    // two chains
     const unsigned char* wp = smem + r * pitch + c * 16;
 #pragma unroll 1
     for (int g = c0; g < c1; g += kAhead) {
 #pragma unroll
         for (int j = 0; j < kAhead; ++j) {
-            if (g + j < c1) {
-                const uint4 b = *reinterpret_cast<const uint4*>(wp + (g + j) * 64);
+            if (g + j >= c1) break;
+            const uint4 b = *reinterpret_cast<const uint4*>(wp + (g + j) * 64);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    const uint4 lo = x[j][2 * mt], hi = x[j][2 * mt + 1];
-                    mma_rows<T>(acc[0][mt], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-                    mma_rows<T>(acc[1][mt], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
-                }
-#pragma unroll
-                for (int i = 0; i < 2 * MT; ++i) x[j][i] = load(i, g + j + kAhead);
+            for (int mt = 0; mt < MT; ++mt) {
+                const uint4 lo = x[j][2 * mt], hi = x[j][2 * mt + 1];
+                mma_rows<T>(acc[0][mt], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+                mma_rows<T>(acc[1][mt], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
             }
+#pragma unroll
+            for (int i = 0; i < 2 * MT; ++i) x[j][i] = load(i, g + j + kAhead);
         }
     }
 #pragma unroll
@@ -338,15 +434,9 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[0][mt][i] += acc[1][mt][i];
     __syncwarp();
-    if (c0 < chunks) store_part<MT>(smem + c0 * 64, pitch, r, c, acc[0]);
+    if (c0 < c1) sl.store(smem, pitch, warp, r, c, acc[0]);
     __syncthreads();
-    if (writes && ok) {
-        const unsigned char* p = smem + part_at(em, pitch) + 4 * (tid & 7);
-        float v = 0.f;
-#pragma unroll 8
-        for (int w = 0; w < active; ++w) v += *reinterpret_cast<const float*>(p + w * per * 64);
-        static_cast<float*>(a.y)[(size_t)em * a.ldy + n] = res + v;
-    }
+    if (writes && ok) static_cast<float*>(a.y)[(size_t)em * a.ldy + n0 + n8] = res + sl.total(smem, pitch, em, n8);
     if (stamp) {
         __syncthreads();
         stamp_end(stamp);
@@ -354,10 +444,8 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (tid == 0 && *abort_flag && a.error) atomicExch(a.error, 7);
 }
 
-int host_pitch(int k) { return (k * 2 + 127) / 128 * 128 + 64; }
-
-// Most shared memory of a launch: what a layer's launches need side by side (152 and 33 KB, 169 and 59 KB), and what a ring may take.
-constexpr int kSharedMost = 172 * 1024;
+// Most shared memory of a launch.  Up to 16 rows a layer's launches fit side by side: 153 and 34 KB, 170 and 59 KB.
+constexpr int kSharedMost = 208 * 1024;
 
 template <typename K>
 int prepare(PerDeviceOnce& once, K kernel) {
@@ -371,18 +459,23 @@ int launch_wide(RowsGemm a, cudaStream_t s, ProfKind kind) {
     B2_TRY(prepare(once, rows_wide_kernel<T, MT, LOAD, EPI, YT>));
     int sms = 0;
     B2_TRY(device_sm_count(&sms));
-    const int unit = EPI == kRowsSwiglu || EPI == kRowsGeglu ? 2 : 1, n_tiles = ceil_div(a.N, 8), tile = 8 * host_pitch(a.K);
-    const int room = kSharedMost - 16 * MT * host_pitch(a.K) - 128;
-    a.tiles = ceil_div(ceil_div(n_tiles, unit), sms) * unit;      // one batch per CTA, one CTA per SM ...
-    a.buffers = 1;
-    if (a.tiles > 8 || a.tiles * tile > room) {                   // ... or, for more columns than a wave holds, batches of four tiles through a ring
-        a.tiles = 4;
-        a.buffers = std::min(4, room / (4 * tile));
-    }
-    const int grid = std::min(sms, ceil_div(n_tiles, a.tiles));
-    const size_t smem = (size_t)a.buffers * a.tiles * tile + 16 * MT * host_pitch(a.K) + 8 * a.buffers + 16;
+    const int unit = EPI == kRowsSwiglu || EPI == kRowsGeglu ? 2 : 1, units = ceil_div(a.N / unit, 8);
+    const int waves = ceil_div(units * unit, 8 * sms), grid = std::min(units, waves * sms);     // one CTA per SM where eight tiles each are enough
+    a.tiles = ceil_div(units, grid) * unit;
+    const size_t smem = (size_t)(8 * a.tiles + 16 * MT) * rows_pitch(a.K) + 16;
     unsigned long long* stamp = prof_stamp_slot(kind);
     launch_pdl_split(true, true, rows_wide_kernel<T, MT, LOAD, EPI, YT>, dim3(grid), dim3(kRowsThreads), smem, s, a, stamp);
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+
+template <typename T, int MT, int LOAD, int EPI>
+int launch_stream(const RowsGemm& a, int sms, cudaStream_t s, ProfKind kind) {
+    static PerDeviceOnce once;
+    B2_TRY(prepare(once, rows_stream_kernel<T, MT, LOAD, EPI>));
+    const size_t smem = (size_t)(8 * kStreamWarps + 16 * MT) * rows_pitch(a.K) + 8 * (2 * kStreamWarps + 16 * MT) + 16;
+    unsigned long long* stamp = prof_stamp_slot(kind);
+    launch_pdl_split(true, true, rows_stream_kernel<T, MT, LOAD, EPI>, dim3(sms), dim3(kStreamWarps * 32), smem, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -392,13 +485,23 @@ int launch_deep(const RowsGemm& a, cudaStream_t s) {
     static PerDeviceOnce once;
     B2_TRY(prepare(once, rows_deep_kernel<T, MT, ADD>));
     unsigned long long* stamp = prof_stamp_slot(PROF_GEMM_RES);
-    launch_pdl_split(true, true, rows_deep_kernel<T, MT, ADD>, dim3(ceil_div(a.N, 8)), dim3(kRowsThreads), (size_t)8 * host_pitch(a.K) + 16, s, a, stamp);
+    int sms = 0;
+    B2_TRY(device_sm_count(&sms));
+    const int grid = std::max(ceil_div(a.N, 8), std::min(a.N, sms));      // up to eight columns a CTA
+    launch_pdl_split(true, true, rows_deep_kernel<T, MT, ADD>, dim3(grid), dim3(kRowsThreads), (size_t)8 * rows_pitch(a.K) + 16, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 template <typename T, int LOAD, int EPI, typename YT>
 int wide(const RowsGemm& a, cudaStream_t s, ProfKind kind) {
+    // Above eight tiles a CTA: the streaming form, for the outputs that such products have.  At 9472 columns and fewer (148 SMs) a CTA holds its
+    // whole slab, which is fetched before the wait, and splitting K over the warps ends sooner.
+    if constexpr ((EPI == kRowsStore && std::is_same_v<YT, float>) || EPI == kRowsArgmax) {
+        int sms = 0;
+        B2_TRY(device_sm_count(&sms));
+        if (a.N > 64 * sms) return a.M <= 16 ? launch_stream<T, 1, LOAD, EPI>(a, sms, s, kind) : launch_stream<T, 2, LOAD, EPI>(a, sms, s, kind);
+    }
     return a.M <= 16 ? launch_wide<T, 1, LOAD, EPI, YT>(a, s, kind) : launch_wide<T, 2, LOAD, EPI, YT>(a, s, kind);
 }
 template <typename T, bool ADD>
@@ -414,14 +517,17 @@ bool gemm_rows_takes(const RowsGemm& a, int epi) {
            (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
 }
 
-int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, bool norm, ElemType out) {
+int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int load, ElemType out) {
     if (!gemm_rows_takes(a, epi)) B2_FAIL(B200ATTN_ERR_UNSUPPORTED, "gemm_rows: unsupported shape %d x %d x %d", a.M, a.N, a.K);
     using B = __nv_bfloat16;
+    const bool norm = load == kLoadNorm;
     if (type == ELEM_F16) {
+        if (epi == kRowsStore && out == ELEM_F32 && load == kLoadF32) return wide<__half, kLoadF32, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsStore && out == ELEM_F32)
             return norm ? wide<__half, kLoadNorm, kRowsStore, float>(a, s, PROF_GEMM_IN) : wide<__half, kLoadAsIs, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsSwiglu && out == ELEM_F16 && norm) return wide<__half, kLoadNorm, kRowsSwiglu, __half>(a, s, PROF_GEMM_FFN);
         if (epi == kRowsResidual) return deep<__half, true>(a, s);
+        if (epi == kRowsDeepStore) return deep<__half, false>(a, s);
         if (epi == kRowsArgmax)
             return norm ? wide<__half, kLoadNorm, kRowsArgmax, float>(a, s, PROF_LM_HEAD) : wide<__half, kLoadAsIs, kRowsArgmax, float>(a, s, PROF_LM_HEAD);
     }

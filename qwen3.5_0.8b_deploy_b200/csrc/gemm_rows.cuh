@@ -8,8 +8,12 @@ namespace b200 {
 constexpr int kRowsGemmMax = 32;        // rows a launch takes
 enum { kRowsStore = 0, kRowsSwiglu, kRowsGeglu, kRowsArgmax, kRowsResidual, kRowsDeepStore };    // the last two: deep K, fp32 Y
 
+// How X comes in: 16-bit rows; fp32 rows to normalise; fp32 rows to which normalised rows `add` are added first, the sums also going to x_out
+// (row m from CTA m); fp32 rows to round.
+enum { kLoadAsIs = 0, kLoadNorm, kLoadAddNorm, kLoadF32 };
+
 struct RowsGemm {
-    const void* x = nullptr;            // [M, K] 16-bit, or fp32 rows to normalise on the way in
+    const void* x = nullptr;            // [M, K]
     int ldx = 0;
     const int* row_index = nullptr;     // row m of X is x + row_index[m] * ldx
     const void* w = nullptr;            // [N, K]; gated: gate and up rows in alternating groups of `group` rows
@@ -25,10 +29,11 @@ struct RowsGemm {
     int group = 0;
     unsigned long long* packed = nullptr;   // argmax words of M rows (see gemm_tc_argmax)
     int* error = nullptr;
-    int tiles = 0, buffers = 0;  // filled in by the launcher
+    bool late = false;                  // let the next launch in only after this one's dependency wait
+    int tiles = 0;                      // most column tiles of a CTA: filled in by the launcher
 };
 
 bool gemm_rows_takes(const RowsGemm& a, int epi);
-int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, bool norm, ElemType out);
+int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int load, ElemType out);
 
 }  // namespace b200

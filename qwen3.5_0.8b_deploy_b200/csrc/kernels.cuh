@@ -115,12 +115,30 @@ struct DecodeOut {
 inline int rows_project(cudaStream_t s, const void* x, bool normed, float eps, const __half* w, float* y, int M, int N, int K, int* error) {
     RowsGemm a;
     a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.eps = eps; a.y = y; a.ldy = N; a.error = error;
-    return gemm_rows(s, a, ELEM_F16, kRowsStore, !normed, ELEM_F32);
+    return gemm_rows(s, a, ELEM_F16, kRowsStore, normed ? kLoadAsIs : kLoadNorm, ELEM_F32);
 }
 inline int rows_residual(cudaStream_t s, const __half* x, const __half* w, float* h, int M, int N, int K, int* error) {
     RowsGemm a;
     a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.y = h; a.ldy = N; a.error = error;
-    return gemm_rows(s, a, ELEM_F16, kRowsResidual, false, ELEM_F32);
+    return gemm_rows(s, a, ELEM_F16, kRowsResidual, kLoadAsIs, ELEM_F32);
+}
+// A layer of its own (no stack around it): fp32 rows in, y = beta y + X W^T with beta 0 or 1 out.  False when the few-row kernels do not take the call.
+// `late`: the attention kernel behind the input projection reads recurrent state before its dependency wait, and nothing but these projections
+// may lie between two calls of the layer, so that the projection has to be the one that waits.
+inline bool rows_layer_in(cudaStream_t s, const float* x, const __half* w, float* y, int M, int N, int K, int* error, int* status) {
+    RowsGemm a;
+    a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.y = y; a.ldy = N; a.error = error; a.late = true;
+    if (!g_flags.decode_gemm_rows || !gemm_rows_takes(a, kRowsStore)) return false;
+    *status = gemm_rows(s, a, ELEM_F16, kRowsStore, kLoadF32, ELEM_F32);
+    return true;
+}
+inline bool rows_layer_out(cudaStream_t s, const __half* x, const __half* w, float* y, float beta, int M, int N, int K, int* error, int* status) {
+    RowsGemm a;
+    a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.y = y; a.ldy = N; a.error = error;
+    const int epi = beta == 0.f ? kRowsDeepStore : kRowsResidual;
+    if (!g_flags.decode_gemm_rows || (beta != 0.f && beta != 1.f) || !gemm_rows_takes(a, epi)) return false;
+    *status = gemm_rows(s, a, ELEM_F16, epi, kLoadAsIs, ELEM_F32);
+    return true;
 }
 
 // ---- operator internals shared with the stack ------------------------------------------------------------------------

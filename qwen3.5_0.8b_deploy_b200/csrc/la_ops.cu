@@ -319,6 +319,9 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
             if (decode && dout)   // decode step of a stack: d_x is the un-normalised residual stream, its RMSNorm scale is applied in the epilogue
                 return gemm_tc_store(s, (const __half*)d_x, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, kLaProjCols, dout->rowsq,
                                      dout->eps, la->d_error);
+            int status = 0;
+            if (decode && !x_is_fp16 && rows_layer_in(s, (const float*)d_x, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, la->d_error, &status))
+                return status;
             const void* xb = d_x;
             if (!x_is_fp16) { B2_TRY(f32_to_f16(s, (const float*)d_x, la->d_xb, (size_t)rows * kHidden)); xb = la->d_xb; }
             return gemm_xwT(s, xb, true, la->d_win_fp16, true, la->d_mixed, false, rows, kLaProjCols, kHidden);
@@ -331,6 +334,9 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
         if (decode && dout)   // residual stream += gated W_out^T, with the fp16 copy and the sums of squares for the next projection
             return gemm_tc_residual(s, (const __half*)la->d_gated, la->d_wout_fp16, d_y, dout->xh, dout->rowsq, rows, kHidden, kLaHeads * kLaVd,
                                     la->d_error);
+        int status = 0;
+        if (fp16 && decode && !x_is_fp16 && rows_layer_out(s, (const __half*)la->d_gated, la->d_wout_fp16, d_y, y_beta, rows, kHidden, kLaHeads * kLaVd, la->d_error, &status))
+            return status;
         if (fp16) return gemm_xwT(s, la->d_gated, true, la->d_wout_fp16, true, d_y, false, rows, kHidden, kLaHeads * kLaVd, y_beta);
         return gemm_xwT(s, la->d_gated, false, la->d_wout_f32, false, d_y, false, rows, kHidden, kLaHeads * kLaVd, y_beta);
     };

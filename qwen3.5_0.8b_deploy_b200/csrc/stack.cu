@@ -532,7 +532,7 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
             g.eps = st->cfg.rms_eps;
             g.y = st->d_act; g.ldy = inter;
             g.error = st->d_error;
-            B2_TRY(gemm_rows(s, g, ELEM_F16, kRowsSwiglu, true, ELEM_F16));
+            B2_TRY(gemm_rows(s, g, ELEM_F16, kRowsSwiglu, kLoadNorm, ELEM_F16));
             B2_TRY(rows_residual(s, st->d_act, st->d_wdown[i], st->d_h, rows, kHidden, inter, st->d_error));
         }
         return 0;
@@ -595,7 +595,7 @@ static int stack_head(b200attn_stack st, int n_seqs, const int* d_row_index, int
     if (few) {
         RowsGemm a = head_product(st, n_seqs, d_row_index, norm_on_load);
         a.packed = st->d_packed;
-        B2_TRY(gemm_rows(s, a, ELEM_F16, kRowsArgmax, norm_on_load, ELEM_F32));
+        B2_TRY(gemm_rows(s, a, ELEM_F16, kRowsArgmax, norm_on_load ? kLoadNorm : kLoadAsIs, ELEM_F32));
         return launch_argmax_unpack(st->d_packed, n_seqs, d_next, s);
     }
     // LM head with the argmax in the GEMM epilogue (the logits never reach memory): 103 us per step against 112 + 31 us for
@@ -636,7 +636,7 @@ static int stack_logits(b200attn_stack st, int n, const int* d_row_index, float*
         RowsGemm a = head_product(st, n, d_row_index, true);
         a.y = d_logits;
         a.ldy = st->cfg.vocab_size;
-        return gemm_rows(s, a, ELEM_F16, kRowsStore, true, ELEM_F32);
+        return gemm_rows(s, a, ELEM_F16, kRowsStore, kLoadNorm, ELEM_F32);
     }
     launch_pdl(rmsnorm_kernel, dim3(n), dim3(256), 0, s, st->d_h, d_row_index, st->d_final_norm, st->cfg.rms_eps, n, st->d_xb, nullptr);
     B2_LAUNCH_CHECK();

@@ -123,3 +123,32 @@ def test_block_rows_of_a_batch(cuda, models, wts, design, rows):
         _, residual, limit = c.expect(tokens[k])
         off = np.sqrt(np.mean(((got[k] - residual[20:]) / c.residual_unit(residual)) ** 2, axis=-1))
         assert (off <= limit[1][20:]).all(), f"row {k}: {off / limit[1][20:]} of the limits"
+
+
+# ---- layers of their own -------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("rows", [1, 8, 9, 17, 32, 33])
+@pytest.mark.parametrize("kind", ["fa16", "fa8", "la"])
+def test_layer_decode_against_library_gemms(ops, cuda, synth, monkeypatch, kind, rows):
+    """Decode steps of one layer back to back, nothing between the calls; fp32 activations, fp16 projections."""
+    torch = cuda
+    w = synth.la_weights(95) if kind == "la" else synth.fa_weights(95)
+    xs = torch.from_numpy(np.stack([synth.hidden_states(95, f"step{d}", rows) for d in range(6)])).cuda()
+    slots = torch.arange(rows, dtype=torch.int32, device="cuda")
+
+    def run():
+        op = (ops.LinearAttention if kind == "la" else ops.FullAttention)(ops.PROJ_FP16, max_batch=rows, max_prefill_rows=64)
+        op.set_weights(w)
+        if kind == "la":
+            cache = ops.LinearAttnState(1, rows)
+        else:
+            cache = ops.KVCache(1, rows, 16, ops.KV_FP16 if kind == "fa16" else ops.KV_INT8)
+            for _ in range(rows):
+                cache.allocate_sequence(16)
+        return torch.stack([op.forward(x, cache, 0, slots) for x in xs])
+
+    monkeypatch.setenv("B200ATTN_DECODE_GEMM", "cublas")
+    want = run()
+    monkeypatch.delenv("B200ATTN_DECODE_GEMM")
+    got = run()
+    # one layer: three rounded vectors on the way, sqrt(3) * 2^-10 where every rounding differs by a unit
+    assert (got - want).norm() <= 2e-3 * want.norm()
