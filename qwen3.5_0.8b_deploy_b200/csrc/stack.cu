@@ -119,8 +119,12 @@ rmsnorm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
 }
 
 // act = silu(gate) * up.  gu rows hold tiles of 64 columns: 32 gate columns followed by the 32 matching up columns
-// (the layout the decode-step GEMM epilogue consumes as well).  fp16.
-__global__ void swiglu_kernel(const __half* __restrict__ gu, int inter, size_t n_oct, __half* __restrict__ act) {
+// (the layout the decode-step GEMM epilogue consumes as well).  fp16.  The fast exponential and division: with expf and the exact quotient the
+// kernel was bound by issue slots, 284 us for 65536 rows of 3584 (1.4 GB, 212 us at the memory rate), now 218 us; their error, 2^-18 at
+// |gate| = 20, is far below the rounding of the result to 11 bits.
+__global__ void __launch_bounds__(256)
+swiglu_kernel(const __half* __restrict__ gu, int inter, size_t n_oct, __half* __restrict__ act) {
+    pdl_enter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // index over (row, inter/8): eight outputs per thread
     if (i >= n_oct) return;
     const size_t per_row = inter / 8;
@@ -134,7 +138,7 @@ __global__ void swiglu_kernel(const __half* __restrict__ gu, int inter, size_t n
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float2 g = __half22float2(gp[e]), u = __half22float2(up[e]);
-        o[e] = __floats2half2_rn(g.x / (1.0f + expf(-g.x)) * u.x, g.y / (1.0f + expf(-g.y)) * u.y);
+        o[e] = __floats2half2_rn(__fdividef(g.x, 1.0f + __expf(-g.x)) * u.x, __fdividef(g.y, 1.0f + __expf(-g.y)) * u.y);
     }
     *reinterpret_cast<uint4*>(act + row * inter + c) = *reinterpret_cast<uint4*>(o);
 }
@@ -557,7 +561,7 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
         B2_LAUNCH_CHECK();
         B2_TRY(gemm_xwT(s, st->d_xb, true, st->d_wgu[i], true, st->d_gu, true, rows, 2 * inter, kHidden));
         const size_t octs = (size_t)rows * inter / 8;
-        swiglu_kernel<<<(unsigned)((octs + 255) / 256), 256, 0, s>>>(st->d_gu, inter, octs, st->d_act);
+        launch_pdl(swiglu_kernel, dim3((unsigned)((octs + 255) / 256)), dim3(256), 0, s, st->d_gu, inter, octs, st->d_act);
         B2_LAUNCH_CHECK();
         B2_TRY(gemm_xwT(s, st->d_act, true, st->d_wdown[i], true, st->d_h, false, rows, kHidden, inter, 1.0f));
     }
