@@ -23,7 +23,7 @@ size_t la_scratch_bytes(const b200attn_la_config& c) {
     n += align_up(R * kLaHeads * kLaVd * 4, 256);       // core
     n += align_up(R * kHidden * 2, 256);                // xb
     n += align_up(R * kLaHeads * kLaVd * 4, 256);       // gated
-    n += align_up((2 * R + 65536) * 4, 256);            // meta
+    n += align_up((4 * R + 65536) * 4, 256);            // meta
     return n;
 }
 
