@@ -268,8 +268,7 @@ int fa_forward_rows(b200attn_fa fa, b200attn_kv_pool pool, int layer, const int*
 
     B2_TRY(fa_project_in(fa, d_x, x_is_fp16, rows, !kv.is_fp16, false, nullptr, pool->d_error, s));
     B2_TRY(launch_fa_q_epilogue(fa->d_qkv_raw, rows, fa->d_qnorm, fa->d_inv_freq, d_row_pos, fa->d_q, fa->d_gate, s));
-    for (int i = 0; i < n_seqs; ++i)
-        B2_TRY(launch_kv_stage_gather(kv, layer, h_slots[i], base[i], ctx0[i], fa->d_kstage, fa->d_vstage, s));
+    B2_TRY(launch_kv_stage_gather(kv, layer, d_slots, d_ctx0, n_seqs, *std::max_element(base.begin(), base.end()), fa->d_kstage, fa->d_vstage, s));
     {
         ProfScope prof(PROF_KV_APPEND, s);
         B2_TRY(launch_kv_append(kv, layer, d_atiles, (int)atiles.size(), d_slots, k_in, kFaQkvCols, v_in, kFaQkvCols, true,

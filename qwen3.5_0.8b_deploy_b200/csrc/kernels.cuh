@@ -24,7 +24,7 @@ int launch_fa_decode_pre(const KvView& kv, int layer, const int* d_slots, int n_
 int launch_kv_advance(const KvView& kv, int layer, const int* d_slots, const int* d_counts, int n_seqs, cudaStream_t s);
 int launch_fa_q_epilogue(const float* qkv_raw, int rows, const float* q_norm_w, const float* inv_freq,
                          const int* d_row_pos, __half* q_out, __half* gate_out, cudaStream_t s);
-int launch_kv_stage_gather(const KvView& kv, int layer, int slot, int base, int stage_row0, __half* kstage,
+int launch_kv_stage_gather(const KvView& kv, int layer, const int* d_slots, const int* d_stage_row0, int n_seqs, int longest, __half* kstage,
                            __half* vstage, cudaStream_t s);
 void build_append_tiles(const std::vector<int>& base, const int* h_counts, int n_seqs, std::vector<AppendTile>& tiles);
 int pool_prepare_append(b200attn_kv_pool p, int layer, const int* h_slots, const int* h_counts, int n_seqs,

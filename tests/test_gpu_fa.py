@@ -280,3 +280,33 @@ def test_errors(ops, cuda, synth):
         fa.forward_batch_prefill(torch.zeros((100, 1024), device="cuda"), kv, 0, [s], [100])   # > max_prefill_rows
     with pytest.raises(ops.InvalidArgument):
         fa.forward(torch.zeros((3, 1024), device="cuda"), kv, 0, torch.zeros(3, dtype=torch.int32, device="cuda"))
+
+
+@pytest.mark.parametrize("kv_dtype", [0, 1])
+def test_prefill_continues_ragged_caches(ops, cuda, synth, kv_dtype):
+    """Second prompts behind caches whose lengths lie around a group of 16 tokens and a page, one of them empty, against one prompt of both parts."""
+    torch = cuda
+    w = synth.fa_weights(97)
+    first, second = [1, 15, 16, 17, 64, 65, 130, 0], [3, 1, 20, 2, 64, 1, 7, 9]
+    n, rows = len(first), sum(first) + sum(second)
+    xs = [synth.hidden_states(97, f"cont{i}", a + b) for i, (a, b) in enumerate(zip(first, second))]
+
+    def run(parts):
+        fa = ops.FullAttention(ops.PROJ_FP32, max_batch=n, max_prefill_rows=rows)
+        fa.set_weights(w)
+        kv = ops.KVCache(1, n, 256, kv_dtype)
+        slots = [kv.allocate_sequence(200) for _ in range(n)][::-1]
+        out = []
+        for lo, hi in parts:
+            x = np.concatenate([x[a:b] for x, a, b in zip(xs, lo, hi)])
+            out.append(fa.forward_batch_prefill(torch.from_numpy(x).cuda(), kv, 0, slots, [b - a for a, b in zip(lo, hi)]).cpu().numpy())
+        return out
+    total = [a + b for a, b in zip(first, second)]
+    whole = run([([0] * n, total)])[0]
+    head, tail = run([([0] * n, first), (first, total)])
+    at = [0, 0, 0]
+    for a, b in zip(first, second):
+        got = np.concatenate([head[at[0]:at[0] + a], tail[at[1]:at[1] + b]])
+        ok, msg = allclose_report(got, whole[at[2]:at[2] + a + b], ATOL, RTOL)
+        assert ok, f"{a} + {b} tokens: {msg}"
+        at = [at[0] + a, at[1] + b, at[2] + a + b]
