@@ -62,10 +62,12 @@ __device__ __forceinline__ int find_seq(const int* s_pref, int n_seqs, int x) { 
 }
 
 // grid (number of SMs).  max_parts = partial slots per (sequence, kv head) in part_o / part_ml (>= 3).
-template <bool kFp16, typename OutT>
+// QT: queries as fp16, or as fp32 that the load rounds (a conversion launch in front of the kernel took 4 of the 58 us of a call at
+// 128 sequences).
+template <bool kFp16, typename OutT, typename QT>
 __global__ void __launch_bounds__(DecodeCfg<kFp16>::kThreads, 1)
 fa_decode_split_kernel(KvView kv, int layer, const int* __restrict__ slots, int n_seqs,
-                       const __half* __restrict__ q, const __half* __restrict__ gate, int max_parts,
+                       const QT* __restrict__ q, const __half* __restrict__ gate, int max_parts,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters,
                        OutT* __restrict__ out, unsigned long long* stamp) {
     using Cfg = DecodeCfg<kFp16>;
@@ -206,11 +208,17 @@ fa_decode_split_kernel(KvView kv, int layer, const int* __restrict__ slots, int 
         // Q^T B-fragments: k-step ks = 4*blk + s covers dims 64*blk + 16*t + 4*s + {0,1 | 2,3}; head = g (< 4).
         uint32_t qf[16][2];
         {
-            const __half* qrow = q + ((size_t)seq * kFaHeads + kvh * 4 + (g & 3)) * kHeadDim;
+            const QT* qrow = q + ((size_t)seq * kFaHeads + kvh * 4 + (g & 3)) * kHeadDim;
 #pragma unroll
             for (int ks = 0; ks < 16; ++ks) {
                 const int p0 = 64 * (ks >> 2) + 16 * t + 4 * (ks & 3);
-                const uint2 v = *reinterpret_cast<const uint2*>(qrow + p0);
+                uint2 v;
+                if constexpr (sizeof(QT) == 2) {
+                    v = *reinterpret_cast<const uint2*>(qrow + p0);
+                } else {
+                    const float4 f = *reinterpret_cast<const float4*>(qrow + p0);
+                    v = make_uint2(pack_half2(f.x, f.y), pack_half2(f.z, f.w));
+                }
                 qf[ks][0] = (g < 4) ? v.x : 0u;
                 qf[ks][1] = (g < 4) ? v.y : 0u;
             }
@@ -494,7 +502,7 @@ fa_decode_split_kernel(KvView kv, int layer, const int* __restrict__ slots, int 
 }
 
 // max_splits = partial slots per (sequence, kv head) pair in part_o / part_ml (kFaDecodeParts in the callers' scratch).
-int launch_fa_decode(const KvView& kv, int layer, const int* d_slots, int n_seqs, const __half* q,
+int launch_fa_decode(const KvView& kv, int layer, const int* d_slots, int n_seqs, const void* q, bool q_fp32,
                      const __half* gate, int max_splits, float* part_o, float* part_ml, int* counters,
                      void* out, bool out_fp16, cudaStream_t s) {
     B2_CHECK_ARG(n_seqs > 0 && n_seqs <= kDecodeMaxSeqs, "decode attention: %d sequences outside (0, %d]", n_seqs, kDecodeMaxSeqs);
@@ -503,17 +511,19 @@ int launch_fa_decode(const KvView& kv, int layer, const int* d_slots, int n_seqs
     B2_TRY(device_sm_count(&n_sm));
     static PerDeviceOnce once;
     B2_PER_DEVICE_ONCE(once,
-        B2_CUDA(cudaFuncSetAttribute(fa_decode_split_kernel<true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeCfg<true>::kSmemBytes));
-        B2_CUDA(cudaFuncSetAttribute(fa_decode_split_kernel<true, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeCfg<true>::kSmemBytes));
-        B2_CUDA(cudaFuncSetAttribute(fa_decode_split_kernel<false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeCfg<false>::kSmemBytes));
-        B2_CUDA(cudaFuncSetAttribute(fa_decode_split_kernel<false, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeCfg<false>::kSmemBytes)));
+#define FA_DEC_SMEM(F16, T, Q) B2_CUDA(cudaFuncSetAttribute(fa_decode_split_kernel<F16, T, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeCfg<F16>::kSmemBytes))
+        FA_DEC_SMEM(true, float, __half); FA_DEC_SMEM(true, __half, __half); FA_DEC_SMEM(false, float, __half); FA_DEC_SMEM(false, __half, __half);
+        FA_DEC_SMEM(true, float, float); FA_DEC_SMEM(false, float, float));
+#undef FA_DEC_SMEM
     dim3 grid(n_sm);
     unsigned long long* stamp = prof_stamp_slot(PROF_FA_DECODE);
-#define FA_DEC_LAUNCH(F16, T)                                                                                          \
-    launch_pdl(fa_decode_split_kernel<F16, T>, grid, dim3(DecodeCfg<F16>::kThreads), DecodeCfg<F16>::kSmemBytes, s,    \
-               kv, layer, d_slots, n_seqs, q, gate, max_splits, part_o, part_ml, counters, (T*)out, stamp)
-    if (kv.is_fp16) { if (out_fp16) FA_DEC_LAUNCH(true, __half); else FA_DEC_LAUNCH(true, float); }
-    else            { if (out_fp16) FA_DEC_LAUNCH(false, __half); else FA_DEC_LAUNCH(false, float); }
+#define FA_DEC_LAUNCH(F16, T, Q)                                                                                          \
+    launch_pdl(fa_decode_split_kernel<F16, T, Q>, grid, dim3(DecodeCfg<F16>::kThreads), DecodeCfg<F16>::kSmemBytes, s,    \
+               kv, layer, d_slots, n_seqs, (const Q*)q, gate, max_splits, part_o, part_ml, counters, (T*)out, stamp)
+    B2_CHECK_ARG(!q_fp32 || !out_fp16, "decode attention: fp32 queries give fp32 outputs");
+    if (q_fp32)          { if (kv.is_fp16) FA_DEC_LAUNCH(true, float, float); else FA_DEC_LAUNCH(false, float, float); }
+    else if (kv.is_fp16) { if (out_fp16) FA_DEC_LAUNCH(true, __half, __half); else FA_DEC_LAUNCH(true, float, __half); }
+    else                 { if (out_fp16) FA_DEC_LAUNCH(false, __half, __half); else FA_DEC_LAUNCH(false, float, __half); }
 #undef FA_DEC_LAUNCH
     B2_LAUNCH_CHECK();
     return 0;

@@ -78,5 +78,5 @@ extern "C" int b200attn_fa_decode_core_static(b200attn_kv_pool pool, int layer, 
     cudaStream_t s = as_stream(stream);
     B2_CUDA(cudaMemsetAsync(counters, 0, kStaticCounterBytes, s));
     B2_TRY(f32_to_f16(s, d_q, q16, (size_t)n_seqs * kFaHeads * kHeadDim));
-    return launch_fa_decode(kv, layer, d_slots, n_seqs, q16, nullptr, kStaticMaxSplits, part_o, part_ml, counters, d_out, false, s);
+    return launch_fa_decode(kv, layer, d_slots, n_seqs, q16, false, nullptr, kStaticMaxSplits, part_o, part_ml, counters, d_out, false, s);
 }

@@ -227,7 +227,7 @@ int fa_forward_rows(b200attn_fa fa, b200attn_kv_pool pool, int layer, const int*
         // kernel then sees the new length already
         B2_TRY(launch_fa_decode_pre(kv, layer, d_slots_in, n_seqs, fa->d_qkv_raw, fa->d_qnorm, fa->d_knorm, fa->d_inv_freq, fa->d_q,
                                     fa->d_gate, s));
-        B2_TRY(launch_fa_decode(kv, layer, d_slots_in, n_seqs, fa->d_q, fa->d_gate, kMaxSplitsCap, fa->d_part_o,
+        B2_TRY(launch_fa_decode(kv, layer, d_slots_in, n_seqs, fa->d_q, false, fa->d_gate, kMaxSplitsCap, fa->d_part_o,
                                 fa->d_part_ml, fa->d_counters, fa->d_attn, fp16, s));
         B2_TRY(fa_project_out(fa, d_y, y_beta, n_seqs, !x_is_fp16, dout, pool->d_error, s));
         pool->lens_dirty = true;
@@ -304,8 +304,9 @@ extern "C" int b200attn_fa_decode_core(b200attn_fa fa, b200attn_kv_pool pool, in
     B2_CHECK_ARG(n_seqs > 0 && n_seqs <= fa->cfg.max_batch, "fa_decode_core: n_seqs %d outside (0, max_batch %d]", n_seqs, fa->cfg.max_batch);
     cudaStream_t s = as_stream(stream);
     const KvView kv = pool->view();
-    B2_TRY(f32_to_f16(s, d_q, fa->d_q, (size_t)n_seqs * kFaHeads * kHeadDim));
-    return launch_fa_decode(kv, layer, d_slots, n_seqs, fa->d_q, nullptr, kMaxSplitsCap, fa->d_part_o, fa->d_part_ml, fa->d_counters,
+    const bool aligned = (reinterpret_cast<uintptr_t>(d_q) & 15) == 0;      // the kernel reads four queries at a time
+    if (!aligned) B2_TRY(f32_to_f16(s, d_q, fa->d_q, (size_t)n_seqs * kFaHeads * kHeadDim));
+    return launch_fa_decode(kv, layer, d_slots, n_seqs, aligned ? (const void*)d_q : (const void*)fa->d_q, aligned, nullptr, kMaxSplitsCap, fa->d_part_o, fa->d_part_ml, fa->d_counters,
                             d_out, false, s);
 }
 

@@ -36,7 +36,7 @@ int kv_pool_create_latent(const std::vector<int>& row_pitch, ElemType elem, int 
 
 // ---- decode attention (fa_decode.cu) -----------------------------------------------------------------------
 constexpr int kFaDecodeParts = 16;      // partial slots per (sequence, kv head) pair the decode kernel may use; sizes part_o / part_ml
-int launch_fa_decode(const KvView& kv, int layer, const int* d_slots, int n_seqs, const __half* q,
+int launch_fa_decode(const KvView& kv, int layer, const int* d_slots, int n_seqs, const void* q, bool q_fp32,
                      const __half* gate, int max_splits, float* part_o, float* part_ml, int* counters,
                      void* out, bool out_fp16, cudaStream_t s);
 
