@@ -70,9 +70,19 @@ struct LaRun {  // up to kConvRun consecutive rows of one sequence
 int launch_la_conv_seq(const float* mixed, const LaRun* d_runs, int n_runs, const LaSeqMeta* d_seqs, const float* conv_layer,
                        size_t conv_stride, const float* conv_w, const float* a_log, const float* dt_bias,
                        float* q, float* k, __half* qh, __half* kh, float* v, __half* vh, float* g, float* beta, cudaStream_t s);
+// The chunked recurrence in two kernels (la_chunk.cu), for batches of few sequences: chunk_list entries {row = chunk, seq} in the order of the
+// sequences, each sequence's first entry, and scratch of la_split_bytes(n_chunks).
+struct LaSplit {
+    int n_chunks = 0;                    // 0: one kernel
+    const LaRun* d_chunks = nullptr;
+    const int* d_first = nullptr;
+    void* scratch = nullptr;
+};
+constexpr size_t kLaSplitBytes = 90112;  // of a chunk and head
+inline size_t la_split_bytes(int n_chunks) { return (size_t)n_chunks * kLaHeads * (kLaSplitBytes + 4); }
 int launch_la_chunk_tc(const __half* q_h, const __half* k_h, const __half* v_h, const float* g, const float* beta,
                        const LaSeqMeta* d_seqs, int n_seqs, int rows, float* rec_layer, size_t rec_stride, float* out,
-                       int* d_error, cudaStream_t s);
+                       int* d_error, const LaSplit& split, cudaStream_t s);
 int launch_la_conv_state_update(const float* mixed, const LaSeqMeta* d_seqs, int n_seqs, float* conv_layer,
                                 size_t conv_stride, cudaStream_t s);
 int launch_la_recurrent_serial(const float* q, const float* k, const float* v, const float* g, const float* beta,

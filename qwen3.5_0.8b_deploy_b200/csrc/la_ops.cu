@@ -13,11 +13,20 @@ namespace b200 {
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// The recurrence in two kernels (la_chunk.cu): most sequences of a batch, and fewest chunks of its longest one.  One kernel / two at 1 x 200 tokens
+// 36.5 / 28.9 us, 1 x 1000 114.5 / 56.5, 3 x 333 49.5 / 36.1, 4 x 193 35.3 / 32.3, 4 x 500 62.3 / 54.0; 8 x 500 63 / 74, and two chunks 20 against
+// 22 us (estimated from 14 us for an own part, 2.6 us a chunk of the walk).
+constexpr int kLaSplitSeqs = 4, kLaSplitChunks = 4;
+// R rows in S sequences are at most R / 64 + S chunks, of 22.5 KB per row; q, k and v hold 24 KB per row.
+constexpr size_t kLaSplitRoom = kLaSplitSeqs * (size_t)kLaHeads * (kLaSplitBytes + 4);
+static_assert(kLaHeads * (kLaSplitBytes + 4) <= 64 * 3 * kLaHeads * kLaKd * 4, "a full chunk's images fit its rows of q, k and v");
+
 size_t la_scratch_bytes(const b200attn_la_config& c) {
     const size_t R = (size_t)std::max(c.max_batch, c.max_prefill_rows);
     size_t n = 0;
     n += align_up(R * kLaProjCols * 4, 256);            // mixed
-    n += 3 * align_up(R * kLaHeads * kLaKd * 4, 256);   // q, k, v
+    n += 3 * align_up(R * kLaHeads * kLaKd * 4, 256);   // q, k, v; in their place the images of the two-kernel recurrence
+    n += align_up(kLaSplitRoom, 256);                   // ... and room for the last, partly filled chunk of each of its sequences
     n += 3 * align_up(R * kLaHeads * kLaKd * 2, 256);   // q, k, v as fp16
     n += 2 * align_up(R * kLaHeads * 4, 256);           // g, beta
     n += align_up(R * kLaHeads * kLaVd * 4, 256);       // core
@@ -37,6 +46,7 @@ void la_carve_scratch(b200attn_la la) {
     la->d_q = (float*)take(R * kLaHeads * kLaKd * 4);
     la->d_k = (float*)take(R * kLaHeads * kLaKd * 4);
     la->d_v = (float*)take(R * kLaHeads * kLaKd * 4);
+    take(kLaSplitRoom);
     la->d_qh = (__half*)take(R * kLaHeads * kLaKd * 2);
     la->d_kh = (__half*)take(R * kLaHeads * kLaKd * 2);
     la->d_vh = (__half*)take(R * kLaHeads * kLaVd * 2);
@@ -261,7 +271,7 @@ static bool la_use_tensor_cores() { return !g_flags.la_prefill_serial; }
 
 static int la_build_meta(b200attn_la la, b200attn_la_state st, const int* h_slots, const int* h_counts, int n_seqs,
                          int* rows_out, std::vector<LaSeqMeta>& seqs, LaSeqMeta** d_seqs, LaRun** d_runs, int* n_runs,
-                         cudaStream_t s) {
+                         LaSplit* split, cudaStream_t s) {
     B2_CHECK_ARG(h_slots && h_counts && n_seqs > 0, "linear attention: bad batch description");
     seqs.resize(n_seqs);
     int rows = 0;
@@ -278,7 +288,18 @@ static int la_build_meta(b200attn_la la, b200attn_la_state st, const int* h_slot
     if (d_runs)
         for (int i = 0; i < n_seqs; ++i)
             for (int j = 0; j < h_counts[i]; j += kConvRun) runs.push_back(LaRun{seqs[i].row0 + j, i});
-    const int need = 3 * n_seqs + 1 + 2 * (int)runs.size();
+    // Few sequences: the chunks' own parts as a launch of their own, handing over through the working buffers of the serial form, which the
+    // tensor-core form does not use.
+    std::vector<LaRun> chunks;
+    std::vector<int> first(n_seqs);
+    if (split && n_seqs <= kLaSplitSeqs && *std::max_element(h_counts, h_counts + n_seqs) > 64 * (kLaSplitChunks - 1)) {
+        for (int i = 0; i < n_seqs; ++i) {
+            first[i] = (int)chunks.size();
+            for (int c = 0; 64 * c < h_counts[i]; ++c) chunks.push_back(LaRun{c, i});
+        }
+    }
+    const int split_ints = chunks.empty() ? 0 : 2 * (int)chunks.size() + n_seqs;
+    const int need = 3 * n_seqs + 1 + 2 * (int)runs.size() + split_ints;
     B2_CHECK_ARG(need <= la->meta_cap, "linear attention: metadata exceeds scratch");
     *d_seqs = reinterpret_cast<LaSeqMeta*>(la->d_meta);
     B2_CUDA(cudaMemcpyAsync(*d_seqs, seqs.data(), (size_t)n_seqs * sizeof(LaSeqMeta), cudaMemcpyHostToDevice, s));
@@ -287,18 +308,25 @@ static int la_build_meta(b200attn_la la, b200attn_la_state st, const int* h_slot
         *n_runs = (int)runs.size();
         if (!runs.empty()) B2_CUDA(cudaMemcpyAsync(*d_runs, runs.data(), runs.size() * sizeof(LaRun), cudaMemcpyHostToDevice, s));
     }
+    if (!chunks.empty()) {
+        LaRun* d_chunks = reinterpret_cast<LaRun*>(la->d_meta + 3 * n_seqs + (n_seqs & 1)) + runs.size();
+        int* d_first = reinterpret_cast<int*>(d_chunks + chunks.size());
+        B2_CUDA(cudaMemcpyAsync(d_chunks, chunks.data(), chunks.size() * sizeof(LaRun), cudaMemcpyHostToDevice, s));
+        B2_CUDA(cudaMemcpyAsync(d_first, first.data(), (size_t)n_seqs * 4, cudaMemcpyHostToDevice, s));
+        *split = LaSplit{(int)chunks.size(), d_chunks, d_first, la->d_q};
+    }
     return 0;
 }
 
 // Runs the delta-rule recurrence over the batch.  tensor_cores: q, k and v must already be in la->d_qh / d_kh / d_vh.
 static int la_recurrence(b200attn_la la, b200attn_la_state st, int layer, const float* q, const float* k, const float* v,
                          const float* g, const float* beta, const LaSeqMeta* d_seqs, int n_seqs, int rows, float* out,
-                         bool tensor_cores, cudaStream_t s) {
+                         bool tensor_cores, const LaSplit& split, cudaStream_t s) {
     float* rec_layer = st->d_recurrent + (size_t)layer * st->cfg.max_seqs * st->rec_stride_slot();
     ProfScope prof(PROF_LA_PREFILL, s);
     if (tensor_cores)
         return launch_la_chunk_tc(la->d_qh, la->d_kh, la->d_vh, g, beta, d_seqs, n_seqs, rows, rec_layer, st->rec_stride_slot(), out,
-                                  la->d_error, s);
+                                  la->d_error, split, s);
     return launch_la_recurrent_serial(q, k, v, g, beta, d_seqs, n_seqs, rec_layer, st->rec_stride_slot(), out, s);
 }
 
@@ -354,15 +382,16 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
     LaSeqMeta* d_seqs = nullptr;
     LaRun* d_runs = nullptr;
     int n_runs = 0;
-    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, &d_runs, &n_runs, s));
+    LaSplit split;
+    const bool tc = la_use_tensor_cores();
+    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, &d_runs, &n_runs, tc ? &split : nullptr, s));
     if (rows == 0) return 0;
     B2_CHECK_ARG(rows <= la->cfg.max_prefill_rows, "la_prefill: %d rows exceed max_prefill_rows %d", rows, la->cfg.max_prefill_rows);
-    const bool tc = la_use_tensor_cores();
     B2_TRY(project_in(rows));
     B2_TRY(launch_la_conv_seq(la->d_mixed, d_runs, n_runs, d_seqs, conv_layer, st->conv_stride_slot(), la->d_conv_w, la->d_a_log,
                               la->d_dt_bias, tc ? nullptr : la->d_q, tc ? nullptr : la->d_k, tc ? la->d_qh : nullptr,
                               tc ? la->d_kh : nullptr, tc ? nullptr : la->d_v, tc ? la->d_vh : nullptr, la->d_g, la->d_beta, s));
-    B2_TRY(la_recurrence(la, st, layer, la->d_q, la->d_k, la->d_v, la->d_g, la->d_beta, d_seqs, n_seqs, rows, la->d_core, tc, s));
+    B2_TRY(la_recurrence(la, st, layer, la->d_q, la->d_k, la->d_v, la->d_g, la->d_beta, d_seqs, n_seqs, rows, la->d_core, tc, split, s));
     B2_TRY(launch_la_conv_state_update(la->d_mixed, d_seqs, n_seqs, conv_layer, st->conv_stride_slot(), s));
     B2_TRY(launch_la_gated_norm(la->d_core, la->d_mixed, la->d_norm, rows, la->d_gated, fp16, s));
     return project_out(rows);
@@ -390,7 +419,8 @@ extern "C" int b200attn_la_prefill_core(b200attn_la la, b200attn_la_state st, in
     int rows = 0;
     std::vector<LaSeqMeta> seqs;
     LaSeqMeta* d_seqs = nullptr;
-    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, nullptr, nullptr, s));
+    LaSplit split;
+    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, nullptr, nullptr, use_tensor_cores ? &split : nullptr, s));
     if (rows == 0) return 0;
     if (use_tensor_cores) {
         B2_TRY(f32_to_f16(s, d_q, la->d_qh, (size_t)rows * kLaHeads * kLaKd));
@@ -398,7 +428,7 @@ extern "C" int b200attn_la_prefill_core(b200attn_la la, b200attn_la_state st, in
         B2_TRY(f32_to_f16(s, d_v, la->d_vh, (size_t)rows * kLaHeads * kLaVd));
         B2_CUDA(cudaMemsetAsync(la->d_error, 0, 4, s));
     }
-    B2_TRY(la_recurrence(la, st, layer, d_q, d_k, d_v, d_g, d_beta, d_seqs, n_seqs, rows, d_out, use_tensor_cores != 0, s));
+    B2_TRY(la_recurrence(la, st, layer, d_q, d_k, d_v, d_g, d_beta, d_seqs, n_seqs, rows, d_out, use_tensor_cores != 0, split, s));
     if (use_tensor_cores) {
         int err = 0;
         B2_CUDA(cudaMemcpyAsync(&err, la->d_error, 4, cudaMemcpyDeviceToHost, s));

@@ -348,3 +348,28 @@ def test_prefill_runs_of_ragged_batches(ops, cuda, oracle, synth, counts):
         ok, msg = allclose_report(np.concatenate([first[at:at + c], then[at:at + c]]), want, ATOL, RTOL)
         assert ok, f"sequence {i} of {c} tokens: {msg}"
         at += c
+
+
+@pytest.mark.parametrize("counts", [[193], [300, 64], [65, 257, 129, 1], [0, 320, 191], [640, 200, 70, 193]])
+def test_two_kernel_recurrence_equals_one_kernel(ops, cuda, synth, counts):
+    """Batches of up to four sequences take the chunks' own parts in a kernel of their own; the same sequences among five take one kernel.  Same
+    products on the same roundings: bit-equal outputs and states."""
+    torch = cuda
+    n, rows = len(counts), sum(counts)
+    q = synth.normal(58, f"q{rows}", (rows, 16, 128)); q /= np.linalg.norm(q, axis=-1, keepdims=True) * np.sqrt(128)
+    k = synth.normal(58, f"k{rows}", (rows, 16, 128)); k /= np.linalg.norm(k, axis=-1, keepdims=True)
+    v = synth.normal(58, f"v{rows}", (rows, 16, 128), 0.5)
+    g = -np.exp(synth.rng(58, f"g{rows}").uniform(-6.0, 2.3, (rows, 16))).astype(np.float32)
+    beta = synth.rng(58, f"b{rows}").uniform(0.0, 1.0, (rows, 16)).astype(np.float32)
+    args = [torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda() for a in (q, k, v, g, beta)]
+    got = []
+    for extra in (0, 5 - n):
+        la = ops.LinearAttention(ops.PROJ_FP32, max_batch=5, max_prefill_rows=rows)
+        st = ops.LinearAttnState(1, 5)
+        for i in range(n):
+            st.import_state(0, i, torch.from_numpy(synth.normal(58, f"s{i}", (16, 128, 128), 0.05)).cuda(), None)
+        out = la.prefill_core(*args, st, 0, list(range(n + extra)), list(counts) + [0] * extra, use_tensor_cores=True).cpu().numpy()
+        got.append((out, [st.export_state(0, i)[0].cpu().numpy() for i in range(n)]))
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1], got[1][1]):
+        np.testing.assert_array_equal(a, b)
