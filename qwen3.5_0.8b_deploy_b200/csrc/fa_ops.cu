@@ -172,9 +172,13 @@ static int fa_project_in(b200attn_fa fa, const void* d_x, bool x_is_fp16, int ro
         const void* xb = d_x;
         const bool compensate = kv_int8 && !x_is_fp16;      // fp32 activations at hand and a quantising cache behind K / V
         int status = 0;
-        if (decode && !x_is_fp16 && !compensate &&
-            rows_layer_in(s, (const float*)d_x, fa->d_wqkv_fp16, fa->d_qkv_raw, rows, kFaQkvCols, kHidden, d_error, &status))
-            return status;
+        if (decode && !x_is_fp16 &&
+            rows_layer_in(s, (const float*)d_x, fa->d_wqkv_fp16, fa->d_qkv_raw, rows, kFaQkvCols, kHidden, d_error, &status)) {
+            const int q_cols = kFaHeads * kHeadDim * 2;
+            if (status != 0 || !compensate) return status;
+            return rows_layer_compensate(s, (const float*)d_x, fa->d_wqkv_fp16 + (size_t)q_cols * kHidden, fa->d_wkv_lo, fa->d_qkv_raw + q_cols, kFaQkvCols, rows,
+                                         2 * kFaKvHeads * kHeadDim, kHidden, d_error);
+        }
         if (!x_is_fp16) {
             if (compensate) B2_TRY(f32_split_f16(s, (const float*)d_x, fa->d_xb, fa->d_xlo, (size_t)rows * kHidden));
             else B2_TRY(f32_to_f16(s, (const float*)d_x, fa->d_xb, (size_t)rows * kHidden));

@@ -122,7 +122,7 @@ __device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, 
                 v[i] = k < a.K ? __ldcg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             float rs = 1.0f;
-            if constexpr (LOAD != kLoadF32) {
+            if constexpr (LOAD < kLoadF32) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
 #pragma unroll
@@ -134,11 +134,14 @@ __device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, 
                 const int k = 4 * (32 * i + lane);
                 if (k < a.K) {
                     float4 w = make_float4(rs, rs, rs, rs);
-                    if (LOAD != kLoadF32 && a.norm_w) {
+                    if (LOAD < kLoadF32 && a.norm_w) {
                         const float4 f = __ldg(reinterpret_cast<const float4*>(a.norm_w + k));
                         w = make_float4(rs * (a.norm_base + f.x), rs * (a.norm_base + f.y), rs * (a.norm_base + f.z), rs * (a.norm_base + f.w));
                     }
                     float4 n = make_float4(v[i].x * w.x, v[i].y * w.y, v[i].z * w.z, v[i].w * w.w);
+                    if constexpr (LOAD == kLoadF32Lo)
+                        n = make_float4((n.x - __half2float(__float2half_rn(n.x))) * kLoScale, (n.y - __half2float(__float2half_rn(n.y))) * kLoScale,
+                                        (n.z - __half2float(__float2half_rn(n.z))) * kLoScale, (n.w - __half2float(__float2half_rn(n.w))) * kLoScale);
                     if constexpr (LOAD == kLoadAddNorm) {
                         const float4 h = __ldcg(reinterpret_cast<const float4*>(xr + k));
                         n = make_float4(h.x + n.x, h.y + n.y, h.z + n.z, h.w + n.w);
@@ -245,6 +248,9 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
             } else {
                 float v = sl.total(tile_at(u), pitch, em, n8) * a.scale;
                 if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
+                if constexpr (EPI == kRowsStore && std::is_same_v<YT, float>) {
+                    if (a.accumulate) v += __ldcg(static_cast<const float*>(a.y) + (size_t)em * a.ldy + n);
+                }
                 if constexpr (EPI == kRowsStore) static_cast<YT*>(a.y)[(size_t)em * a.ldy + n] = to_out<YT>(v);
                 else if (v > -INFINITY) best = max(best, pack_max(v, n));
             }
@@ -500,7 +506,7 @@ int wide(const RowsGemm& a, cudaStream_t s, ProfKind kind) {
     if constexpr ((EPI == kRowsStore && std::is_same_v<YT, float>) || EPI == kRowsArgmax) {
         int sms = 0;
         B2_TRY(device_sm_count(&sms));
-        if (a.N > 64 * sms) return a.M <= 16 ? launch_stream<T, 1, LOAD, EPI>(a, sms, s, kind) : launch_stream<T, 2, LOAD, EPI>(a, sms, s, kind);
+        if (a.N > 64 * sms && !a.accumulate) return a.M <= 16 ? launch_stream<T, 1, LOAD, EPI>(a, sms, s, kind) : launch_stream<T, 2, LOAD, EPI>(a, sms, s, kind);
     }
     return a.M <= 16 ? launch_wide<T, 1, LOAD, EPI, YT>(a, s, kind) : launch_wide<T, 2, LOAD, EPI, YT>(a, s, kind);
 }
@@ -522,6 +528,7 @@ int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int loa
     using B = __nv_bfloat16;
     const bool norm = load == kLoadNorm;
     if (type == ELEM_F16) {
+        if (epi == kRowsStore && out == ELEM_F32 && load == kLoadF32Lo) return wide<__half, kLoadF32Lo, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsStore && out == ELEM_F32 && load == kLoadF32) return wide<__half, kLoadF32, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsStore && out == ELEM_F32)
             return norm ? wide<__half, kLoadNorm, kRowsStore, float>(a, s, PROF_GEMM_IN) : wide<__half, kLoadAsIs, kRowsStore, float>(a, s, PROF_GEMM_IN);

@@ -9,8 +9,8 @@ constexpr int kRowsGemmMax = 32;        // rows a launch takes
 enum { kRowsStore = 0, kRowsSwiglu, kRowsGeglu, kRowsArgmax, kRowsResidual, kRowsDeepStore };    // the last two: deep K, fp32 Y
 
 // How X comes in: 16-bit rows; fp32 rows to normalise; fp32 rows to which normalised rows `add` are added first, the sums also going to x_out
-// (row m from CTA m); fp32 rows to round.
-enum { kLoadAsIs = 0, kLoadNorm, kLoadAddNorm, kLoadF32 };
+// (row m from CTA m); fp32 rows to round; what rounding them to fp16 takes away, times kLoScale.
+enum { kLoadAsIs = 0, kLoadNorm, kLoadAddNorm, kLoadF32, kLoadF32Lo };
 
 struct RowsGemm {
     const void* x = nullptr;            // [M, K]
@@ -24,6 +24,7 @@ struct RowsGemm {
     const float* add = nullptr;         // [M, K] fp32: X = x + norm(add), kept in x_out (another buffer than x)
     float* x_out = nullptr;
     float scale = 1.f, cap = 0.f;       // store: y = cap tanh(scale v / cap), no cap at 0
+    bool accumulate = false;            // store, fp32: added to what is there
     void* y = nullptr;                  // store: [M, N]; gated: [M, N / 2]; residual: fp32 [M, N], added to
     int ldy = 0;
     int group = 0;

@@ -142,6 +142,16 @@ inline bool rows_layer_in(cudaStream_t s, const float* x, const __half* w, float
     *status = gemm_rows(s, a, ELEM_F16, kRowsStore, kLoadF32, ELEM_F32);
     return true;
 }
+// y's columns += (x_lo W_hi^T + x_hi W_lo^T) / kLoScale, the operands' low-order fp16 halves times kLoScale (f32_split_f16): behind rows_layer_in.
+inline int rows_layer_compensate(cudaStream_t s, const float* x, const __half* w_hi, const __half* w_lo, float* y, int ldy, int M, int N, int K, int* error) {
+    RowsGemm a;
+    a.x = x; a.ldx = K; a.w = w_hi; a.M = M; a.N = N; a.K = K; a.y = y; a.ldy = ldy; a.error = error;
+    a.scale = 1.0f / kLoScale;
+    a.accumulate = true;
+    B2_TRY(gemm_rows(s, a, ELEM_F16, kRowsStore, kLoadF32Lo, ELEM_F32));
+    a.w = w_lo;
+    return gemm_rows(s, a, ELEM_F16, kRowsStore, kLoadF32, ELEM_F32);
+}
 inline bool rows_layer_out(cudaStream_t s, const __half* x, const __half* w, float* y, float beta, int M, int N, int K, int* error, int* status) {
     RowsGemm a;
     a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.y = y; a.ldy = N; a.error = error;
