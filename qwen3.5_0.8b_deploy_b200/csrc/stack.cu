@@ -119,9 +119,10 @@ rmsnorm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
 }
 
 // act = silu(gate) * up.  gu rows hold tiles of 64 columns: 32 gate columns followed by the 32 matching up columns
-// (the layout the decode-step GEMM epilogue consumes as well).  fp16.  The fast exponential and division: with expf and the exact quotient the
-// kernel was bound by issue slots, 284 us for 65536 rows of 3584 (1.4 GB, 212 us at the memory rate), now 218 us; their error, 2^-18 at
-// |gate| = 20, is far below the rounding of the result to 11 bits.
+// (the layout the decode-step GEMM epilogue consumes as well).  fp16.  expf and the exact quotient, as in the epilogue of the few-row product
+// (gemm_rows.cu): the kernel is bound by issue slots with them, 284 us for 65536 rows of 3584 against 218 us with __expf and __fdividef (1.4 GB,
+// 212 us at the memory rate), but those leave errors up to 2^-20 of the value in front of the rounding (large negative gates), the library
+// functions 2^-22.
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const __half* __restrict__ gu, int inter, size_t n_oct, __half* __restrict__ act) {
     pdl_enter();
@@ -138,7 +139,7 @@ swiglu_kernel(const __half* __restrict__ gu, int inter, size_t n_oct, __half* __
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float2 g = __half22float2(gp[e]), u = __half22float2(up[e]);
-        o[e] = __floats2half2_rn(__fdividef(g.x, 1.0f + __expf(-g.x)) * u.x, __fdividef(g.y, 1.0f + __expf(-g.y)) * u.y);
+        o[e] = __floats2half2_rn(g.x / (1.0f + expf(-g.x)) * u.x, g.y / (1.0f + expf(-g.y)) * u.y);
     }
     *reinterpret_cast<uint4*>(act + row * inter + c) = *reinterpret_cast<uint4*>(o);
 }

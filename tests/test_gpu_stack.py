@@ -237,3 +237,37 @@ def test_stack_errors(ops, cuda, synth):
     with pytest.raises(ops.InvalidArgument):
         st.set_layer_weights(99, dict(input_norm=np.zeros(1024), post_norm=np.zeros(1024)),
                              dict(gate=np.zeros((INTER, 1024)), up=np.zeros((INTER, 1024)), down=np.zeros((1024, INTER))))
+
+
+def test_swiglu_of_prompts_keeps_fp32_accuracy(ops, cuda, synth):
+    """Gate and up values that reach the activation exactly: attention outputs of zero, one-hot residual rows of 1024 whose norm is 32, and an identity
+    behind the activation.  What the fp16 result may be off beside its own rounding: 2 ulp of expf and half an ulp each of the sum, the quotient
+    and the product, 3.5 * 2^-23 < 2^-21 of the value."""
+    torch = cuda
+    n, H, V = 128, 1024, 128
+    la = dict(synth.la_weights(64))
+    la["w_out"] = np.zeros_like(la["w_out"])
+    # the gates with the largest errors of a fast exponential, 2^-20 of the value (log2(e) g is rounded to 2^-20)
+    g = (np.round(synth.rng(64, "gates").uniform(-17, -11.2, (H, n)) * 64) / 64).astype(np.float16)
+    sil = g.astype(np.float64) / (1.0 + np.exp(-g.astype(np.float64)))
+    # up values that bring the products near one, so that none is rounded as an fp16 denormal
+    up = (synth.rng(64, "ups").uniform(1, 2, (H, n)) * 2.0 ** np.clip(-np.floor(np.log2(np.abs(sil) + 1e-30)), -2, 14)).astype(np.float16)
+    gate_w, up_w = np.zeros((H, H), np.float32), np.zeros((H, H), np.float32)
+    gate_w[:, :n], up_w[:, :n] = g.astype(np.float32) / 32, up.astype(np.float32) / 32
+    assert (gate_w.astype(np.float16).astype(np.float32) == gate_w).all() and (up_w.astype(np.float16).astype(np.float32) == up_w).all()
+    st = ops.HybridStack(num_layers=1, intermediate_size=H, vocab_size=V, max_seqs=n, max_seq_len=8, prefill_chunk_seqs=n, kv_dtype=ops.KV_FP16, int8_weights=False)
+    zero = np.zeros(H, np.float32)
+    st.set_layer_weights(0, dict(input_norm=zero, post_norm=zero), dict(gate=gate_w, up=up_w, down=np.eye(H, dtype=np.float32)), la=la)
+    st.set_embedding(1024.0 * np.eye(V, H, dtype=np.float32), zero)
+    hidden = st.forward_batch_prefill(torch.arange(n, dtype=torch.int32, device="cuda").reshape(n, 1), want_hidden=True)[1].double().cpu().numpy()
+    assert st.device_status() == 0
+    want = sil * up.astype(np.float64)                                    # [H, n]
+    x = 1024.0 * np.eye(n, H) + want.T
+    got = (hidden * np.sqrt((x ** 2).mean(1, keepdims=True) + 1e-6)).T    # the residual rows behind the layer, to about 2^-21
+    got = got.astype(np.float16).astype(np.float64)
+    keep = ~np.eye(H, n, dtype=bool) & (np.abs(want) > 2.0 ** -10)
+    assert keep.mean() > 0.9
+    off = np.abs(got - want)
+    half_ulp = 0.5 * 2.0 ** (np.floor(np.log2(np.abs(want) + 1e-30)) - 10)
+    bad = (off > half_ulp + 2.0 ** -21 * np.abs(want)) & keep
+    assert not bad.any(), f"{int(bad.sum())} of {int(keep.sum())} values beyond their rounding"
