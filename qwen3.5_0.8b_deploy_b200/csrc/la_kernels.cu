@@ -253,7 +253,9 @@ la_decode_kernel(const float* __restrict__ mixed, const int* __restrict__ slots,
     const int h = blockIdx.x, b = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = slots[b];
-    if (slot < 0 || slot >= max_seqs) return;
+    // A row without a sequence waits as well: left at once, a launch of such rows alone would complete before its predecessor, and the
+    // kernel behind, which waits for this one only, would run beside the input projection.
+    if (slot < 0 || slot >= max_seqs) { pdl_enter(); return; }
     __shared__ __align__(16) float s_qkv[3][kLaKd];
     constexpr int kWarpsR = 128 / kRows, kThreadsR = 32 * kWarpsR;
     if (stagger_ns) {
@@ -447,9 +449,10 @@ int launch_la_decode(const float* mixed, const int* d_slots, int n_seqs, int max
     // sequences with the start offset: 51.7 us without, 48.5 / 48.2 / 48.7 / 49.5 / 51.8 / 54.4 us at 148 / 222 / 296 /
     // 444 / 592 / 888 units.
     const unsigned l2_ahead = g_flags.la_l2_ahead;
-    // The kernel requests its state before the programmatic-launch wait.  That is only sound when another kernel that
-    // executes the wait runs between two writers of the same state (the decode step of a stack).  A caller that may
-    // launch this kernel twice in a row on one layer (the core entry) takes the ordinary stream order instead.
+    // The kernel requests its state before the programmatic-launch wait.  That is only sound when a kernel that waits BEFORE it lets the next
+    // launch in runs between two writers of the same state: the embedding launch of a step, or a projection launched with RowsGemm::late where the
+    // layer is called alone.  Kernels that let their successor in first (gemm_rows.cu) give no order, however many of them lie between.  A caller
+    // that may launch this kernel twice in a row on one layer (the core entry) takes the ordinary stream order instead.
 #define LA_DEC(T) launch_pdl_split(early_state_loads, n_seqs <= kRowsGemmMax, la_decode_kernel<T, 3, 16>, grid, dim3(256), 0, s, mixed, d_slots, max_seqs, rec_layer, \
                                 rec_stride, conv_layer, conv_stride, conv_w, a_log, dt_bias, norm_w, (T*)out, stagger_ns, (unsigned)n_sm, l2_ahead, stamp)
     if (out_fp16) LA_DEC(__half); else LA_DEC(float);

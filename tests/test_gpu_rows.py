@@ -152,3 +152,65 @@ def test_layer_decode_against_library_gemms(ops, cuda, synth, monkeypatch, kind,
     got = run()
     # one layer: three rounded vectors on the way, sqrt(3) * 2^-10 where every rounding differs by a unit
     assert (got - want).norm() <= 2e-3 * want.norm()
+
+
+# ---- steps whose rows are all without a sequence ------------------------------------------------------------------------------------
+@pytest.mark.parametrize("kind", ["fa16", "fa8", "la"])
+def test_layer_calls_of_inactive_rows(ops, cuda, synth, kind):
+    """Calls of slots -1 alone between calls of active rows, nothing else between them: the active ones give what they give without."""
+    torch = cuda
+    rows = 8
+    w = synth.la_weights(96) if kind == "la" else synth.fa_weights(96)
+    xs = torch.from_numpy(np.stack([synth.hidden_states(96, f"step{d}", rows) for d in range(8)])).cuda()
+    slots, none = torch.arange(rows, dtype=torch.int32, device="cuda"), torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+
+    def run(idle):
+        op = (ops.LinearAttention if kind == "la" else ops.FullAttention)(ops.PROJ_FP16, max_batch=rows, max_prefill_rows=64)
+        op.set_weights(w)
+        if kind == "la":
+            cache = ops.LinearAttnState(1, rows)
+        else:
+            cache = ops.KVCache(1, rows, 16, ops.KV_FP16 if kind == "fa16" else ops.KV_INT8)
+            for _ in range(rows):
+                cache.allocate_sequence(16)
+        out = []
+        for x in xs:
+            for _ in range(idle):
+                op.forward(x, cache, 0, none)
+            out.append(op.forward(x, cache, 0, slots))
+        return torch.stack(out)
+    want = run(0)
+    assert torch.equal(run(1), want) and torch.equal(run(3), want)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_steps_of_inactive_rows(ops, cuda, synth, captured):
+    """Steps behind the last sequence's end, then new sequences: their tokens are those of a stack that ran no such steps."""
+    torch = cuda
+    weights = _weights(synth, 97, 256, 512)
+    prompts = torch.from_numpy(synth.rng(97, "prompts").integers(0, 512, (4, T)).astype(np.int32)).cuda()
+
+    def run(idle):
+        st = _stack(ops, weights, 256, 512, 2)
+        st.begin_batching()
+        if captured:
+            st.capture_decode(2)
+        picks = []
+        for a in (0, 2):
+            for p in prompts[a:a + 2]:
+                st.admit(p.contiguous(), T + STEPS + 1)
+            for _ in range(STEPS):
+                st.step(2)
+                picks.append(st.get_tokens(2).clone())
+            st.retire(1)
+            st.retire(0)
+            for _ in range(idle):
+                st.step(2)
+        torch.cuda.synchronize()
+        assert st.device_status() == 0
+        return torch.stack(picks)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert torch.equal(run(3), run(0))
+    torch.cuda.synchronize()
