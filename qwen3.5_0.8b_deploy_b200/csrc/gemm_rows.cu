@@ -96,6 +96,15 @@ __device__ __forceinline__ float rows_act(float g) {
     else return times_sigmoid<A>(g, g);
 }
 
+// The next kernel of the stream may take its place at once.  If it is one of these it fetches weights and waits; any other waits before it touches
+// what a step writes, or reads recurrent state that was written before the step's embedding launch, which waits first (la_decode_kernel).  Where no
+// such launch lies between two calls (RowsGemm::late) this one waits first, whichever of the kernels the shape takes.
+__device__ __forceinline__ void rows_enter(bool late) {
+    if (!late) pdl_launch_dependents();
+    pdl_wait();
+    if (late) pdl_launch_dependents();
+}
+
 constexpr int kRowsThreads = 512, kRowsWarps = 16;
 
 // X into shared memory as 16-bit rows, a warp per row.
@@ -188,11 +197,7 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
                 bulk_g2s(smem_u32(smem) + half + i * pitch, static_cast<const T*>(a.w) + (size_t)(from + a.group) * a.K, (uint32_t)row_bytes, smem_u32(bar));
         }
     }
-    // The next kernel of the stream may take its place now.  If it is one of these it fetches weights and waits; any other waits before
-    // it touches what a step writes, or reads recurrent state that a kernel writes only after a wait of its own (la_decode_kernel).
-    if (!a.late) pdl_launch_dependents();
-    pdl_wait();
-    if (a.late) pdl_launch_dependents();
+    rows_enter(a.late);
     stamp_begin(stamp);
     load_rows<T, LOAD, kRowsWarps>(a, sx, pitch, warp, lane);
     __syncthreads();
@@ -303,8 +308,7 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (tid < 16 * MT) s_best[tid] = 0ull;
     __syncwarp();
     if (first < n_tiles) { fetch(first, 0); fetch(first, 1); }
-    pdl_launch_dependents();                     // see rows_wide_kernel
-    pdl_wait();
+    rows_enter(a.late);
     stamp_begin(stamp);
     load_rows<T, LOAD, kStreamWarps>(a, sx, pitch, warp, lane);
     __syncthreads();
@@ -398,8 +402,7 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
         if (lane < cols)
             bulk_g2s(smem_u32(smem) + lane * pitch, static_cast<const T*>(a.w) + (size_t)(n0 + lane) * a.K, (uint32_t)a.K * 2, smem_u32(bar));
     }
-    pdl_launch_dependents();                     // see rows_wide_kernel
-    pdl_wait();
+    rows_enter(a.late);
     stamp_begin(stamp);
     const Slices<MT> sl(a.K, kRowsWarps);
     const int c0 = sl.begin(warp), c1 = sl.begin(warp + 1);

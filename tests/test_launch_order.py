@@ -76,3 +76,11 @@ def test_no_way_out_before_the_wait(file, name):
     wait = WAIT.search(body)
     assert wait, "launched as a programmatic dependent, never waits"
     assert not re.search(r"\breturn\s*;", body[:wait.start()]), "leaves before it waits for its predecessor"
+
+
+@pytest.mark.parametrize("file,name", sorted(k for k, b in KERNELS.items() if "pdl_launch_dependents" in b or "rows_enter" in b))
+def test_the_next_launch_is_let_in_behind_the_wait(file, name):
+    """... or through rows_enter, which keeps that order for launches that ask for it."""
+    body = KERNELS[file, name]
+    lets = body.find("pdl_launch_dependents")
+    assert lets < 0 or WAIT.search(body).start() < lets
