@@ -1,4 +1,4 @@
-// Y = X W^T for the few rows of a decode step (M <= 32) on mma.sync, 16-bit operands, fp32 sums.
+// Y = X W^T for the few rows of a decode step (M <= 16) on mma.sync, 16-bit operands, fp32 sums.
 //
 // At a few rows a projection is one pass over its weights: the 17 MB of an input projection take 2.5 us at the memory rate.  A library
 // GEMM of this shape takes 5.5 to 8 us, because it starts to read them only after the kernel in front of it has finished, and the norm
@@ -14,8 +14,10 @@
 // 5.2 us, output projections (1024 x 2048 and 1024 x 3584) 3.1 us; the step of four layers and the head 237 -> 134 us.
 // Taken back: X in registers with one column tile at a time (eight warps through 2000 instructions each: 8.6, 9.5 and 4.1 us); asking L2 for the
 // weights of the launch after next (no change: the copies are not what a launch waits for).
-// tcgen05 would pad the rows to 64 or 128 and pay for a TMEM round trip (the kernels of gemm_tc.cu: 9.0, 10.8 and 10.5 us).  From 33 rows on X no
-// longer fits beside the slabs, and the library GEMMs serve the step.
+// Why 16 rows: a step of the hybrid stack at 1 / 8 / 16 rows takes 126 / 138 / 163 us against 194 / 191 / 200 us on library GEMMs.  Two row tiles (17 to 32
+// rows) need 203 KB beside the widest slab, so the next launch no longer fits an SM, and 64 registers no longer hold them: at 17 / 24 / 32 rows 228 / 241 /
+// 272 us against 193 / 204 / 221 (bf16 stacks 256 to 337 against 206 to 256), the head 25 to 29 us against 18; layers called alone gained 7 % at best.
+// Taken out: the library GEMMs serve those steps.  tcgen05 would pad the rows to 64 or 128 and pay for a TMEM round trip (gemm_tc.cu: 9.0, 10.8 and 10.5 us).
 #include "gemm_rows.cuh"
 #include "elem.cuh"
 #include "kernels.cuh"
@@ -59,25 +61,20 @@ __device__ __host__ __forceinline__ int rows_pitch(int k) { return (k * 2 + 127)
 // launch put two CTAs on each idle SM and left no registers there for the one behind it, which then came late.
 __device__ __forceinline__ int part_begin(int i, int n, int items) { return (int)((long long)i * items / n); }
 
-// K in slices of `per` chunks of 32, one per warp.  A tile's partial sums of one warp, 16 MT x 8 floats, lie in the eight weight rows they came
-// from, in the slice that this warp alone has read (the last one may reach into the padding): row m % 8, with the halves m / 8 swapped in every
-// other pair of rows against bank conflicts.
-template <int MT>
+// K in slices of `per` chunks of 32, one per warp.  A tile's partial sums of one warp, 16 x 8 floats, lie in the eight weight rows they came
+// from, in the slice that this warp alone has read: row m % 8, with the halves m / 8 swapped in every other pair of rows against bank conflicts.
 struct Slices {
     int chunks, per, active;      // active slices
     __device__ __forceinline__ Slices(int k, int warps) : chunks(k / 32) {
-        per = max(MT, (chunks + warps - 1) / warps);
+        per = (chunks + warps - 1) / warps;
         active = (chunks + per - 1) / per;
     }
     __device__ __forceinline__ int begin(int w) const { return min(chunks, w * per); }
     __device__ __forceinline__ static int at(int m, int pitch) { return (m & 7) * pitch + (((m >> 3) ^ ((m >> 1) & 1)) * 32); }
-    __device__ __forceinline__ void store(unsigned char* tile, int pitch, int w, int r, int c, const float (&acc)[MT][4]) const {
+    __device__ __forceinline__ void store(unsigned char* tile, int pitch, int w, int r, int c, const float (&acc)[4]) const {
         unsigned char* slice = tile + w * per * 64 + 8 * c;
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-            *reinterpret_cast<float2*>(slice + at(16 * mt + r, pitch)) = make_float2(acc[mt][0], acc[mt][1]);
-            *reinterpret_cast<float2*>(slice + at(16 * mt + 8 + r, pitch)) = make_float2(acc[mt][2], acc[mt][3]);
-        }
+        *reinterpret_cast<float2*>(slice + at(r, pitch)) = make_float2(acc[0], acc[1]);
+        *reinterpret_cast<float2*>(slice + at(8 + r, pitch)) = make_float2(acc[2], acc[3]);
     }
     __device__ __forceinline__ float total(const unsigned char* tile, int pitch, int m, int n) const {
         const unsigned char* p = tile + at(m, pitch) + 4 * n;
@@ -105,7 +102,8 @@ __device__ __forceinline__ void rows_enter(bool late) {
     if (late) pdl_launch_dependents();
 }
 
-constexpr int kRowsThreads = 512, kRowsWarps = 16;
+constexpr int kRowsThreads = 512, kRowsWarps = 16, kRows = kRowsGemmMax;
+static_assert(kRows == 16, "one row tile of mma.m16n8k16");
 
 // X into shared memory as 16-bit rows, a warp per row.
 template <typename T, int LOAD, int WARPS>
@@ -166,10 +164,9 @@ __device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, 
 // Many columns, K <= 1024: X in shared memory, up to eight column tiles per CTA.  A warp multiplies four tiles (two groups of eight warps when a
 // launch has CTAs with more than four) over its slice of K.  Gated: units of two tiles, 8 gate rows of the weights and the 8 up rows that
 // belong to them; the slab holds all gate rows, then all up rows.
-template <typename T, int MT, int LOAD, int EPI, typename YT>
+template <typename T, int LOAD, int EPI, typename YT>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
-    constexpr int kRows = 16 * MT;
     constexpr bool kGated = EPI == kRowsSwiglu || EPI == kRowsGeglu;
     extern __shared__ __align__(128) unsigned char smem[];
     const int pitch = rows_pitch(a.K), row_bytes = a.K * 2;
@@ -205,33 +202,24 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
 
     // ---- products --------------------------------------------------------------------------------------------------------
     const int groups = a.tiles > 4 ? 2 : 1, splits = kRowsWarps / groups, split = warp % splits, tile0 = (warp / splits) * 4;
-    const Slices<MT> sl(a.K, splits);
+    const Slices sl(a.K, splits);
     const int c0 = sl.begin(split), c1 = sl.begin(split + 1);
     const bool high = a.M > 8;
     auto tile_at = [&](int t) { return smem + (kGated ? (t & 1) * half + 8 * (t >> 1) * pitch : 8 * t * pitch); };
     const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
-    float acc[4][MT][4] = {};
+    float acc[4][4] = {};
     const unsigned char* xp = sx + r * pitch + c * 16;
-    auto x_frag = [&](int mt, int ch, uint4& lo, uint4& hi) {
-        lo = *reinterpret_cast<const uint4*>(xp + 16 * mt * pitch + ch * 64);
-        hi = make_uint4(0u, 0u, 0u, 0u);
-        if (high) hi = *reinterpret_cast<const uint4*>(xp + (16 * mt + 8) * pitch + ch * 64);
-    };
-    auto multiply = [&](float (&d)[4], const uint4& lo, const uint4& hi, const uint4& b) {
-        mma_rows<T>(d, lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-        mma_rows<T>(d, lo.z, hi.z, lo.w, hi.w, b.z, b.w);
-    };
-#pragma unroll(MT == 1 ? 2 : 1)
+#pragma unroll 2
     for (int ch = c0; ch < c1; ++ch) {
-        uint4 lo[MT], hi[MT];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) x_frag(mt, ch, lo[mt], hi[mt]);
+        const uint4 lo = *reinterpret_cast<const uint4*>(xp + ch * 64);
+        uint4 hi = make_uint4(0u, 0u, 0u, 0u);
+        if (high) hi = *reinterpret_cast<const uint4*>(xp + 8 * pitch + ch * 64);
 #pragma unroll
         for (int t = 0; t < 4; ++t)
             if (tile0 + t < tiles) {
                 const uint4 b = *reinterpret_cast<const uint4*>(tile_at(tile0 + t) + r * pitch + c * 16 + ch * 64);
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt) multiply(acc[t][mt], lo[mt], hi[mt], b);
+                mma_rows<T>(acc[t], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+                mma_rows<T>(acc[t], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
             }
     }
     __syncwarp();                                // every lane has read the slice: it may be overwritten
@@ -278,16 +266,16 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
 // in flight all the time, and no barrier of the CTA and no reduction stands between two tiles.
 // 32768 columns at 8 rows: 15.5 us from the dependency wait on, 67 MB; a ring at whose batches of tiles all warps met took 19.4 us, gemm_tc.cu's 20.9 us.
 constexpr int kStreamWarps = 8;
-template <typename T, int MT, int LOAD, int EPI>
+template <typename T, int LOAD, int EPI>
 __global__ void __launch_bounds__(kStreamWarps * 32)
 rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int pitch = rows_pitch(a.K), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
     unsigned char* sw = smem + warp * 8 * pitch;
     unsigned char* sx = smem + kStreamWarps * 8 * pitch;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sx + 16 * MT * pitch);              // two per warp
-    unsigned long long* s_best = reinterpret_cast<unsigned long long*>(bars + 2 * kStreamWarps);     // [16 MT]
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(s_best + 16 * MT);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sx + kRows * pitch);                // two per warp
+    unsigned long long* s_best = reinterpret_cast<unsigned long long*>(bars + 2 * kStreamWarps);     // [kRows]
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(s_best + kRows);
     const uint32_t bar = smem_u32(bars + 2 * warp);
     const int chunks = a.K / 32, mid = (chunks + 1) / 2, n_tiles = (a.N + 7) / 8, step = gridDim.x * kStreamWarps;
     const int first = blockIdx.x + gridDim.x * warp;
@@ -305,7 +293,7 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
         if (warp == 0) *abort_flag = 0;
         mbar_fence_init();
     }
-    if (tid < 16 * MT) s_best[tid] = 0ull;
+    if (tid < kRows) s_best[tid] = 0ull;
     __syncwarp();
     if (first < n_tiles) { fetch(first, 0); fetch(first, 1); }
     rows_enter(a.late);
@@ -314,15 +302,13 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
     __syncthreads();
 
     const bool high = a.M > 8;
-    unsigned long long best[2 * MT];
-#pragma unroll
-    for (int i = 0; i < 2 * MT; ++i) best[i] = pack_max(-INFINITY, 0);       // a row without a number above -inf gives token 0
+    unsigned long long best[2] = {pack_max(-INFINITY, 0), pack_max(-INFINITY, 0)};       // a row without a number above -inf gives token 0
     const unsigned char* xp = sx + r * pitch + c * 16;
     const unsigned char* wp = sw + r * pitch + c * 16;
     uint32_t parity = 0;
     bool ok = true;
     for (int tile = first; ok && tile < n_tiles; tile += step, parity ^= 1u) {
-        float acc[2][MT][4] = {};                // two chains
+        float acc[2][4] = {};                    // two chains
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
             const int c0 = half ? mid : 0, c1 = half ? chunks : mid;
@@ -332,14 +318,11 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
 #pragma unroll 4
             for (int ch = c0; ch < c1; ++ch) {
                 const uint4 b = *reinterpret_cast<const uint4*>(wp + ch * 64);
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    const uint4 lo = *reinterpret_cast<const uint4*>(xp + 16 * mt * pitch + ch * 64);
-                    uint4 hi = make_uint4(0u, 0u, 0u, 0u);
-                    if (high) hi = *reinterpret_cast<const uint4*>(xp + (16 * mt + 8) * pitch + ch * 64);
-                    mma_rows<T>(acc[0][mt], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-                    mma_rows<T>(acc[1][mt], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
-                }
+                const uint4 lo = *reinterpret_cast<const uint4*>(xp + ch * 64);
+                uint4 hi = make_uint4(0u, 0u, 0u, 0u);
+                if (high) hi = *reinterpret_cast<const uint4*>(xp + 8 * pitch + ch * 64);
+                mma_rows<T>(acc[0], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+                mma_rows<T>(acc[1], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
             }
             __syncwarp();                        // every lane has read the half
             if (tile + step < n_tiles) {
@@ -349,29 +332,27 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
         }
         if (!ok) break;
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int m = 16 * mt + 8 * (i >> 1) + r, n = 8 * tile + 2 * c + (i & 1);
-                float v = (acc[0][mt][i] + acc[1][mt][i]) * a.scale;
-                if (m >= a.M || n >= a.N) continue;
-                if constexpr (EPI == kRowsStore) {
-                    if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
-                    static_cast<float*>(a.y)[(size_t)m * a.ldy + n] = v;
-                } else if (v > -INFINITY) {
-                    best[2 * mt + (i >> 1)] = max(best[2 * mt + (i >> 1)], pack_max(v, n));
-                }
+        for (int i = 0; i < 4; ++i) {
+            const int m = 8 * (i >> 1) + r, n = 8 * tile + 2 * c + (i & 1);
+            float v = (acc[0][i] + acc[1][i]) * a.scale;
+            if (m >= a.M || n >= a.N) continue;
+            if constexpr (EPI == kRowsStore) {
+                if (a.cap > 0.f) v = a.cap * tanhf(v / a.cap);
+                static_cast<float*>(a.y)[(size_t)m * a.ldy + n] = v;
+            } else if (v > -INFINITY) {
+                best[i >> 1] = max(best[i >> 1], pack_max(v, n));
             }
+        }
     }
     if constexpr (EPI == kRowsArgmax) {
 #pragma unroll
-        for (int i = 0; i < 2 * MT; ++i) {
+        for (int i = 0; i < 2; ++i) {
             best[i] = max(best[i], __shfl_xor_sync(0xffffffffu, best[i], 1));
             best[i] = max(best[i], __shfl_xor_sync(0xffffffffu, best[i], 2));
             if (c == 0) atomicMax(s_best + 8 * i + r, best[i]);
         }
         __syncthreads();
-        if (tid < 16 * MT && tid < a.M) atomicMax(a.packed + tid, s_best[tid]);
+        if (tid < a.M) atomicMax(a.packed + tid, s_best[tid]);
     }
     __syncthreads();
     stamp_end(stamp);
@@ -380,10 +361,10 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
 
 // Few columns, deep K <= 4096: fp32 Y[M, N] = X W^T, added to what is there with ADD.  Up to eight columns per CTA (six or seven of 1024 on 148
 // SMs), the 16 warps split K, X goes from L2 straight into the registers of the warp that multiplies it, kAhead chunks at a time.
-template <typename T, int MT, bool ADD>
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
-    constexpr int kRows = 16 * MT, kAhead = MT == 1 ? 4 : 2;
+    constexpr int kAhead = 4;
     extern __shared__ __align__(128) unsigned char smem[];
     const int pitch = rows_pitch(a.K);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 8 * pitch);
@@ -404,7 +385,7 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     }
     rows_enter(a.late);
     stamp_begin(stamp);
-    const Slices<MT> sl(a.K, kRowsWarps);
+    const Slices sl(a.K, kRowsWarps);
     const int c0 = sl.begin(warp), c1 = sl.begin(warp + 1);
     const bool writes = tid < 8 * kRows && em < a.M && n8 < cols;
     float res = 0.f;
@@ -413,14 +394,14 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     auto load = [&](int i, int ch) {             // rows 8 i + r, chunk ch
         return 8 * i + r < a.M && ch < c1 ? __ldcg(reinterpret_cast<const uint4*>(xp + (size_t)8 * i * a.ldx + 32 * ch)) : make_uint4(0u, 0u, 0u, 0u);
     };
-    uint4 x[kAhead][2 * MT];
+    uint4 x[kAhead][2];
 #pragma unroll
     for (int j = 0; j < kAhead; ++j)
 #pragma unroll
-        for (int i = 0; i < 2 * MT; ++i) x[j][i] = load(i, c0 + j);
+        for (int i = 0; i < 2; ++i) x[j][i] = load(i, c0 + j);
     __syncthreads();                             // the barrier is initialised
     const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
-    float acc[2][MT][4] = {};                    // two chains
+    float acc[2][4] = {};                        // two chains
     const unsigned char* wp = smem + r * pitch + c * 16;
 #pragma unroll 1
     for (int g = c0; g < c1; g += kAhead) {
@@ -428,20 +409,15 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
         for (int j = 0; j < kAhead; ++j) {
             if (g + j >= c1) break;
             const uint4 b = *reinterpret_cast<const uint4*>(wp + (g + j) * 64);
+            const uint4 lo = x[j][0], hi = x[j][1];
+            mma_rows<T>(acc[0], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+            mma_rows<T>(acc[1], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                const uint4 lo = x[j][2 * mt], hi = x[j][2 * mt + 1];
-                mma_rows<T>(acc[0][mt], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-                mma_rows<T>(acc[1][mt], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
-            }
-#pragma unroll
-            for (int i = 0; i < 2 * MT; ++i) x[j][i] = load(i, g + j + kAhead);
+            for (int i = 0; i < 2; ++i) x[j][i] = load(i, g + j + kAhead);
         }
     }
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[0][mt][i] += acc[1][mt][i];
+    for (int i = 0; i < 4; ++i) acc[0][i] += acc[1][i];
     __syncwarp();
     if (c0 < c1) sl.store(smem, pitch, warp, r, c, acc[0]);
     __syncthreads();
@@ -453,8 +429,8 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (tid == 0 && *abort_flag && a.error) atomicExch(a.error, 7);
 }
 
-// Most shared memory of a launch.  Up to 16 rows a layer's launches fit side by side: 153 and 34 KB, 170 and 59 KB.
-constexpr int kSharedMost = 208 * 1024;
+// Most shared memory of a launch: 64 weight rows and 16 of X.  A layer's launches fit side by side: 153 and 34 KB, 170 and 59 KB.
+constexpr int kSharedMost = 176 * 1024;
 
 template <typename K>
 int prepare(PerDeviceOnce& once, K kernel) {
@@ -462,42 +438,42 @@ int prepare(PerDeviceOnce& once, K kernel) {
     return 0;
 }
 
-template <typename T, int MT, int LOAD, int EPI, typename YT>
+template <typename T, int LOAD, int EPI, typename YT>
 int launch_wide(RowsGemm a, cudaStream_t s, ProfKind kind) {
     static PerDeviceOnce once;
-    B2_TRY(prepare(once, rows_wide_kernel<T, MT, LOAD, EPI, YT>));
+    B2_TRY(prepare(once, rows_wide_kernel<T, LOAD, EPI, YT>));
     int sms = 0;
     B2_TRY(device_sm_count(&sms));
     const int unit = EPI == kRowsSwiglu || EPI == kRowsGeglu ? 2 : 1, units = ceil_div(a.N / unit, 8);
     const int waves = ceil_div(units * unit, 8 * sms), grid = std::min(units, waves * sms);     // one CTA per SM where eight tiles each are enough
     a.tiles = ceil_div(units, grid) * unit;
-    const size_t smem = (size_t)(8 * a.tiles + 16 * MT) * rows_pitch(a.K) + 16;
+    const size_t smem = (size_t)(8 * a.tiles + kRows) * rows_pitch(a.K) + 16;
     unsigned long long* stamp = prof_stamp_slot(kind);
-    launch_pdl_split(true, true, rows_wide_kernel<T, MT, LOAD, EPI, YT>, dim3(grid), dim3(kRowsThreads), smem, s, a, stamp);
+    launch_pdl_split(true, true, rows_wide_kernel<T, LOAD, EPI, YT>, dim3(grid), dim3(kRowsThreads), smem, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
-template <typename T, int MT, int LOAD, int EPI>
+template <typename T, int LOAD, int EPI>
 int launch_stream(const RowsGemm& a, int sms, cudaStream_t s, ProfKind kind) {
     static PerDeviceOnce once;
-    B2_TRY(prepare(once, rows_stream_kernel<T, MT, LOAD, EPI>));
-    const size_t smem = (size_t)(8 * kStreamWarps + 16 * MT) * rows_pitch(a.K) + 8 * (2 * kStreamWarps + 16 * MT) + 16;
+    B2_TRY(prepare(once, rows_stream_kernel<T, LOAD, EPI>));
+    const size_t smem = (size_t)(8 * kStreamWarps + kRows) * rows_pitch(a.K) + 8 * (2 * kStreamWarps + kRows) + 16;
     unsigned long long* stamp = prof_stamp_slot(kind);
-    launch_pdl_split(true, true, rows_stream_kernel<T, MT, LOAD, EPI>, dim3(sms), dim3(kStreamWarps * 32), smem, s, a, stamp);
+    launch_pdl_split(true, true, rows_stream_kernel<T, LOAD, EPI>, dim3(sms), dim3(kStreamWarps * 32), smem, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
-template <typename T, int MT, bool ADD>
+template <typename T, bool ADD>
 int launch_deep(const RowsGemm& a, cudaStream_t s) {
     static PerDeviceOnce once;
-    B2_TRY(prepare(once, rows_deep_kernel<T, MT, ADD>));
+    B2_TRY(prepare(once, rows_deep_kernel<T, ADD>));
     unsigned long long* stamp = prof_stamp_slot(PROF_GEMM_RES);
     int sms = 0;
     B2_TRY(device_sm_count(&sms));
     const int grid = std::max(ceil_div(a.N, 8), std::min(a.N, sms));      // up to eight columns a CTA
-    launch_pdl_split(true, true, rows_deep_kernel<T, MT, ADD>, dim3(grid), dim3(kRowsThreads), (size_t)8 * rows_pitch(a.K) + 16, s, a, stamp);
+    launch_pdl_split(true, true, rows_deep_kernel<T, ADD>, dim3(grid), dim3(kRowsThreads), (size_t)8 * rows_pitch(a.K) + 16, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -509,13 +485,9 @@ int wide(const RowsGemm& a, cudaStream_t s, ProfKind kind) {
     if constexpr ((EPI == kRowsStore && std::is_same_v<YT, float>) || EPI == kRowsArgmax) {
         int sms = 0;
         B2_TRY(device_sm_count(&sms));
-        if (a.N > 64 * sms && !a.accumulate) return a.M <= 16 ? launch_stream<T, 1, LOAD, EPI>(a, sms, s, kind) : launch_stream<T, 2, LOAD, EPI>(a, sms, s, kind);
+        if (a.N > 64 * sms && !a.accumulate) return launch_stream<T, LOAD, EPI>(a, sms, s, kind);
     }
-    return a.M <= 16 ? launch_wide<T, 1, LOAD, EPI, YT>(a, s, kind) : launch_wide<T, 2, LOAD, EPI, YT>(a, s, kind);
-}
-template <typename T, bool ADD>
-int deep(const RowsGemm& a, cudaStream_t s) {
-    return a.M <= 16 ? launch_deep<T, 1, ADD>(a, s) : launch_deep<T, 2, ADD>(a, s);
+    return launch_wide<T, LOAD, EPI, YT>(a, s, kind);
 }
 
 }  // namespace
@@ -536,8 +508,8 @@ int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int loa
         if (epi == kRowsStore && out == ELEM_F32)
             return norm ? wide<__half, kLoadNorm, kRowsStore, float>(a, s, PROF_GEMM_IN) : wide<__half, kLoadAsIs, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsSwiglu && out == ELEM_F16 && norm) return wide<__half, kLoadNorm, kRowsSwiglu, __half>(a, s, PROF_GEMM_FFN);
-        if (epi == kRowsResidual) return deep<__half, true>(a, s);
-        if (epi == kRowsDeepStore) return deep<__half, false>(a, s);
+        if (epi == kRowsResidual) return launch_deep<__half, true>(a, s);
+        if (epi == kRowsDeepStore) return launch_deep<__half, false>(a, s);
         if (epi == kRowsArgmax)
             return norm ? wide<__half, kLoadNorm, kRowsArgmax, float>(a, s, PROF_LM_HEAD) : wide<__half, kLoadAsIs, kRowsArgmax, float>(a, s, PROF_LM_HEAD);
     }
@@ -550,8 +522,8 @@ int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int loa
 #undef ROWS_LOADS
         if (epi == kRowsStore && out == ELEM_BF16 && !a.add)
             return norm ? wide<B, kLoadNorm, kRowsStore, B>(a, s, PROF_GEMM_IN) : wide<B, kLoadAsIs, kRowsStore, B>(a, s, PROF_GEMM_IN);
-        if (epi == kRowsResidual) return deep<B, true>(a, s);
-        if (epi == kRowsDeepStore) return deep<B, false>(a, s);
+        if (epi == kRowsResidual) return launch_deep<B, true>(a, s);
+        if (epi == kRowsDeepStore) return launch_deep<B, false>(a, s);
     }
     B2_FAIL(B200ATTN_ERR_UNSUPPORTED, "gemm_rows: unsupported types");
 }

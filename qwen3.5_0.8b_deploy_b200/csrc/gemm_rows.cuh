@@ -5,7 +5,7 @@
 
 namespace b200 {
 
-constexpr int kRowsGemmMax = 32;        // rows a launch takes
+constexpr int kRowsGemmMax = 16;        // rows a launch takes (the figures: gemm_rows.cu)
 enum { kRowsStore = 0, kRowsSwiglu, kRowsGeglu, kRowsArgmax, kRowsResidual, kRowsDeepStore };    // the last two: deep K, fp32 Y
 
 // How X comes in: 16-bit rows; fp32 rows to normalise; fp32 rows to which normalised rows `add` are added first, the sums also going to x_out

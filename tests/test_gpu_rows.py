@@ -76,6 +76,18 @@ def test_decode_rows_against_library_gemms(ops, cuda, synth, monkeypatch, rows, 
     assert ((got_t >= 0) & (got_t < vocab)).all()
 
 
+@pytest.mark.parametrize("rows", [17, 32])
+def test_more_rows_than_one_tile_take_the_library_gemms(ops, cuda, synth, monkeypatch, rows):
+    """Above 16 rows the library GEMMs are the faster ones: the step is theirs, bit for bit."""
+    torch = cuda
+    weights = _weights(synth, 70 + rows, 256, 512)
+    tokens = torch.from_numpy(synth.rng(70 + rows, "tokens").integers(0, 512, (rows, T + STEPS)).astype(np.int32)).cuda()
+    got = _decode(torch, ops, weights, 256, 512, rows, tokens)
+    monkeypatch.setenv("B200ATTN_DECODE_GEMM", "cublas")
+    want = _decode(torch, ops, weights, 256, 512, rows, tokens)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 # ---- layer-described stacks (bf16) -------------------------------------------------------------------------------------------------
 def _gutenex_layers():
     return [gutenex.lightning(2, 32, 48, ff=96), gutenex.delta(4, 2, 32, 32, conv=4, a_rank=20, g_rank=12, ff=70), gutenex.diff(4, 2, 32, 64, 16, 30, 5, ff=64),
