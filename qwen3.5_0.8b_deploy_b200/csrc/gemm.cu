@@ -180,31 +180,34 @@ int gemm_xwT(cudaStream_t stream, const void* X, bool x_fp16, const void* W, boo
 }
 
 // x -> hi = fp16(x), lo = fp16((x - hi) * 2^11): hi + lo * 2^-11 carries about 22 significant bits of x.
-__global__ void f32_split_f16_kernel(const float* __restrict__ in, __half* __restrict__ hi, __half* __restrict__ lo, size_t n) {
+// `wide`: the input lies on a boundary of the vector loads; a caller's tensor may not (a view that starts at an odd element).
+__global__ void f32_split_f16_kernel(const float* __restrict__ in, __half* __restrict__ hi, __half* __restrict__ lo, size_t n, bool wide) {
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    if (i + 1 < n) {
+    if (wide && i + 1 < n) {
         const float2 v = *reinterpret_cast<const float2*>(in + i);
         const __half2 h = __floats2half2_rn(v.x, v.y);
         const float2 hf = __half22float2(h);
         *reinterpret_cast<__half2*>(hi + i) = h;
         *reinterpret_cast<__half2*>(lo + i) = __floats2half2_rn((v.x - hf.x) * kLoScale, (v.y - hf.y) * kLoScale);
-    } else if (i < n) {
-        const __half h = __float2half_rn(in[i]);
-        hi[i] = h;
-        lo[i] = __float2half_rn((in[i] - __half2float(h)) * kLoScale);
+    } else {
+        for (size_t j = i; j < n && j < i + 2; ++j) {
+            const __half h = __float2half_rn(in[j]);
+            hi[j] = h;
+            lo[j] = __float2half_rn((in[j] - __half2float(h)) * kLoScale);
+        }
     }
 }
 int f32_split_f16(cudaStream_t s, const float* in, __half* hi, __half* lo, size_t n) {
     if (n == 0) return 0;
     const size_t threads = (n + 1) / 2;
-    f32_split_f16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(in, hi, lo, n);
+    f32_split_f16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(in, hi, lo, n, (reinterpret_cast<uintptr_t>(in) & 7) == 0);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
-__global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restrict__ out, size_t n) {
+__global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restrict__ out, size_t n, bool wide) {
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i + 3 < n) {
+    if (wide && i + 3 < n) {
         const float4 v = *reinterpret_cast<const float4*>(in + i);
         __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
         uint2 pk;
@@ -212,14 +215,14 @@ __global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restri
         pk.y = *reinterpret_cast<uint32_t*>(&b);
         *reinterpret_cast<uint2*>(out + i) = pk;
     } else {
-        for (size_t j = i; j < n; ++j) out[j] = __float2half_rn(in[j]);
+        for (size_t j = i; j < n && j < i + 4; ++j) out[j] = __float2half_rn(in[j]);
     }
 }
 
 int f32_to_f16(cudaStream_t s, const float* in, __half* out, size_t n) {
     if (n == 0) return 0;
     const size_t threads = (n + 3) / 4;
-    f32_to_f16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(in, out, n);
+    f32_to_f16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(in, out, n, (reinterpret_cast<uintptr_t>(in) & 15) == 0);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -310,3 +310,22 @@ def test_prefill_continues_ragged_caches(ops, cuda, synth, kv_dtype):
         ok, msg = allclose_report(got, whole[at[2]:at[2] + a + b], ATOL, RTOL)
         assert ok, f"{a} + {b} tokens: {msg}"
         at = [at[0] + a, at[1] + b, at[2] + a + b]
+
+
+@pytest.mark.parametrize("kv_dtype", [0, 1])
+def test_decode_core_takes_unaligned_queries(ops, cuda, synth, kv_dtype):
+    """Queries that do not start on a 16-byte boundary are rounded by a launch of their own, to the same values: equal outputs."""
+    torch = cuda
+    n, lengths = 5, [1, 63, 64, 130, 200]
+    fa = ops.FullAttention(ops.PROJ_FP32, max_batch=n, max_prefill_rows=64)
+    kv = ops.KVCache(1, n, 256, kv_dtype)
+    slots = [kv.allocate_sequence(256) for _ in range(n)]
+    k, v = (torch.from_numpy(synth.normal(99, name, (sum(lengths), 512))).float().cuda() for name in "kv")
+    kv.append(0, slots, lengths, k, v)
+    d_slots = torch.tensor(slots, dtype=torch.int32, device="cuda")
+    q = torch.from_numpy(synth.normal(99, "q", (n, 8, 256))).float().cuda()
+    want = fa.decode_core(q, kv, 0, d_slots)
+    for shift in (1, 2, 3):
+        base = torch.empty(q.numel() + shift, device="cuda")
+        got = fa.decode_core(base[shift:].view(q.shape).copy_(q), kv, 0, d_slots)
+        assert torch.equal(got, want), f"queries {4 * shift} bytes behind a boundary"

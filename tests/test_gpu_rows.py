@@ -166,6 +166,39 @@ def test_layer_decode_against_library_gemms(ops, cuda, synth, monkeypatch, kind,
     assert (got - want).norm() <= 2e-3 * want.norm()
 
 
+@pytest.mark.parametrize("kind", ["fa16", "fa8", "la"])
+@pytest.mark.parametrize("rows", [1, 8, 17])
+def test_layer_calls_on_unaligned_rows(ops, cuda, synth, kind, rows):
+    """Inputs that start one, two and three floats behind a 16-byte boundary, prompts and decode rows: the products of before the few-row kernels."""
+    torch = cuda
+    w = synth.la_weights(98) if kind == "la" else synth.fa_weights(98)
+    xs = torch.from_numpy(np.stack([synth.hidden_states(98, f"step{d}", rows) for d in range(4)])).cuda()
+    slots = torch.arange(rows, dtype=torch.int32, device="cuda")
+
+    def at(x, shift):
+        base = torch.empty(x.numel() + shift, device="cuda")
+        out = base[shift:].view(x.shape)
+        assert (out.data_ptr() - base.data_ptr()) == 4 * shift
+        return out.copy_(x)
+
+    def run(shift):
+        op = (ops.LinearAttention if kind == "la" else ops.FullAttention)(ops.PROJ_FP16, max_batch=rows, max_prefill_rows=64)
+        op.set_weights(w)
+        if kind == "la":
+            cache = ops.LinearAttnState(1, rows)
+        else:
+            cache = ops.KVCache(1, rows, 16, ops.KV_FP16 if kind == "fa16" else ops.KV_INT8)
+            for _ in range(rows):
+                cache.allocate_sequence(16)
+        prefill = op.forward_batch if kind == "la" else op.forward_batch_prefill
+        return torch.stack([prefill(at(xs[0], shift), cache, 0, list(range(rows)), [1] * rows)] + [op.forward(at(x, shift), cache, 0, slots) for x in xs])
+    want = run(0)
+    for shift in (1, 2, 3):
+        got = run(shift)
+        assert torch.equal(got[0], want[0])                        # a prompt takes the same products
+        assert (got - want).norm() <= 2e-3 * want.norm()           # as test_layer_decode_against_library_gemms
+
+
 # ---- steps whose rows are all without a sequence ------------------------------------------------------------------------------------
 @pytest.mark.parametrize("kind", ["fa16", "fa8", "la"])
 def test_layer_calls_of_inactive_rows(ops, cuda, synth, kind):
