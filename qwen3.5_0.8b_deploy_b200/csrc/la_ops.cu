@@ -18,7 +18,8 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // 22 us (estimated from 14 us for an own part, 2.6 us a chunk of the walk).
 constexpr int kLaSplitSeqs = 4, kLaSplitChunks = 4;
 // R rows in S sequences are at most R / 64 + S chunks, of 22.5 KB per row; q, k and v hold 24 KB per row.
-constexpr size_t kLaSplitRoom = kLaSplitSeqs * (size_t)kLaHeads * (kLaSplitBytes + 4);
+// Room for the last, partly filled chunk of each sequence, 5.8 MB; an operator of fewer rows than the longest sequence needs never takes that form.
+static size_t la_split_room(size_t rows) { return rows > 64 * (kLaSplitChunks - 1) ? kLaSplitSeqs * (size_t)kLaHeads * (kLaSplitBytes + 4) : 0; }
 static_assert(kLaHeads * (kLaSplitBytes + 4) <= 64 * 3 * kLaHeads * kLaKd * 4, "a full chunk's images fit its rows of q, k and v");
 
 size_t la_scratch_bytes(const b200attn_la_config& c) {
@@ -26,7 +27,7 @@ size_t la_scratch_bytes(const b200attn_la_config& c) {
     size_t n = 0;
     n += align_up(R * kLaProjCols * 4, 256);            // mixed
     n += 3 * align_up(R * kLaHeads * kLaKd * 4, 256);   // q, k, v; in their place the images of the two-kernel recurrence
-    n += align_up(kLaSplitRoom, 256);                   // ... and room for the last, partly filled chunk of each of its sequences
+    n += align_up(la_split_room(R), 256);
     n += 3 * align_up(R * kLaHeads * kLaKd * 2, 256);   // q, k, v as fp16
     n += 2 * align_up(R * kLaHeads * 4, 256);           // g, beta
     n += align_up(R * kLaHeads * kLaVd * 4, 256);       // core
@@ -46,7 +47,7 @@ void la_carve_scratch(b200attn_la la) {
     la->d_q = (float*)take(R * kLaHeads * kLaKd * 4);
     la->d_k = (float*)take(R * kLaHeads * kLaKd * 4);
     la->d_v = (float*)take(R * kLaHeads * kLaKd * 4);
-    take(kLaSplitRoom);
+    take(la_split_room(R));
     la->d_qh = (__half*)take(R * kLaHeads * kLaKd * 2);
     la->d_kh = (__half*)take(R * kLaHeads * kLaKd * 2);
     la->d_vh = (__half*)take(R * kLaHeads * kLaVd * 2);

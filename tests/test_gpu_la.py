@@ -373,3 +373,18 @@ def test_two_kernel_recurrence_equals_one_kernel(ops, cuda, synth, counts):
     np.testing.assert_array_equal(got[0][0], got[1][0])
     for a, b in zip(got[0][1], got[1][1]):
         np.testing.assert_array_equal(a, b)
+
+
+def test_scratch_of_the_two_kernel_recurrence(ops, cuda):
+    """Its 5.8 MB are held by operators that can be given a sequence of more than 192 tokens, and by no other."""
+    torch = cuda
+
+    def held(rows):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        la = [ops.LinearAttention(ops.PROJ_FP16, max_batch=4, max_prefill_rows=rows) for _ in range(4)]
+        used = before - torch.cuda.mem_get_info()[0]
+        del la
+        return used / 4
+    held(64)                                                       # what the first operator of a process sets up
+    assert held(193) - held(192) > 4e6                             # one row is 0.1 MB; allocations are rounded up to 2 MB
