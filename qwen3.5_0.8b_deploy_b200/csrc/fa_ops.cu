@@ -165,7 +165,7 @@ static int fa_check(b200attn_fa fa, b200attn_kv_pool pool, int layer) {
 static int fa_project_in(b200attn_fa fa, const void* d_x, bool x_is_fp16, int rows, bool kv_int8, bool decode, DecodeOut* fused, int* d_error,
                          cudaStream_t s) {
     if (fa->cfg.proj_precision == B200ATTN_PROJ_FP16) {
-        if (fused && fused->rows) return rows_project(s, d_x, x_is_fp16, fused->eps, fa->d_wqkv_fp16, fa->d_qkv_raw, rows, kFaQkvCols, kHidden, d_error);
+        if (fused && fused->rows) return rows_project(s, d_x, fused->eps, fa->d_wqkv_fp16, fa->d_qkv_raw, rows, kFaQkvCols, kHidden, d_error);
         if (fused)   // decode step of a stack: d_x is the un-normalised residual stream, its RMSNorm scale is applied in the epilogue
             return gemm_tc_store(s, (const __half*)d_x, fa->d_wqkv_fp16, fa->d_qkv_raw, rows, kFaQkvCols, kHidden, kFaQkvCols, fused->rowsq,
                                  fused->eps, d_error);

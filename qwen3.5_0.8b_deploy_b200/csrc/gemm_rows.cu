@@ -505,8 +505,7 @@ int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int loa
     if (type == ELEM_F16) {
         if (epi == kRowsStore && out == ELEM_F32 && load == kLoadF32Lo) return wide<__half, kLoadF32Lo, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsStore && out == ELEM_F32 && load == kLoadF32) return wide<__half, kLoadF32, kRowsStore, float>(a, s, PROF_GEMM_IN);
-        if (epi == kRowsStore && out == ELEM_F32)
-            return norm ? wide<__half, kLoadNorm, kRowsStore, float>(a, s, PROF_GEMM_IN) : wide<__half, kLoadAsIs, kRowsStore, float>(a, s, PROF_GEMM_IN);
+        if (epi == kRowsStore && out == ELEM_F32 && norm) return wide<__half, kLoadNorm, kRowsStore, float>(a, s, PROF_GEMM_IN);
         if (epi == kRowsSwiglu && out == ELEM_F16 && norm) return wide<__half, kLoadNorm, kRowsSwiglu, __half>(a, s, PROF_GEMM_FFN);
         if (epi == kRowsResidual) return launch_deep<__half, true>(a, s);
         if (epi == kRowsDeepStore) return launch_deep<__half, false>(a, s);

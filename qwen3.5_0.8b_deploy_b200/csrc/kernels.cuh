@@ -71,7 +71,7 @@ int launch_la_conv_seq(const float* mixed, const LaRun* d_runs, int n_runs, cons
                        size_t conv_stride, const float* conv_w, const float* a_log, const float* dt_bias,
                        float* q, float* k, __half* qh, __half* kh, float* v, __half* vh, float* g, float* beta, cudaStream_t s);
 // The chunked recurrence in two kernels (la_chunk.cu), for batches of few sequences: chunk_list entries {row = chunk, seq} in the order of the
-// sequences, each sequence's first entry, and scratch of la_split_bytes(n_chunks).
+// sequences, each sequence's first entry, and scratch of kLaHeads * (kLaSplitBytes + 4) bytes per chunk.
 struct LaSplit {
     int n_chunks = 0;                    // 0: one kernel
     const LaRun* d_chunks = nullptr;
@@ -79,7 +79,6 @@ struct LaSplit {
     void* scratch = nullptr;
 };
 constexpr size_t kLaSplitBytes = 90112;  // of a chunk and head
-inline size_t la_split_bytes(int n_chunks) { return (size_t)n_chunks * kLaHeads * (kLaSplitBytes + 4); }
 int launch_la_chunk_tc(const __half* q_h, const __half* k_h, const __half* v_h, const float* g, const float* beta,
                        const LaSeqMeta* d_seqs, int n_seqs, int rows, float* rec_layer, size_t rec_stride, float* out,
                        int* d_error, const LaSplit& split, cudaStream_t s);
@@ -117,15 +116,14 @@ struct DecodeOut {
     __half* xh;        // [rows, hidden] fp16 copy of the residual stream (read as d_x, rewritten by the output projection)
     float* rowsq;      // [128][kRowsqParts] partial sums of squares of the residual rows
     float eps;         // RMSNorm epsilon
-    bool rows = false; // few rows (gemm_rows.cu): d_x is the fp32 residual stream, normalised by the projection itself, or already normalised
-                       // fp16 rows; xh and rowsq are not used
+    bool rows = false; // few rows (gemm_rows.cu): d_x is the fp32 residual stream, normalised by the projection itself; xh and rowsq are not used
 };
 
-// The same over few rows: Y = norm(X) W^T or X W^T, and h += X W^T.
-inline int rows_project(cudaStream_t s, const void* x, bool normed, float eps, const __half* w, float* y, int M, int N, int K, int* error) {
+// The same over few rows: Y = norm(X) W^T, and h += X W^T.
+inline int rows_project(cudaStream_t s, const void* x, float eps, const __half* w, float* y, int M, int N, int K, int* error) {
     RowsGemm a;
     a.x = x; a.ldx = K; a.w = w; a.M = M; a.N = N; a.K = K; a.eps = eps; a.y = y; a.ldy = N; a.error = error;
-    return gemm_rows(s, a, ELEM_F16, kRowsStore, normed ? kLoadAsIs : kLoadNorm, ELEM_F32);
+    return gemm_rows(s, a, ELEM_F16, kRowsStore, kLoadNorm, ELEM_F32);
 }
 inline int rows_residual(cudaStream_t s, const __half* x, const __half* w, float* h, int M, int N, int K, int* error) {
     RowsGemm a;

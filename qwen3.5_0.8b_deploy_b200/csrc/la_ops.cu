@@ -344,7 +344,7 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
     auto project_in = [&](int rows) -> int {
         if (fp16) {
             if (decode && dout && dout->rows)
-                return rows_project(s, d_x, x_is_fp16, dout->eps, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, la->d_error);
+                return rows_project(s, d_x, dout->eps, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, la->d_error);
             if (decode && dout)   // decode step of a stack: d_x is the un-normalised residual stream, its RMSNorm scale is applied in the epilogue
                 return gemm_tc_store(s, (const __half*)d_x, la->d_win_fp16, la->d_mixed, rows, kLaProjCols, kHidden, kLaProjCols, dout->rowsq,
                                      dout->eps, la->d_error);
