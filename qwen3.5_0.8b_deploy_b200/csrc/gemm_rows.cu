@@ -207,6 +207,7 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
     const bool high = a.M > 8;
     auto tile_at = [&](int t) { return smem + (kGated ? (t & 1) * half + 8 * (t >> 1) * pitch : 8 * t * pitch); };
     const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
+    if (!ok) mbar_drain(smem_u32(bar), 0);
     float acc[4][4] = {};
     const unsigned char* xp = sx + r * pitch + c * 16;
 #pragma unroll 2
@@ -314,7 +315,11 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
             const int c0 = half ? mid : 0, c1 = half ? chunks : mid;
             if (c0 == c1) continue;
             ok = mbar_wait_warp(bar + 8 * half, parity, abort_flag);
-            if (!ok) break;
+            if (!ok) {                           // this half's copies, and the other half's: of this tile behind it, or of the next
+                mbar_drain(bar + 8 * half, parity);
+                if (half ? tile + step < n_tiles : mid < chunks) mbar_drain(bar + 8 * (half ^ 1), parity ^ half);
+                break;
+            }
 #pragma unroll 4
             for (int ch = c0; ch < c1; ++ch) {
                 const uint4 b = *reinterpret_cast<const uint4*>(wp + ch * 64);
@@ -401,6 +406,7 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
         for (int i = 0; i < 2; ++i) x[j][i] = load(i, c0 + j);
     __syncthreads();                             // the barrier is initialised
     const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
+    if (!ok) mbar_drain(smem_u32(bar), 0);
     float acc[2][4] = {};                        // two chains
     const unsigned char* wp = smem + r * pitch + c * 16;
 #pragma unroll 1

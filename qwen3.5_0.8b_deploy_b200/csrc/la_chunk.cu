@@ -706,7 +706,11 @@ la_chunk_own_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_after();
         tmem_dealloc(tm_x, 128);
     }
-    if (tid == 0 && *abort_flag) atomicExch(error_word, 6);
+    if (tid == 0 && *abort_flag) {
+        mbar_drain(bar(G_FULL_KQ), 0);
+        mbar_drain(bar(G_FULL_V), 0);
+        atomicExch(error_word, 6);
+    }
 }
 
 // grid (heads, n_seqs), block 288: eight compute warps as in la_chunk_tc_kernel, one warp for copies and MMAs.  Two images in flight.
@@ -762,7 +766,8 @@ la_chunk_walk_kernel(const unsigned char* __restrict__ images, const float* __re
             };
             load(0);
             if (n_chunks > 1) load(1);
-            for (int c = 0; c < n_chunks; ++c) {
+            int c = 0;
+            for (; c < n_chunks; ++c) {
                 const uint32_t par = c & 1, kq = base + 1024 + par * kImgTiles, w = kq + 32768, mq = kq + 49152, tm_x = tm_o + par * 64;
                 if (!mbar_wait(bar(W_FULL0 + par), (c >> 1) & 1, abort_flag)) break;
                 if (!mbar_wait(bar(W_B2), par, abort_flag)) break;
@@ -792,6 +797,7 @@ la_chunk_walk_kernel(const unsigned char* __restrict__ images, const float* __re
                     load(c + 2);
                 }
             }
+            for (int e = c; e < min(c + 2, n_chunks); ++e) mbar_drain(bar(W_FULL0 + (e & 1)), (e >> 1) & 1);     // after a wait that ran out
         }
     } else {
         const int r = tid & 127, hf = tid >> 7;

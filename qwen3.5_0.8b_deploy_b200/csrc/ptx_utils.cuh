@@ -83,6 +83,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// After a wait that ran out: a second, shorter limit for the copies that are still on their way to this CTA's shared memory, which another CTA
+// may be given as soon as this one leaves.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, uint64_t limit_ns = 50000000ull) {
+    const uint64_t t0 = global_timer_ns();
+    while (!mbar_try_wait(bar, parity) && global_timer_ns() - t0 < limit_ns) {}
+}
+
 // Warp-uniform form for roles whose next instruction is warp-collective (.sync.aligned): either every
 // lane proceeds or every lane gives up.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {

@@ -84,3 +84,10 @@ def test_the_next_launch_is_let_in_behind_the_wait(file, name):
     body = KERNELS[file, name]
     lets = body.find("pdl_launch_dependents")
     assert lets < 0 or WAIT.search(body).start() < lets
+
+
+@pytest.mark.parametrize("file,name", [("gemm_rows.cu", "rows_wide_kernel"), ("gemm_rows.cu", "rows_stream_kernel"), ("gemm_rows.cu", "rows_deep_kernel"),
+                                       ("la_chunk.cu", "la_chunk_own_kernel"), ("la_chunk.cu", "la_chunk_walk_kernel")])
+def test_a_wait_that_runs_out_leaves_no_copy_behind(file, name):
+    """A CTA that gives up waits once more for its copies: its shared memory may be another's as soon as it leaves."""
+    assert "mbar_drain" in KERNELS[file, name]
