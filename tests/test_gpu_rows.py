@@ -1,5 +1,6 @@
-"""GPU: the few-row projections of a decode step against the library GEMMs, at the edges of their row tiles (8 / 9, 16 / 17, 32 / 33 rows) and
-of their column tiles (feed-forward widths of one gate / up group and of a ragged last batch, vocabularies below and above a wave)."""
+"""GPU: the few-row projections of a decode step against the library GEMMs and the plain implementations, at the edges of their row tile (8 / 9,
+16 / 17 rows) and of their column tiles: feed-forward widths of one gate / up group, of a ragged last batch and of more than one wave; vocabularies that one
+slab per CTA holds and, above 64 columns per SM (9472 on 148), streamed ones."""
 import os
 import sys
 
@@ -9,6 +10,7 @@ import pytest
 sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 import test_gpu_gutenex as gutenex  # noqa: E402
 import test_gpu_nuzopel as nuzopel  # noqa: E402
+import test_gpu_stack as stack_tests  # noqa: E402
 from test_gpu_nuzopel import models, wts  # noqa: E402,F401
 
 pytestmark = pytest.mark.gpu
@@ -86,6 +88,88 @@ def test_more_rows_than_one_tile_take_the_library_gemms(ops, cuda, synth, monkey
     monkeypatch.setenv("B200ATTN_DECODE_GEMM", "cublas")
     want = _decode(torch, ops, weights, 256, 512, rows, tokens)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_few_row_steps_against_cpu_composition(ops, cuda, oracle, synth, monkeypatch):
+    monkeypatch.delenv("B200ATTN_DECODE_GEMM", raising=False)
+    stack_tests.test_prefill_and_decode_against_cpu_composition(ops, cuda, oracle, synth, None)
+
+
+# ---- vocabularies that are streamed ------------------------------------------------------------------------------------------------
+def _head_limits(torch, hidden, embed):
+    """float64 logits of normed rows; what sums of 1024 products in fp32 may be off (2^-23 of their absolute sum each); that sum itself."""
+    x = hidden.half().double()
+    absolute = x.abs() @ embed.abs().T
+    return x @ embed.T, 1024 * 2.0 ** -23 * absolute, absolute
+
+
+@pytest.mark.parametrize("vocab", [9473, 20001, 32768])
+def test_streamed_head(ops, cuda, synth, vocab):
+    """Picks over one column of a last tile, over ragged and over whole tiles, several tiles a warp: maximal under float64 logits of the same rows."""
+    torch = cuda
+    weights = _weights(synth, 33, 64, vocab)
+    embed = torch.from_numpy(weights["embed"]).cuda().half().double()
+    for rows in (1, 8, 9, 16, 17):
+        tokens = torch.from_numpy(synth.rng(33, f"tokens{rows}").integers(0, vocab, (rows, T + 1)).astype(np.int32)).cuda()
+        st = _stack(ops, weights, 64, vocab, rows)
+        prompt = tokens[:, :T].contiguous()
+        with_hidden, hidden = st.forward_batch_prefill(prompt, want_hidden=True)
+        st.reset_cache()
+        alone = st.forward_batch_prefill(prompt)
+        stepped = st.forward_batch_decode(tokens[:, T].contiguous())
+        st.reset_cache()
+        then = st.forward_batch_prefill(tokens, want_hidden=True)[1]
+        assert st.device_status() == 0
+        logits, limit, absolute = _head_limits(torch, hidden, embed)
+        at = torch.arange(rows, device="cuda")
+        assert (logits[at, with_hidden.long()] >= logits.amax(1) - 2 * limit.amax(1)).all()
+        # the norm on the way in may round a value to its neighbour, 2^-10 of it
+        assert (logits[at, alone.long()] >= logits.amax(1) - 2 * (limit + 2.0 ** -10 * absolute).amax(1)).all()
+        # a step against a prompt of the same tokens: other products in the layers, four of them
+        logits = _head_limits(torch, then, embed)[0]
+        assert (logits[at, stepped.long()] >= logits.amax(1) - 0.05 * (logits.amax(1) - logits.mean(1))).all()
+
+
+@pytest.mark.parametrize("vocab", [9473, 20001, 32768])
+def test_streamed_logits(ops, cuda, synth, monkeypatch, vocab):
+    """Logits of 1 to 17 places of a prompt: the last place against float64 from its normed row, all of them against the library GEMM's."""
+    torch = cuda
+    n = 20
+    weights = _weights(synth, 34, 64, vocab)
+    embed = torch.from_numpy(weights["embed"]).cuda().half().double()
+    tokens = torch.from_numpy(synth.rng(34, "tokens").integers(0, vocab, (1, n)).astype(np.int32)).cuda()
+    hidden = _stack(ops, weights, 64, vocab, 2).forward_batch_prefill(tokens, want_hidden=True)[1]
+    logits, limit, absolute = _head_limits(torch, hidden, embed)
+
+    def run(places):
+        st = _stack(ops, weights, 64, vocab, 2)
+        st.begin_batching()
+        out = st.extend(st.open(n), tokens[0].contiguous(), range(n - places, n)).clone().reshape(places, vocab)
+        assert st.device_status() == 0
+        return out
+    for places in (1, 8, 9, 16, 17):
+        got = run(places)
+        assert ((got[-1].double() - logits[0]).abs() <= (limit + 2.0 ** -10 * absolute)[0]).all()
+        monkeypatch.setenv("B200ATTN_DECODE_GEMM", "cublas")
+        want = run(places)
+        monkeypatch.delenv("B200ATTN_DECODE_GEMM")
+        assert (got - want).norm() <= 2.0 ** -11 * want.norm()         # the same rows: a rounding of the norm now and then
+
+
+@pytest.mark.parametrize("design", [0, 1])
+def test_wide_layers_and_streamed_logits_of_block_stacks(cuda, models, wts, design):
+    """A feed-forward width of two waves with a ragged end, a vocabulary that is streamed, and (Gutenex) its soft cap."""
+    mod, make = ((nuzopel, nuzopel.make), (gutenex, gutenex.make))[design]
+    layers = [nuzopel.mlstm(2, 32, 48, ff=4802)] if design == 0 else [gutenex.lightning(2, 32, 48, ff=4802)]
+    c = mod.Case(models, wts, *make(layers, width=64, vocab=20001, seed=35), "bfloat16")
+    toks = c.tokens(34)
+    want = c.expect(toks)
+    with nuzopel.on_stream(cuda):
+        c.stack.begin_batching()
+        for cuts in ([1], [9, 1, 16]):
+            row = c.stack.open()
+            c.judge(c.run(cuda, row, toks, cuts), want, f"cuts {cuts}")
+            c.stack.retire(row)
 
 
 # ---- layer-described stacks (bf16) -------------------------------------------------------------------------------------------------
