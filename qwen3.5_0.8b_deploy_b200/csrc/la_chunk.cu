@@ -138,129 +138,129 @@ __device__ __forceinline__ void solve_column_group(const float* BM, float* TF, i
 // matrices; kq: the K / Q tiles.
 __device__ __forceinline__ void chunk_own_part(unsigned char* sm, unsigned char* kq, unsigned char* wr, float* AM, float* TF, const float* s_b, const float* s_beta,
                                                const float* s_eb, uint32_t tm_ut, uint32_t lane_base, int tid, int warp, int lane, int r, int hf) {
-                {
-                    uint32_t d1[32];
-                    tmem_ld32(tm_ut + lane_base + hf * 32, d1);
-                    tmem_wait_ld();
-                    if (r < 64) {
-                        const float bi = s_b[r], be = s_beta[r];
-    #pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            float a4[4];
-                            const float4 bj4 = *reinterpret_cast<const float4*>(&s_b[hf * 32 + j4 * 4]);
-                            const float bj[4] = {bj4.x, bj4.y, bj4.z, bj4.w};
-    #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int j = hf * 32 + j4 * 4 + e;
-                                a4[e] = (j < r) ? be * ex2_approx((bi - bj[e]) * kLog2e) * __uint_as_float(d1[j4 * 4 + e]) : 0.f;
-                            }
-                            *reinterpret_cast<float4*>(AM + r * kLd + hf * 32 + j4 * 4) = make_float4(a4[0], a4[1], a4[2], a4[3]);
-                        }
-                    } else {
-                        const int i = r - 64;
-                        const float bi = s_b[i];
-                        unsigned char* row_ptr = sm + kOffMQ + i * 128;
-    #pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) {
-                            uint32_t pk[4];
-                            const float4 bl = *reinterpret_cast<const float4*>(&s_b[hf * 32 + cc * 8]);
-                            const float4 bh = *reinterpret_cast<const float4*>(&s_b[hf * 32 + cc * 8 + 4]);
-                            const float bj[8] = {bl.x, bl.y, bl.z, bl.w, bh.x, bh.y, bh.z, bh.w};
-    #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int j0 = hf * 32 + cc * 8 + 2 * e, j1 = j0 + 1;
-                                const float m0 = (j0 <= i) ? ex2_approx((bi - bj[2 * e]) * kLog2e) * __uint_as_float(d1[cc * 8 + 2 * e]) : 0.f;
-                                const float m1 = (j1 <= i) ? ex2_approx((bi - bj[2 * e + 1]) * kLog2e) * __uint_as_float(d1[cc * 8 + 2 * e + 1]) : 0.f;
-                                pk[e] = pack_half2(m0, m1);
-                            }
-                            *reinterpret_cast<uint4*>(row_ptr + (((hf * 4 + cc) ^ (i & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                        }
-                    }
+    {
+        uint32_t d1[32];
+        tmem_ld32(tm_ut + lane_base + hf * 32, d1);
+        tmem_wait_ld();
+        if (r < 64) {
+            const float bi = s_b[r], be = s_beta[r];
+#pragma unroll
+            for (int j4 = 0; j4 < 8; ++j4) {
+                float a4[4];
+                const float4 bj4 = *reinterpret_cast<const float4*>(&s_b[hf * 32 + j4 * 4]);
+                const float bj[4] = {bj4.x, bj4.y, bj4.z, bj4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = hf * 32 + j4 * 4 + e;
+                    a4[e] = (j < r) ? be * ex2_approx((bi - bj[e]) * kLog2e) * __uint_as_float(d1[j4 * 4 + e]) : 0.f;
                 }
-                named_sync_256();
-                // ---- T = (I + A)^-1, blocked 16 x 16.  Two warps invert the diagonal blocks by forward substitution (one
-                //      thread per column); meanwhile the other six scale the Q tile: every element of row i times e^{b_i}
-                //      (the swizzle only permutes 16-byte pieces inside a row). ----
-                if (tid < 64) {
-                    const int b0 = (tid >> 4) * 16, col = tid & 15;      // column `col` of diagonal block b0 / 16
-                    float t[16];
-    #pragma unroll
-                    for (int i = 0; i < 16; ++i) t[i] = (i == col) ? 1.f : 0.f;
-    #pragma unroll
-                    for (int i = 1; i < 16; ++i) {
-                        const float* arow = AM + (b0 + i) * kLd + b0;
-                        float acc0 = 0.f, acc1 = 0.f;
-    #pragma unroll
-                        for (int j4 = 0; 4 * j4 < i; ++j4) {
-                            const float4 a4 = *reinterpret_cast<const float4*>(arow + 4 * j4);   // entries at and above the diagonal are zero
-                            acc0 += a4.x * t[4 * j4] + a4.z * t[4 * j4 + 2];
-                            acc1 += a4.y * t[4 * j4 + 1] + a4.w * t[4 * j4 + 3];
-                        }
-                        t[i] -= acc0 + acc1;   // rows <= col keep their start value: A is strictly lower and t[j < col] = 0
-                    }
-    #pragma unroll
-                    for (int i = 0; i < 16; ++i) TF[(b0 + i) * kLd + b0 + col] = t[i];
-                } else {
-                    for (int idx = tid - 64; idx < 1024; idx += 192) {
-                        const int blk = idx >> 9, i = (idx >> 3) & 63;
-                        const float sc = s_eb[i];
-                        uint4* p4 = reinterpret_cast<uint4*>(kq + blk * 16384 + 8192 + i * 128 + ((idx & 7) << 4));
-                        uint4 x = *p4;
-                        __half2* hx = reinterpret_cast<__half2*>(&x);
-    #pragma unroll
-                        for (int w2 = 0; w2 < 4; ++w2) {
-                            const float2 f = __half22float2(hx[w2]);
-                            hx[w2] = __floats2half2_rn(f.x * sc, f.y * sc);
-                        }
-                        *p4 = x;
-                    }
+                *reinterpret_cast<float4*>(AM + r * kLd + hf * 32 + j4 * 4) = make_float4(a4[0], a4[1], a4[2], a4[3]);
+            }
+        } else {
+            const int i = r - 64;
+            const float bi = s_b[i];
+            unsigned char* row_ptr = sm + kOffMQ + i * 128;
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+                uint32_t pk[4];
+                const float4 bl = *reinterpret_cast<const float4*>(&s_b[hf * 32 + cc * 8]);
+                const float4 bh = *reinterpret_cast<const float4*>(&s_b[hf * 32 + cc * 8 + 4]);
+                const float bj[8] = {bl.x, bl.y, bl.z, bl.w, bh.x, bh.y, bh.z, bh.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j0 = hf * 32 + cc * 8 + 2 * e, j1 = j0 + 1;
+                    const float m0 = (j0 <= i) ? ex2_approx((bi - bj[2 * e]) * kLog2e) * __uint_as_float(d1[cc * 8 + 2 * e]) : 0.f;
+                    const float m1 = (j1 <= i) ? ex2_approx((bi - bj[2 * e + 1]) * kLog2e) * __uint_as_float(d1[cc * 8 + 2 * e + 1]) : 0.f;
+                    pk[e] = pack_half2(m0, m1);
                 }
-                named_sync_256();
-                if (warp < 6) scale_blocks(AM, TF, warp, lane);
-                named_sync_256();
-                // every warp takes a group of columns of T and works down its block rows: the four leftmost groups of 4 columns
-                // have the longest way (six 16 x 16 x 4 products), the others less
-                if (warp < 4) solve_column_group<4, 0>(AM, TF, 4 * warp, lane);
-                else if (warp < 6) solve_column_group<8, 1>(AM, TF, 16 + 8 * (warp - 4), lane);
-                else solve_column_group<8, 2>(AM, TF, 32 + 8 * (warp - 6), lane);
-                named_sync_256();
-                {   // T diag(beta) and T diag(beta e^b) -> fp16 hi + lo tiles (row = i, K = j), written over A and T
-                    const int i = tid >> 2, qd = tid & 3;
-                    float tv[16];
-    #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        float4 t4 = *reinterpret_cast<const float4*>(&TF[i * kLd + qd * 16 + 4 * e]);
-                        if (qd > (i >> 4)) t4 = make_float4(0.f, 0.f, 0.f, 0.f);      // blocks above the diagonal are never written
-                        tv[4 * e] = t4.x; tv[4 * e + 1] = t4.y; tv[4 * e + 2] = t4.z; tv[4 * e + 3] = t4.w;
-                    }
-                    float bt[16], ebv[16];       // beta_j and e^{b_j} of this thread's 16 columns
-    #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float4 b4 = *reinterpret_cast<const float4*>(&s_beta[qd * 16 + 4 * e]);
-                        const float4 e4 = *reinterpret_cast<const float4*>(&s_eb[qd * 16 + 4 * e]);
-                        bt[4 * e] = b4.x; bt[4 * e + 1] = b4.y; bt[4 * e + 2] = b4.z; bt[4 * e + 3] = b4.w;
-                        ebv[4 * e] = e4.x; ebv[4 * e + 1] = e4.y; ebv[4 * e + 2] = e4.z; ebv[4 * e + 3] = e4.w;
-                    }
-                    named_sync_256();     // every thread holds its part of T: the tiles may overwrite it
-    #pragma unroll
-                    for (int cc = 0; cc < 2; ++cc) {
-                        uint32_t uh[4], ul[4], wh[4], wl[4];
-    #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float u0 = tv[cc * 8 + 2 * e] * bt[cc * 8 + 2 * e], u1 = tv[cc * 8 + 2 * e + 1] * bt[cc * 8 + 2 * e + 1];
-                            const float w0 = u0 * ebv[cc * 8 + 2 * e], w1 = u1 * ebv[cc * 8 + 2 * e + 1];
-                            const float uh0 = __half2float(__float2half_rn(u0)), uh1 = __half2float(__float2half_rn(u1));
-                            const float wh0 = __half2float(__float2half_rn(w0)), wh1 = __half2float(__float2half_rn(w1));
-                            uh[e] = pack_half2(uh0, uh1); ul[e] = pack_half2(u0 - uh0, u1 - uh1);
-                            wh[e] = pack_half2(wh0, wh1); wl[e] = pack_half2(w0 - wh0, w1 - wh1);
-                        }
-                        const uint32_t o16 = i * 128 + (((qd * 2 + cc) ^ (i & 7)) << 4);
-                        *reinterpret_cast<uint4*>(wr + o16) = make_uint4(uh[0], uh[1], uh[2], uh[3]);
-                        *reinterpret_cast<uint4*>(wr + 8192 + o16) = make_uint4(ul[0], ul[1], ul[2], ul[3]);
-                        *reinterpret_cast<uint4*>(wr + 16384 + o16) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                        *reinterpret_cast<uint4*>(wr + 24576 + o16) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-                    }
-                }
+                *reinterpret_cast<uint4*>(row_ptr + (((hf * 4 + cc) ^ (i & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            }
+        }
+    }
+    named_sync_256();
+    // ---- T = (I + A)^-1, blocked 16 x 16.  Two warps invert the diagonal blocks by forward substitution (one
+    //      thread per column); meanwhile the other six scale the Q tile: every element of row i times e^{b_i}
+    //      (the swizzle only permutes 16-byte pieces inside a row). ----
+    if (tid < 64) {
+        const int b0 = (tid >> 4) * 16, col = tid & 15;      // column `col` of diagonal block b0 / 16
+        float t[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) t[i] = (i == col) ? 1.f : 0.f;
+#pragma unroll
+        for (int i = 1; i < 16; ++i) {
+            const float* arow = AM + (b0 + i) * kLd + b0;
+            float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+            for (int j4 = 0; 4 * j4 < i; ++j4) {
+                const float4 a4 = *reinterpret_cast<const float4*>(arow + 4 * j4);   // entries at and above the diagonal are zero
+                acc0 += a4.x * t[4 * j4] + a4.z * t[4 * j4 + 2];
+                acc1 += a4.y * t[4 * j4 + 1] + a4.w * t[4 * j4 + 3];
+            }
+            t[i] -= acc0 + acc1;   // rows <= col keep their start value: A is strictly lower and t[j < col] = 0
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) TF[(b0 + i) * kLd + b0 + col] = t[i];
+    } else {
+        for (int idx = tid - 64; idx < 1024; idx += 192) {
+            const int blk = idx >> 9, i = (idx >> 3) & 63;
+            const float sc = s_eb[i];
+            uint4* p4 = reinterpret_cast<uint4*>(kq + blk * 16384 + 8192 + i * 128 + ((idx & 7) << 4));
+            uint4 x = *p4;
+            __half2* hx = reinterpret_cast<__half2*>(&x);
+#pragma unroll
+            for (int w2 = 0; w2 < 4; ++w2) {
+                const float2 f = __half22float2(hx[w2]);
+                hx[w2] = __floats2half2_rn(f.x * sc, f.y * sc);
+            }
+            *p4 = x;
+        }
+    }
+    named_sync_256();
+    if (warp < 6) scale_blocks(AM, TF, warp, lane);
+    named_sync_256();
+    // every warp takes a group of columns of T and works down its block rows: the four leftmost groups of 4 columns
+    // have the longest way (six 16 x 16 x 4 products), the others less
+    if (warp < 4) solve_column_group<4, 0>(AM, TF, 4 * warp, lane);
+    else if (warp < 6) solve_column_group<8, 1>(AM, TF, 16 + 8 * (warp - 4), lane);
+    else solve_column_group<8, 2>(AM, TF, 32 + 8 * (warp - 6), lane);
+    named_sync_256();
+    {   // T diag(beta) and T diag(beta e^b) -> fp16 hi + lo tiles (row = i, K = j), written over A and T
+        const int i = tid >> 2, qd = tid & 3;
+        float tv[16];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float4 t4 = *reinterpret_cast<const float4*>(&TF[i * kLd + qd * 16 + 4 * e]);
+            if (qd > (i >> 4)) t4 = make_float4(0.f, 0.f, 0.f, 0.f);      // blocks above the diagonal are never written
+            tv[4 * e] = t4.x; tv[4 * e + 1] = t4.y; tv[4 * e + 2] = t4.z; tv[4 * e + 3] = t4.w;
+        }
+        float bt[16], ebv[16];       // beta_j and e^{b_j} of this thread's 16 columns
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float4 b4 = *reinterpret_cast<const float4*>(&s_beta[qd * 16 + 4 * e]);
+            const float4 e4 = *reinterpret_cast<const float4*>(&s_eb[qd * 16 + 4 * e]);
+            bt[4 * e] = b4.x; bt[4 * e + 1] = b4.y; bt[4 * e + 2] = b4.z; bt[4 * e + 3] = b4.w;
+            ebv[4 * e] = e4.x; ebv[4 * e + 1] = e4.y; ebv[4 * e + 2] = e4.z; ebv[4 * e + 3] = e4.w;
+        }
+        named_sync_256();     // every thread holds its part of T: the tiles may overwrite it
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+            uint32_t uh[4], ul[4], wh[4], wl[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float u0 = tv[cc * 8 + 2 * e] * bt[cc * 8 + 2 * e], u1 = tv[cc * 8 + 2 * e + 1] * bt[cc * 8 + 2 * e + 1];
+                const float w0 = u0 * ebv[cc * 8 + 2 * e], w1 = u1 * ebv[cc * 8 + 2 * e + 1];
+                const float uh0 = __half2float(__float2half_rn(u0)), uh1 = __half2float(__float2half_rn(u1));
+                const float wh0 = __half2float(__float2half_rn(w0)), wh1 = __half2float(__float2half_rn(w1));
+                uh[e] = pack_half2(uh0, uh1); ul[e] = pack_half2(u0 - uh0, u1 - uh1);
+                wh[e] = pack_half2(wh0, wh1); wl[e] = pack_half2(w0 - wh0, w1 - wh1);
+            }
+            const uint32_t o16 = i * 128 + (((qd * 2 + cc) ^ (i & 7)) << 4);
+            *reinterpret_cast<uint4*>(wr + o16) = make_uint4(uh[0], uh[1], uh[2], uh[3]);
+            *reinterpret_cast<uint4*>(wr + 8192 + o16) = make_uint4(ul[0], ul[1], ul[2], ul[3]);
+            *reinterpret_cast<uint4*>(wr + 16384 + o16) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+            *reinterpret_cast<uint4*>(wr + 24576 + o16) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+        }
+    }
 }
 
 // Per-chunk scalars by warp 0, two consecutive tokens per lane: b = cumsum(g), beta, e^b, e^{b_C - b}.
