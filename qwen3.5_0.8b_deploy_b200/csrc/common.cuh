@@ -87,7 +87,8 @@ struct ProfScope {   // brackets the launches issued during its lifetime when pr
 // before it builds its operators, and no launch path touches the environment.
 struct RuntimeFlags {
     bool pdl = true;                 // B200ATTN_PDL=0: ordinary stream order instead of programmatic dependent launch
-    bool decode_gemm_tc = false;     // B200ATTN_DECODE_GEMM=tc: the fused decode step on the tcgen05 skinny GEMMs (default: library GEMMs + norm / SwiGLU kernels)
+    bool decode_gemm_tc = false;     // B200ATTN_DECODE_GEMM=tc: the fused decode step on the tcgen05 skinny GEMMs (default: the few-row products of gemm_rows.cu
+                                     // up to 16 rows, library GEMMs + norm / SwiGLU kernels above)
     bool decode_gemm_rows = true;    // B200ATTN_DECODE_GEMM=cublas: library GEMMs for few rows too
     bool lm_head_cublas = false;     // B200ATTN_LM_HEAD=cublas: library GEMM + argmax kernel instead of the fused epilogue
     bool la_prefill_serial = false;  // B200ATTN_LA_PREFILL=serial: token-serial fp32 recurrence instead of the chunked tensor-core kernels
@@ -118,7 +119,8 @@ void per_device_once_end(PerDeviceOnce& o, int dev);
 //
 // `share_sm`: the launch asks for the largest shared-memory part of the L1 store.  An SM keeps the split that it was given until it is
 // empty, so with one split for a chain of kernels the next one can become resident, and fetch its weights, beside the one that still
-// runs: a decode step of 8 rows took 196 us with the splits that the driver chose and 149 us with one.
+// runs: a decode step of 8 rows took 196 us with the splits that the driver chose and 149 us with one (then; columns cut evenly over the SMs took it
+// further, gemm_rows.cu).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl_split(bool on, bool share_sm, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
