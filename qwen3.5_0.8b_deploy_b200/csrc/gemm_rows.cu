@@ -11,7 +11,8 @@
 //   * the fp32 residual rows are normalised on the way in (the rounding point is the norm kernel's: one rounding of the normalised value), and
 //     SwiGLU and the residual addition sit in the epilogue.  A layer of a step is five launches in place of eight or nine.
 // Measured in a captured step of 8 rows, from the dependency wait on: input projection (8224 x 1024) 5.3 us, gate / up with SwiGLU (7168 x 1024)
-// 5.2 us, output projections (1024 x 2048 and 1024 x 3584) 3.1 us; the step of four layers and the head 237 -> 134 us.
+// 5.0 us, output projections (1024 x 2048 and 1024 x 3584) 3.7 us; the step of four layers and the head 191 -> 138 us (fp16 cache, 50 tokens), 193 -> 141 us
+// behind 500 tokens of an INT8 cache.
 // Taken back: X in registers with one column tile at a time (eight warps through 2000 instructions each: 8.6, 9.5 and 4.1 us); asking L2 for the
 // weights of the launch after next (no change: the copies are not what a launch waits for).
 // Why 16 rows: a step of the hybrid stack at 1 / 8 / 16 rows takes 126 / 138 / 163 us against 194 / 191 / 200 us on library GEMMs.  Two row tiles (17 to 32
@@ -210,17 +211,25 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (!ok) mbar_drain(smem_u32(bar), 0);
     float acc[4][4] = {};
     const unsigned char* xp = sx + r * pitch + c * 16;
+    // These two as functions: written out in the loop, ptxas spilled in the variants on 16-bit rows, 1.5 us more a step of the bf16 stacks.
+    auto x_frag = [&](int ch, uint4& lo, uint4& hi) {
+        lo = *reinterpret_cast<const uint4*>(xp + ch * 64);
+        hi = make_uint4(0u, 0u, 0u, 0u);
+        if (high) hi = *reinterpret_cast<const uint4*>(xp + 8 * pitch + ch * 64);
+    };
+    auto multiply = [&](float (&d)[4], const uint4& lo, const uint4& hi, const uint4& b) {
+        mma_rows<T>(d, lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+        mma_rows<T>(d, lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+    };
 #pragma unroll 2
     for (int ch = c0; ch < c1; ++ch) {
-        const uint4 lo = *reinterpret_cast<const uint4*>(xp + ch * 64);
-        uint4 hi = make_uint4(0u, 0u, 0u, 0u);
-        if (high) hi = *reinterpret_cast<const uint4*>(xp + 8 * pitch + ch * 64);
+        uint4 lo, hi;
+        x_frag(ch, lo, hi);
 #pragma unroll
         for (int t = 0; t < 4; ++t)
             if (tile0 + t < tiles) {
                 const uint4 b = *reinterpret_cast<const uint4*>(tile_at(tile0 + t) + r * pitch + c * 16 + ch * 64);
-                mma_rows<T>(acc[t], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-                mma_rows<T>(acc[t], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+                multiply(acc[t], lo, hi, b);
             }
     }
     __syncwarp();                                // every lane has read the slice: it may be overwritten
@@ -265,7 +274,8 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
 // More columns than a wave of CTAs holds at eight tiles each (the LM head), K <= 1024: the warps work on tiles of their own.  A warp streams
 // its tiles' weights through one slab in two halves of K, each refilled as soon as it has been multiplied, so that most of the 135 KB are
 // in flight all the time, and no barrier of the CTA and no reduction stands between two tiles.
-// 32768 columns at 8 rows: 15.5 us from the dependency wait on, 67 MB; a ring at whose batches of tiles all warps met took 19.4 us, gemm_tc.cu's 20.9 us.
+// From the dependency wait on, this / gemm_tc.cu's kernel, which needs a norm launch in front: 32768 columns at 8 rows 16.4 / 18.3 us (67 MB), 248320 at 1 / 8 / 16 rows
+// 78 / 81 / 89 against 104 / 111 / 111 us (509 MB).  A ring at whose batches of tiles all warps met took 19.4 us at 32768.
 constexpr int kStreamWarps = 8;
 template <typename T, int LOAD, int EPI>
 __global__ void __launch_bounds__(kStreamWarps * 32)
