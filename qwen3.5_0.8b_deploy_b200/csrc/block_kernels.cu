@@ -214,18 +214,6 @@ int launch_softcap(float* logits, size_t n, float cap, cudaStream_t s) {
     return 0;
 }
 
-// 0.5 z (1 + tanh y) = z / (1 + e^{-2y}), y = sqrt(2 / pi) (z + 0.044715 z^3)
-template <typename T>
-__device__ __forceinline__ float gelu_tanh(float z) {
-    return times_sigmoid<T>(z, 1.5957691216057308f * (z + 0.044715f * z * z * z));
-}
-
-template <typename T, int kAct>
-__device__ __forceinline__ float activated(float z) {
-    if constexpr (kAct == B200ATTN_ACT_SILU) return times_sigmoid<T>(z, z);
-    else return gelu_tanh<T>(z);
-}
-
 // Blocks of 128 threads: one per row, or (few rows) several along it.
 template <typename T, int kAct>
 __global__ void __launch_bounds__(128)

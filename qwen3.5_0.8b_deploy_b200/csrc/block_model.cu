@@ -1,6 +1,7 @@
 // Layer-described models: construction from descriptions, weights by name, the layer loop, and the mixers with norms on their outputs.
 #include "stack.cuh"
 #include "elem.cuh"
+#include "gemm_pair.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -591,6 +592,8 @@ static int run_layers(BlockModel& m, const PassRows& pass, cudaStream_t s) {
             a.group = L.ff;
             a.y = m.act.p; a.ldy = L.ff;
             B2_TRY(gemm_rows(s, a, m.elem, L.act == B200ATTN_ACT_SILU ? kRowsSwiglu : kRowsGeglu, a.x != m.xt.p ? kLoadNorm : kLoadAsIs, m.elem));
+        } else if (!p.decode && gemm_glu_takes(m.elem, m.xt.p, L.w_gu.p, m.act.p, R, L.ff, W)) {
+            B2_TRY(gemm_glu(s, m.elem, L.act, m.xt.p, L.w_gu.p, m.act.p, R, L.ff, W, true, m.error.i()));
         } else {
             B2_TRY(gemm_typed(s, m.xt.p, W, L.w_gu.p, m.gu.p, 2 * L.ff, m.elem, m.elem, R, 2 * L.ff, W));
             B2_TRY(launch_act_mul(m.elem, L.act, m.gu.p, R, L.ff, m.act.p, s));

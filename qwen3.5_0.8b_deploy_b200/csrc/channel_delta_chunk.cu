@@ -875,7 +875,7 @@ int launch_delta_chunk(const DeltaShape& sh, const void* qkv, const float* a, co
         const uint64_t dims[2] = {(uint64_t)sh.off_b(), (uint64_t)rows};
         const uint64_t str[1] = {(uint64_t)sh.off_b() * 2};
         const uint32_t box[2] = {(uint32_t)cols, 67};
-        return make_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, qkv, dims, str, box, false);
+        return make_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, qkv, dims, str, box, 0);
     };
     B2_TRY(map(&mk, 64 * it.nd));
     B2_TRY(map(&mv, 64 * it.nv));

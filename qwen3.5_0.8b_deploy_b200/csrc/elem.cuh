@@ -45,6 +45,18 @@ template <typename T> __device__ __forceinline__ float times_sigmoid(float x, fl
 template <> __device__ __forceinline__ float times_sigmoid<float>(float x, float z) { return x / (1.0f + expf(-z)); }
 template <> __device__ __forceinline__ float times_sigmoid<__nv_bfloat16>(float x, float z) { return __fdividef(x, 1.0f + __expf(-z)); }
 
+// 0.5 z (1 + tanh y) = z / (1 + e^{-2y}), y = sqrt(2 / pi) (z + 0.044715 z^3)
+template <typename T>
+__device__ __forceinline__ float gelu_tanh(float z) {
+    return times_sigmoid<T>(z, 1.5957691216057308f * (z + 0.044715f * z * z * z));
+}
+
+template <typename T, int kAct>
+__device__ __forceinline__ float activated(float z) {
+    if constexpr (kAct == B200ATTN_ACT_SILU) return times_sigmoid<T>(z, z);
+    else return gelu_tanh<T>(z);
+}
+
 template <typename F>
 inline void dispatch_elem(ElemType t, F&& f) {
     if (t == ELEM_F32) f(float{});

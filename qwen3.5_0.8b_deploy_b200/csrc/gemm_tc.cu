@@ -231,11 +231,6 @@ constexpr uint32_t kResSmem = kResStages * kResStage + 256 + 1024;
 static_assert(128 * kResLd * 4 <= kResStages * kResStage, "the partial tile reuses the operand ring");
 static_assert(kHidden / kResBN == kRowsqParts, "one sum-of-squares part per output tile of the residual GEMM");
 
-__device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_smem_addr, uint32_t cta_rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta_rank));
-    return r;
-}
 __device__ __forceinline__ float4 dsmem_ld_f4(uint32_t addr) {
     float4 v;
     // not volatile: the loads of one thread are independent and may be issued as a batch; they cannot move above the
@@ -243,12 +238,6 @@ __device__ __forceinline__ float4 dsmem_ld_f4(uint32_t addr) {
     asm("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
-// Every thread of every CTA of the cluster (threads that have exited do not count).
-__device__ __forceinline__ void cluster_sync_all() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 template <int S>
 __global__ void __launch_bounds__(192)
 gemm_residual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int M, int N, int nk,
@@ -350,7 +339,7 @@ gemm_residual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         const uint32_t local = smem_u32(part + rrow * kResLd + rseg * kCols);
 #pragma unroll
         for (int sp = 0; sp < S; ++sp) {
-            const uint32_t remote = dsmem_addr(local, (uint32_t)sp);
+            const uint32_t remote = cluster_smem_addr(local, (uint32_t)sp);
 #pragma unroll
             for (int c4 = 0; c4 < kV4; ++c4) pv[sp][c4] = dsmem_ld_f4(remote + 16 * c4);
         }

@@ -9,6 +9,7 @@
 // [6144][3] with index 0 = newest.  Conv taps: w[d][3] * x_t + w[d][0] * x_{t-1} + w[d][1] * x_{t-2}
 // + w[d][2] * x_{t-3} (language_linear_attn.cpp:145-152).
 #include "kernels.cuh"
+#include "la_math.cuh"
 #include "ptx_utils.cuh"
 
 #include <algorithm>
@@ -21,13 +22,6 @@ __device__ __forceinline__ float warp_sum_f(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-// SiLU on the special-function unit (ex2.approx + rcp.approx, about 2 ulp): the sequence-form conv kernel evaluates it
-// 6144 times per token and is otherwise bound by these instructions, not by memory.
-__device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : logf(1.0f + expf(x)); }
-
 // ---- C1, sequence form -------------------------------------------------------------------------------
 // One warp per (run of up to kConvRun consecutive rows of one sequence, head, part) with part = q, k or v channels of the head: conv +
 // SiLU, L2 norm of q and k (eps inside the sqrt), q * 1/sqrt(128); the v warps also produce beta and the log-decay g.

@@ -90,11 +90,47 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, uint64
     while (!mbar_try_wait(bar, parity) && global_timer_ns() - t0 < limit_ns) {}
 }
 
+// The same without a memory fence: neither CTA goes on before the other has come this far.
+__device__ __forceinline__ void cluster_meet_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// Address of the same shared-memory location in CTA `rank` of the cluster, and an arrival on a barrier there.  The arrival orders what the
+// asynchronous units did (copies that this thread has seen land, TMEM reads behind their fence), not ordinary writes for a reader in the other CTA:
+// with .release.cluster it waits for those as well, which held a hand-over per 64-deep slice of a product to 0.8 us.
+__device__ __forceinline__ uint32_t cluster_smem_addr(uint32_t local_smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
+// Every thread of every CTA of the cluster (threads that have exited do not count).
+__device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Warp-uniform form for roles whose next instruction is warp-collective (.sync.aligned): either every
 // lane proceeds or every lane gives up.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     const bool r = mbar_wait(bar, parity, abort_flag);
     return __all_sync(0xffffffffu, r);
+}
+
+// One lane of a warp whose lanes are all here, always the same one.  Code that a whole warp walks through, with this around the issue of a copy or a
+// product alone, keeps addresses and descriptors in the warp's uniform registers, where those instructions read them.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
 }
 
 // ---- programmatic dependent launch ---------------------------------------------------------------------------

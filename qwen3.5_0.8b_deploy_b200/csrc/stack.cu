@@ -7,6 +7,7 @@
 // per-layer weights, prefill over token batches, a decode step for the whole batch, reset_cache, and a
 // graph-captured step (there: prefill, :391-479; here: decode with device-resident lengths and tokens).
 // The residual stream is fp32; GEMM operands are fp16 with fp32 accumulation (cuBLAS).
+#include "gemm_pair.cuh"
 #include "stack.cuh"
 #include "ptx_utils.cuh"
 
@@ -560,10 +561,14 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
         else
             launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, st->d_h, nullptr, st->d_post_norm[i], st->cfg.rms_eps, rows, st->d_xb, nullptr);
         B2_LAUNCH_CHECK();
-        B2_TRY(gemm_xwT(s, st->d_xb, true, st->d_wgu[i], true, st->d_gu, true, rows, 2 * inter, kHidden));
-        const size_t octs = (size_t)rows * inter / 8;
-        launch_pdl(swiglu_kernel, dim3((unsigned)((octs + 255) / 256)), dim3(256), 0, s, st->d_gu, inter, octs, st->d_act);
-        B2_LAUNCH_CHECK();
+        if (!decode && gemm_glu_takes(ELEM_F16, st->d_xb, st->d_wgu[i], st->d_act, rows, inter, kHidden)) {
+            B2_TRY(gemm_glu(s, ELEM_F16, B200ATTN_ACT_SILU, st->d_xb, st->d_wgu[i], st->d_act, rows, inter, kHidden, false, st->d_error));
+        } else {
+            B2_TRY(gemm_xwT(s, st->d_xb, true, st->d_wgu[i], true, st->d_gu, true, rows, 2 * inter, kHidden));
+            const size_t octs = (size_t)rows * inter / 8;
+            launch_pdl(swiglu_kernel, dim3((unsigned)((octs + 255) / 256)), dim3(256), 0, s, st->d_gu, inter, octs, st->d_act);
+            B2_LAUNCH_CHECK();
+        }
         B2_TRY(gemm_xwT(s, st->d_act, true, st->d_wdown[i], true, st->d_h, false, rows, kHidden, inter, 1.0f));
     }
     return 0;
