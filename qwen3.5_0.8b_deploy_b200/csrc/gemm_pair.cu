@@ -4,6 +4,9 @@
 // 0.94 GB each way.  Here the accumulators go through the function on their way out of TMEM while the tensor cores work on the next tile: 613 us (1.57
 // PFLOP/s, bound by the tensor cores' 512 cycles a slice and, over seconds, by the power limit) in place of 682 + 285 us.  fp16 products reach the function
 // unrounded; bf16 ones are rounded first, as the two kernels did: outputs of the layer-described stacks stay the same bit for bit.
+//   kPairConv   the DeltaNet input projection with the causal convolution, SiLU, L2 norms and gates behind it (fp16).  Here the channels of W are the
+//               rows of the product and the tokens its columns: a thread holds one channel and finds the taps of a token in its own registers.
+//               65536 rows 950 us (projection 878 and convolution 502 before, 3.2 GB between them), 3 x 333 23 (33), 9 x 466 67 (111), 45 14 (12).
 //
 // A cluster of two CTAs owns a 256 x 256 tile (cta_group::2, M = 256): each CTA fetches its 128 rows of both operands and holds 128 rows of the
 // result, so that an operand byte in shared memory serves twice the products that it would in a tile of one CTA.  Two accumulators of 256 columns
@@ -20,16 +23,28 @@
 namespace b200 {
 namespace {
 
-constexpr int kStages = 6;                              // ring of 64-deep slices, 32 KB each per CTA
 constexpr uint32_t kOperand = 128 * 128;                // 128 rows of 64 two-byte elements
 constexpr uint32_t kStage = 2 * kOperand;
 constexpr int kEpiWarps = 16;
-constexpr uint32_t kOutBytes = kEpiWarps * 2048;
-constexpr uint32_t kBars = kStages * kStage + kOutBytes;
-constexpr uint32_t kSmem = kBars + 256 + 1024;
 constexpr int kThreads = 32 * (kEpiWarps + 2);          // epilogue warps, one for loads, one for products (CTA 0) or the hand-over of slices (CTA 1)
 
-enum { kPairGlu = 0 };
+enum { kPairGlu = 0, kPairConv = 1 };
+constexpr int kConvTokens = 253;                        // of a tile of 256 columns: the first three are the taps of the fourth
+constexpr int kMaxSeqRows = 512;                        // first rows and slots of the sequences kept in shared memory, up to so many sequences
+
+template <int EPI>
+struct PairSmem {
+    static constexpr int kStages = EPI == kPairConv ? 5 : 6;               // ring of 64-deep slices, 32 KB each per CTA
+    static constexpr uint32_t kOut = kStages * kStage;                     // 2 KB per epilogue warp
+    static constexpr uint32_t kExtra = kOut + kEpiWarps * 2048;            // kPairConv: the tables of conv_part
+    static constexpr uint32_t kBars = kExtra + (EPI == kPairConv ? 4096 + 4096 + 2048 + 8 * kMaxSeqRows : 0);
+    static constexpr int kReaders = EPI == kPairConv ? kEpiWarps / 2 : kEpiWarps;     // epilogue warps of one tile
+    static constexpr uint32_t kBytes = kBars + 256 + 1024;
+};
+struct PairMaps {
+    CUtensorMap a, b, b32;         // operands: rows of the product, its columns, those in boxes of 32 rows
+    CUtensorMap out[4];            // results: kPairGlu one, kPairConv q, k, v, mixed
+};
 
 struct PairArgs {
     int row_tiles, col_tiles;      // tiles of X rows and of W rows
@@ -39,6 +54,7 @@ struct PairArgs {
     int rows, cols;                // of the result
     int up;                        // kPairGlu: W row of the first up column (0: groups of 32 gate and 32 up rows)
     int* error;
+    LaConvArgs la;                 // kPairConv
 };
 
 // One unit of work: a tile, or a part of it `width` columns of the product wide.
@@ -95,14 +111,215 @@ __device__ __forceinline__ void glu_part(const PairArgs& p, const CUtensorMap* m
         tma_store_2d(map_y, out_smem, col, row);
         bulk_commit_group();
     }
+    __syncwarp();
+}
+
+// What the convolution has to know of a token: place in its sequence's rows of this call, up to 3, and rows behind it, up to 3.
+constexpr int kTokenPlain = 15, kTokenNone = 16;
+__device__ __forceinline__ int sequence_of(const LaConvArgs& a, const int* first_rows, int t) {
+    int lo = 0, hi = a.n_seqs - 1;                       // the last sequence that starts at or before row t (empty ones start where the next does)
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if ((a.n_seqs <= kMaxSeqRows ? first_rows[mid] : a.seqs[mid].row0) <= t) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+__device__ __forceinline__ int slot_of(const LaConvArgs& a, const int* first_rows, int t) {
+    const int i = sequence_of(a, first_rows, t);
+    return a.n_seqs <= kMaxSeqRows ? first_rows[kMaxSeqRows + i] : a.seqs[i].slot;
+}
+__device__ __forceinline__ int token_info(const LaConvArgs& a, const int* first_rows, int rows, int t) {
+    if (t < 0 || t >= rows) return kTokenNone;
+    const int i = sequence_of(a, first_rows, t), row0 = a.n_seqs <= kMaxSeqRows ? first_rows[i] : a.seqs[i].row0;
+    const int next = i + 1 == a.n_seqs ? rows : a.n_seqs <= kMaxSeqRows ? first_rows[i + 1] : a.seqs[i + 1].row0;
+    return min(next - 1 - t, 3) << 2 | min(t - row0, 3);
+}
+
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Taps of four tokens, the newest one's weight last in the reference's order, and SiLU.
+__device__ __forceinline__ float conv_tap(const float4& w, float x0, float x1, float x2, float x3) {
+    float y = w.w * x0;
+    y += w.x * x1;
+    y += w.y * x2;
+    y += w.z * x3;
+    return silu_sfu(y);
+}
+
+// Sum over the lanes of v[j]^2, token j's in lane j: every step halves the tokens that a lane still carries.
+__device__ __forceinline__ float squares_by_token(const float (&v)[32], int lane) {
+    float s[16];
+    const bool up16 = lane & 16;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const float keep = up16 ? v[j + 16] : v[j], give = up16 ? v[j] : v[j + 16];
+        s[j] = keep * keep + __shfl_xor_sync(0xffffffffu, give * give, 16);
+    }
+#pragma unroll
+    for (int n = 8; n > 0; n >>= 1) {
+        const bool up = lane & n;
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+            const float keep = up ? s[j + n] : s[j], give = up ? s[j] : s[j + n];
+            s[j] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+        }
+    }
+    return s[0];
+}
+
+// This warp's 32 channels and 128 tokens of a tile, 32 tokens at a time.  `info`: of the tile's 256 tokens; `sums`: 2 x 4 x 32 floats shared by the
+// four warps of these tokens (all 128 channels of a head), which meet at barrier `bar`; `scale`: 32 floats of this warp; `stage`: its 2 KB, from where TMA
+// writes the results (stores of 2 bytes a lane straight to memory took 4.4 cycles each of the SM's one load / store unit).  Without `ok` it only keeps
+// its place at the barriers.
+template <typename Release>
+__device__ __forceinline__ void conv_part(const LaConvArgs& a, const PairMaps& maps, bool ok, uint32_t acc, int tile, int t_tile, int rows, int rank, int q, int part,
+                                          int lane, const int* info, const int* first_rows, float* sums, int bar, float* scale, unsigned char* stage,
+                                          Release&& release) {
+    const int ch = tile * 256 + rank * 128 + 32 * q + lane, kind = min(tile >> 3, 3);       // 0 q, 1 k, 2 v, 3 z and (tile 32) the gates' inputs
+    const bool wanted = ok && ch - lane < kLaProjCols;
+    float* raw = reinterpret_cast<float*>(stage);
+    if (kind == 3) {
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {
+            const int col = 128 * part + 16 * c, t0 = t_tile + col;
+            const bool live = wanted && t0 < rows;
+            uint32_t r[16];
+            if (live) {
+                tmem_ld16(acc + col, r);
+                tmem_wait_ld();
+            }
+            if (c == 7) release();
+            if (!live) continue;
+            if (col == 0) {                              // its first three tokens are the tile's before
+                float* dst = a.mixed + (long long)t0 * kLaProjCols + ch;
+#pragma unroll
+                for (int j = 3; j < 16; ++j)
+                    if (t0 + j < rows) dst[(long long)j * kLaProjCols] = __uint_as_float(r[j]);
+                continue;
+            }
+            if (lane == 0) bulk_wait_group_read0();
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) raw[32 * j + lane] = __uint_as_float(r[j]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_2d(&maps.out[3], smem_u32(stage), ch, t0);
+                bulk_commit_group();
+            }
+            __syncwarp();
+        }
+        return;
+    }
+    const float4 w = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch * kLaConvK);
+    float h[3] = {0.f, 0.f, 0.f};                        // the three tokens in front, oldest first
+    if (ok && part > 0) {
+        uint32_t r[4];
+        tmem_ld4(acc + 128 * part - 4, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 3; ++i) h[i] = __uint_as_float(r[i + 1]);
+    }
+    const int out_ch = (tile & 7) * 256 + rank * 128 + 32 * q;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        const int col = 128 * part + 32 * c, t0 = t_tile + col;
+        const bool live = wanted && t0 < rows;           // the same for all warps of these tokens
+        float v[32];
+        if (live) {
+            uint32_t r[32];
+            tmem_ld32(acc + col, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        }
+        if (c == 3) release();
+        if (live) {
+            const float last[3] = {v[29], v[30], v[31]};
+            const int f = info[col + lane];
+            const unsigned tails = __ballot_sync(0xffffffffu, f < 12 && col + lane >= 3);               // of their sequence's last three rows
+            const unsigned starts = __ballot_sync(0xffffffffu, f < kTokenNone && (f & 3) < 3);          // of its first three
+            if (tails) {
+                float* dst = a.mixed + (long long)t0 * kLaProjCols + ch;
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (tails >> j & 1) dst[(long long)j * kLaProjCols] = v[j];
+            }
+            if (starts == 0) {
+#pragma unroll
+                for (int j = 31; j >= 3; --j) v[j] = conv_tap(w, v[j], v[j - 1], v[j - 2], v[j - 3]);
+                v[2] = conv_tap(w, v[2], v[1], v[0], h[2]);
+                v[1] = conv_tap(w, v[1], v[0], h[2], h[1]);
+                v[0] = conv_tap(w, v[0], h[2], h[1], h[0]);
+            } else {
+                int of = -1;                             // first row of the sequence whose last inputs are in s0 (oldest) .. s2
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+#pragma unroll
+                for (int j = 31; j >= 0; --j) {
+                    float x1 = j >= 1 ? v[j >= 1 ? j - 1 : 0] : h[2], x2 = j >= 2 ? v[j >= 2 ? j - 2 : 0] : h[j == 1 ? 2 : 1];
+                    float x3 = j >= 3 ? v[j >= 3 ? j - 3 : 0] : h[j < 3 ? j : 0];
+                    if (starts >> j & 1) {
+                        const int pos = info[col + j] & 3, first = t0 + j - pos;
+                        if (first != of) {
+                            of = first;
+                            const float* st = a.conv_state + (size_t)slot_of(a, first_rows, t0 + j) * a.conv_stride + ch;
+                            s0 = st[0]; s1 = st[kLaConvDim]; s2 = st[2 * kLaConvDim];
+                        }
+                        x3 = pos == 0 ? s0 : pos == 1 ? s1 : s2;
+                        if (pos < 2) x2 = pos == 0 ? s1 : s2;
+                        if (pos < 1) x1 = s2;
+                    }
+                    v[j] = conv_tap(w, v[j], x1, x2, x3);
+                }
+            }
+            h[0] = last[0]; h[1] = last[1]; h[2] = last[2];
+        }
+        if (kind < 2) {
+            float* sum = sums + (c & 1) * 128;
+            if (live) sum[32 * q + lane] = squares_by_token(v, lane);
+            bar_sync(bar, 128);
+            if (live) {
+                const float ss = (sum[lane] + sum[32 + lane]) + (sum[64 + lane] + sum[96 + lane]);
+                scale[lane] = (kind == 0 ? 1.0f / sqrtf((float)kLaKd) : 1.0f) / sqrtf(ss + 1e-6f);
+                __syncwarp();
+#pragma unroll
+                for (int j4 = 0; j4 < 8; ++j4) {
+                    const float4 s4 = *reinterpret_cast<const float4*>(scale + 4 * j4);
+                    v[4 * j4] *= s4.x; v[4 * j4 + 1] *= s4.y; v[4 * j4 + 2] *= s4.z; v[4 * j4 + 3] *= s4.w;
+                }
+            }
+        }
+        if (!live) continue;
+        if (col == 0) {                                  // without the tile's first three tokens, which are the tile's before
+            __half* dst = (kind == 0 ? a.q : kind == 1 ? a.k : a.v) + (long long)t0 * (kLaHeads * kLaKd) + out_ch + lane;
+#pragma unroll
+            for (int j = 3; j < 32; ++j)
+                if (t0 + j < rows) dst[j * (kLaHeads * kLaKd)] = __float2half_rn(v[j]);
+            continue;
+        }
+        if (lane == 0) bulk_wait_group_read0();
+        __syncwarp();
+        __half* out = reinterpret_cast<__half*>(stage);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) out[32 * j + lane] = __float2half_rn(v[j]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(&maps.out[kind], smem_u32(stage), out_ch, t0);
+            bulk_commit_group();
+        }
+        __syncwarp();
+    }
 }
 
 // grid 2 x pairs, clusters of two.  Rank 0 of a pair issues the products once its own slice and its neighbour's have landed; the neighbour's
-// product warp passes that on (its loads signal its own barrier).  map_w32: boxes of 32 rows, for the narrower parts.
+// product warp passes that on (its loads signal its own barrier).  Operand a gives the rows of the product (X, kPairConv: W), b its columns.
 template <int EPI, typename T, int kAct>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w32,
-                 const __grid_constant__ CUtensorMap map_y, const PairArgs p) {
+gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
+    using Smem = PairSmem<EPI>;
+    constexpr int kStages = Smem::kStages;
+    constexpr uint32_t kBars = Smem::kBars;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -125,8 +342,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         mbar_init(acc_full(0), 1);
         mbar_init(acc_full(1), 1);
-        mbar_init(acc_empty(0), 2 * kEpiWarps);
-        mbar_init(acc_empty(1), 2 * kEpiWarps);
+        mbar_init(acc_empty(0), 2 * Smem::kReaders);
+        mbar_init(acc_empty(1), 2 * Smem::kReaders);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -134,7 +351,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         tmem_alloc_pair(smem_u32(tmem_slot), 512);
         tmem_relinquish_pair();
     }
-    if (warp == kEpiWarps && lane == 0) { tma_prefetch_desc(&map_x); tma_prefetch_desc(&map_w); tma_prefetch_desc(&map_w32); tma_prefetch_desc(&map_y); }
+    if (warp == kEpiWarps && lane == 0) { 
+        tma_prefetch_desc(&maps.a);
+        tma_prefetch_desc(&maps.b);
+        tma_prefetch_desc(&maps.out[0]);
+    }
     const PairItem first(p, pair);
     tc_fence_before();
     __syncthreads();
@@ -153,25 +374,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         PairItem w = first;
         for (int t = pair; t < p.items && ok; t += pairs) {
             if (t != pair) w = PairItem(p, t);
-            const int x_row = w.row * 256 + rank * 128;
-            const int w_row = p.up ? w.col / 2 + rank * p.up : w.col + rank * w.width / 2;
+            const int a_row = (EPI == kPairConv ? w.col : w.row * 256) + rank * 128;
+            const int b_row = EPI == kPairConv ? w.row * kConvTokens - 3 + rank * 128 : p.up ? w.col / 2 + rank * p.up : w.col + rank * w.width / 2;
             const uint32_t bytes = kOperand + w.width * 64;
             for (int k = 0; k < 64 * p.k_steps; k += 64) {
                 if (!mbar_wait_warp(empty(s), parity, abort_flag)) { ok = false; break; }
                 const uint32_t dst = base + s * kStage, bar = full(s);
                 if (elect_one()) {
                     mbar_arrive_expect_tx(bar, bytes);
-                    tma_load_2d(dst, &map_x, bar, k, x_row);
-                    if (w.width == 256) tma_load_2d(dst + kOperand, &map_w, bar, k, w_row);
+                    tma_load_2d(dst, &maps.a, bar, k, a_row);
+                    if (w.width == 256) tma_load_2d(dst + kOperand, &maps.b, bar, k, b_row);
                     else
-                        for (int r = 0; r < w.width / 2; r += 32) tma_load_2d(dst + kOperand + r * 128, &map_w32, bar, k, w_row + r);
+                        for (int r = 0; r < w.width / 2; r += 32) tma_load_2d(dst + kOperand + r * 128, &maps.b32, bar, k, b_row + r);
                 }
                 ++issued;
                 if (++s == kStages) { s = 0; parity ^= 1; }
             }
         }
-        if (!ok && lane == 0)
-            for (int j = max(0, issued - kStages); j < issued; ++j) mbar_drain(full(j % kStages), (j / kStages) & 1);
+        // A copy or an arrival of the neighbour's that is still under way must not find this CTA gone.
+        if (lane == 0)
+            for (int j = max(0, issued - kStages); j < issued; ++j) {
+                if (!ok) mbar_drain(full(j % kStages), (j / kStages) & 1);
+                else mbar_wait(empty(j % kStages), (j / kStages) & 1, abort_flag);
+            }
     } else if (warp == kEpiWarps + 1) {
         int s = 0;
         uint32_t parity = 0;
@@ -185,7 +410,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const int b = i & 1;
                 if (t != pair) w = PairItem(p, t);
                 const uint32_t idesc = umma_idesc(fmt, 256, w.width, 0, 0);
-                if (!mbar_wait_warp(acc_empty(b), ((i >> 1) & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_warp(acc_empty(b), ((i >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d = tmem + b * 256;
                 for (int ks = 0; ks < p.k_steps; ++ks) {
@@ -203,6 +428,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 if (ok && elect_one()) umma_commit_pair(acc_full(b));
             }
+            for (int j = max(0, i - 2); ok && j < i; ++j) ok = mbar_wait_warp(acc_empty(j & 1), (j >> 1) & 1, abort_flag);     // the neighbour's arrivals
         } else {
             const uint32_t theirs = cluster_smem_addr(full(0), 0);
             for (int left = (p.items - pair + pairs - 1) / pairs * p.k_steps; left > 0; --left) {
@@ -213,21 +439,51 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
     } else {
         const int q = warp & 3, part = warp >> 2;          // TMEM lanes 32 q .. 32 q + 31, a quarter of the columns
-        unsigned char* out = sm + kStages * kStage + warp * 2048;
-        const uint32_t out_smem = base + kStages * kStage + warp * 2048;
-        int i = 0;
-        for (int t = pair; t < p.items; t += pairs, ++i) {
+        unsigned char* out = sm + Smem::kOut + warp * 2048;
+        const uint32_t out_smem = base + Smem::kOut + warp * 2048;
+        // kPairConv: the two halves of these warps take turns at the tiles.  One half's special functions then run beside the other's shuffles, loads
+        // and stores; all on one tile went through them in step.
+        int i = EPI == kPairConv ? warp >> 3 : 0;
+        bool ok = true;
+        if constexpr (EPI == kPairConv) {
+            int* first_rows = reinterpret_cast<int*>(sm + Smem::kExtra + 10240);
+            for (int j = threadIdx.x; j < min(p.la.n_seqs, kMaxSeqRows); j += 32 * kEpiWarps) {
+                first_rows[j] = p.la.seqs[j].row0;
+                first_rows[kMaxSeqRows + j] = p.la.seqs[j].slot;
+            }
+            __syncwarp();
+            bar_sync(1, 32 * kEpiWarps);
+        }
+        for (int t = pair + i * pairs; t < p.items; t += EPI == kPairConv ? 2 * pairs : pairs, i += EPI == kPairConv ? 2 : 1) {
             const int b = i & 1;
             const PairItem w = t == pair ? first : PairItem(p, t);
-            if (!mbar_wait_warp(acc_full(b), (i >> 1) & 1, abort_flag)) break;
-            tc_fence_after();
+            auto release = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(cluster_smem_addr(acc_empty(b), 0));
+            };
             const uint32_t acc = tmem + b * 256 + ((uint32_t)(32 * q) << 16);
-            if (64 * part < w.width)
-                glu_part<T, kAct>(p, &map_y, acc + (p.up ? 32 : 64) * part, acc + (p.up ? 32 * part + w.width / 2 : 64 * part + 32), out_smem, out,
-                                  w.row * 256 + rank * 128 + 32 * q, w.col / 2 + 32 * part, lane);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(cluster_smem_addr(acc_empty(b), 0));
+            if constexpr (EPI == kPairConv) {
+                const int half = b, side = part & 1;                           // these warps' half, and their half of the tokens
+                int* info = reinterpret_cast<int*>(sm + Smem::kExtra) + (2 * half + (i >> 1 & 1)) * 256;
+                float* sums = reinterpret_cast<float*>(sm + Smem::kExtra + 4096) + (2 * half + side) * 256;
+                float* scale = reinterpret_cast<float*>(sm + Smem::kExtra + 8192) + 32 * warp;
+                const int* first_rows = reinterpret_cast<const int*>(sm + Smem::kExtra + 10240);
+                const int t_tile = w.row * kConvTokens - 3, mine = threadIdx.x & 255;
+                info[mine] = token_info(p.la, first_rows, p.rows, t_tile + mine);
+                __syncwarp();
+                bar_sync(2 + half, 256);
+                ok = ok && mbar_wait_warp(acc_full(b), (i >> 1) & 1, abort_flag);
+                tc_fence_after();
+                conv_part(p.la, maps, ok, acc, w.col >> 8, t_tile, p.rows, rank, q, side, lane, info, first_rows, sums, 4 + 2 * half + side, scale, out, release);
+            } else {
+                if (!mbar_wait_warp(acc_full(b), (i >> 1) & 1, abort_flag)) break;
+                tc_fence_after();
+                if (64 * part < w.width)
+                    glu_part<T, kAct>(p, &maps.out[0], acc + (p.up ? 32 : 64) * part, acc + (p.up ? 32 * part + w.width / 2 : 64 * part + 32), out_smem, out,
+                                      w.row * 256 + rank * 128 + 32 * q, w.col / 2 + 32 * part, lane);
+                release();
+            }
         }
         if (lane == 0) bulk_wait_group0();
     }
@@ -242,20 +498,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 }
 
 template <int EPI, typename T, int kAct>
-int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mw32, const CUtensorMap& my, PairArgs p, cudaStream_t s) {
+int launch_pair(const PairMaps& maps, PairArgs p, cudaStream_t s) {
     static PerDeviceOnce once;
-    B2_PER_DEVICE_ONCE(once, B2_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<EPI, T, kAct>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)));
+    B2_PER_DEVICE_ONCE(once, B2_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<EPI, T, kAct>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<EPI>::kBytes)));
     int sms = 0;
     B2_TRY(device_sm_count(&sms));
     cudaLaunchConfig_t cfg = {};
     // Whole rounds of tiles, then the rest in parts as narrow as it takes to give every pair one (at least 64 columns).
     const int tiles = p.row_tiles * p.col_tiles, pairs = sms / 2, rest = tiles % pairs;
-    p.split_log2 = rest == 0 ? 0 : rest * 4 <= pairs ? 2 : rest * 2 <= pairs ? 1 : 0;
+    p.split_log2 = rest == 0 || EPI == kPairConv ? 0 : rest * 4 <= pairs ? 2 : rest * 2 <= pairs ? 1 : 0;
     p.whole = tiles - rest;
     p.items = p.whole + (rest << p.split_log2);
     cfg.gridDim = dim3(2 * std::min(p.items, pairs));
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmem;
+    cfg.dynamicSmemBytes = PairSmem<EPI>::kBytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -264,16 +520,17 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap&
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_flags.pdl ? 2 : 1;
-    B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, T, kAct>, mx, mw, mw32, my, p));
+    B2_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, T, kAct>, maps, p));
     count_launch();
     return 0;
 }
 
-// [rows, cols] of two-byte elements, row pitch = cols, in boxes of 64 or (results) 32 columns
-int map_rows(CUtensorMap* m, ElemType t, const void* p, long long rows, int cols, int box_cols, int box_rows) {
-    const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows}, str[1] = {(uint64_t)cols * 2};
+// [rows, cols] row-major, in boxes of so many columns and rows; a swizzle as wide as the box for operands and (64 bytes) results of kPairGlu
+int map_rows(CUtensorMap* m, ElemType t, const void* p, long long rows, int cols, int box_cols, int box_rows, bool swizzle = true) {
+    const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows}, str[1] = {(uint64_t)cols * elem_bytes(t)};
     const uint32_t box[2] = {(uint32_t)box_cols, (uint32_t)box_rows};
-    return make_tensor_map(m, t == ELEM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p, dims, str, box, box_cols * 2);
+    return make_tensor_map(m, t == ELEM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : t == ELEM_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+                           p, dims, str, box, swizzle ? box_cols * 2 : 0);
 }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -286,11 +543,11 @@ bool gemm_glu_takes(ElemType t, const void* x, const void* w, const void* act, i
 }
 
 int gemm_glu(cudaStream_t s, ElemType t, int act_kind, const void* x, const void* w, void* act, int rows, int ff, int K, bool split, int* error) {
-    CUtensorMap mx, mw, mw32, my;
-    B2_TRY(map_rows(&mx, t, x, rows, K, 64, 128));
-    B2_TRY(map_rows(&mw, t, w, 2LL * ff, K, 64, 128));
-    B2_TRY(map_rows(&mw32, t, w, 2LL * ff, K, 64, 32));
-    B2_TRY(map_rows(&my, t, act, rows, ff, 32, 32));
+    PairMaps m{};
+    B2_TRY(map_rows(&m.a, t, x, rows, K, 64, 128));
+    B2_TRY(map_rows(&m.b, t, w, 2LL * ff, K, 64, 128));
+    B2_TRY(map_rows(&m.b32, t, w, 2LL * ff, K, 64, 32));
+    B2_TRY(map_rows(&m.out[0], t, act, rows, ff, 32, 32));
     PairArgs p{};
     p.row_tiles = ceil_div(rows, 256);
     p.col_tiles = ceil_div(ff, 128);
@@ -299,9 +556,29 @@ int gemm_glu(cudaStream_t s, ElemType t, int act_kind, const void* x, const void
     p.cols = ff;
     p.up = split ? ff : 0;
     p.error = error;
-    if (t == ELEM_F16) return launch_pair<kPairGlu, __half, B200ATTN_ACT_SILU>(mx, mw, mw32, my, p, s);
-    if (act_kind == B200ATTN_ACT_SILU) return launch_pair<kPairGlu, __nv_bfloat16, B200ATTN_ACT_SILU>(mx, mw, mw32, my, p, s);
-    return launch_pair<kPairGlu, __nv_bfloat16, B200ATTN_ACT_GELU_TANH>(mx, mw, mw32, my, p, s);
+    if (t == ELEM_F16) return launch_pair<kPairGlu, __half, B200ATTN_ACT_SILU>(m, p, s);
+    if (act_kind == B200ATTN_ACT_SILU) return launch_pair<kPairGlu, __nv_bfloat16, B200ATTN_ACT_SILU>(m, p, s);
+    return launch_pair<kPairGlu, __nv_bfloat16, B200ATTN_ACT_GELU_TANH>(m, p, s);
+}
+
+bool gemm_la_conv_takes(const void* x, const void* w) { return aligned16(x) && aligned16(w); }
+
+int gemm_la_conv(cudaStream_t s, const __half* x, const __half* w, int rows, const LaConvArgs& la, int* error) {
+    PairMaps m{};
+    B2_TRY(map_rows(&m.a, ELEM_F16, w, kLaProjCols, kHidden, 64, 128));
+    B2_TRY(map_rows(&m.b, ELEM_F16, x, rows, kHidden, 64, 128));
+    __half* const out[3] = {la.q, la.k, la.v};
+    for (int i = 0; i < 3; ++i) B2_TRY(map_rows(&m.out[i], ELEM_F16, out[i], rows, kLaHeads * kLaKd, 32, 32, false));
+    B2_TRY(map_rows(&m.out[3], ELEM_F32, la.mixed, rows, kLaProjCols, 32, 16, false));
+    PairArgs p{};
+    p.row_tiles = ceil_div(rows, kConvTokens);
+    p.col_tiles = ceil_div(kLaProjCols, 256);
+    p.k_steps = kHidden / 64;
+    p.rows = rows;
+    p.cols = kLaProjCols;
+    p.error = error;
+    p.la = la;
+    return launch_pair<kPairConv, __half, B200ATTN_ACT_SILU>(m, p, s);
 }
 
 }  // namespace b200

@@ -1,7 +1,7 @@
 // Prompt-sized products on pairs of CTAs with their element-wise successor in the epilogue (gemm_pair.cu).
 #pragma once
 
-#include "common.cuh"
+#include "kernels.cuh"
 
 namespace b200 {
 
@@ -9,5 +9,20 @@ namespace b200 {
 // rows.  f: act_kind (B200ATTN_ACT_*); SiLU for fp16.
 bool gemm_glu_takes(ElemType t, const void* x, const void* w, const void* act, int rows, int ff, int K);
 int gemm_glu(cudaStream_t s, ElemType t, int act_kind, const void* x, const void* w, void* act, int rows, int ff, int K, bool split, int* error);
+
+// The DeltaNet input projection of prompts with its convolution: X[rows, 1024] W[8224, 1024]^T, then for every token q, k, v (conv + SiLU, L2 norms,
+// q / sqrt(128)) as fp16; z and the gates' inputs go to their columns of mixed [rows, 8224], and so do the unconvolved q, k, v of each sequence's last
+// three rows (launch_la_conv_tail).  The sequences' rows follow one another without gaps.
+struct LaConvArgs {
+    const LaSeqMeta* seqs;
+    int n_seqs;
+    const float* conv_state;       // of the layer, conv_stride floats a slot
+    size_t conv_stride;
+    const float* conv_w;
+    __half *q, *k, *v;
+    float* mixed;
+};
+bool gemm_la_conv_takes(const void* x, const void* w);
+int gemm_la_conv(cudaStream_t s, const __half* x, const __half* w, int rows, const LaConvArgs& la, int* error);
 
 }  // namespace b200

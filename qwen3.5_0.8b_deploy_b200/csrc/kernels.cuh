@@ -82,8 +82,8 @@ constexpr size_t kLaSplitBytes = 90112;  // of a chunk and head
 int launch_la_chunk_tc(const __half* q_h, const __half* k_h, const __half* v_h, const float* g, const float* beta,
                        const LaSeqMeta* d_seqs, int n_seqs, int rows, float* rec_layer, size_t rec_stride, float* out,
                        int* d_error, const LaSplit& split, cudaStream_t s);
-int launch_la_conv_state_update(const float* mixed, const LaSeqMeta* d_seqs, int n_seqs, float* conv_layer,
-                                size_t conv_stride, cudaStream_t s);
+int launch_la_conv_tail(const float* mixed, const LaSeqMeta* d_seqs, int n_seqs, float* conv_layer, size_t conv_stride, int gate_rows, const float* a_log,
+                        const float* dt_bias, float* g, float* beta, cudaStream_t s);
 int launch_la_recurrent_serial(const float* q, const float* k, const float* v, const float* g, const float* beta,
                                const LaSeqMeta* d_seqs, int n_seqs, float* rec_layer, size_t rec_stride, float* out,
                                cudaStream_t s);

@@ -23,6 +23,7 @@ __device__ __forceinline__ float warp_sum_f(float v) {
     return v;
 }
 // ---- C1, sequence form -------------------------------------------------------------------------------
+// For fp32 projections and the serial recurrence; the fp16 layers convolve in the epilogue of their projection (gemm_pair.cu).
 // One warp per (run of up to kConvRun consecutive rows of one sequence, head, part) with part = q, k or v channels of the head: conv +
 // SiLU, L2 norm of q and k (eps inside the sqrt), q * 1/sqrt(128); the v warps also produce beta and the log-decay g.
 // A warp requests its whole input window (the run's rows plus three rows of history, 16 bytes per lane and row) before
@@ -134,9 +135,20 @@ la_conv_seq_kernel(const float* __restrict__ mixed, const LaRun* __restrict__ ru
     }
 }
 
-// Conv state after a chunk: the last three inputs of the sequence. grid (n_seqs, 6144/256), block 256.
-__global__ void la_conv_state_update_kernel(const float* __restrict__ mixed, const LaSeqMeta* __restrict__ seqs,
-                                            float* __restrict__ conv_state_layer, size_t conv_stride_slot) {
+// Conv state after a chunk: the last three inputs of the sequence. grid (n_seqs, 6144/256), block 256.  With gate_rows > 0 the blocks behind those
+// of the sequences (rows of the grid from n_seqs on) also turn the projections a and b of 16 x 6144/256 rows each into log-decay and beta.
+__global__ void __launch_bounds__(256)
+la_conv_tail_kernel(const float* __restrict__ mixed, const LaSeqMeta* __restrict__ seqs, int n_seqs, float* __restrict__ conv_state_layer,
+                    size_t conv_stride_slot, int gate_rows, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                    float* __restrict__ g_out, float* __restrict__ beta_out) {
+    if (blockIdx.x >= n_seqs) {
+        const int row = ((blockIdx.x - n_seqs) * gridDim.y + blockIdx.y) * 16 + (threadIdx.x >> 4), h = threadIdx.x & 15;
+        if (row >= gate_rows) return;
+        const float a = mixed[(size_t)row * kLaProjCols + kLaAOff + h], b = mixed[(size_t)row * kLaProjCols + kLaBOff + h];
+        beta_out[(size_t)row * kLaHeads + h] = sigmoid_f(b);
+        g_out[(size_t)row * kLaHeads + h] = -expf(a_log[h]) * softplus_f(a + dt_bias[h]);
+        return;
+    }
     const LaSeqMeta sm = seqs[blockIdx.x];
     const int d = blockIdx.y * blockDim.x + threadIdx.x;
     if (d >= kLaConvDim || sm.count <= 0) return;
@@ -401,10 +413,11 @@ int launch_la_conv_seq(const float* mixed, const LaRun* d_runs, int n_runs, cons
     B2_LAUNCH_CHECK();
     return 0;
 }
-int launch_la_conv_state_update(const float* mixed, const LaSeqMeta* d_seqs, int n_seqs, float* conv_layer,
-                                size_t conv_stride, cudaStream_t s) {
-    dim3 grid(n_seqs, kLaConvDim / 256);
-    la_conv_state_update_kernel<<<grid, 256, 0, s>>>(mixed, d_seqs, conv_layer, conv_stride);
+int launch_la_conv_tail(const float* mixed, const LaSeqMeta* d_seqs, int n_seqs, float* conv_layer, size_t conv_stride, int gate_rows, const float* a_log,
+                        const float* dt_bias, float* g, float* beta, cudaStream_t s) {
+    constexpr int kCols = kLaConvDim / 256;
+    la_conv_tail_kernel<<<dim3(n_seqs + ceil_div(gate_rows, 16 * kCols), kCols), 256, 0, s>>>(mixed, d_seqs, n_seqs, conv_layer, conv_stride, gate_rows, a_log,
+                                                                                            dt_bias, g, beta);
     B2_LAUNCH_CHECK();
     return 0;
 }

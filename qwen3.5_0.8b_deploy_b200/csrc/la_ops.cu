@@ -3,6 +3,7 @@
 // Mirrors qwen::cuda::CudaLinearAttention / CudaLinearAttentionV2 / CudaLinearAttnState
 // (src/backend/cuda/kernels/linear_attention_cuda.cu:266-326,412-684, linear_attention_v2.cu:734-883 in
 // the reference).
+#include "gemm_pair.cuh"
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -385,15 +386,23 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
     int n_runs = 0;
     LaSplit split;
     const bool tc = la_use_tensor_cores();
-    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, &d_runs, &n_runs, tc ? &split : nullptr, s));
+    const bool fused = tc && fp16 && gemm_la_conv_takes(x_is_fp16 ? d_x : la->d_xb, la->d_win_fp16);
+    B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, fused ? nullptr : &d_runs, &n_runs, tc ? &split : nullptr, s));
     if (rows == 0) return 0;
     B2_CHECK_ARG(rows <= la->cfg.max_prefill_rows, "la_prefill: %d rows exceed max_prefill_rows %d", rows, la->cfg.max_prefill_rows);
-    B2_TRY(project_in(rows));
-    B2_TRY(launch_la_conv_seq(la->d_mixed, d_runs, n_runs, d_seqs, conv_layer, st->conv_stride_slot(), la->d_conv_w, la->d_a_log,
-                              la->d_dt_bias, tc ? nullptr : la->d_q, tc ? nullptr : la->d_k, tc ? la->d_qh : nullptr,
-                              tc ? la->d_kh : nullptr, tc ? nullptr : la->d_v, tc ? la->d_vh : nullptr, la->d_g, la->d_beta, s));
+    if (fused) {
+        const void* xb = d_x;
+        if (!x_is_fp16) { B2_TRY(f32_to_f16(s, (const float*)d_x, la->d_xb, (size_t)rows * kHidden)); xb = la->d_xb; }
+        B2_TRY(gemm_la_conv(s, (const __half*)xb, la->d_win_fp16, rows,
+                            LaConvArgs{d_seqs, n_seqs, conv_layer, st->conv_stride_slot(), la->d_conv_w, la->d_qh, la->d_kh, la->d_vh, la->d_mixed}, la->d_error));
+    } else {
+        B2_TRY(project_in(rows));
+        B2_TRY(launch_la_conv_seq(la->d_mixed, d_runs, n_runs, d_seqs, conv_layer, st->conv_stride_slot(), la->d_conv_w, la->d_a_log,
+                                  la->d_dt_bias, tc ? nullptr : la->d_q, tc ? nullptr : la->d_k, tc ? la->d_qh : nullptr,
+                                  tc ? la->d_kh : nullptr, tc ? nullptr : la->d_v, tc ? la->d_vh : nullptr, la->d_g, la->d_beta, s));
+    }
+    B2_TRY(launch_la_conv_tail(la->d_mixed, d_seqs, n_seqs, conv_layer, st->conv_stride_slot(), fused ? rows : 0, la->d_a_log, la->d_dt_bias, la->d_g, la->d_beta, s));
     B2_TRY(la_recurrence(la, st, layer, la->d_q, la->d_k, la->d_v, la->d_g, la->d_beta, d_seqs, n_seqs, rows, la->d_core, tc, split, s));
-    B2_TRY(launch_la_conv_state_update(la->d_mixed, d_seqs, n_seqs, conv_layer, st->conv_stride_slot(), s));
     B2_TRY(launch_la_gated_norm(la->d_core, la->d_mixed, la->d_norm, rows, la->d_gated, fp16, s));
     return project_out(rows);
 }

@@ -1,5 +1,5 @@
-"""GPU: prompt-sized products on pairs of CTAs with their successor in the epilogue, at the edges of their tiles (256 rows, 128 outputs, parts of 32) and of
-their dispatch (more than 128 rows)."""
+"""GPU: prompt-sized products on pairs of CTAs with their successor in the epilogue, at the edges of their tiles (feed-forward: 256 rows, 128 outputs, parts
+of 32; DeltaNet projection: 253 tokens behind 3 that only serve as taps, 32 at a time) and of their dispatch (feed-forward: more than 128 rows)."""
 import os
 import sys
 
@@ -47,3 +47,50 @@ def test_feed_forward_widths(cuda, models, wts, ff, width, rows):      # noqa: F
         c.stack.begin_batching()
         row = c.stack.open(rows)
         c.judge(c.run(cuda, row, toks, [rows]), want, f"ff {ff} width {width}")
+
+
+# fp16 operands against fp32 ones: each of the about 10 roundings between a row's input and its output moves it by up to 2^-11, 5e-3 in all; a tap taken
+# from the wrong place moves the row by a good part of itself.
+ROW_REL = 5e-3
+
+
+@pytest.mark.parametrize("counts", [
+    [1], [2, 1, 3], [31, 1, 33, 64], [247, 16, 5], [248, 2, 3, 1, 20], [249, 1, 40], [250, 3, 252, 7], [251, 2, 1, 1, 1, 90], [252, 260], [253, 253, 4], [254, 0, 40, 0],
+    [16] * 40, [1] * 70, [506, 33], [600],
+])
+def test_convolution_at_the_edges_of_tiles_and_sequences(ops, cuda, synth, counts):
+    """Sequence starts and ends at every place around a tile's first tokens, in the middle of its chunks, several to a chunk; two calls, the second with
+    the state that the first left behind, against the layer with fp32 projections (convolution in a kernel of its own)."""
+    torch, n = cuda, len(counts)
+    w = synth.la_weights(77)
+    out, conv = [], []
+    for proj in (ops.PROJ_FP32, ops.PROJ_FP16):
+        la = ops.LinearAttention(proj, max_batch=n, max_prefill_rows=sum(counts))
+        la.set_weights(w)
+        st = ops.LinearAttnState(1, n + 1)
+        slots = [n - i for i in range(n)]
+        y = []
+        for call in range(2):
+            x = torch.from_numpy(synth.hidden_states(77, f"edges.{call}", sum(counts))).cuda()
+            y.append(la.forward_batch(x, st, 0, slots, counts))
+        assert la.device_status() == 0
+        out.append(torch.cat(y))
+        conv.append(torch.stack([st.export_state(0, s)[1] for s in slots]))
+    worst = ((out[1] - out[0]).norm(dim=1) / out[0].norm(dim=1)).max()
+    assert worst <= ROW_REL, worst
+    assert (conv[1] - conv[0]).norm() <= ROW_REL * conv[0].norm()
+
+
+def test_more_sequences_than_the_tables_on_chip_hold(ops, cuda, synth):
+    """Above 512 sequences their first rows and slots are read from memory."""
+    torch, n = cuda, 600
+    w = synth.la_weights(78)
+    counts = [1 + i % 3 for i in range(n)]
+    x = torch.from_numpy(synth.hidden_states(78, "many", sum(counts))).cuda()
+    out = []
+    for proj in (ops.PROJ_FP32, ops.PROJ_FP16):
+        la = ops.LinearAttention(proj, max_batch=n, max_prefill_rows=sum(counts))
+        la.set_weights(w)
+        st = ops.LinearAttnState(1, n)
+        out.append([la.forward_batch(x, st, 0, list(range(n)), counts) for _ in range(2)][1])
+    assert ((out[1] - out[0]).norm(dim=1) / out[0].norm(dim=1)).max() <= ROW_REL
