@@ -50,7 +50,7 @@ diff_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     float* x_l = reinterpret_cast<float*>(sm + L.off_bar + 512);       // row sums of the two maps, then sums of squares of the two column halves
     auto bar = [&](int i) { return base + L.off_bar + 8u * i; };
     if (*reinterpret_cast<volatile int*>(error_word) != 0) return;     // an earlier launch gave up: do not queue more bounded waits
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int cta = blockIdx.x, n_cta = gridDim.x;
     const int n_my = (cta < n_items) ? (n_items - cta + n_cta - 1) / n_cta : 0;
     struct Item { DiffTile t; int head, kept, w0, n_kt; };             // pages of kept positions, first page behind them, pages in all
@@ -130,26 +130,34 @@ diff_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
         }
     } else if (warp == 9) {
-        // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // ------------------------------ MMA issuer: the warp as one, an elected lane at each issue (elect_one) ------------------------------
+        // Twenty products a key step: a thread on its own took some 80 cycles for each, more than the products themselves (247 -> 220 us at 16 x 1024 tokens).
+        {
+            const uint64_t q_k = umma_smem_desc(base, 16, 1024), k_k = umma_smem_desc(base + L.off_k, 16, 1024), p_k = umma_smem_desc(base + L.off_p, 16, 1024);
+            const uint64_t v_mn = umma_smem_desc(base + L.off_v, kDKBlk, 1024);
             constexpr uint32_t id_s = umma_idesc(kFmtBF16, kDM, kDN, 0, 0);
             const uint32_t id_pv = umma_idesc(kFmtBF16, kDM, 64 * L.nv, 0, 1);
             // PV products of global step g; `first` overwrites O (the previous item's epilogue has read it), after `last` O is final
             auto issue_pv = [&](int g, bool first, bool last, int it) -> bool {
                 const int b = g & 1, s = g % NST;
-                if (!mbar_wait(bar(D_VF + s), (g / NST) & 1, abort_flag)) return false;
-                if (first && it > 0 && !mbar_wait(bar(D_OD), (it - 1) & 1, abort_flag)) return false;
+                if (!mbar_wait_warp(bar(D_VF + s), (g / NST) & 1, abort_flag)) return false;
+                if (first && it > 0 && !mbar_wait_warp(bar(D_OD), (it - 1) & 1, abort_flag)) return false;
+                const uint64_t v = v_mn + s * L.nv * desc_step(kDKBlk);
                 for (int m = 0; m < 2; ++m) {
-                    if (!mbar_wait(bar(D_PF + 2 * m + b), (g >> 1) & 1, abort_flag)) return false;
+                    if (!mbar_wait_warp(bar(D_PF + 2 * m + b), (g >> 1) & 1, abort_flag)) return false;
                     tc_fence_after();
+                    const uint64_t a = p_k + (2 * m + b) * desc_step(kDPBuf);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ++ks)
-                        umma_f16(tmem_o + m * 64 * L.nv, umma_smem_desc(base + L.off_p + (2 * m + b) * kDPBuf + ks * 32, 16, 1024),
-                                 umma_smem_desc(base + L.off_v + s * L.nv * kDKBlk + ks * 2048, kDKBlk, 1024), id_pv, (!first || ks > 0) ? 1u : 0u);
-                    umma_commit(bar(D_PV + 2 * m + b));
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_f16(tmem_o + m * 64 * L.nv, a + desc_step(ks * 32), v + desc_step(ks * 2048), id_pv, (!first || ks > 0) ? 1u : 0u);
+                        umma_commit(bar(D_PV + 2 * m + b));
+                    }
                 }
-                umma_commit(bar(D_VE + s));
-                if (last) umma_commit(bar(D_OF));
+                if (elect_one()) {
+                    umma_commit(bar(D_VE + s));
+                    if (last) umma_commit(bar(D_OF));
+                }
                 return true;
             };
             bool ok = true, pending = false, pfirst = false, plast = false;
@@ -160,23 +168,28 @@ diff_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
                     pending = false;
                 }
-                if (!mbar_wait(bar(D_Q), i & 1, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_warp(bar(D_Q), i & 1, abort_flag)) { ok = false; break; }
                 for (int j = 0; ok && j < n_kt; ++j, ++gs) {
                     const int b = gs & 1, s = gs % NST;
-                    if (!mbar_wait(bar(D_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar(D_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
                     for (int m = 0; m < 2; ++m) {
-                        if (gs >= 2 && !mbar_wait(bar(D_SE + 2 * m + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                        if (gs >= 2 && !mbar_wait_warp(bar(D_SE + 2 * m + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
                         tc_fence_after();
-                        for (int blk = 0; blk < L.nd; ++blk)
+                        const uint64_t q0 = q_k + m * L.nd * desc_step(kDQBlk), k0 = k_k + (s * 2 + m) * L.nd * desc_step(kDKBlk);
+                        if (elect_one()) {
+                            for (int blk = 0; blk < L.nd; ++blk)
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks)
-                                umma_f16(tmem + (2 * m + b) * kDN, umma_smem_desc(base + (m * L.nd + blk) * kDQBlk + ks * 32, 16, 1024),
-                                         umma_smem_desc(base + L.off_k + ((s * 2 + m) * L.nd + blk) * kDKBlk + ks * 32, 16, 1024), id_s, (blk > 0 || ks > 0) ? 1u : 0u);
-                        umma_commit(bar(D_SF + 2 * m + b));
+                                for (int ks = 0; ks < 4; ++ks)
+                                    umma_f16(tmem + (2 * m + b) * kDN, q0 + blk * desc_step(kDQBlk) + desc_step(ks * 32), k0 + blk * desc_step(kDKBlk) + desc_step(ks * 32), id_s,
+                                             (blk > 0 || ks > 0) ? 1u : 0u);
+                            umma_commit(bar(D_SF + 2 * m + b));
+                        }
                     }
                     if (!ok) break;
-                    umma_commit(bar(D_KE + s));
-                    if (j == n_kt - 1) umma_commit(bar(D_QE));
+                    if (elect_one()) {
+                        umma_commit(bar(D_KE + s));
+                        if (j == n_kt - 1) umma_commit(bar(D_QE));
+                    }
                     if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
                     pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
                 }

@@ -47,7 +47,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     float* x_mx = reinterpret_cast<float*>(sm + L.off_bar + 256);      // row-maximum exchange [2 tiles][2 halves][128]
     auto bar = [&](int i) { return base + L.off_bar + 8u * i; };
     if (*reinterpret_cast<volatile int*>(error_word) != 0) return;     // an earlier launch gave up: do not queue more bounded waits
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int cta = blockIdx.x, n_cta = gridDim.x;
     const int n_my = (cta < n_items) ? (n_items - cta + n_cta - 1) / n_cta : 0;
     const int nq = L.nd + L.nr;
@@ -126,26 +126,28 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             }
         }
     } else if (warp == 9) {
-        // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // ------------------------------ MMA issuer: the warp as one, an elected lane at each issue (elect_one) ------------------------------
+        // Twenty products a key step: a thread on its own took some 80 cycles for each, more than the products themselves (55.7 -> 45.7 us at 5 x 771 tokens).
+        {
+            const uint64_t q_k = umma_smem_desc(base, 16, 1024), k_k = umma_smem_desc(base + L.off_k, 16, 1024), p_k = umma_smem_desc(base + L.off_p, 16, 1024);
+            const uint64_t v_mn = umma_smem_desc(base + L.off_v, kKBlk, 1024);
             constexpr uint32_t id_s = umma_idesc(kFmtBF16, kLM, kLN, 0, 0);
             const uint32_t id_pv = umma_idesc(kFmtBF16, kLM, 64 * L.nv, 0, 1);
             // PV product of global step g; `first` overwrites O (the previous item's epilogue has read it), after `last` O is final
             auto issue_pv = [&](int g, bool first, bool last, int it) -> bool {
                 const int b = g & 1, s = g % NST;
-                if (!mbar_wait(bar(L_VF + s), (g / NST) & 1, abort_flag)) return false;
-                if (!mbar_wait(bar(L_PF + b), (g >> 1) & 1, abort_flag)) return false;
-                if (first && it > 0 && !mbar_wait(bar(L_OD), (it - 1) & 1, abort_flag)) return false;
+                if (!mbar_wait_warp(bar(L_VF + s), (g / NST) & 1, abort_flag)) return false;
+                if (!mbar_wait_warp(bar(L_PF + b), (g >> 1) & 1, abort_flag)) return false;
+                if (first && it > 0 && !mbar_wait_warp(bar(L_OD), (it - 1) & 1, abort_flag)) return false;
                 tc_fence_after();
+                const uint64_t a = p_k + b * desc_step(kPBuf), v = v_mn + s * L.nv * desc_step(kKBlk);
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    const uint64_t a = umma_smem_desc(base + L.off_p + b * kPBuf + ks * 32, 16, 1024);
-                    const uint64_t v = umma_smem_desc(base + L.off_v + s * L.nv * kKBlk + ks * 2048, kKBlk, 1024);
-                    umma_f16(tmem_o, a, v, id_pv, (!first || ks > 0) ? 1u : 0u);
+                    for (int ks = 0; ks < 4; ++ks) umma_f16(tmem_o, a + desc_step(ks * 32), v + desc_step(ks * 2048), id_pv, (!first || ks > 0) ? 1u : 0u);
+                    umma_commit(bar(L_PV + b));
+                    umma_commit(bar(L_VE + s));
+                    if (last) umma_commit(bar(L_OF));
                 }
-                umma_commit(bar(L_PV + b));
-                umma_commit(bar(L_VE + s));
-                if (last) umma_commit(bar(L_OF));
                 return true;
             };
             bool ok = true, pending = false, pfirst = false, plast = false;
@@ -156,22 +158,23 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
                     pending = false;
                 }
-                if (!mbar_wait(bar(L_Q), i & 1, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_warp(bar(L_Q), i & 1, abort_flag)) { ok = false; break; }
                 for (int j = 0; j < n_kt; ++j, ++gs) {
                     const int b = gs & 1, s = gs % NST;
-                    if (!mbar_wait(bar(L_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
-                    if (gs >= 2 && !mbar_wait(bar(L_SE + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar(L_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
+                    if (gs >= 2 && !mbar_wait_warp(bar(L_SE + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    for (int blk = 0; blk < nq; ++blk)
+                    const uint64_t k0 = k_k + s * nq * desc_step(kKBlk);
+                    if (elect_one()) {
+                        for (int blk = 0; blk < nq; ++blk)
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            const uint64_t a = umma_smem_desc(base + blk * kQBlk + ks * 32, 16, 1024);
-                            const uint64_t k = umma_smem_desc(base + L.off_k + (s * nq + blk) * kKBlk + ks * 32, 16, 1024);
-                            umma_f16(tmem + b * kLN, a, k, id_s, (blk > 0 || ks > 0) ? 1u : 0u);
-                        }
-                    umma_commit(bar(L_SF + b));
-                    umma_commit(bar(L_KE + s));
-                    if (j == n_kt - 1) umma_commit(bar(L_QE));
+                            for (int ks = 0; ks < 4; ++ks)
+                                umma_f16(tmem + b * kLN, q_k + blk * desc_step(kQBlk) + desc_step(ks * 32), k0 + blk * desc_step(kKBlk) + desc_step(ks * 32), id_s,
+                                         (blk > 0 || ks > 0) ? 1u : 0u);
+                        umma_commit(bar(L_SF + b));
+                        umma_commit(bar(L_KE + s));
+                        if (j == n_kt - 1) umma_commit(bar(L_QE));
+                    }
                     if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
                     pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
                 }

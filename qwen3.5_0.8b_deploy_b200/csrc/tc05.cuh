@@ -27,6 +27,9 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr, uint32_t 
     return d;
 }
 
+// What a descriptor grows by when its tile starts so many bytes further on.
+__host__ __device__ constexpr uint32_t desc_step(uint32_t bytes) { return bytes >> 4; }
+
 // ---- instruction descriptor (32-bit) for kind::f16 / kind::tf32, fp32 accumulation ---------------------------
 //   [4,6) D format: 1 = f32   [7,10) A format, [10,13) B format: 0 = f16, 1 = bf16, 2 = tf32
 //   [15] A major, [16] B major: 0 = K, 1 = MN   [17,23) N >> 3   [24,29) M >> 4
