@@ -10,12 +10,12 @@
 //     reduction over warps needs no shared memory of its own, and its order is fixed;
 //   * the fp32 residual rows are normalised on the way in (the rounding point is the norm kernel's: one rounding of the normalised value), and
 //     SwiGLU and the residual addition sit in the epilogue.  A layer of a step is five launches in place of eight or nine.
-// Measured in a captured step of 8 rows, from the dependency wait on: input projection (8224 x 1024) 5.3 us, gate / up with SwiGLU (7168 x 1024)
-// 5.0 us, output projections (1024 x 2048 and 1024 x 3584) 3.7 us; the step of four layers and the head 191 -> 138 us (fp16 cache, 50 tokens), 193 -> 141 us
-// behind 500 tokens of an INT8 cache.
+// Measured in a captured step of 8 rows, one CTA's stamps from the dependency wait on: input projection (8224 x 1024) 4.0 us, gate / up with SwiGLU
+// (7168 x 1024) 3.7 us, output projections (1024 x 2048 and 1024 x 3584) 2.5 and 3.8 us; the step of four layers and the head 191 us on library GEMMs, 128 us
+// here (fp16 cache, 50 tokens).  A Gutenex step of 1 / 16 rows takes 131 / 172 us (165 / 205 with the norms' weights read behind the wait).
 // Taken back: X in registers with one column tile at a time (eight warps through 2000 instructions each: 8.6, 9.5 and 4.1 us); asking L2 for the
 // weights of the launch after next (no change: the copies are not what a launch waits for).
-// Why 16 rows: a step of the hybrid stack at 1 / 8 / 16 rows takes 126 / 138 / 163 us against 194 / 191 / 200 us on library GEMMs.  Two row tiles (17 to 32
+// Why 16 rows: a step of the hybrid stack at 1 / 8 / 16 rows took 126 / 138 / 163 us (before the copies were shared out) against 194 / 191 / 200 us on library GEMMs.  Two row tiles (17 to 32
 // rows) need 203 KB beside the widest slab, so the next launch no longer fits an SM, and 64 registers no longer hold them: at 17 / 24 / 32 rows 228 / 241 /
 // 272 us against 193 / 204 / 221 (bf16 stacks 256 to 337 against 206 to 256), the head 25 to 29 us against 18; layers called alone gained 7 % at best.
 // Taken out: the library GEMMs serve those steps.  tcgen05 would pad the rows to 64 or 128 and pay for a TMEM round trip (gemm_tc.cu: 9.0, 10.8 and 10.5 us).
@@ -106,9 +106,17 @@ __device__ __forceinline__ void rows_enter(bool late) {
 constexpr int kRowsThreads = 512, kRowsWarps = 16, kRows = kRowsGemmMax;
 static_assert(kRows == 16, "one row tile of mma.m16n8k16");
 
-// X into shared memory as 16-bit rows, a warp per row.
+// The norm's weights, which no kernel of a step writes, come into shared memory by a copy that is issued with those of the product's weights.  Read from L2
+// behind the dependency wait (which empties L1), one load after the other between the stores of the normalised row, they took 3.5 us of a launch.
+template <int LOAD>
+__device__ __forceinline__ bool norms_with_weights(const RowsGemm& a) { return (LOAD == kLoadNorm || LOAD == kLoadAddNorm) && a.norm_w; }
+inline size_t norm_bytes(const RowsGemm& a) { return a.norm_w ? (size_t)a.K * 4 : 0; }
+
+// X into shared memory as 16-bit rows, a warp per row.  s_norm: the norm's weights, there once norm_bar's first phase is over.  False: they did not come.
 template <typename T, int LOAD, int WARPS>
-__device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, int pitch, int warp, int lane) {
+__device__ __forceinline__ bool load_rows(const RowsGemm& a, unsigned char* sx, int pitch, int warp, int lane, const float* s_norm, uint32_t norm_bar,
+                                          volatile int* abort_flag) {
+    bool ok = true;
 #pragma unroll 1
     for (int m = warp; m < a.M; m += WARPS) {
         const size_t at = (size_t)(a.row_index ? a.row_index[m] : m) * a.ldx;
@@ -136,14 +144,25 @@ __device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, 
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
                 rs = 1.0f / sqrtf(ss / (float)a.K + a.eps);
+                if (norms_with_weights<LOAD>(a) && ok) ok = mbar_wait_warp(norm_bar, 0, abort_flag);
             }
+            float4 h[4];                         // kLoadAddNorm: what is added to, half a row at a time
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int k = 4 * (32 * i + lane);
+                if constexpr (LOAD == kLoadAddNorm) {
+                    if ((i & 3) == 0) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int kj = k + 128 * j;
+                            h[j] = kj < a.K ? __ldcg(reinterpret_cast<const float4*>(xr + kj)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+                    }
+                }
                 if (k < a.K) {
                     float4 w = make_float4(rs, rs, rs, rs);
                     if (LOAD < kLoadF32 && a.norm_w) {
-                        const float4 f = __ldg(reinterpret_cast<const float4*>(a.norm_w + k));
+                        const float4 f = *reinterpret_cast<const float4*>(s_norm + k);
                         w = make_float4(rs * (a.norm_base + f.x), rs * (a.norm_base + f.y), rs * (a.norm_base + f.z), rs * (a.norm_base + f.w));
                     }
                     float4 n = make_float4(v[i].x * w.x, v[i].y * w.y, v[i].z * w.z, v[i].w * w.w);
@@ -151,8 +170,7 @@ __device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, 
                         n = make_float4((n.x - __half2float(__float2half_rn(n.x))) * kLoScale, (n.y - __half2float(__float2half_rn(n.y))) * kLoScale,
                                         (n.z - __half2float(__float2half_rn(n.z))) * kLoScale, (n.w - __half2float(__float2half_rn(n.w))) * kLoScale);
                     if constexpr (LOAD == kLoadAddNorm) {
-                        const float4 h = __ldcg(reinterpret_cast<const float4*>(xr + k));
-                        n = make_float4(h.x + n.x, h.y + n.y, h.z + n.z, h.w + n.w);
+                        n = make_float4(h[i & 3].x + n.x, h[i & 3].y + n.y, h[i & 3].z + n.z, h[i & 3].w + n.w);
                         if (blockIdx.x == m % gridDim.x) *reinterpret_cast<float4*>(a.x_out + (size_t)m * a.K + k) = n;
                     }
                     *reinterpret_cast<uint2*>(dst + 2 * k) = make_uint2(pack2<T>(n.x, n.y), pack2<T>(n.z, n.w));
@@ -160,6 +178,8 @@ __device__ __forceinline__ void load_rows(const RowsGemm& a, unsigned char* sx, 
             }
         }
     }
+    if (!ok) mbar_drain(norm_bar, 0);
+    return ok;
 }
 
 // Many columns, K <= 1024: X in shared memory, up to eight column tiles per CTA.  A warp multiplies four tiles (two groups of eight warps when a
@@ -172,42 +192,48 @@ rows_wide_kernel(const RowsGemm a, unsigned long long* stamp) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int pitch = rows_pitch(a.K), row_bytes = a.K * 2;
     unsigned char* sx = smem + 8 * a.tiles * pitch;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sx + kRows * pitch);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar + 1);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sx + kRows * pitch);                          // of the weights, of the norm's
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar + 2);
+    float* s_norm = reinterpret_cast<float*>(sx + kRows * pitch + 32);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
     const int cols = kGated ? a.N / 2 : a.N, units = (cols + 7) / 8;                         // output columns, and eights of them
     const int u0 = part_begin(blockIdx.x, gridDim.x, units), u1 = part_begin(blockIdx.x + 1, gridDim.x, units);
     const int col0 = 8 * u0, n_cols = min(cols, 8 * u1) - col0, half = 8 * (u1 - u0) * pitch;      // gated: the up rows' place
     const int tiles = (kGated ? 2 : 1) * (u1 - u0);
 
-    if (warp == 0 && n_cols > 0) {
-        if (lane == 0) {
-            mbar_init(smem_u32(bar), 1);
-            *abort_flag = 0;
-            mbar_fence_init();
-            mbar_arrive_expect_tx(smem_u32(bar), (uint32_t)((kGated ? 2 : 1) * n_cols * row_bytes));
-        }
-        __syncwarp();
-        for (int i = lane; i < n_cols; i += 32) {
-            const int n = col0 + i, from = kGated ? n + n / a.group * a.group : n;
-            bulk_g2s(smem_u32(smem) + i * pitch, static_cast<const T*>(a.w) + (size_t)from * a.K, (uint32_t)row_bytes, smem_u32(bar));
-            if (kGated)
-                bulk_g2s(smem_u32(smem) + half + i * pitch, static_cast<const T*>(a.w) + (size_t)(from + a.group) * a.K, (uint32_t)row_bytes, smem_u32(bar));
+    if (tid == 0) {
+        mbar_init(smem_u32(bar), 1);
+        mbar_init(smem_u32(bar + 1), 1);
+        *abort_flag = 0;
+        mbar_fence_init();
+        if (n_cols > 0) mbar_arrive_expect_tx(smem_u32(bar), (uint32_t)((kGated ? 2 : 1) * n_cols * row_bytes));
+        if (norms_with_weights<LOAD>(a)) {
+            mbar_arrive_expect_tx(smem_u32(bar + 1), (uint32_t)a.K * 4);
+            bulk_g2s(smem_u32(s_norm), a.norm_w, (uint32_t)a.K * 4, smem_u32(bar + 1));
         }
     }
+    __syncthreads();
+    // A lane's copy takes 45 ns to issue, whoever of the warp is next: all warps share them.
+    for (int i = warp + kRowsWarps * lane; i < n_cols; i += 32 * kRowsWarps) {
+        const int n = col0 + i, from = kGated ? n + n / a.group * a.group : n;
+        bulk_g2s(smem_u32(smem) + i * pitch, static_cast<const T*>(a.w) + (size_t)from * a.K, (uint32_t)row_bytes, smem_u32(bar));
+        if (kGated)
+            bulk_g2s(smem_u32(smem) + half + i * pitch, static_cast<const T*>(a.w) + (size_t)(from + a.group) * a.K, (uint32_t)row_bytes, smem_u32(bar));
+    }
+    __syncwarp();
+    const int wide_log2 = a.tiles > 4 ? 3 : 4, splits = 1 << wide_log2, split = warp & (splits - 1), tile0 = (warp >> wide_log2) * 4;
+    const Slices sl(a.K, splits);
+    const int c0 = sl.begin(split), c1 = sl.begin(split + 1);
+    const bool high = a.M > 8;
     rows_enter(a.late);
     stamp_begin(stamp);
-    load_rows<T, LOAD, kRowsWarps>(a, sx, pitch, warp, lane);
+    const bool rows_ok = load_rows<T, LOAD, kRowsWarps>(a, sx, pitch, warp, lane, s_norm, smem_u32(bar + 1), abort_flag);
     __syncthreads();
     if (n_cols <= 0) return;
 
     // ---- products --------------------------------------------------------------------------------------------------------
-    const int groups = a.tiles > 4 ? 2 : 1, splits = kRowsWarps / groups, split = warp % splits, tile0 = (warp / splits) * 4;
-    const Slices sl(a.K, splits);
-    const int c0 = sl.begin(split), c1 = sl.begin(split + 1);
-    const bool high = a.M > 8;
     auto tile_at = [&](int t) { return smem + (kGated ? (t & 1) * half + 8 * (t >> 1) * pitch : 8 * t * pitch); };
-    const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
+    const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag) && rows_ok;
     if (!ok) mbar_drain(smem_u32(bar), 0);
     float acc[4][4] = {};
     const unsigned char* xp = sx + r * pitch + c * 16;
@@ -286,7 +312,9 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
     unsigned char* sx = smem + kStreamWarps * 8 * pitch;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sx + kRows * pitch);                // two per warp
     unsigned long long* s_best = reinterpret_cast<unsigned long long*>(bars + 2 * kStreamWarps);     // [kRows]
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(s_best + kRows);
+    uint64_t* norm_bar = reinterpret_cast<uint64_t*>(s_best + kRows);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(norm_bar + 1);
+    float* s_norm = reinterpret_cast<float*>(norm_bar + 2);
     const uint32_t bar = smem_u32(bars + 2 * warp);
     const int chunks = a.K / 32, mid = (chunks + 1) / 2, n_tiles = (a.N + 7) / 8, step = gridDim.x * kStreamWarps;
     const int first = blockIdx.x + gridDim.x * warp;
@@ -304,12 +332,20 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
         if (warp == 0) *abort_flag = 0;
         mbar_fence_init();
     }
+    if (tid == 0) {
+        mbar_init(smem_u32(norm_bar), 1);
+        mbar_fence_init();
+        if (norms_with_weights<LOAD>(a)) {
+            mbar_arrive_expect_tx(smem_u32(norm_bar), (uint32_t)a.K * 4);
+            bulk_g2s(smem_u32(s_norm), a.norm_w, (uint32_t)a.K * 4, smem_u32(norm_bar));
+        }
+    }
     if (tid < kRows) s_best[tid] = 0ull;
-    __syncwarp();
+    __syncthreads();
     if (first < n_tiles) { fetch(first, 0); fetch(first, 1); }
     rows_enter(a.late);
     stamp_begin(stamp);
-    load_rows<T, LOAD, kStreamWarps>(a, sx, pitch, warp, lane);
+    const bool rows_ok = load_rows<T, LOAD, kStreamWarps>(a, sx, pitch, warp, lane, s_norm, smem_u32(norm_bar), abort_flag);
     __syncthreads();
 
     const bool high = a.M > 8;
@@ -318,7 +354,11 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
     const unsigned char* wp = sw + r * pitch + c * 16;
     uint32_t parity = 0;
     bool ok = true;
-    for (int tile = first; ok && tile < n_tiles; tile += step, parity ^= 1u) {
+    if (!rows_ok && first < n_tiles) {           // its first copies are on their way
+        mbar_drain(bar, 0);
+        if (mid < chunks) mbar_drain(bar + 8, 0);
+    }
+    for (int tile = first; ok && rows_ok && tile < n_tiles; tile += step, parity ^= 1u) {
         float acc[2][4] = {};                    // two chains
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
@@ -375,11 +415,12 @@ rows_stream_kernel(const RowsGemm a, unsigned long long* stamp) {
 }
 
 // Few columns, deep K <= 4096: fp32 Y[M, N] = X W^T, added to what is there with ADD.  Up to eight columns per CTA (six or seven of 1024 on 148
-// SMs), the 16 warps split K, X goes from L2 straight into the registers of the warp that multiplies it, kAhead chunks at a time.
-template <typename T, bool ADD>
+// SMs), the 16 warps split K, X goes from L2 straight into the registers of the warp that multiplies it, kAhead chunks at a time: all that a warp has
+// for up to eight rows, in two round trips to L2 for more rows (HIGH) and K above 2048.
+template <typename T, bool ADD, bool HIGH>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
-    constexpr int kAhead = 4;
+    constexpr int kHalves = HIGH ? 2 : 1, kAhead = HIGH ? 4 : 8;
     extern __shared__ __align__(128) unsigned char smem[];
     const int pitch = rows_pitch(a.K);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 8 * pitch);
@@ -398,10 +439,10 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
         if (lane < cols)
             bulk_g2s(smem_u32(smem) + lane * pitch, static_cast<const T*>(a.w) + (size_t)(n0 + lane) * a.K, (uint32_t)a.K * 2, smem_u32(bar));
     }
-    rows_enter(a.late);
-    stamp_begin(stamp);
     const Slices sl(a.K, kRowsWarps);
     const int c0 = sl.begin(warp), c1 = sl.begin(warp + 1);
+    rows_enter(a.late);
+    stamp_begin(stamp);
     const bool writes = tid < 8 * kRows && em < a.M && n8 < cols;
     float res = 0.f;
     if (ADD && writes) res = __ldcg(static_cast<const float*>(a.y) + (size_t)em * a.ldy + n0 + n8);
@@ -409,11 +450,11 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     auto load = [&](int i, int ch) {             // rows 8 i + r, chunk ch
         return 8 * i + r < a.M && ch < c1 ? __ldcg(reinterpret_cast<const uint4*>(xp + (size_t)8 * i * a.ldx + 32 * ch)) : make_uint4(0u, 0u, 0u, 0u);
     };
-    uint4 x[kAhead][2];
+    uint4 x[kAhead][kHalves];
 #pragma unroll
     for (int j = 0; j < kAhead; ++j)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) x[j][i] = load(i, c0 + j);
+        for (int i = 0; i < kHalves; ++i) x[j][i] = load(i, c0 + j);
     __syncthreads();                             // the barrier is initialised
     const bool ok = mbar_wait(smem_u32(bar), 0, abort_flag);
     if (!ok) mbar_drain(smem_u32(bar), 0);
@@ -425,11 +466,11 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
         for (int j = 0; j < kAhead; ++j) {
             if (g + j >= c1) break;
             const uint4 b = *reinterpret_cast<const uint4*>(wp + (g + j) * 64);
-            const uint4 lo = x[j][0], hi = x[j][1];
+            const uint4 lo = x[j][0], hi = HIGH ? x[j][kHalves - 1] : make_uint4(0u, 0u, 0u, 0u);
             mma_rows<T>(acc[0], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
             mma_rows<T>(acc[1], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) x[j][i] = load(i, g + j + kAhead);
+            for (int i = 0; i < kHalves; ++i) x[j][i] = load(i, g + j + kAhead);
         }
     }
 #pragma unroll
@@ -445,7 +486,8 @@ rows_deep_kernel(const RowsGemm a, unsigned long long* stamp) {
     if (tid == 0 && *abort_flag && a.error) atomicExch(a.error, 7);
 }
 
-// Most shared memory of a launch: 64 weight rows and 16 of X.  A layer's launches fit side by side: 153 and 34 KB, 170 and 59 KB.
+// Most shared memory of a launch: 64 weight rows, 16 of X, the norm's weights.  A layer's launches fit side by side: 153 and 34 KB, 169 and 57 KB (of 228
+// with 1 KB reserved for each, so that the norm's 4 KB just fit).
 constexpr int kSharedMost = 176 * 1024;
 
 template <typename K>
@@ -463,7 +505,7 @@ int launch_wide(RowsGemm a, cudaStream_t s, ProfKind kind) {
     const int unit = EPI == kRowsSwiglu || EPI == kRowsGeglu ? 2 : 1, units = ceil_div(a.N / unit, 8);
     const int waves = ceil_div(units * unit, 8 * sms), grid = std::min(units, waves * sms);     // one CTA per SM where eight tiles each are enough
     a.tiles = ceil_div(units, grid) * unit;
-    const size_t smem = (size_t)(8 * a.tiles + kRows) * rows_pitch(a.K) + 16;
+    const size_t smem = (size_t)(8 * a.tiles + kRows) * rows_pitch(a.K) + 32 + norm_bytes(a);
     unsigned long long* stamp = prof_stamp_slot(kind);
     launch_pdl_split(true, true, rows_wide_kernel<T, LOAD, EPI, YT>, dim3(grid), dim3(kRowsThreads), smem, s, a, stamp);
     B2_LAUNCH_CHECK();
@@ -474,24 +516,28 @@ template <typename T, int LOAD, int EPI>
 int launch_stream(const RowsGemm& a, int sms, cudaStream_t s, ProfKind kind) {
     static PerDeviceOnce once;
     B2_TRY(prepare(once, rows_stream_kernel<T, LOAD, EPI>));
-    const size_t smem = (size_t)(8 * kStreamWarps + kRows) * rows_pitch(a.K) + 8 * (2 * kStreamWarps + kRows) + 16;
+    const size_t smem = (size_t)(8 * kStreamWarps + kRows) * rows_pitch(a.K) + 8 * (2 * kStreamWarps + kRows) + 16 + norm_bytes(a);
     unsigned long long* stamp = prof_stamp_slot(kind);
     launch_pdl_split(true, true, rows_stream_kernel<T, LOAD, EPI>, dim3(sms), dim3(kStreamWarps * 32), smem, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
-template <typename T, bool ADD>
-int launch_deep(const RowsGemm& a, cudaStream_t s) {
+template <typename T, bool ADD, bool HIGH>
+int launch_deep_rows(const RowsGemm& a, cudaStream_t s) {
     static PerDeviceOnce once;
-    B2_TRY(prepare(once, rows_deep_kernel<T, ADD>));
+    B2_TRY(prepare(once, rows_deep_kernel<T, ADD, HIGH>));
     unsigned long long* stamp = prof_stamp_slot(PROF_GEMM_RES);
     int sms = 0;
     B2_TRY(device_sm_count(&sms));
     const int grid = std::max(ceil_div(a.N, 8), std::min(a.N, sms));      // up to eight columns a CTA
-    launch_pdl_split(true, true, rows_deep_kernel<T, ADD>, dim3(grid), dim3(kRowsThreads), (size_t)8 * rows_pitch(a.K) + 16, s, a, stamp);
+    launch_pdl_split(true, true, rows_deep_kernel<T, ADD, HIGH>, dim3(grid), dim3(kRowsThreads), (size_t)8 * rows_pitch(a.K) + 16, s, a, stamp);
     B2_LAUNCH_CHECK();
     return 0;
+}
+template <typename T, bool ADD>
+int launch_deep(const RowsGemm& a, cudaStream_t s) {
+    return a.M > 8 ? launch_deep_rows<T, ADD, true>(a, s) : launch_deep_rows<T, ADD, false>(a, s);
 }
 
 template <typename T, int LOAD, int EPI, typename YT>
@@ -511,7 +557,7 @@ int wide(const RowsGemm& a, cudaStream_t s, ProfKind kind) {
 bool gemm_rows_takes(const RowsGemm& a, int epi) {
     const bool deep = epi == kRowsResidual || epi == kRowsDeepStore;
     return a.M > 0 && a.M <= kRowsGemmMax && a.N > 0 && a.K > 0 && a.K % 32 == 0 && a.K <= (deep ? 4096 : 1024) && a.ldx % 8 == 0 &&
-           (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
+           ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15) == 0;
 }
 
 int gemm_rows(cudaStream_t s, const RowsGemm& a, ElemType type, int epi, int load, ElemType out) {
