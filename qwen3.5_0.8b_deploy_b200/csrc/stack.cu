@@ -543,7 +543,9 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
         }
         return 0;
     }
-    const bool many_rows = !decode && rows > 128;      // prefill: warp-per-row norm
+    // The warp-per-row norm where blocks of a row each no longer run side by side: a prompt pass of four layers at 256 / 1000 / 4000 / 8000 / 16000 / 32000
+    // rows took 421 / 608 / 1099 / 1894 / 3434 / 6995 us with it and 373 / 560 / 1077 / 1889 / 3540 / 7100 us with a block per row.
+    const bool many_rows = !decode && rows > 8192;
     for (int i = 0; i < st->cfg.num_layers; ++i) {
         if (many_rows)
             rmsnorm_rows_kernel<<<ceil_div(rows, 4), 128, 0, s>>>(st->d_h, st->d_in_norm[i], st->cfg.rms_eps, rows, st->d_xb);
