@@ -62,7 +62,7 @@ int lightning_forward(BlockModel& m, MlstmOp& op, const LayerRun& run, const Pas
     const int W = m.cfg.width;
     float* state = m.state->d_recurrent + m.state->block_offset[run.state_layer];
     if (!p.decode && op.chunk && p.max_count >= 16) {
-        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.cols(), op.elem, ELEM_BF16, p.rows, sh.cols(), W));
+        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.cols(), op.elem, ELEM_BF16, p.rows, sh.cols(), W, 0.0f, 1.0f, m.error.i()));
         B2_TRY(launch_silu_cols(op.elem, m.proj.p, p.rows, sh.off_g(), sh.cols(), s));
         {
             ProfScope prof(PROF_LA_PREFILL, s);
@@ -165,10 +165,10 @@ int delta_forward(BlockModel& m, DeltaOp& op, const LayerRun& run, const PassRow
         float *a = m.gates.f(), *b = a + (size_t)p.rows * acols;
         void* g = b + ((size_t)p.rows * sh.heads + 3) / 4 * 4;
         const size_t e = elem_bytes(op.elem);
-        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, qkv, op.elem, op.elem, p.rows, qkv, W));
+        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, qkv, op.elem, op.elem, p.rows, qkv, W, 0.0f, 1.0f, m.error.i()));
         B2_TRY(gemm_typed(s, m.xt.p, W, (const char*)op.w_in.p + (size_t)qkv * W * e, b, sh.heads, op.elem, ELEM_F32, p.rows, sh.heads, W));
-        B2_TRY(gemm_typed(s, m.low.p, sh.low(), op.w_gate.p, a, acols, op.elem, ELEM_F32, p.rows, acols, sh.low()));
-        B2_TRY(gemm_typed(s, m.low.p, sh.low(), (const char*)op.w_gate.p + (size_t)acols * sh.low() * e, g, gcols, op.elem, op.elem, p.rows, gcols, sh.low()));
+        B2_TRY(gemm_typed(s, m.low.p, sh.low(), op.w_gate.p, a, acols, op.elem, ELEM_F32, p.rows, acols, sh.low(), 0.0f, 1.0f, m.error.i()));
+        B2_TRY(gemm_typed(s, m.low.p, sh.low(), (const char*)op.w_gate.p + (size_t)acols * sh.low() * e, g, gcols, op.elem, op.elem, p.rows, gcols, sh.low(), 0.0f, 1.0f, m.error.i()));
         {
             ProfScope prof(PROF_DELTA_PREFILL, s);
             B2_TRY(launch_delta_chunk(sh, m.proj.p, a, b, sh.taps <= 4 ? op.conv4.f() : op.conv.f(), op.a_log.f(), op.dt_bias.f(), p.d_seqs, p.n_seqs, p.max_count, p.rows, m.cfg.max_seqs, state,

@@ -380,7 +380,7 @@ static int mlstm_forward(BlockModel& m, MlstmOp& op, const LayerRun& run, const 
     float* state = m.state->d_recurrent + m.state->block_offset[run.state_layer];
     if (!p.decode && op.chunk && p.max_count >= 16) {
         // q | k | v | g in bf16 for the tensor cores, the gate pre-activations in fp32
-        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.cols(), op.elem, ELEM_BF16, p.rows, sh.cols(), W));
+        B2_TRY(gemm_typed(s, m.xt.p, W, op.w_in.p, m.proj.p, sh.cols(), op.elem, ELEM_BF16, p.rows, sh.cols(), W, 0.0f, 1.0f, m.error.i()));
         B2_TRY(gemm_typed(s, m.xt.p, W, (const char*)op.w_in.p + (size_t)sh.off_i() * W * elem_bytes(op.elem), m.gates.p, 2 * sh.heads, op.elem, ELEM_F32,
                           p.rows, 2 * sh.heads, W));
         {
@@ -466,8 +466,8 @@ static int latent_expanded(BlockModel& m, LatentOp& op, const LayerRun& run, con
     }
     B2_CUDA(cudaMemcpyAsync(m.tiles(), tiles.data(), tiles.size() * sizeof(LatentTile), cudaMemcpyHostToDevice, s));
     const int kcols = sh.heads * sh.dp, vcols = sh.heads * sh.vp;
-    B2_TRY(gemm_typed(s, m.c_stage.p, sh.rank, op.w_uk.p, m.k_up.p, kcols, op.elem, op.elem, ctx, kcols, sh.rank));
-    B2_TRY(gemm_typed(s, m.c_stage.p, sh.rank, op.w_uv.p, m.v_up.p, vcols, op.elem, op.elem, ctx, vcols, sh.rank));
+    B2_TRY(gemm_typed(s, m.c_stage.p, sh.rank, op.w_uk.p, m.k_up.p, kcols, op.elem, op.elem, ctx, kcols, sh.rank, 0.0f, 1.0f, m.error.i()));
+    B2_TRY(gemm_typed(s, m.c_stage.p, sh.rank, op.w_uv.p, m.v_up.p, vcols, op.elem, op.elem, ctx, vcols, sh.rank, 0.0f, 1.0f, m.error.i()));
     ProfScope prof(PROF_FA_PREFILL, s);
     return launch_latent_prefill(sh, m.q.p, p.rows, m.k_up.p, m.r_stage.p, m.v_up.p, ctx, m.tiles(), (int)tiles.size(), m.mixed.p, m.error.i(), s);
 }
@@ -486,7 +486,7 @@ static bool rows_step(const BlockModel& m, int rows) {
 
 int block_project(BlockModel& m, const PassRows& p, const void* w, int cols, void* out, ElemType out_type, cudaStream_t s) {
     const int W = m.cfg.width;
-    if (!p.in) return gemm_typed(s, m.xt.p, W, w, out, cols, m.elem, out_type, p.rows, cols, W);
+    if (!p.in) return gemm_typed(s, m.xt.p, W, w, out, cols, m.elem, out_type, p.rows, cols, W, 0.0f, 1.0f, m.error.i());
     RowsGemm a = *p.in;
     a.w = w; a.N = cols;
     a.y = out; a.ldy = cols;
@@ -559,7 +559,7 @@ static int run_layers(BlockModel& m, const PassRows& pass, cudaStream_t s) {
         a.error = m.error.i();
         const int epi = pre ? kRowsResidual : kRowsDeepStore;
         if (few && gemm_rows_takes(a, epi)) B2_TRY(gemm_rows(s, a, m.elem, epi, kLoadAsIs, ELEM_F32));
-        else B2_TRY(gemm_typed(s, from, cols, w.p, a.y, W, m.elem, ELEM_F32, R, W, cols, pre ? 1.0f : 0.0f));
+        else B2_TRY(gemm_typed(s, from, cols, w.p, a.y, W, m.elem, ELEM_F32, R, W, cols, pre ? 1.0f : 0.0f, 1.0f, m.error.i()));
         if (pre) return 0;
         pending = &norm;
         return few ? 0 : add_pending();

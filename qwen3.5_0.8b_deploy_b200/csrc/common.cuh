@@ -157,14 +157,15 @@ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // ---- GEMM (cuBLAS) --------------------------------------------------------------------------------
 // Y[rows, out] = X[rows, in] * W[out, in]^T, row-major.  x_fp16/w_fp16/y_fp16 select the storage
 // types; accumulation is fp32.  fp32 inputs use full fp32 math (no TF32).
-// Y = alpha * X W^T + beta * Y; ld_out > 0 gives the row pitch of Y (elements) when it is a column block of a wider matrix.
+// Y = alpha * X W^T + beta * Y; ld_out > 0 gives the row pitch of Y (elements) when it is a column block of a wider matrix.  With a device word for
+// what goes wrong there (`error`), large products run on the kernels of gemm_pair.cu.
 int gemm_xwT(cudaStream_t stream, const void* X, bool x_fp16, const void* W, bool w_fp16, void* Y,
-             bool y_fp16, int rows, int out, int in, float beta = 0.f, float alpha = 1.f, int ld_out = 0);
+             bool y_fp16, int rows, int out, int in, float beta = 0.f, float alpha = 1.f, int ld_out = 0, int* error = nullptr);
 // The same product with named element types (accumulation fp32; fp32 inputs in full fp32 math): X has row pitch ldx, Y row pitch ldy.
 enum ElemType { ELEM_F16 = 0, ELEM_BF16, ELEM_F32 };
 inline size_t elem_bytes(ElemType t) { return t == ELEM_F32 ? 4 : 2; }
 int gemm_typed(cudaStream_t stream, const void* X, int ldx, const void* W, void* Y, int ldy, ElemType in_type, ElemType out_type, int rows,
-               int out, int in, float beta = 0.f, float alpha = 1.f);
+               int out, int in, float beta = 0.f, float alpha = 1.f, int* error = nullptr);
 // One product per head, strided batched: Y_h[rows, out] = X_h[rows, in] W_h^T with W_h [out, in], or X_h W_h with W_h [in, out]
 // when w_in_major.  Head h starts x_stride / y_stride elements behind head h - 1 inside a row; the W_h lie back to back.
 int gemm_heads(cudaStream_t stream, const void* X, int ldx, int x_stride, const void* W, bool w_in_major, void* Y, int ldy, int y_stride,

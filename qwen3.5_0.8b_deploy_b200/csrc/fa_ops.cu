@@ -184,7 +184,7 @@ static int fa_project_in(b200attn_fa fa, const void* d_x, bool x_is_fp16, int ro
             else B2_TRY(f32_to_f16(s, (const float*)d_x, fa->d_xb, (size_t)rows * kHidden));
             xb = fa->d_xb;
         }
-        B2_TRY(gemm_xwT(s, xb, true, fa->d_wqkv_fp16, true, fa->d_qkv_raw, false, rows, kFaQkvCols, kHidden));
+        B2_TRY(gemm_xwT(s, xb, true, fa->d_wqkv_fp16, true, fa->d_qkv_raw, false, rows, kFaQkvCols, kHidden, 0.0f, 1.0f, 0, d_error));
         if (compensate) {
             // K | V columns += (x_lo W_hi^T + x_hi W_lo^T) / kLoScale
             const int q_cols = kFaHeads * kHeadDim * 2, kv_cols = 2 * kFaKvHeads * kHeadDim;
@@ -207,7 +207,7 @@ static int fa_project_out(b200attn_fa fa, float* d_y, float beta, int rows, bool
         rows_layer_out(s, (const __half*)fa->d_attn, fa->d_wo_fp16, d_y, beta, rows, kHidden, kFaHeads * kHeadDim, d_error, &status))
         return status;
     if (fa->cfg.proj_precision == B200ATTN_PROJ_FP16)
-        return gemm_xwT(s, fa->d_attn, true, fa->d_wo_fp16, true, d_y, false, rows, kHidden, kFaHeads * kHeadDim, beta);
+        return gemm_xwT(s, fa->d_attn, true, fa->d_wo_fp16, true, d_y, false, rows, kHidden, kFaHeads * kHeadDim, beta, 1.0f, 0, d_error);
     return gemm_xwT(s, fa->d_attn, false, fa->d_wo_f32, false, d_y, false, rows, kHidden, kFaHeads * kHeadDim, beta);
 }
 

@@ -1,6 +1,7 @@
 // Library GEMMs (cuBLAS) for the projections around the attention cores, error text, launch counter and
 // small conversion helpers.
 #include "common.cuh"
+#include "gemm_pair.cuh"
 #include <cstdlib>
 
 #include <algorithm>
@@ -141,8 +142,14 @@ int cublas_init() { return cublas_for_current_device(nullptr); }
 static cudaDataType cuda_type(ElemType t) { return t == ELEM_F16 ? CUDA_R_16F : t == ELEM_BF16 ? CUDA_R_16BF : CUDA_R_32F; }
 
 int gemm_typed(cudaStream_t stream, const void* X, int ldx, const void* W, void* Y, int ldy, ElemType in_type, ElemType out_type, int rows,
-               int out, int in, float beta, float alpha) {
+               int out, int in, float beta, float alpha, int* error) {
     if (rows <= 0 || out <= 0) return 0;
+    // From four rounds of 256 x 256 tiles on (74 pairs of CTAs), the pairs are the faster ones: pair / library in us, 16-bit operands, 5120 x 1024 at 3855 / 8192 /
+    // 65536 rows 37.7 / 37.5, 74.5 / 83.0, 559 / 718 (fp32 out); 8192 x 1024 at 1000 / 3000 / 16384 rows 15.2 / 15.4, 36.9 / 38.5, 182 / 206 (bf16 out).  Products
+    // that are added to Y stay: 1024 x 3584 at 3855 / 8192 / 16384 rows 26.3 / 22.0, 49.6 / 47.6, 97.3 / 96.6, within a pass of 65536 rows 289 / 288.
+    if (error && alpha == 1.0f && beta == 0.0f && (long long)ceil_div(rows, 256) * ceil_div(out, 256) >= 300 &&
+        gemm_pair_takes(X, ldx, W, Y, ldy, in_type, out_type, in))
+        return gemm_pair(stream, X, ldx, W, Y, ldy, in_type, out_type, rows, out, in, error);
     cublasHandle_t handle = nullptr;
     B2_TRY(cublas_for_current_device(&handle));
     cublasStatus_t st = cublasSetStream(handle, stream);
@@ -173,10 +180,10 @@ int gemm_heads(cudaStream_t stream, const void* X, int ldx, int x_stride, const 
 }
 
 int gemm_xwT(cudaStream_t stream, const void* X, bool x_fp16, const void* W, bool w_fp16, void* Y, bool y_fp16, int rows,
-             int out, int in, float beta, float alpha, int ld_out) {
+             int out, int in, float beta, float alpha, int ld_out, int* error) {
     if (x_fp16 != w_fp16) B2_FAIL(B200ATTN_ERR_INVALID, "gemm: activation and weight types must match");
     return gemm_typed(stream, X, in, W, Y, ld_out > 0 ? ld_out : out, x_fp16 ? ELEM_F16 : ELEM_F32, y_fp16 ? ELEM_F16 : ELEM_F32, rows, out,
-                      in, beta, alpha);
+                      in, beta, alpha, error);
 }
 
 // x -> hi = fp16(x), lo = fp16((x - hi) * 2^11): hi + lo * 2^-11 carries about 22 significant bits of x.

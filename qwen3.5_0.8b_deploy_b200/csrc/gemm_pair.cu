@@ -4,6 +4,7 @@
 // 0.94 GB each way.  Here the accumulators go through the function on their way out of TMEM while the tensor cores work on the next tile: 613 us (1.57
 // PFLOP/s, bound by the tensor cores' 512 cycles a slice and, over seconds, by the power limit) in place of 682 + 285 us.  fp16 products reach the function
 // unrounded; bf16 ones are rounded first, as the two kernels did: outputs of the layer-described stacks stay the same bit for bit.
+//   kPairStore16, kPairStore32   the product alone, as 16-bit or fp32 values (large products, gemm_typed)
 //   kPairConv   the DeltaNet input projection with the causal convolution, SiLU, L2 norms and gates behind it (fp16).  Here the channels of W are the
 //               rows of the product and the tokens its columns: a thread holds one channel and finds the taps of a token in its own registers.
 //               65536 rows 950 us (projection 878 and convolution 502 before, 3.2 GB between them), 3 x 333 23 (33), 9 x 466 67 (111), 45 14 (12).
@@ -28,7 +29,7 @@ constexpr uint32_t kStage = 2 * kOperand;
 constexpr int kEpiWarps = 16;
 constexpr int kThreads = 32 * (kEpiWarps + 2);          // epilogue warps, one for loads, one for products (CTA 0) or the hand-over of slices (CTA 1)
 
-enum { kPairGlu = 0, kPairConv = 1 };
+enum { kPairGlu = 0, kPairConv, kPairStore16, kPairStore32 };
 constexpr int kConvTokens = 253;                        // of a tile of 256 columns: the first three are the taps of the fourth
 constexpr int kMaxSeqRows = 512;                        // first rows and slots of the sequences kept in shared memory, up to so many sequences
 
@@ -112,6 +113,39 @@ __device__ __forceinline__ void glu_part(const PairArgs& p, const CUtensorMap* m
         bulk_commit_group();
     }
     __syncwarp();
+}
+
+// 32 rows of up to 64 columns as they are, 16-bit or fp32 rows of 64 bytes at a time.
+template <typename T, int EPI>
+__device__ __forceinline__ void plain_part(const PairArgs& p, const CUtensorMap* map_y, uint32_t acc, uint32_t out_smem, unsigned char* out, int row, int col, int lane) {
+    constexpr int kCols = EPI == kPairStore16 ? 32 : 16;
+    if (row >= p.rows) return;
+#pragma unroll 1
+    for (int c = 0; c < 64 && col + c < p.cols; c += kCols) {
+        uint32_t o[16];
+        if constexpr (EPI == kPairStore16) {
+            uint32_t v[32];
+            tmem_ld32(acc + c, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] = pack2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), T{});
+        } else {
+            tmem_ld16(acc + c, o);
+            tmem_wait_ld();
+        }
+        if (lane == 0) bulk_wait_group_read0();          // the last rows have left this place
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<uint4*>(out + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(map_y, out_smem, col + c, row);
+            bulk_commit_group();
+        }
+        __syncwarp();
+    }
 }
 
 // What the convolution has to know of a token: place in its sequence's rows of this call, up to 3, and rows behind it, up to 3.
@@ -479,7 +513,10 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
             } else {
                 if (!mbar_wait_warp(acc_full(b), (i >> 1) & 1, abort_flag)) break;
                 tc_fence_after();
-                if (64 * part < w.width)
+                if constexpr (EPI != kPairGlu) {
+                    if (64 * part < w.width)
+                        plain_part<T, EPI>(p, &maps.out[0], acc + 64 * part, out_smem, out, w.row * 256 + rank * 128 + 32 * q, w.col + 64 * part, lane);
+                } else if (64 * part < w.width)
                     glu_part<T, kAct>(p, &maps.out[0], acc + (p.up ? 32 : 64) * part, acc + (p.up ? 32 * part + w.width / 2 : 64 * part + 32), out_smem, out,
                                       w.row * 256 + rank * 128 + 32 * q, w.col / 2 + 32 * part, lane);
                 release();
@@ -525,12 +562,12 @@ int launch_pair(const PairMaps& maps, PairArgs p, cudaStream_t s) {
     return 0;
 }
 
-// [rows, cols] row-major, in boxes of so many columns and rows; a swizzle as wide as the box for operands and (64 bytes) results of kPairGlu
-int map_rows(CUtensorMap* m, ElemType t, const void* p, long long rows, int cols, int box_cols, int box_rows, bool swizzle = true) {
-    const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows}, str[1] = {(uint64_t)cols * elem_bytes(t)};
+// [rows, cols] row-major, in boxes of so many columns and rows; a swizzle as wide as the box for operands and (64 bytes) results but those of kPairConv
+int map_rows(CUtensorMap* m, ElemType t, const void* p, long long rows, int cols, int box_cols, int box_rows, bool swizzle = true, int pitch = 0) {
+    const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows}, str[1] = {(uint64_t)(pitch ? pitch : cols) * elem_bytes(t)};
     const uint32_t box[2] = {(uint32_t)box_cols, (uint32_t)box_rows};
     return make_tensor_map(m, t == ELEM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : t == ELEM_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-                           p, dims, str, box, swizzle ? box_cols * 2 : 0);
+                           p, dims, str, box, swizzle ? (int)(box_cols * elem_bytes(t)) : 0);
 }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -579,6 +616,29 @@ int gemm_la_conv(cudaStream_t s, const __half* x, const __half* w, int rows, con
     p.error = error;
     p.la = la;
     return launch_pair<kPairConv, __half, B200ATTN_ACT_SILU>(m, p, s);
+}
+
+bool gemm_pair_takes(const void* x, int ldx, const void* w, const void* y, int ldy, ElemType in_type, ElemType out_type, int in) {
+    return in_type != ELEM_F32 && (out_type == ELEM_F32 || out_type == in_type) && ldx % 8 == 0 && in % 8 == 0 && ldy * elem_bytes(out_type) % 16 == 0 &&
+           aligned16(x) && aligned16(w) && aligned16(y);
+}
+
+int gemm_pair(cudaStream_t s, const void* x, int ldx, const void* w, void* y, int ldy, ElemType in_type, ElemType out_type, int rows, int out, int in, int* error) {
+    PairMaps m{};
+    B2_TRY(map_rows(&m.a, in_type, x, rows, in, 64, 128, true, ldx));
+    B2_TRY(map_rows(&m.b, in_type, w, out, in, 64, 128));
+    B2_TRY(map_rows(&m.b32, in_type, w, out, in, 64, 32));
+    B2_TRY(map_rows(&m.out[0], out_type, y, rows, out, out_type == ELEM_F32 ? 16 : 32, 32, true, ldy));
+    PairArgs p{};
+    p.row_tiles = ceil_div(rows, 256);
+    p.col_tiles = ceil_div(out, 256);
+    p.k_steps = ceil_div(in, 64);
+    p.rows = rows;
+    p.cols = out;
+    p.error = error;
+    constexpr int kNone = B200ATTN_ACT_SILU;
+    if (in_type == ELEM_F16) return out_type == ELEM_F32 ? launch_pair<kPairStore32, __half, kNone>(m, p, s) : launch_pair<kPairStore16, __half, kNone>(m, p, s);
+    return out_type == ELEM_F32 ? launch_pair<kPairStore32, __nv_bfloat16, kNone>(m, p, s) : launch_pair<kPairStore16, __nv_bfloat16, kNone>(m, p, s);
 }
 
 }  // namespace b200

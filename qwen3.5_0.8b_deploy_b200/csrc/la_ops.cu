@@ -367,7 +367,7 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
         int status = 0;
         if (fp16 && decode && !x_is_fp16 && rows_layer_out(s, (const __half*)la->d_gated, la->d_wout_fp16, d_y, y_beta, rows, kHidden, kLaHeads * kLaVd, la->d_error, &status))
             return status;
-        if (fp16) return gemm_xwT(s, la->d_gated, true, la->d_wout_fp16, true, d_y, false, rows, kHidden, kLaHeads * kLaVd, y_beta);
+        if (fp16) return gemm_xwT(s, la->d_gated, true, la->d_wout_fp16, true, d_y, false, rows, kHidden, kLaHeads * kLaVd, y_beta, 1.0f, 0, la->d_error);
         return gemm_xwT(s, la->d_gated, false, la->d_wout_f32, false, d_y, false, rows, kHidden, kLaHeads * kLaVd, y_beta);
     };
     if (decode) {

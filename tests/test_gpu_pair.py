@@ -94,3 +94,26 @@ def test_more_sequences_than_the_tables_on_chip_hold(ops, cuda, synth):
         st = ops.LinearAttnState(1, n)
         out.append([la.forward_batch(x, st, 0, list(range(n)), counts) for _ in range(2)][1])
     assert ((out[1] - out[0]).norm(dim=1) / out[0].norm(dim=1)).max() <= ROW_REL
+
+
+@pytest.mark.parametrize("rows,fp16_kv", [(14 * 256, 1), (14 * 256 + 1, 0), (38 * 256 - 1, 1), (75 * 256 + 3, 1)])
+def test_large_products_of_a_layer_equal_smaller_ones(ops, cuda, synth, rows, fp16_kv):
+    """Attention layer on both sides of where its products move to the pairs (300 tiles: the input projection above 14 x 256 rows, the output projection above
+    74 x 256), in one call and a sequence at a time: the same sums in the same order, whatever the kernel, so outputs agree to the bit."""
+    torch = cuda
+    w, per = synth.fa_weights(79), 1024
+    counts = [per] * (rows // per) + ([rows % per] if rows % per else [])
+    x = torch.from_numpy(synth.hidden_states(79, "large", rows)).cuda()
+    out = []
+    for chunk in (len(counts), 1):
+        fa = ops.FullAttention(ops.PROJ_FP16, max_batch=len(counts), max_prefill_rows=rows)
+        fa.set_weights(w)
+        kv = ops.KVCache(1, len(counts), per, ops.KV_FP16 if fp16_kv else ops.KV_INT8)
+        slots = [kv.allocate_sequence(per) for _ in counts]
+        y, at = [], 0
+        for i in range(0, len(counts), chunk):
+            n = sum(counts[i:i + chunk])
+            y.append(fa.forward_batch_prefill(x[at:at + n].contiguous(), kv, 0, slots[i:i + chunk], counts[i:i + chunk]))
+            at += n
+        out.append(torch.cat(y))
+    assert torch.equal(out[0], out[1])
