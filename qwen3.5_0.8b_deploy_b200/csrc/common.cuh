@@ -229,6 +229,11 @@ struct b200attn_kv_pool_s {
     b200::LatentView latent_view(int layer) const;
     b200::KvView view() const;
     int sync_lens();                // refresh h_lens from the device when dirty
+    // A step that is over appended `tokens` to the slot in every layer, and nothing else did since the mirror was up to date: it is again.
+    void advance_mirror(int slot, int tokens) {
+        for (int l = 0; l < cfg.num_layers; ++l) h_lens[(size_t)l * cfg.max_seqs + slot] += tokens;
+        lens_dirty = false;
+    }
     size_t layer_stride_elems() const {
         return (size_t)cfg.num_pages * cfg.num_kv_heads * b200::kPageTokens * cfg.head_dim;
     }

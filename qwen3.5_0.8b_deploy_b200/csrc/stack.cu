@@ -822,6 +822,7 @@ extern "C" int b200attn_stack_extend(b200attn_stack st, int row, const int* d_to
     size_t out = 0;
     for (int t = 0, w = 0, n; t < n_tokens; t += n) {
         n = std::min(st->max_rows, n_tokens - t);
+        const bool known = n == 1 && st->pool && !st->pool->lens_dirty;
         if (n == 1) {
             B2_TRY(stack_decode_layers(st, 1, d_tokens + t, st->d_slots + row, s));
         } else if (st->blocks) {
@@ -836,14 +837,17 @@ extern "C" int b200attn_stack_extend(b200attn_stack st, int row, const int* d_to
         if (t + n == n_tokens && d_next) idx.push_back(n - 1);
         const int have = (int)idx.size() - ((t + n == n_tokens && d_next) ? 1 : 0);
         if (idx.empty()) continue;
-        B2_CUDA(cudaMemcpyAsync(st->d_want, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        const int* d_want = n > 1 ? st->d_want : nullptr;              // a single token's outputs are of row 0: no index to bring over
+        if (d_want) B2_CUDA(cudaMemcpyAsync(st->d_want, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, s));
         for (int r0 = 0, k; r0 < have; r0 += k) {                  // the head's row buffer holds max_rows rows
             k = std::min(st->max_rows, have - r0);
-            B2_TRY(stack_logits(st, k, st->d_want + r0, d_logits + out * st->cfg.vocab_size, s));
+            B2_TRY(stack_logits(st, k, d_want ? d_want + r0 : nullptr, d_logits + out * st->cfg.vocab_size, s));
             out += k;
         }
-        if ((int)idx.size() > have) B2_TRY(stack_head(st, 1, st->d_want + have, d_next, nullptr, s));
-        B2_CUDA(cudaStreamSynchronize(s));                          // the index vector goes out of scope
+        if ((int)idx.size() > have) B2_TRY(stack_head(st, 1, d_want ? d_want + have : nullptr, d_next, nullptr, s));
+        B2_CUDA(cudaStreamSynchronize(s));                          // the outputs are there when the call returns; the index vector goes out of scope
+        // The step is over, and with its pages reserved it appended one token in every layer: the next call need not wait for the device and ask.
+        if (known) st->pool->advance_mirror(slot, 1);
     }
     return 0;
 }

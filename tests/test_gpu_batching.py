@@ -87,3 +87,40 @@ def test_admission_errors(ops, cuda, synth):
     st.retire(0)
     n, slots = st.rows()
     assert n == 1 and slots[0] == 1 and slots[1] == -1    # the second sequence moved into row 0
+
+
+def test_lengths_between_single_token_calls(ops, cuda, synth):
+    """Single tokens with and without outputs, a captured step for all rows and portions in turn: what the host believes of the lengths (the limit of the
+    row, its pages) is what the device holds, and the tokens land where a run in one portion puts them."""
+    torch, vocab = cuda, 400
+    from oracle import cpu_stack
+    w = cpu_stack.make_stack_weights(synth, 31, 4, 256, vocab, int8=False, norm_std=0.1)
+
+    def build():
+        st = ops.HybridStack(num_layers=4, intermediate_size=256, vocab_size=vocab, max_seqs=2, max_seq_len=70, prefill_chunk_seqs=2, kv_dtype=1, int8_weights=False)
+        for i, lw in enumerate(w["layers"]):
+            st.set_layer_weights(i, lw, lw["ffn"], fa=lw.get("fa"), la=lw.get("la"))
+        st.set_embedding(w["embed"], w["final_norm"])
+        st.begin_batching()
+        return st
+    toks = torch.from_numpy(synth.rng(31, "toks").integers(0, vocab, 70).astype(np.int32)).cuda()
+    one, many = build(), build()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        want = one.extend(one.open(0), toks, [69])
+        row, at = many.open(0), 0
+        for n, wanted in ((1, True), (1, False), (1, True), (5, True), (1, False), (1, False), (2, False), (1, True)):
+            many.extend(row, toks[at:at + n].contiguous(), [n - 1] if wanted else [])
+            at += n
+        many.set_tokens(toks[at:at + 1].contiguous())
+        many.step(1)
+        at += 1
+        while at < 69:
+            many.extend(row, toks[at:at + 1].contiguous(), [0])
+            at += 1
+        got = many.extend(row, toks[69:].contiguous(), [0])
+        with pytest.raises(ops.InvalidArgument):
+            many.extend(row, toks[:1].contiguous(), [0])          # the row is full, on the host's account too
+        torch.cuda.synchronize()
+    assert many.device_status() == 0
+    # 70 tokens through steps on one side and a prompt pass on the other: fp16 roundings at the same places, sums in another order
+    assert (got - want).norm() <= 2e-2 * want.norm()
