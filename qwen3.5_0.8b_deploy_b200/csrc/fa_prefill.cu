@@ -52,6 +52,7 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t base = smem_u32(smem_raw);
     unsigned char* sm = smem_raw;
+    pdl_enter();
     if (base & 1023u) {            // the 128-byte swizzle needs 1024-byte aligned tiles
         if (threadIdx.x == 0) atomicExch(error_word, 8);
         return;
@@ -553,9 +554,9 @@ int launch_fa_prefill_tc(const __half* q, int rows, const __half* kstage, const 
     const int n_items = n_tiles * kFaHeads;
     dim3 grid(std::min(n_items, n_sm));
     if (out_fp16)
-        fa_prefill_tc_kernel<__half><<<grid, kF1Threads, kF1Smem, s>>>(mq, mk, mv, mo, d_tiles, n_items, gate, (__half*)out, d_error);
+        launch_pdl_if(rows <= kPdlRows, fa_prefill_tc_kernel<__half>, dim3(grid), dim3(kF1Threads), kF1Smem, s, mq, mk, mv, mo, d_tiles, n_items, gate, (__half*)out, d_error);
     else
-        fa_prefill_tc_kernel<float><<<grid, kF1Threads, kF1Smem, s>>>(mq, mk, mv, mo, d_tiles, n_items, gate, (float*)out, d_error);
+        launch_pdl_if(rows <= kPdlRows, fa_prefill_tc_kernel<float>, dim3(grid), dim3(kF1Threads), kF1Smem, s, mq, mk, mv, mo, d_tiles, n_items, gate, (float*)out, d_error);
     B2_LAUNCH_CHECK();
     return 0;
 }

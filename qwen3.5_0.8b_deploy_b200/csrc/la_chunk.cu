@@ -320,6 +320,7 @@ la_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + G_BAR_COUNT);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     auto bar = [&](int i) { return base + kOffBarG + 8u * i; };
+    pdl_enter();
 
     const int h = blockIdx.x;
     const LaSeqMeta sq = seqs[blockIdx.y];
@@ -603,6 +604,7 @@ la_chunk_own_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + G_BAR_COUNT);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     auto bar = [&](int i) { return base + kOffBarG + 8u * i; };
+    pdl_enter();
     const int h = blockIdx.x;
     const LaRun ck = chunk_list[blockIdx.y];
     const LaSeqMeta sq = seqs[ck.seq];
@@ -743,6 +745,7 @@ la_chunk_walk_kernel(const unsigned char* __restrict__ images, const float* __re
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + W_BAR_COUNT);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     auto bar = [&](int i) { return base + 8u * i; };
+    pdl_enter();
     const int h = blockIdx.x;
     const LaSeqMeta sq = seqs[blockIdx.y];
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
@@ -934,13 +937,13 @@ int launch_la_chunk_tc(const __half* q_h, const __half* k_h, const __half* v_h, 
         B2_PER_DEVICE_ONCE(walk, B2_CUDA(cudaFuncSetAttribute(la_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem)));
         unsigned char* images = static_cast<unsigned char*>(split.scratch);
         float* decay = reinterpret_cast<float*>(images + (size_t)split.n_chunks * kLaHeads * kImg);
-        la_chunk_own_kernel<<<dim3(kLaHeads, split.n_chunks), kG1Threads, kG1Smem, s>>>(mq, mk, mv, g, beta, d_seqs, split.d_chunks, images, decay, d_error);
+        launch_pdl_if(rows <= kPdlRows, la_chunk_own_kernel, dim3(kLaHeads, split.n_chunks), dim3(kG1Threads), kG1Smem, s, mq, mk, mv, g, beta, d_seqs, split.d_chunks, images, decay, d_error);
         B2_LAUNCH_CHECK();
-        la_chunk_walk_kernel<<<grid, kG1Threads, kWalkSmem, s>>>(images, decay, d_seqs, split.d_first, rec_layer, rec_stride, out, d_error);
+        launch_pdl_if(rows <= kPdlRows, la_chunk_walk_kernel, grid, dim3(kG1Threads), kWalkSmem, s, images, decay, d_seqs, split.d_first, rec_layer, rec_stride, out, d_error);
         B2_LAUNCH_CHECK();
         return 0;
     }
-    la_chunk_tc_kernel<<<grid, kG1Threads, kG1Smem, s>>>(mq, mk, mv, g, beta, d_seqs, rec_layer, rec_stride, out, d_error);
+    launch_pdl_if(rows <= kPdlRows, la_chunk_tc_kernel, grid, dim3(kG1Threads), kG1Smem, s, mq, mk, mv, g, beta, d_seqs, rec_layer, rec_stride, out, d_error);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 namespace b200 {
 
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(256)
 la_conv_tail_kernel(const float* __restrict__ mixed, const LaSeqMeta* __restrict__ seqs, int n_seqs, float* __restrict__ conv_state_layer,
                     size_t conv_stride_slot, int gate_rows, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                     float* __restrict__ g_out, float* __restrict__ beta_out) {
+    pdl_enter();
     if (blockIdx.x >= n_seqs) {
         const int row = ((blockIdx.x - n_seqs) * gridDim.y + blockIdx.y) * 16 + (threadIdx.x >> 4), h = threadIdx.x & 15;
         if (row >= gate_rows) return;
@@ -222,10 +224,12 @@ la_recurrent_serial_kernel(const float* __restrict__ q, const float* __restrict_
 }
 
 // ---- gated RMSNorm epilogue: o * rsqrt(mean(o^2)+1e-6) * w * silu(z), one warp per (row, head) ------------
-template <typename OutT>
+// kDependent: launched as a programmatic dependent (few rows; 65536 rows take 271 us with the wait in it and 224 without).
+template <typename OutT, bool kDependent>
 __global__ void __launch_bounds__(128)
 la_gated_norm_kernel(const float* __restrict__ core, const float* __restrict__ mixed, const float* __restrict__ norm_w,
                      int rows, OutT* __restrict__ out) {
+    if constexpr (kDependent) pdl_enter();
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (gw >= rows * kLaHeads) return;
@@ -416,8 +420,8 @@ int launch_la_conv_seq(const float* mixed, const LaRun* d_runs, int n_runs, cons
 int launch_la_conv_tail(const float* mixed, const LaSeqMeta* d_seqs, int n_seqs, float* conv_layer, size_t conv_stride, int gate_rows, const float* a_log,
                         const float* dt_bias, float* g, float* beta, cudaStream_t s) {
     constexpr int kCols = kLaConvDim / 256;
-    la_conv_tail_kernel<<<dim3(n_seqs + ceil_div(gate_rows, 16 * kCols), kCols), 256, 0, s>>>(mixed, d_seqs, n_seqs, conv_layer, conv_stride, gate_rows, a_log,
-                                                                                            dt_bias, g, beta);
+    launch_pdl_if(gate_rows <= kPdlRows, la_conv_tail_kernel, dim3(n_seqs + ceil_div(gate_rows, 16 * kCols), kCols), dim3(256), 0, s, mixed, d_seqs, n_seqs, conv_layer, conv_stride,
+               gate_rows, a_log, dt_bias, g, beta);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -431,11 +435,13 @@ int launch_la_recurrent_serial(const float* q, const float* k, const float* v, c
 }
 int launch_la_gated_norm(const float* core, const float* mixed, const float* norm_w, int rows, void* out,
                          bool out_fp16, cudaStream_t s) {
-    const int blocks = ceil_div(rows * kLaHeads, 4);
-    if (out_fp16)
-        la_gated_norm_kernel<__half><<<blocks, 128, 0, s>>>(core, mixed, norm_w, rows, (__half*)out);
-    else
-        la_gated_norm_kernel<float><<<blocks, 128, 0, s>>>(core, mixed, norm_w, rows, (float*)out);
+    const dim3 grid(ceil_div(rows * kLaHeads, 4)), block(128);
+    auto launch = [&](auto* typed) {
+        using T = std::remove_pointer_t<decltype(typed)>;
+        if (rows <= kPdlRows) launch_pdl(la_gated_norm_kernel<T, true>, grid, block, 0, s, core, mixed, norm_w, rows, typed);
+        else la_gated_norm_kernel<T, false><<<grid, block, 0, s>>>(core, mixed, norm_w, rows, typed);
+    };
+    if (out_fp16) launch((__half*)out); else launch((float*)out);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -201,6 +201,7 @@ __global__ void iota_kernel(int* p, int n) {
     if (i < n) p[i] = i;
 }
 __global__ void last_row_index_kernel(int* idx, int n_seqs, int len) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_seqs) idx[i] = i * len + len - 1;
 }
@@ -668,7 +669,7 @@ static int stack_prefill_slots(b200attn_stack st, const int* h_slots, int n_seqs
                 n = std::min(st->max_rows, prompt_len - t);
                 B2_TRY(block_prefill_rows(*st->blocks, 1, h_slots + i, &n, d_tokens + (size_t)i * prompt_len + t, s));
                 if (t + n < prompt_len) continue;
-                last_row_index_kernel<<<1, 128, 0, s>>>(st->d_last_idx, 1, n);
+                launch_pdl_if(n <= kPdlRows, last_row_index_kernel, dim3(1), dim3(128), 0, s, st->d_last_idx, 1, n);
                 count_launch();
                 B2_TRY(stack_head(st, 1, st->d_last_idx, d_next + i, d_hidden_out, s));
             }
@@ -690,7 +691,7 @@ static int stack_prefill_slots(b200attn_stack st, const int* h_slots, int n_seqs
             rc = stack_layers(st, rows, h_slots + s0, counts.data(), n, nullptr, false, s);
         }
         if (rc != 0) break;
-        last_row_index_kernel<<<ceil_div(n, 128), 128, 0, s>>>(d_idx, n, prompt_len);
+        launch_pdl_if(rows <= kPdlRows, last_row_index_kernel, dim3(ceil_div(n, 128)), dim3(128), 0, s, d_idx, n, prompt_len);
         count_launch();
         rc = stack_head(st, n, d_idx, d_next + s0, d_hidden_out ? d_hidden_out + (size_t)s0 * kHidden : nullptr, s);
     }
