@@ -27,7 +27,7 @@ namespace {
 constexpr uint32_t kOperand = 128 * 128;                // 128 rows of 64 two-byte elements
 constexpr uint32_t kStage = 2 * kOperand;
 constexpr int kEpiWarps = 16;
-constexpr int kThreads = 32 * (kEpiWarps + 2);          // epilogue warps, one for loads, one for products (CTA 0) or the hand-over of slices (CTA 1)
+constexpr int kThreads = 32 * (kEpiWarps + 2);          // epilogue warps, one for loads, one for TMEM and (CTA 0) the products
 
 enum { kPairGlu = 0, kPairConv, kPairStore16, kPairStore32 };
 constexpr int kConvTokens = 253;                        // of a tile of 256 columns: the first three are the taps of the fourth
@@ -346,8 +346,9 @@ __device__ __forceinline__ void conv_part(const LaConvArgs& a, const PairMaps& m
     }
 }
 
-// grid 2 x pairs, clusters of two.  Rank 0 of a pair issues the products once its own slice and its neighbour's have landed; the neighbour's
-// product warp passes that on (its loads signal its own barrier).  Operand a gives the rows of the product (X, kPairConv: W), b its columns.
+// grid 2 x pairs, clusters of two.  Rank 0 of a pair issues the products once its own slice and its neighbour's have landed: the copies of both CTAs
+// complete on its barrier.  Every barrier here is signalled from the other CTA too, so all waits are of cluster scope.  Operand a gives the rows of
+// the product (X, kPairConv: W), b its columns.
 template <int EPI, typename T, int kAct>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
@@ -361,7 +362,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + kBars + 248);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kBars + 252);
     const uint32_t bar0 = base + kBars;
-    auto full = [&](int s) { return bar0 + 8u * s; };                          // this CTA's slice has landed, in rank 0 the neighbour's too
+    auto full = [&](int s) { return bar0 + 8u * s; };                          // rank 0: the slices of both CTAs have landed
     auto empty = [&](int s) { return bar0 + 8u * (kStages + s); };             // the products that read it are done
     auto acc_full = [&](int b) { return bar0 + 8u * (2 * kStages + b); };
     auto acc_empty = [&](int b) { return bar0 + 8u * (2 * kStages + 2 + b); }; // rank 0: the epilogue warps of both CTAs have read it
@@ -371,7 +372,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
-            mbar_init(full(i), 2 - rank);
+            mbar_init(full(i), 1);
             mbar_init(empty(i), 1);
         }
         mbar_init(acc_full(0), 1);
@@ -393,7 +394,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
     const PairItem first(p, pair);
     tc_fence_before();
     __syncthreads();
-    cluster_meet_all();                   // the barriers of both CTAs are in place
+    cluster_sync_all();                   // the barriers and the TMEM of both CTAs are in place
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_wait();
@@ -404,37 +405,40 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
     if (warp == kEpiWarps) {
         int s = 0, issued = 0;
         uint32_t parity = 1;
+        const uint32_t landed = cluster_smem_addr(full(0), 0);
         bool ok = true;
         PairItem w = first;
         for (int t = pair; t < p.items && ok; t += pairs) {
             if (t != pair) w = PairItem(p, t);
             const int a_row = (EPI == kPairConv ? w.col : w.row * 256) + rank * 128;
             const int b_row = EPI == kPairConv ? w.row * kConvTokens - 3 + rank * 128 : p.up ? w.col / 2 + rank * p.up : w.col + rank * w.width / 2;
-            const uint32_t bytes = kOperand + w.width * 64;
+            const uint32_t bytes = 2 * (kOperand + w.width * 64);              // of both CTAs
             for (int k = 0; k < 64 * p.k_steps; k += 64) {
-                if (!mbar_wait_warp(empty(s), parity, abort_flag)) { ok = false; break; }
-                const uint32_t dst = base + s * kStage, bar = full(s);
+                if (!mbar_wait_warp<kClusterScope>(empty(s), parity, abort_flag)) { ok = false; break; }
+                const uint32_t dst = base + s * kStage, bar = landed + 8u * s;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(bar, bytes);
-                    tma_load_2d(dst, &maps.a, bar, k, a_row);
-                    if (w.width == 256) tma_load_2d(dst + kOperand, &maps.b, bar, k, b_row);
+                    if (rank == 0) mbar_arrive_expect_tx(full(s), bytes);          // the neighbour's bytes may come in first: the phase waits for this arrival
+                    tma_load_2d_pair(dst, &maps.a, bar, k, a_row);
+                    if (w.width == 256) tma_load_2d_pair(dst + kOperand, &maps.b, bar, k, b_row);
                     else
-                        for (int r = 0; r < w.width / 2; r += 32) tma_load_2d(dst + kOperand + r * 128, &maps.b32, bar, k, b_row + r);
+                        for (int r = 0; r < w.width / 2; r += 32) tma_load_2d_pair(dst + kOperand + r * 128, &maps.b32, bar, k, b_row + r);
                 }
                 ++issued;
                 if (++s == kStages) { s = 0; parity ^= 1; }
             }
         }
-        // A copy or an arrival of the neighbour's that is still under way must not find this CTA gone.
-        if (lane == 0)
-            for (int j = max(0, issued - kStages); j < issued; ++j) {
-                if (!ok) mbar_drain(full(j % kStages), (j / kStages) & 1);
-                else mbar_wait(empty(j % kStages), (j / kStages) & 1, abort_flag);
-            }
+        // A copy or an arrival of the neighbour's that is still under way must not find this CTA gone.  When a wait has run out, rank 0 waits for the
+        // copies of both, then for as long again (a phase that nothing completes) for what the neighbour may have asked for beyond.
+        if (lane == 0) {
+            if (ok)
+                for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait<kClusterScope>(empty(j % kStages), (j / kStages) & 1, abort_flag);
+            else if (rank == 0)
+                for (int j = max(0, issued - kStages); j <= issued; ++j) mbar_drain(full(j % kStages), (j / kStages) & 1);
+        }
     } else if (warp == kEpiWarps + 1) {
-        int s = 0;
-        uint32_t parity = 0;
         if (rank == 0) {
+            int s = 0;
+            uint32_t parity = 0;
             constexpr uint32_t fmt = std::is_same<T, __half>::value ? kFmtF16 : kFmtBF16;
             const uint64_t a0 = umma_smem_desc(base, 16, 1024), w0 = umma_smem_desc(base + kOperand, 16, 1024);
             int i = 0;
@@ -444,11 +448,11 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
                 const int b = i & 1;
                 if (t != pair) w = PairItem(p, t);
                 const uint32_t idesc = umma_idesc(fmt, 256, w.width, 0, 0);
-                if (!mbar_wait_warp(acc_empty(b), ((i >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_warp<kClusterScope>(acc_empty(b), ((i >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d = tmem + b * 256;
                 for (int ks = 0; ks < p.k_steps; ++ks) {
-                    if (!mbar_wait_warp(full(s), parity, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp<kClusterScope>(full(s), parity, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint64_t a = a0 + s * (kStage >> 4), wd = w0 + s * (kStage >> 4);
                     const uint32_t done = empty(s);
@@ -462,14 +466,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
                 }
                 if (ok && elect_one()) umma_commit_pair(acc_full(b));
             }
-            for (int j = max(0, i - 2); ok && j < i; ++j) ok = mbar_wait_warp(acc_empty(j & 1), (j >> 1) & 1, abort_flag);     // the neighbour's arrivals
-        } else {
-            const uint32_t theirs = cluster_smem_addr(full(0), 0);
-            for (int left = (p.items - pair + pairs - 1) / pairs * p.k_steps; left > 0; --left) {
-                if (!mbar_wait_warp(full(s), parity, abort_flag)) break;
-                if (elect_one()) mbar_arrive_cluster(theirs + 8u * s);
-                if (++s == kStages) { s = 0; parity ^= 1; }
-            }
+            for (int j = max(0, i - 2); ok && j < i; ++j) ok = mbar_wait_warp<kClusterScope>(acc_empty(j & 1), (j >> 1) & 1, abort_flag);     // the neighbour's arrivals
         }
     } else {
         const int q = warp & 3, part = warp >> 2;          // TMEM lanes 32 q .. 32 q + 31, a quarter of the columns
@@ -507,11 +504,11 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
                 info[mine] = token_info(p.la, first_rows, p.rows, t_tile + mine);
                 __syncwarp();
                 bar_sync(2 + half, 256);
-                ok = ok && mbar_wait_warp(acc_full(b), (i >> 1) & 1, abort_flag);
+                ok = ok && mbar_wait_warp<kClusterScope>(acc_full(b), (i >> 1) & 1, abort_flag);
                 tc_fence_after();
                 conv_part(p.la, maps, ok, acc, w.col >> 8, t_tile, p.rows, rank, q, side, lane, info, first_rows, sums, 4 + 2 * half + side, scale, out, release);
             } else {
-                if (!mbar_wait_warp(acc_full(b), (i >> 1) & 1, abort_flag)) break;
+                if (!mbar_wait_warp<kClusterScope>(acc_full(b), (i >> 1) & 1, abort_flag)) break;
                 tc_fence_after();
                 if constexpr (EPI != kPairGlu) {
                     if (64 * part < w.width)
@@ -526,7 +523,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
     }
     tc_fence_before();
     __syncthreads();
-    cluster_meet_all();                   // neither CTA reads the other's shared memory, arrives on its barriers or works on its TMEM any more
+    cluster_sync_all();                   // neither CTA reads the other's shared memory, arrives on its barriers or works on its TMEM any more
     if (warp == kEpiWarps + 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem, 512);

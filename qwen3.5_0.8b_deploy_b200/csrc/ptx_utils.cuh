@@ -40,15 +40,27 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// kClusterScope: of a barrier that the other CTAs of the cluster signal as well; what they did in front of their signal is then seen by this thread.
+enum MbarScope { kCtaScope, kClusterScope };
+template <MbarScope SCOPE = kCtaScope>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if constexpr (SCOPE == kClusterScope)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 // Non-blocking probe (try_wait may park the thread for a while when the phase is not complete; a producer that
@@ -66,13 +78,14 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 }
 // Bounded wait: gives up after `limit_ns` or as soon as another thread of the CTA raised *abort_flag.
 // Returns false on give-up (and raises the flag), so every role can fall through to the common exit.
+template <MbarScope SCOPE = kCtaScope>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           uint64_t limit_ns = 500000000ull) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<SCOPE>(bar, parity)) return true;
     const uint64_t t0 = global_timer_ns();
     uint32_t it = 0;
     while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait<SCOPE>(bar, parity)) return true;
         if ((++it & 63u) == 0u) {
             if (*abort_flag) return false;
             if (global_timer_ns() - t0 > limit_ns) {
@@ -90,22 +103,15 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, uint64
     while (!mbar_try_wait(bar, parity) && global_timer_ns() - t0 < limit_ns) {}
 }
 
-// The same without a memory fence: neither CTA goes on before the other has come this far.
-__device__ __forceinline__ void cluster_meet_all() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
-
-// Address of the same shared-memory location in CTA `rank` of the cluster, and an arrival on a barrier there.  The arrival orders what the
-// asynchronous units did (copies that this thread has seen land, TMEM reads behind their fence), not ordinary writes for a reader in the other CTA:
-// with .release.cluster it waits for those as well, which held a hand-over per 64-deep slice of a product to 0.8 us.
+// Address of the same shared-memory location in CTA `rank` of the cluster, and an arrival on a barrier there, behind everything that this thread did
+// before (to be waited for at kClusterScope).
 __device__ __forceinline__ uint32_t cluster_smem_addr(uint32_t local_smem_addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
     return r;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // Every thread of every CTA of the cluster (threads that have exited do not count).
@@ -116,8 +122,9 @@ __device__ __forceinline__ void cluster_sync_all() {
 
 // Warp-uniform form for roles whose next instruction is warp-collective (.sync.aligned): either every
 // lane proceeds or every lane gives up.
+template <MbarScope SCOPE = kCtaScope>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    const bool r = mbar_wait(bar, parity, abort_flag);
+    const bool r = mbar_wait<SCOPE>(bar, parity, abort_flag);
     return __all_sync(0xffffffffu, r);
 }
 

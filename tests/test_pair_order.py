@@ -1,0 +1,34 @@
+"""What passes between the two CTAs of a pair is ordered for a reader in the other one: signals release and waits acquire at the scope of the cluster, and the
+copies of both CTAs complete on the barrier that the products wait for.  Read from the sources: an order that is missing cannot be provoked."""
+import re
+
+from test_launch_order import KERNELS, SOURCES, CSRC
+
+import glob
+import os
+
+
+def _texts():
+    headers = {os.path.basename(p): open(p).read() for p in glob.glob(os.path.join(CSRC, "*.cuh"))}
+    return {**headers, **{f: open(os.path.join(CSRC, f)).read() for f in SOURCES}}
+
+
+def test_arrivals_at_another_cta_release_to_it():
+    found = [(f, m.group()) for f, text in _texts().items() for m in re.finditer(r"mbarrier\.arrive[\w.:]*shared::cluster[\w.:]*", text)]
+    assert found
+    assert not [x for x in found if ".release.cluster" not in x[1]]
+
+
+def test_every_wait_of_a_pair_is_of_cluster_scope():
+    pairs = {k: body for k, body in KERNELS.items() if re.search(r"\bumma_f16_pair\b", body)}
+    assert pairs
+    for kernel, body in pairs.items():
+        waits = re.findall(r"\bmbar_(?:try_|test_)?wait(?:_warp)?\b\s*(<\w+>)?", body)
+        assert waits and set(waits) == {"<kClusterScope>"}, kernel
+        assert not re.search(r"\bcluster_\w*meet\w*\b", body), kernel
+        loads = set(re.findall(r"\btma_load_2d\w*\b", body))
+        assert loads == {"tma_load_2d_pair"}, kernel
+        signal = re.search(r"const uint32_t dst = [^;]*, bar = (\w+) \+ 8u \* s;", body)
+        assert signal and re.search(r"\b%s = cluster_smem_addr\(full\(0\), 0\);" % signal.group(1), body), kernel
+    wait = re.search(r"bool mbar_try_wait\(.*?\n}\n", _texts()["ptx_utils.cuh"], re.S).group()
+    assert re.search(r"SCOPE == kClusterScope\).*?try_wait\.parity\.acquire\.cluster\.", wait, re.S)
