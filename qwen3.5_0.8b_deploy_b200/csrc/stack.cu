@@ -838,7 +838,7 @@ extern "C" int b200attn_stack_extend(b200attn_stack st, int row, const int* d_to
         if (t + n == n_tokens && d_next) idx.push_back(n - 1);
         const int have = (int)idx.size() - ((t + n == n_tokens && d_next) ? 1 : 0);
         if (idx.empty()) continue;
-        const int* d_want = n > 1 ? st->d_want : nullptr;              // a single token's outputs are of row 0: no index to bring over
+        const int* d_want = n > 1 || have > 1 ? st->d_want : nullptr;  // a single token's output is of row 0: no index to bring over (unless it is wanted repeatedly)
         if (d_want) B2_CUDA(cudaMemcpyAsync(st->d_want, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, s));
         for (int r0 = 0, k; r0 < have; r0 += k) {                  // the head's row buffer holds max_rows rows
             k = std::min(st->max_rows, have - r0);

@@ -124,3 +124,29 @@ def test_lengths_between_single_token_calls(ops, cuda, synth):
     assert many.device_status() == 0
     # 70 tokens through steps on one side and a prompt pass on the other: fp16 roundings at the same places, sums in another order
     assert (got - want).norm() <= 2e-2 * want.norm()
+
+
+@pytest.mark.parametrize("stack", ["hybrid", "layers"])
+def test_places_wanted_more_than_once(ops, cuda, synth, stack):
+    """Wanted places may repeat, also in a single-token call and in a pass that ends with one token (33 tokens in passes of 32 rows)."""
+    torch = cuda
+    if stack == "hybrid":
+        from oracle import cpu_stack
+        w = cpu_stack.make_stack_weights(synth, 32, 4, 256, 400, int8=False, norm_std=0.1)
+        st = ops.HybridStack(num_layers=4, intermediate_size=256, vocab_size=400, max_seqs=2, max_seq_len=70, prefill_chunk_seqs=2, kv_dtype=1, int8_weights=False)
+        for i, lw in enumerate(w["layers"]):
+            st.set_layer_weights(i, lw, lw["ffn"], fa=lw.get("fa"), la=lw.get("la"))
+        st.set_embedding(w["embed"], w["final_norm"])
+    else:
+        import test_gpu_nuzopel as nuzopel
+        models, wts = (importlib.import_module(f"{entry.PKG_NAME}.{m}") for m in ("models", "weights"))
+        st = nuzopel.Case(models, wts, *nuzopel.make([nuzopel.mlstm(2, 32, 32, ff=64)], width=96, vocab=400, seed=3), "bfloat16", max_pass_rows=32).stack
+    st.begin_batching()
+    toks = torch.from_numpy(synth.rng(32, "toks").integers(0, 400, 36).astype(np.int32)).cuda()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        row = st.open(40)
+        first = st.extend(row, toks[:33].contiguous(), [0, 31, 32, 32, 32])
+        got, token = st.extend(row, toks[33:34].contiguous(), [0, 0, 0], want_next=True)
+        torch.cuda.synchronize()
+    assert torch.equal(first[2], first[3]) and torch.equal(first[2], first[4]) and not torch.equal(first[1], first[2])
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2]) and int(token) == int(got[0].argmax())
