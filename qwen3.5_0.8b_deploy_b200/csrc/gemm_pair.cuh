@@ -26,7 +26,7 @@ struct LaConvArgs {
     __half *q, *k, *v;
     float* mixed;
 };
-bool gemm_la_conv_takes(const void* x, const void* w);
+bool gemm_la_conv_takes(const void* x, const void* w, long long rows, int n_seqs);
 int gemm_la_conv(cudaStream_t s, const __half* x, const __half* w, int rows, const LaConvArgs& la, int* error);
 
 }  // namespace b200

@@ -24,7 +24,7 @@ __device__ __forceinline__ float warp_sum_f(float v) {
     return v;
 }
 // ---- C1, sequence form -------------------------------------------------------------------------------
-// For fp32 projections and the serial recurrence; the fp16 layers convolve in the epilogue of their projection (gemm_pair.cu).
+// For fp32 projections, the serial recurrence and short passes of several sequences; others of fp16 layers convolve in the epilogue of their projection (gemm_pair.cu).
 // One warp per (run of up to kConvRun consecutive rows of one sequence, head, part) with part = q, k or v channels of the head: conv +
 // SiLU, L2 norm of q and k (eps inside the sqrt), q * 1/sqrt(128); the v warps also produce beta and the log-decay g.
 // A warp requests its whole input window (the run's rows plus three rows of history, 16 bytes per lane and row) before

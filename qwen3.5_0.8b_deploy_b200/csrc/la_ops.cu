@@ -386,7 +386,9 @@ int la_forward_rows(b200attn_la la, b200attn_la_state st, int layer, const int* 
     int n_runs = 0;
     LaSplit split;
     const bool tc = la_use_tensor_cores();
-    const bool fused = tc && fp16 && gemm_la_conv_takes(x_is_fp16 ? d_x : la->d_xb, la->d_win_fp16);
+    long long all_rows = 0;
+    for (int i = 0; h_counts && i < n_seqs; ++i) all_rows += h_counts[i];
+    const bool fused = tc && fp16 && gemm_la_conv_takes(x_is_fp16 ? d_x : la->d_xb, la->d_win_fp16, all_rows, n_seqs);
     B2_TRY(la_build_meta(la, st, h_slots, h_counts, n_seqs, &rows, seqs, &d_seqs, fused ? nullptr : &d_runs, &n_runs, tc ? &split : nullptr, s));
     if (rows == 0) return 0;
     B2_CHECK_ARG(rows <= la->cfg.max_prefill_rows, "la_prefill: %d rows exceed max_prefill_rows %d", rows, la->cfg.max_prefill_rows);

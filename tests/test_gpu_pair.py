@@ -1,5 +1,6 @@
 """GPU: prompt-sized products on pairs of CTAs with their successor in the epilogue, at the edges of their tiles (feed-forward: 256 rows, 128 outputs, parts
-of 32; DeltaNet projection: 253 tokens behind 3 that only serve as taps, 32 at a time) and of their dispatch (feed-forward: more than 128 rows)."""
+of 32; DeltaNet projection: 253 tokens behind 3 that only serve as taps, 32 at a time) and of their dispatch (feed-forward: more than 128 rows; DeltaNet
+projection: one sequence, or from 300 rows and 36 more for each sequence on, at most 3000, and 24 rows a sequence)."""
 import os
 import sys
 
@@ -56,13 +57,22 @@ def test_feed_forward_widths(cuda, models, wts, ff, width, rows):      # noqa: F
 ROW_REL = 5e-3
 
 
+def fused_rows(n):
+    """From so many rows on, a pass of n sequences takes the projection with the convolution in its epilogue."""
+    return max(min(300 + 36 * n, 3000), 24 * n) if n > 1 else 1
+
+
+@pytest.mark.parametrize("fused", [False, True])
 @pytest.mark.parametrize("counts", [
     [1], [2, 1, 3], [31, 1, 33, 64], [247, 16, 5], [248, 2, 3, 1, 20], [249, 1, 40], [250, 3, 252, 7], [251, 2, 1, 1, 1, 90], [252, 260], [253, 253, 4], [254, 0, 40, 0],
     [16] * 40, [1] * 70, [506, 33], [600],
 ])
-def test_convolution_at_the_edges_of_tiles_and_sequences(ops, cuda, synth, counts):
+def test_convolution_at_the_edges_of_tiles_and_sequences(ops, cuda, synth, counts, fused):
     """Sequence starts and ends at every place around a tile's first tokens, in the middle of its chunks, several to a chunk; two calls, the second with
-    the state that the first left behind, against the layer with fp32 projections (convolution in a kernel of its own)."""
+    the state that the first left behind, against the layer with fp32 projections (convolution in a kernel of its own).  fused: with one more sequence
+    behind them, which brings the pass to the fewest rows that the fused projection takes; without it most of them are below."""
+    if fused:
+        counts = counts + [max(1, fused_rows(len(counts) + 1) - sum(counts))]
     torch, n = cuda, len(counts)
     w = synth.la_weights(77)
     out, conv = [], []
@@ -84,10 +94,11 @@ def test_convolution_at_the_edges_of_tiles_and_sequences(ops, cuda, synth, count
 
 
 def test_more_sequences_than_the_tables_on_chip_hold(ops, cuda, synth):
-    """Above 512 sequences their first rows and slots are read from memory."""
-    torch, n = cuda, 600
+    """Above 512 sequences their first rows and slots are read from memory.  The last one is as long as the fused projection needs."""
+    torch, n = cuda, 514
     w = synth.la_weights(78)
-    counts = [1 + i % 3 for i in range(n)]
+    counts = [1 + i % 3 for i in range(n - 1)]
+    counts.append(fused_rows(n) - sum(counts))
     x = torch.from_numpy(synth.hidden_states(78, "many", sum(counts))).cuda()
     out = []
     for proj in (ops.PROJ_FP32, ops.PROJ_FP16):
