@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/b200attn.h"
+#include "len_mirror.h"
 
 namespace b200 {
 
@@ -221,7 +222,7 @@ struct b200attn_kv_pool_s {
     int* d_meta = nullptr;          // scratch for slots / cu_rows of append & export calls
     int meta_cap = 0;
     std::vector<int> h_lens;        // [layers][max_seqs] mirror
-    bool lens_dirty = false;        // device lengths advanced without the host (decode / graph replay)
+    b200::MirrorMarks lens_marks;   // device lengths advanced without the host (decode / graph replay)
     std::vector<std::vector<int>> seq_pages;
     std::vector<char> slot_used;
     std::vector<int> free_pages;
@@ -233,11 +234,12 @@ struct b200attn_kv_pool_s {
     std::vector<int> latent_pitch;       // elements per row
     b200::LatentView latent_view(int layer) const;
     b200::KvView view() const;
-    int sync_lens();                // refresh h_lens from the device when dirty
-    // A step that is over appended `tokens` to the slot in every layer, and nothing else did since the mirror was up to date: it is again.
-    void advance_mirror(int slot, int tokens) {
-        for (int l = 0; l < cfg.num_layers; ++l) h_lens[(size_t)l * cfg.max_seqs + slot] += tokens;
-        lens_dirty = false;
+    int sync_lens();                // refresh h_lens from the device when it may be behind
+    // This thread's steps since `at`, where the mirror was up to date, are over: they appended `tokens` to the slot in every layer.
+    void advance_mirror(b200::MirrorMarks::Point at, int slot, int tokens) {
+        lens_marks.enter_own(at, [&] {
+            for (int l = 0; l < cfg.num_layers; ++l) h_lens[(size_t)l * cfg.max_seqs + slot] += tokens;
+        });
     }
     size_t layer_stride_elems() const {
         return (size_t)cfg.num_pages * cfg.num_kv_heads * b200::kPageTokens * cfg.head_dim;

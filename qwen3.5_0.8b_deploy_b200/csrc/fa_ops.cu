@@ -234,7 +234,7 @@ int fa_forward_rows(b200attn_fa fa, b200attn_kv_pool pool, int layer, const int*
         B2_TRY(launch_fa_decode(kv, layer, d_slots_in, n_seqs, fa->d_q, false, fa->d_gate, kMaxSplitsCap, fa->d_part_o,
                                 fa->d_part_ml, fa->d_counters, fa->d_attn, fp16, s));
         B2_TRY(fa_project_out(fa, d_y, y_beta, n_seqs, !x_is_fp16, dout, pool->d_error, s));
-        pool->lens_dirty = true;
+        pool->lens_marks.mark();
         return 0;
     }
     std::vector<int> base;

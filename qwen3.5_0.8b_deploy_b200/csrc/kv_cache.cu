@@ -455,13 +455,13 @@ b200::KvView b200attn_kv_pool_s::view() const {
 }
 
 int b200attn_kv_pool_s::sync_lens() {
-    if (!lens_dirty) return 0;
     // Decode steps and graph replays advance the lengths on streams the pool does not know (non-blocking streams do not
     // order against the legacy stream a plain cudaMemcpy uses), so wait for the whole device first.
-    B2_CUDA(cudaDeviceSynchronize());
-    B2_CUDA(cudaMemcpy(h_lens.data(), d_lens, h_lens.size() * sizeof(int), cudaMemcpyDeviceToHost));
-    lens_dirty = false;
-    return 0;
+    return lens_marks.refresh([&]() -> int {
+        B2_CUDA(cudaDeviceSynchronize());
+        B2_CUDA(cudaMemcpy(h_lens.data(), d_lens, h_lens.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        return 0;
+    });
 }
 
 b200::LatentView b200attn_kv_pool_s::latent_view(int layer) const {
@@ -668,8 +668,7 @@ extern "C" int b200attn_kv_seq_shrink(b200attn_kv_pool p, int slot, int new_len)
 extern "C" int b200attn_kv_clear(b200attn_kv_pool p, b200attn_stream stream) {
     B2_CHECK_ARG(p, "kv_clear: null pool");
     B2_CUDA(cudaMemsetAsync(p->d_lens, 0, p->h_lens.size() * sizeof(int), as_stream(stream)));
-    std::fill(p->h_lens.begin(), p->h_lens.end(), 0);
-    p->lens_dirty = false;
+    p->lens_marks.set_both([&] { std::fill(p->h_lens.begin(), p->h_lens.end(), 0); });
     return 0;
 }
 

@@ -624,7 +624,7 @@ static int stack_head(b200attn_stack st, int n_seqs, const int* d_row_index, int
 // The layers of one decode step over n rows whose slots are d_slots[0 .. n).
 static int stack_decode_layers(b200attn_stack st, int n_seqs, const int* d_tokens_in, const int* d_slots, cudaStream_t s) {
     if (st->blocks) {
-        if (st->pool) st->pool->lens_dirty = true;
+        if (st->pool) st->pool->lens_marks.mark();
         return block_decode_rows(*st->blocks, n_seqs, d_tokens_in, d_slots, s);
     }
     if (n_seqs <= 128 && gemm_tc_enabled())
@@ -633,7 +633,7 @@ static int stack_decode_layers(b200attn_stack st, int n_seqs, const int* d_token
     else
         launch_pdl_split(true, n_seqs <= kRowsGemmMax, embed_gather_kernel, dim3(n_seqs), dim3(256), 0, s, d_tokens_in, st->d_embed, st->cfg.vocab_size, st->d_h);
     B2_LAUNCH_CHECK();
-    if (st->pool) st->pool->lens_dirty = true;
+    if (st->pool) st->pool->lens_marks.mark();
     return stack_layers(st, n_seqs, nullptr, nullptr, n_seqs, d_slots, true, s);
 }
 
@@ -823,7 +823,7 @@ extern "C" int b200attn_stack_extend(b200attn_stack st, int row, const int* d_to
     size_t out = 0;
     for (int t = 0, w = 0, n; t < n_tokens; t += n) {
         n = std::min(st->max_rows, n_tokens - t);
-        const bool known = n == 1 && st->pool && !st->pool->lens_dirty;
+        const MirrorMarks::Point at = st->pool ? st->pool->lens_marks.here() : MirrorMarks::Point{};
         if (n == 1) {
             B2_TRY(stack_decode_layers(st, 1, d_tokens + t, st->d_slots + row, s));
         } else if (st->blocks) {
@@ -848,7 +848,7 @@ extern "C" int b200attn_stack_extend(b200attn_stack st, int row, const int* d_to
         if ((int)idx.size() > have) B2_TRY(stack_head(st, 1, d_want ? d_want + have : nullptr, d_next, nullptr, s));
         B2_CUDA(cudaStreamSynchronize(s));                          // the outputs are there when the call returns; the index vector goes out of scope
         // The step is over, and with its pages reserved it appended one token in every layer: the next call need not wait for the device and ask.
-        if (known) st->pool->advance_mirror(slot, 1);
+        if (n == 1 && st->pool) st->pool->advance_mirror(at, slot, 1);
     }
     return 0;
 }
@@ -926,7 +926,7 @@ extern "C" int b200attn_decode_graph_launch(b200attn_stack st, int steps, b200at
     B2_CHECK_ARG(steps > 0, "decode_graph_launch: steps must be > 0");
     for (int i = 0; i < steps; ++i) B2_CUDA(cudaGraphLaunch(st->graph_exec, as_stream(stream)));
     g_launches += st->graph_nodes * steps;
-    if (st->pool) st->pool->lens_dirty = true;
+    if (st->pool) st->pool->lens_marks.mark();
     return 0;
 }
 
