@@ -366,6 +366,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
     auto empty = [&](int s) { return bar0 + 8u * (kStages + s); };             // the products that read it are done
     auto acc_full = [&](int b) { return bar0 + 8u * (2 * kStages + b); };
     auto acc_empty = [&](int b) { return bar0 + 8u * (2 * kStages + 2 + b); }; // rank 0: the epilogue warps of both CTAs have read it
+    const uint32_t halted = bar0 + 8u * (2 * kStages + 4);                     // rank 0, after a wait that ran out: no product is under way any more
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -379,6 +380,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
         mbar_init(acc_full(1), 1);
         mbar_init(acc_empty(0), 2 * Smem::kReaders);
         mbar_init(acc_empty(1), 2 * Smem::kReaders);
+        mbar_init(halted, 1);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -467,6 +469,10 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
                 if (ok && elect_one()) umma_commit_pair(acc_full(b));
             }
             for (int j = max(0, i - 2); ok && j < i; ++j) ok = mbar_wait_warp<kClusterScope>(acc_empty(j & 1), (j >> 1) & 1, abort_flag);     // the neighbour's arrivals
+            if (!ok) {                    // products under way read shared memory and write TMEM that others are given when these CTAs leave
+                if (elect_one()) umma_commit_pair(halted, 1);
+                mbar_drain(halted, 0);
+            }
         }
     } else {
         const int q = warp & 3, part = warp >> 2;          // TMEM lanes 32 q .. 32 q + 31, a quarter of the columns

@@ -96,9 +96,9 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// Arrives on the barrier at this place in both CTAs once every product issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+// Arrives on the barrier at this place in both CTAs (or those of `ranks`) once every product issued so far by this thread has completed.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t ranks = 3) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(ranks)
                  : "memory");
 }
 

@@ -32,3 +32,14 @@ def test_every_wait_of_a_pair_is_of_cluster_scope():
         assert signal and re.search(r"\b%s = cluster_smem_addr\(full\(0\), 0\);" % signal.group(1), body), kernel
     wait = re.search(r"bool mbar_try_wait\(.*?\n}\n", _texts()["ptx_utils.cuh"], re.S).group()
     assert re.search(r"SCOPE == kClusterScope\).*?try_wait\.parity\.acquire\.cluster\.", wait, re.S)
+
+
+def test_no_product_is_under_way_when_a_pair_gives_up():
+    """After a wait that ran out, the warp that issues products waits (with a limit) for those it has issued before it goes to the exit."""
+    for kernel, body in KERNELS.items():
+        if not re.search(r"\bumma_f16_pair\b", body):
+            continue
+        last = max(m.end() for m in re.finditer(r"\bumma_f16_pair\b|umma_commit_pair\(acc_full", body))
+        given_up = re.search(r"if \(!ok\) \{\s*if \(elect_one\(\)\) umma_commit_pair\((\w+), 1\);\s*mbar_drain\(\1, 0\);", body[last:])
+        assert given_up, kernel
+        assert re.search(r"mbar_init\(%s, 1\);" % given_up.group(1), body), kernel
