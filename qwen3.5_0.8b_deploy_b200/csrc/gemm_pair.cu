@@ -577,9 +577,11 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 }  // namespace
 
 // Up to 128 rows the library's smaller tiles and the activation behind them are faster: 8.3 us at 128 rows of 1024 and 2 x 3584 columns (bf16)
-// against 8.9 here; 9.7 / 9.0 at 256, 21.8 / 17.1 at 999, 53.7 / 39.9 at 3855, 130 / 78 at 8192 (the product alone 92).
+// against 8.9 here; 9.7 / 9.0 at 256, 21.8 / 17.1 at 999, 53.7 / 39.9 at 3855, 130 / 78 at 8192 (the product alone 92).  The deeper the product, the less the
+// activation weighs and the more the library's rate, the higher one in deep products: a prompt pass of three layers of width 2048 and 5632 outputs takes 351 / 346
+// us at 400 rows, 538 / 482 at 1000, 806 / 768 at 2000; of 4096 and 11008 656 / 673, 1022 / 1092 and 1842 / 2035; of 4096 and 1024 at 200 341 / 357.
 bool gemm_glu_takes(ElemType t, const void* x, const void* w, const void* act, int rows, int ff, int K) {
-    return rows > 128 && t != ELEM_F32 && K % 8 == 0 && ff % 8 == 0 && aligned16(x) && aligned16(w) && aligned16(act);
+    return rows > 128 && K <= 2048 && t != ELEM_F32 && K % 8 == 0 && ff % 8 == 0 && aligned16(x) && aligned16(w) && aligned16(act);
 }
 
 int gemm_glu(cudaStream_t s, ElemType t, int act_kind, const void* x, const void* w, void* act, int rows, int ff, int K, bool split, int* error) {
