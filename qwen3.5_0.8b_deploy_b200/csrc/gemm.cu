@@ -144,11 +144,7 @@ static cudaDataType cuda_type(ElemType t) { return t == ELEM_F16 ? CUDA_R_16F : 
 int gemm_typed(cudaStream_t stream, const void* X, int ldx, const void* W, void* Y, int ldy, ElemType in_type, ElemType out_type, int rows,
                int out, int in, float beta, float alpha, int* error) {
     if (rows <= 0 || out <= 0) return 0;
-    // From four rounds of 256 x 256 tiles on (74 pairs of CTAs), the pairs are the faster ones: pair / library in us, 16-bit operands, 5120 x 1024 at 3855 / 8192 /
-    // 65536 rows 37.7 / 37.5, 74.5 / 83.0, 559 / 718 (fp32 out); 8192 x 1024 at 1000 / 3000 / 16384 rows 15.2 / 15.4, 36.9 / 38.5, 182 / 206 (bf16 out).  Products
-    // that are added to Y stay: 1024 x 3584 at 3855 / 8192 / 16384 rows 26.3 / 22.0, 49.6 / 47.6, 97.3 / 96.6, within a pass of 65536 rows 289 / 288.
-    if (error && alpha == 1.0f && beta == 0.0f && (long long)ceil_div(rows, 256) * ceil_div(out, 256) >= 300 &&
-        gemm_pair_takes(X, ldx, W, Y, ldy, in_type, out_type, in))
+    if (error && alpha == 1.0f && beta == 0.0f && gemm_pair_takes(X, ldx, W, Y, ldy, in_type, out_type, rows, out, in))
         return gemm_pair(stream, X, ldx, W, Y, ldy, in_type, out_type, rows, out, in, error);
     cublasHandle_t handle = nullptr;
     B2_TRY(cublas_for_current_device(&handle));

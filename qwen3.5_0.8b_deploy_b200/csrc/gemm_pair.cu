@@ -634,9 +634,18 @@ int gemm_la_conv(cudaStream_t s, const __half* x, const __half* w, int rows, con
     return launch_pair<kPairConv, __half, B200ATTN_ACT_SILU>(m, p, s);
 }
 
-bool gemm_pair_takes(const void* x, int ldx, const void* w, const void* y, int ldy, ElemType in_type, ElemType out_type, int in) {
-    return in_type != ELEM_F32 && (out_type == ELEM_F32 || out_type == in_type) && ldx % 8 == 0 && in % 8 == 0 && ldy * elem_bytes(out_type) % 16 == 0 &&
-           aligned16(x) && aligned16(w) && aligned16(y);
+// From four rounds of tiles over the device's pairs on, and of depths at which neither the stores (below 512) nor the products alone (above 3584) decide.
+// Pairs / library (cuBLAS 12.8, which a process with PyTorch has) in us back to back, fp32 results: 5120 x 1024 of 3855 / 8192 / 65536 rows 42 / 45, 77 / 98, 599 /
+// 754; 8192 x 2048 of 8192 rows 216 / 246; 1024 x 2048 of 65536 rows 213 / 245; 5120 x 512 of 3855 / 65536 rows 30 / 31, 399 / 479; bf16 results: 5120 x 1024 of 3855 /
+// 65536 rows 32 / 34, 460 / 539; 8192 x 512 of 16384 rows 116 / 133.  Depth 128, bf16 results: 5120 outputs of 3855 / 65536 rows 14.9 / 12.5, 180 / 143, 1024 of 65536 rows
+// 43 / 32 (fp32 results even); depth 3584, 1024 outputs of 40960 rows 202 / 222; depth 4096, 8192 x 8192 376 / 359.  An attention layer of 16384 rows takes
+// 506 us with and 520 without them, of 65536 rows 1676 / 1710.  cuBLAS 12.9 alone (a program without PyTorch) is up to 13 % ahead of the pairs instead.
+// Products that are added to Y stay with the library: 1024 x 3584 at 3855 / 8192 / 16384 rows 26.3 / 22.0, 49.6 / 47.6, 97.3 / 96.6.
+bool gemm_pair_takes(const void* x, int ldx, const void* w, const void* y, int ldy, ElemType in_type, ElemType out_type, int rows, int out, int in) {
+    if (in_type == ELEM_F32 || !(out_type == ELEM_F32 || (in_type == ELEM_BF16 && out_type == ELEM_BF16)) || in < 512 || in > 3584) return false;
+    if (ldx % 8 != 0 || in % 8 != 0 || ldy * elem_bytes(out_type) % 16 != 0 || !aligned16(x) || !aligned16(w) || !aligned16(y)) return false;
+    int sms = 0;
+    return device_sm_count(&sms) == 0 && (long long)ceil_div(rows, 256) * ceil_div(out, 256) > 4 * (sms / 2);
 }
 
 int gemm_pair(cudaStream_t s, const void* x, int ldx, const void* w, void* y, int ldy, ElemType in_type, ElemType out_type, int rows, int out, int in, int* error) {
@@ -653,7 +662,7 @@ int gemm_pair(cudaStream_t s, const void* x, int ldx, const void* w, void* y, in
     p.cols = out;
     p.error = error;
     constexpr int kNone = B200ATTN_ACT_SILU;
-    if (in_type == ELEM_F16) return out_type == ELEM_F32 ? launch_pair<kPairStore32, __half, kNone>(m, p, s) : launch_pair<kPairStore16, __half, kNone>(m, p, s);
+    if (in_type == ELEM_F16) return launch_pair<kPairStore32, __half, kNone>(m, p, s);
     return out_type == ELEM_F32 ? launch_pair<kPairStore32, __nv_bfloat16, kNone>(m, p, s) : launch_pair<kPairStore16, __nv_bfloat16, kNone>(m, p, s);
 }
 

@@ -10,8 +10,8 @@ namespace b200 {
 bool gemm_glu_takes(ElemType t, const void* x, const void* w, const void* act, int rows, int ff, int K);
 int gemm_glu(cudaStream_t s, ElemType t, int act_kind, const void* x, const void* w, void* act, int rows, int ff, int K, bool split, int* error);
 
-// Y[rows, out] = X[rows, in] W[out, in]^T, X and Y with row pitches.  gemm_typed asks for it where it is the faster route.
-bool gemm_pair_takes(const void* x, int ldx, const void* w, const void* y, int ldy, ElemType in_type, ElemType out_type, int in);
+// Y[rows, out] = X[rows, in] W[out, in]^T, X and Y with row pitches.  fp32 results, or bf16 ones of bf16 operands; `takes`: where it is the faster route as well.
+bool gemm_pair_takes(const void* x, int ldx, const void* w, const void* y, int ldy, ElemType in_type, ElemType out_type, int rows, int out, int in);
 int gemm_pair(cudaStream_t s, const void* x, int ldx, const void* w, void* y, int ldy, ElemType in_type, ElemType out_type, int rows, int out, int in, int* error);
 
 // The DeltaNet input projection of prompts with its convolution: X[rows, 1024] W[8224, 1024]^T, then for every token q, k, v (conv + SiLU, L2 norms,

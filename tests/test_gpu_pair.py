@@ -1,6 +1,7 @@
 """GPU: prompt-sized products on pairs of CTAs with their successor in the epilogue, at the edges of their tiles (feed-forward: 256 rows, 128 outputs, parts
 of 32; DeltaNet projection: 253 tokens behind 3 that only serve as taps, 32 at a time) and of their dispatch (feed-forward: more than 128 rows; DeltaNet
 projection: one sequence, or from 300 rows and 36 more for each sequence on, at most 3000, and 24 rows a sequence)."""
+import ctypes as C
 import os
 import sys
 
@@ -111,8 +112,8 @@ def test_more_sequences_than_the_tables_on_chip_hold(ops, cuda, synth):
 
 @pytest.mark.parametrize("rows,fp16_kv", [(14 * 256, 1), (14 * 256 + 1, 0), (38 * 256 - 1, 1), (75 * 256 + 3, 1)])
 def test_large_products_of_a_layer_equal_smaller_ones(ops, cuda, synth, rows, fp16_kv):
-    """Attention layer on both sides of where its products move to the pairs (300 tiles: the input projection above 14 x 256 rows, the output projection above
-    74 x 256), in one call and a sequence at a time: the same sums in the same order, whatever the kernel, so outputs agree to the bit."""
+    """Attention layer on both sides of where its products move to the pairs (296 tiles are four rounds: the input projection above 14 x 256 rows, the output
+    projection above 74 x 256), in one call and a sequence at a time: the same sums in the same order, whatever the kernel, so outputs agree to the bit."""
     torch = cuda
     w, per = synth.fa_weights(79), 1024
     counts = [per] * (rows // per) + ([rows % per] if rows % per else [])
@@ -130,3 +131,16 @@ def test_large_products_of_a_layer_equal_smaller_ones(ops, cuda, synth, rows, fp
             at += n
         out.append(torch.cat(y))
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("kind,out_kind,rows,out,depth,taken", [
+    (0, 2, 15 * 256, 5120, 1024, True), (0, 2, 14 * 256, 5120, 1024, False), (1, 1, 75 * 256, 1024, 2048, True), (1, 1, 74 * 256, 1024, 2048, False),
+    (1, 1, 65536, 2048, 128, False), (1, 2, 65536, 2048, 504, False), (1, 2, 65536, 2048, 512, True), (1, 2, 65536, 2048, 4096, False),
+    (0, 0, 65536, 2048, 1024, False), (2, 2, 65536, 2048, 1024, False), (1, 2, 65536, 2048, 1028, False),
+])
+def test_large_products_go_to_the_pairs_where_these_are_faster(ops, cuda, kind, out_kind, rows, out, depth, taken):
+    """Kinds 0 fp16, 1 bf16, 2 fp32; four rounds of tiles on this device, depths 512 to 3584."""
+    f = C.CDLL(ops.LIB_PATH)["_ZN4b20015gemm_pair_takesEPKviS1_S1_iNS_8ElemTypeES2_iii"]
+    f.restype, f.argtypes = C.c_bool, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]
+    assert cuda.cuda.get_device_properties(0).multi_processor_count == 148
+    assert f(16, depth, 32, 48, out, kind, out_kind, rows, out, depth) == taken
