@@ -144,3 +144,76 @@ def test_large_products_go_to_the_pairs_where_these_are_faster(ops, cuda, kind, 
     f.restype, f.argtypes = C.c_bool, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]
     assert cuda.cuda.get_device_properties(0).multi_processor_count == 148
     assert f(16, depth, 32, 48, out, kind, out_kind, rows, out, depth) == taken
+
+
+# ---- the kernel's forms one by one, against float64 of the same operands: tiles whole, halved and quartered (74 pairs: as many to a round) ------------------
+def _operands(torch, rows, cols, dtype, seed, scale, pitch=None):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    whole = (torch.randn(rows, pitch or cols, device="cuda", generator=g) * scale).to(dtype)
+    return whole, whole[:, :cols].double()
+
+
+def _call(ops, torch, name, *args):
+    """A launcher of the library on the current stream; its device word must stay clean."""
+    word = torch.zeros(1, dtype=torch.int32, device="cuda")
+    conv = [C.c_void_p(a.data_ptr()) if torch.is_tensor(a) else C.c_bool(a) if isinstance(a, bool) else C.c_int(a) for a in args]
+    f = C.CDLL(ops.LIB_PATH)[name]
+    assert f(C.c_void_p(torch.cuda.current_stream().cuda_stream), *conv, C.c_void_p(word.data_ptr())) == 0
+    torch.cuda.synchronize()
+    assert int(word) == 0
+
+
+# Sums of K fp32 products: within 2^-18 of the sum of their magnitudes (K <= 4096 roundings of 2^-24 in some order, at most sqrt(K) of them in one direction).
+SUM = 2.0 ** -18
+
+
+@pytest.mark.parametrize("form", ["fp16 silu", "bf16 silu", "bf16 gelu"])
+@pytest.mark.parametrize("rows,ff,depth", [
+    (130, 64, 64), (257, 264, 72),              # one tile, five: quarters
+    (130, 4712, 136),                           # 37 tiles: halves
+    (600, 2400, 1024),                          # 57: one part-empty round of whole tiles
+    (2304, 1160, 136), (2305, 1304, 72), (2600, 1384, 200),          # 90, 110, 121: a whole round, then quarters, halves, whole ones
+    (4099, 2424, 520),                          # 323: four rounds and halves
+])
+def test_feed_forward_forms(ops, cuda, form, rows, ff, depth):
+    """Gate rows in front of up rows (bf16) and groups of 32 of each (fp16).  Rounding to 11 (fp16) or 8 bits (bf16) moves a value by up to 2^-11 or 2^-8 of it.
+    bf16 products are rounded in front of the activation: gate, up and the result by so much each, where the activations' slopes are at most 1.13."""
+    torch = cuda
+    half, silu = form.startswith("fp16"), form.endswith("silu")
+    dtype, unit = (torch.float16, 2.0 ** -11) if half else (torch.bfloat16, 2.0 ** -8)
+    if half:
+        ff = -(-ff // 32) * 32
+    x, xd = _operands(torch, rows, depth, dtype, 1, 1.0)
+    w, wd = _operands(torch, 2 * ff, depth, dtype, 2, 1.5 / depth ** 0.5)
+    gate, up = (wd.view(-1, 2, 32, depth)[:, i].reshape(ff, depth) for i in (0, 1)) if half else (wd[:ff], wd[ff:])
+    y = torch.full((rows + 2, ff), 7.0, dtype=dtype, device="cuda")
+    _call(ops, torch, "_ZN4b2008gemm_gluEP11CUstream_stNS_8ElemTypeEiPKvS4_PviiibPi", 0 if half else 1, 1 if silu else 0, x, w, y, rows, ff, depth, not half)
+    assert (y[rows:] == 7.0).all()
+    g, u = xd @ gate.t(), xd @ up.t()
+    f = g * torch.sigmoid(g) if silu else torch.nn.functional.gelu(g, approximate="tanh")
+    want = f * u
+    sums = SUM * (1.13 * (xd.abs() @ gate.abs().t()) * u.abs() + (xd.abs() @ up.abs().t()) * f.abs())
+    rounded = unit * want.abs() + (0.0 if half else unit * (1.13 * (g * u).abs() + want.abs()))
+    excess = (y[:rows].double() - want).abs() - 1.05 * (rounded + sums) - 1e-5       # two roundings compound; the special functions are good to 2^-20
+    assert excess.max() <= 0, float(excess.max())
+
+
+@pytest.mark.parametrize("kind,out_kind", [(0, 2), (1, 1), (1, 2)])
+@pytest.mark.parametrize("rows,out,depth,x_more,y_more", [
+    (255, 264, 72, 0, 0), (1025, 264, 520, 8, 16),                   # one and two columns of tiles, quarters
+    (9 * 256 + 1, 4 * 256 - 8, 128, 0, 8),                           # 40: whole
+    (8 * 256 + 3, 10 * 256, 512, 24, 0), (9 * 256, 11 * 256 + 40, 200, 0, 24),       # 90: a round and quarters; 108: and halves
+    (15 * 256 - 5, 20 * 256, 1024, 0, 0),                            # 300
+])
+def test_plain_forms(ops, cuda, kind, out_kind, rows, out, depth, x_more, y_more):
+    """fp16 to fp32, bf16 to bf16 and fp32, with row pitches on either side; what lies outside the matrix is left alone."""
+    torch = cuda
+    dtype, out_dtype = (torch.float16 if kind == 0 else torch.bfloat16), (torch.float32 if out_kind == 2 else torch.bfloat16)
+    x, xd = _operands(torch, rows, depth, dtype, 3, 1.0, depth + x_more)
+    w, wd = _operands(torch, out, depth, dtype, 4, 1.0)
+    y = torch.full((rows + 1, out + y_more), 7.0, dtype=out_dtype, device="cuda")
+    _call(ops, torch, "_ZN4b2009gemm_pairEP11CUstream_stPKviS3_PviNS_8ElemTypeES5_iiiPi", x, depth + x_more, w, y, out + y_more, kind, out_kind, rows, out, depth)
+    assert (y[rows:] == 7.0).all() and (y[:, out:] == 7.0).all()
+    want, sums = xd @ wd.t(), SUM * (xd.abs() @ wd.abs().t())
+    excess = (y[:rows, :out].double() - want).abs() - sums - (2.0 ** -8 * want.abs() * 1.01 if out_kind == 1 else 0.0)       # 8 bits
+    assert excess.max() <= 0, float(excess.max())

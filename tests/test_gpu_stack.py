@@ -129,6 +129,29 @@ def test_plain_stream_order_gives_the_same_tokens(ops, cuda, synth, monkeypatch)
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("n,tokens", [(3, 333), (1, 700), (9, 300), (2, 5)])
+def test_plain_stream_order_gives_the_same_hidden_rows(ops, cuda, synth, monkeypatch, n, tokens):
+    """Prompt passes bit for bit: up to four sequences with one of more than 192 tokens (the recurrence in two kernels), more sequences (in one), few rows."""
+    torch = cuda
+    from oracle import cpu_stack
+    weights = cpu_stack.make_stack_weights(synth, 64, L, INTER, VOCAB, int8=False)
+    toks = torch.from_numpy(synth.rng(64, "tokens").integers(0, VOCAB, (n, tokens)).astype(np.int32)).cuda()
+    hidden = []
+    for pdl in ("1", "0"):
+        monkeypatch.setenv("B200ATTN_PDL", pdl)
+        st = ops.HybridStack(num_layers=L, intermediate_size=INTER, vocab_size=VOCAB, max_seqs=n, max_seq_len=tokens, prefill_chunk_seqs=n, kv_dtype=1, int8_weights=False)
+        for i, lw in enumerate(weights["layers"]):
+            st.set_layer_weights(i, lw, lw["ffn"], fa=lw.get("fa"), la=lw.get("la"))
+        st.set_embedding(weights["embed"], weights["final_norm"])
+        for _ in range(3):                                 # the caches differ from pass to pass in their places, not in what they hold
+            st.reset_cache()
+            hidden.append(st.forward_batch_prefill(toks, want_hidden=True)[1].clone())
+        torch.cuda.synchronize()
+        assert st.device_status() == 0
+    for h in hidden[1:]:
+        assert torch.equal(h, hidden[0])
+
+
 def test_decode_after_a_prefill_that_fills_the_working_buffers(ops, cuda, oracle, synth):
     """The operators of one stack overlay their working buffers on one area.  A prefill that uses (nearly) every row of
     it must leave nothing behind that the decode step depends on: the split counters and status words live outside it.
