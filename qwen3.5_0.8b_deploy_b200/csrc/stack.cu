@@ -322,7 +322,8 @@ extern "C" int b200attn_stack_create(const b200attn_stack_config* cfg, b200attn_
     const size_t R = st->max_rows;
     ST_CUDA(cudaMalloc(&st->d_h, R * kHidden * 4));
     ST_CUDA(cudaMalloc(&st->d_xb, R * kHidden * 2));
-    ST_CUDA(cudaMalloc(&st->d_gu, R * 2 * cfg->intermediate_size * 2));
+    st->gu_rows = std::max((int)std::min<size_t>(R, 128), cfg->max_seqs);      // longer passes take the product with the activation in its epilogue
+    ST_CUDA(cudaMalloc(&st->d_gu, (size_t)st->gu_rows * 2 * cfg->intermediate_size * 2));
     ST_CUDA(cudaMalloc(&st->d_act, R * cfg->intermediate_size * 2));
     ST_CUDA(cudaMalloc(&st->d_last, (size_t)cfg->max_seqs * kHidden * 4));
     ST_CUDA(cudaMalloc(&st->d_logits, (size_t)cfg->max_seqs * cfg->vocab_size * 4));
@@ -567,6 +568,7 @@ static int stack_layers(b200attn_stack st, int rows, const int* h_slots, const i
         if (!decode && gemm_glu_takes(ELEM_F16, st->d_xb, st->d_wgu[i], st->d_act, rows, inter, kHidden)) {
             B2_TRY(gemm_glu(s, ELEM_F16, B200ATTN_ACT_SILU, st->d_xb, st->d_wgu[i], st->d_act, rows, inter, kHidden, false, st->d_error));
         } else {
+            if (rows > st->gu_rows) B2_FAIL(B200ATTN_ERR_UNSUPPORTED, "stack: %d rows exceed the %d of the gate / up buffer", rows, st->gu_rows);
             B2_TRY(gemm_xwT(s, st->d_xb, true, st->d_wgu[i], true, st->d_gu, true, rows, 2 * inter, kHidden));
             const size_t octs = (size_t)rows * inter / 8;
             launch_pdl(swiglu_kernel, dim3((unsigned)((octs + 255) / 256)), dim3(256), 0, s, st->d_gu, inter, octs, st->d_act);

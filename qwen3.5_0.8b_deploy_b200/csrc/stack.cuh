@@ -27,7 +27,8 @@ struct b200attn_stack_s {
     int max_rows = 0;
     float* d_h = nullptr;              // [max_rows, hidden] residual stream
     __half* d_xb = nullptr;     // [max_rows, hidden]
-    __half* d_gu = nullptr;     // [max_rows, 2*inter]
+    __half* d_gu = nullptr;     // [gu_rows, 2*inter]: decode steps and passes of up to 128 rows
+    int gu_rows = 0;
     __half* d_act = nullptr;    // [max_rows, inter]
     float* d_last = nullptr;           // [max_seqs, hidden]
     float* d_logits = nullptr;         // [max_seqs, vocab]
