@@ -118,7 +118,8 @@ int b200attn_kv_pages(b200attn_kv_pool pool, int* total_out, int* used_out);
 /* Reads (and clears) the pool's device-side status word: 0 = clean, 1 = slot out of range seen by a
  * kernel, 2 = append beyond the reserved pages (the write was skipped), 3/4 = a bounded wait inside
  * the decode / prefill attention kernel ran out, 8 = the prefill kernel found its shared-memory window
- * misaligned and did nothing.  Synchronises the device.  No reference counterpart:
+ * misaligned and did nothing, 7 = a bounded wait inside a product of an attention layer ran out (few rows, or the paired
+ * products of large passes).  Synchronises the device.  No reference counterpart:
  * the reference's kernels report nothing (full_attention_cuda.cu:11-17 prints and continues). */
 int b200attn_kv_device_status(b200attn_kv_pool pool, int* code_out);
 /* Quantise-on-append of already normalised/rotated K and raw V rows, the arithmetic of
@@ -343,7 +344,7 @@ int b200attn_stack_init_embedding_random(b200attn_stack st, uint64_t seed, float
                                          const float* h_final_norm);
 /* Reads (and clears) the device-side status words of the stack (its KV pool, its DeltaNet operators and its own
  * GEMM kernels): 0 = clean, otherwise the first non-zero code found (codes as in b200attn_kv_device_status /
- * b200attn_la_device_status; 7 = a bounded wait inside a decode-step GEMM ran out, 9 = one inside the chunked mLSTM prefill).  Synchronises the device.
+ * b200attn_la_device_status; 7 = a bounded wait inside a product ran out, of a decode step or a prompt, 9 = one inside the chunked mLSTM prefill).  Synchronises the device.
  * No reference counterpart. */
 int b200attn_stack_device_status(b200attn_stack st, int* code_out);
 /* CudaEngine::reset_cache (cuda_engine.cu:514-519). */

@@ -132,70 +132,68 @@ diff_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     } else if (warp == 9) {
         // ------------------------------ MMA issuer: the warp as one, an elected lane at each issue (elect_one) ------------------------------
         // Twenty products a key step: a thread on its own took some 80 cycles for each, more than the products themselves (247 -> 220 us at 16 x 1024 tokens).
-        {
-            const uint64_t q_k = umma_smem_desc(base, 16, 1024), k_k = umma_smem_desc(base + L.off_k, 16, 1024), p_k = umma_smem_desc(base + L.off_p, 16, 1024);
-            const uint64_t v_mn = umma_smem_desc(base + L.off_v, kDKBlk, 1024);
-            constexpr uint32_t id_s = umma_idesc(kFmtBF16, kDM, kDN, 0, 0);
-            const uint32_t id_pv = umma_idesc(kFmtBF16, kDM, 64 * L.nv, 0, 1);
-            // PV products of global step g; `first` overwrites O (the previous item's epilogue has read it), after `last` O is final
-            auto issue_pv = [&](int g, bool first, bool last, int it) -> bool {
-                const int b = g & 1, s = g % NST;
-                if (!mbar_wait_warp(bar(D_VF + s), (g / NST) & 1, abort_flag)) return false;
-                if (first && it > 0 && !mbar_wait_warp(bar(D_OD), (it - 1) & 1, abort_flag)) return false;
-                const uint64_t v = v_mn + s * L.nv * desc_step(kDKBlk);
-                for (int m = 0; m < 2; ++m) {
-                    if (!mbar_wait_warp(bar(D_PF + 2 * m + b), (g >> 1) & 1, abort_flag)) return false;
-                    tc_fence_after();
-                    const uint64_t a = p_k + (2 * m + b) * desc_step(kDPBuf);
-                    if (elect_one()) {
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks)
-                            umma_f16(tmem_o + m * 64 * L.nv, a + desc_step(ks * 32), v + desc_step(ks * 2048), id_pv, (!first || ks > 0) ? 1u : 0u);
-                        umma_commit(bar(D_PV + 2 * m + b));
-                    }
-                }
+        const uint64_t q_k = umma_smem_desc(base, 16, 1024), k_k = umma_smem_desc(base + L.off_k, 16, 1024), p_k = umma_smem_desc(base + L.off_p, 16, 1024);
+        const uint64_t v_mn = umma_smem_desc(base + L.off_v, kDKBlk, 1024);
+        constexpr uint32_t id_s = umma_idesc(kFmtBF16, kDM, kDN, 0, 0);
+        const uint32_t id_pv = umma_idesc(kFmtBF16, kDM, 64 * L.nv, 0, 1);
+        // PV products of global step g; `first` overwrites O (the previous item's epilogue has read it), after `last` O is final
+        auto issue_pv = [&](int g, bool first, bool last, int it) -> bool {
+            const int b = g & 1, s = g % NST;
+            if (!mbar_wait_warp(bar(D_VF + s), (g / NST) & 1, abort_flag)) return false;
+            if (first && it > 0 && !mbar_wait_warp(bar(D_OD), (it - 1) & 1, abort_flag)) return false;
+            const uint64_t v = v_mn + s * L.nv * desc_step(kDKBlk);
+            for (int m = 0; m < 2; ++m) {
+                if (!mbar_wait_warp(bar(D_PF + 2 * m + b), (g >> 1) & 1, abort_flag)) return false;
+                tc_fence_after();
+                const uint64_t a = p_k + (2 * m + b) * desc_step(kDPBuf);
                 if (elect_one()) {
-                    umma_commit(bar(D_VE + s));
-                    if (last) umma_commit(bar(D_OF));
-                }
-                return true;
-            };
-            bool ok = true, pending = false, pfirst = false, plast = false;
-            int pg = 0, pitem = 0, gs = 0;
-            for (int i = 0; ok && i < n_my; ++i) {
-                const int n_kt = item(i).n_kt;
-                if (pending) {         // the previous item's last PV goes out before the wait for this item's Q tile
-                    if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
-                    pending = false;
-                }
-                if (!mbar_wait_warp(bar(D_Q), i & 1, abort_flag)) { ok = false; break; }
-                for (int j = 0; ok && j < n_kt; ++j, ++gs) {
-                    const int b = gs & 1, s = gs % NST;
-                    if (!mbar_wait_warp(bar(D_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
-                    for (int m = 0; m < 2; ++m) {
-                        if (gs >= 2 && !mbar_wait_warp(bar(D_SE + 2 * m + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint64_t q0 = q_k + m * L.nd * desc_step(kDQBlk), k0 = k_k + (s * 2 + m) * L.nd * desc_step(kDKBlk);
-                        if (elect_one()) {
-                            for (int blk = 0; blk < L.nd; ++blk)
 #pragma unroll
-                                for (int ks = 0; ks < 4; ++ks)
-                                    umma_f16(tmem + (2 * m + b) * kDN, q0 + blk * desc_step(kDQBlk) + desc_step(ks * 32), k0 + blk * desc_step(kDKBlk) + desc_step(ks * 32), id_s,
-                                             (blk > 0 || ks > 0) ? 1u : 0u);
-                            umma_commit(bar(D_SF + 2 * m + b));
-                        }
-                    }
-                    if (!ok) break;
-                    if (elect_one()) {
-                        umma_commit(bar(D_KE + s));
-                        if (j == n_kt - 1) umma_commit(bar(D_QE));
-                    }
-                    if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
-                    pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
+                    for (int ks = 0; ks < 4; ++ks)
+                        umma_f16(tmem_o + m * 64 * L.nv, a + desc_step(ks * 32), v + desc_step(ks * 2048), id_pv, (!first || ks > 0) ? 1u : 0u);
+                    umma_commit(bar(D_PV + 2 * m + b));
                 }
             }
-            if (ok && pending) issue_pv(pg, pfirst, plast, pitem);
+            if (elect_one()) {
+                umma_commit(bar(D_VE + s));
+                if (last) umma_commit(bar(D_OF));
+            }
+            return true;
+        };
+        bool ok = true, pending = false, pfirst = false, plast = false;
+        int pg = 0, pitem = 0, gs = 0;
+        for (int i = 0; ok && i < n_my; ++i) {
+            const int n_kt = item(i).n_kt;
+            if (pending) {         // the previous item's last PV goes out before the wait for this item's Q tile
+                if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
+                pending = false;
+            }
+            if (!mbar_wait_warp(bar(D_Q), i & 1, abort_flag)) { ok = false; break; }
+            for (int j = 0; ok && j < n_kt; ++j, ++gs) {
+                const int b = gs & 1, s = gs % NST;
+                if (!mbar_wait_warp(bar(D_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
+                for (int m = 0; m < 2; ++m) {
+                    if (gs >= 2 && !mbar_wait_warp(bar(D_SE + 2 * m + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t q0 = q_k + m * L.nd * desc_step(kDQBlk), k0 = k_k + (s * 2 + m) * L.nd * desc_step(kDKBlk);
+                    if (elect_one()) {
+                        for (int blk = 0; blk < L.nd; ++blk)
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks)
+                                umma_f16(tmem + (2 * m + b) * kDN, q0 + blk * desc_step(kDQBlk) + desc_step(ks * 32), k0 + blk * desc_step(kDKBlk) + desc_step(ks * 32), id_s,
+                                         (blk > 0 || ks > 0) ? 1u : 0u);
+                        umma_commit(bar(D_SF + 2 * m + b));
+                    }
+                }
+                if (!ok) break;
+                if (elect_one()) {
+                    umma_commit(bar(D_KE + s));
+                    if (j == n_kt - 1) umma_commit(bar(D_QE));
+                }
+                if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
+                pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
+            }
         }
+        if (ok && pending) issue_pv(pg, pfirst, plast, pitem);
     } else {
         // ------------------------------ softmax / correction / epilogue ------------------------------
         const int r = threadIdx.x & 127;                 // query row == TMEM lane

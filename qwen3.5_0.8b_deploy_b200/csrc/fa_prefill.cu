@@ -149,66 +149,64 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     } else if (warp == 9) {
         // ------------------------------ MMA issuer: the warp as one, an elected lane at each issue (elect_one) ------------------------------
         // Twenty products a key step: a thread on its own took some 80 cycles for each, more than the products themselves (445 -> 386 us at 64 x 1024 tokens).
-        {
-            const uint64_t p_k = umma_smem_desc(base + kOffP, 16, 1024), v_mn = umma_smem_desc(base + kOffV, kBN * 128, 1024);
-            const uint64_t q_k = umma_smem_desc(base + kOffQ, 16, 1024), k_k = umma_smem_desc(base + kOffK, 16, 1024);
-            constexpr uint32_t idesc_s = umma_idesc(kFmtF16, kBM, kBN, 0, 0);
-            constexpr uint32_t idesc_pv = umma_idesc(kFmtF16, kBM, kHeadDim, 0, 1);
-            // PV product of global step g; `first`: first key step of its item (overwrites O, which the previous item's
-            // epilogue must have read), `last`: last key step of its item (O is final afterwards)
-            auto issue_pv = [&](int g, bool first, bool last, int item) -> bool {
-                const int b = g & 1;
-                const uint32_t par = (g >> 1) & 1;
-                if (!mbar_wait_warp(bar(BAR_VF + b), par, abort_flag)) return false;
-                if (!mbar_wait_warp(bar(BAR_PF + b), par, abort_flag)) return false;
-                if (first && item > 0 && !mbar_wait_warp(bar(BAR_OD), (item - 1) & 1, abort_flag)) return false;
+        const uint64_t p_k = umma_smem_desc(base + kOffP, 16, 1024), v_mn = umma_smem_desc(base + kOffV, kBN * 128, 1024);
+        const uint64_t q_k = umma_smem_desc(base + kOffQ, 16, 1024), k_k = umma_smem_desc(base + kOffK, 16, 1024);
+        constexpr uint32_t idesc_s = umma_idesc(kFmtF16, kBM, kBN, 0, 0);
+        constexpr uint32_t idesc_pv = umma_idesc(kFmtF16, kBM, kHeadDim, 0, 1);
+        // PV product of global step g; `first`: first key step of its item (overwrites O, which the previous item's
+        // epilogue must have read), `last`: last key step of its item (O is final afterwards)
+        auto issue_pv = [&](int g, bool first, bool last, int item) -> bool {
+            const int b = g & 1;
+            const uint32_t par = (g >> 1) & 1;
+            if (!mbar_wait_warp(bar(BAR_VF + b), par, abort_flag)) return false;
+            if (!mbar_wait_warp(bar(BAR_PF + b), par, abort_flag)) return false;
+            if (first && item > 0 && !mbar_wait_warp(bar(BAR_OD), (item - 1) & 1, abort_flag)) return false;
+            tc_fence_after();
+            const uint64_t a = p_k + b * desc_step(kPBytes), bd = v_mn + b * desc_step(kKVBytes);
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) umma_f16(tmem_o, a + desc_step(ks * 32), bd + desc_step(ks * 2048), idesc_pv, (!first || ks > 0) ? 1u : 0u);
+                umma_commit(bar(BAR_PV + b));
+                umma_commit(bar(BAR_VE + b));
+                if (last) umma_commit(bar(BAR_OF));
+            }
+            return true;
+        };
+        bool ok = true, pending = false;
+        int pg = 0, pitem = 0;
+        bool pfirst = false, plast = false;
+        int gs = 0;
+        for (int i = 0; ok && i < n_my; ++i) {
+            int head;
+            const PrefillTile tile = item_tile(i, head);
+            const int n_kt = key_tiles(tile);
+            // the previous item's last PV product goes out before the wait for this item's Q tile, so that its
+            // epilogue runs while Q and the first S product are on their way
+            if (pending) {
+                if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
+                pending = false;
+            }
+            if (!mbar_wait_warp(bar(BAR_Q), i & 1, abort_flag)) { ok = false; break; }
+            for (int j = 0; j < n_kt; ++j, ++gs) {
+                const int b = gs & 1;
+                if (!mbar_wait_warp(bar(BAR_KF + b), (gs >> 1) & 1, abort_flag)) { ok = false; break; }
+                if (gs >= 2 && !mbar_wait_warp(bar(BAR_SE + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t a = p_k + b * desc_step(kPBytes), bd = v_mn + b * desc_step(kKVBytes);
+                const uint64_t kd = k_k + b * desc_step(kKVBytes);
                 if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) umma_f16(tmem_o, a + desc_step(ks * 32), bd + desc_step(ks * 2048), idesc_pv, (!first || ks > 0) ? 1u : 0u);
-                    umma_commit(bar(BAR_PV + b));
-                    umma_commit(bar(BAR_VE + b));
-                    if (last) umma_commit(bar(BAR_OF));
+                    for (int ks = 0; ks < 16; ++ks)
+                        umma_f16(tmem + b * kBN, q_k + desc_step((ks >> 2) * (kBM * 128) + (ks & 3) * 32), kd + desc_step((ks >> 2) * (kBN * 128) + (ks & 3) * 32), idesc_s,
+                                 ks > 0 ? 1u : 0u);
+                    umma_commit(bar(BAR_SF + b));
+                    umma_commit(bar(BAR_KE + b));
+                    if (j == n_kt - 1) umma_commit(bar(BAR_QE));      // the Q tile is free once this item's S products are done
                 }
-                return true;
-            };
-            bool ok = true, pending = false;
-            int pg = 0, pitem = 0;
-            bool pfirst = false, plast = false;
-            int gs = 0;
-            for (int i = 0; ok && i < n_my; ++i) {
-                int head;
-                const PrefillTile tile = item_tile(i, head);
-                const int n_kt = key_tiles(tile);
-                // the previous item's last PV product goes out before the wait for this item's Q tile, so that its
-                // epilogue runs while Q and the first S product are on their way
-                if (pending) {
-                    if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
-                    pending = false;
-                }
-                if (!mbar_wait_warp(bar(BAR_Q), i & 1, abort_flag)) { ok = false; break; }
-                for (int j = 0; j < n_kt; ++j, ++gs) {
-                    const int b = gs & 1;
-                    if (!mbar_wait_warp(bar(BAR_KF + b), (gs >> 1) & 1, abort_flag)) { ok = false; break; }
-                    if (gs >= 2 && !mbar_wait_warp(bar(BAR_SE + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t kd = k_k + b * desc_step(kKVBytes);
-                    if (elect_one()) {
-#pragma unroll
-                        for (int ks = 0; ks < 16; ++ks)
-                            umma_f16(tmem + b * kBN, q_k + desc_step((ks >> 2) * (kBM * 128) + (ks & 3) * 32), kd + desc_step((ks >> 2) * (kBN * 128) + (ks & 3) * 32), idesc_s,
-                                     ks > 0 ? 1u : 0u);
-                        umma_commit(bar(BAR_SF + b));
-                        umma_commit(bar(BAR_KE + b));
-                        if (j == n_kt - 1) umma_commit(bar(BAR_QE));      // the Q tile is free once this item's S products are done
-                    }
-                    if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
-                    pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
-                }
+                if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
+                pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
             }
-            if (ok && pending) issue_pv(pg, pfirst, plast, pitem);
         }
+        if (ok && pending) issue_pv(pg, pfirst, plast, pitem);
     } else {
         // ------------------------------ softmax / correction / epilogue ------------------------------
         const int r = threadIdx.x & 127;                 // query row == TMEM lane

@@ -4,14 +4,14 @@
 // 0.94 GB each way.  Here the accumulators go through the function on their way out of TMEM while the tensor cores work on the next tile: 613 us (1.57
 // PFLOP/s, bound by the tensor cores' 512 cycles a slice and, over seconds, by the power limit) in place of 682 + 285 us.  fp16 products reach the function
 // unrounded; bf16 ones are rounded first, as the two kernels did: outputs of the layer-described stacks stay the same bit for bit.
-//   kPairStore16, kPairStore32   the product alone, as 16-bit or fp32 values (large products, gemm_typed)
+//   kPairStore16, kPairStore32   the product alone, as bf16 or fp32 values (large products, gemm_typed)
 //   kPairConv   the DeltaNet input projection with the causal convolution, SiLU, L2 norms and gates behind it (fp16).  Here the channels of W are the
 //               rows of the product and the tokens its columns: a thread holds one channel and finds the taps of a token in its own registers.
 //               65536 rows 950 us (projection 878 and convolution 502 before, 3.2 GB between them), 3 x 333 23 (33), 9 x 466 67 (111).
 //
 // A cluster of two CTAs owns a 256 x 256 tile (cta_group::2, M = 256): each CTA fetches its 128 rows of both operands and holds 128 rows of the
 // result, so that an operand byte in shared memory serves twice the products that it would in a tile of one CTA.  Two accumulators of 256 columns
-// fill TMEM; eight warps empty one while the other is being filled.  Persistent: one CTA per SM, tiles in a fixed order.
+// fill TMEM; sixteen warps (kPairConv: eight, in turns) empty one while the other is being filled.  Persistent: one CTA per SM, tiles in a fixed order.
 #include "elem.cuh"
 #include "gemm_pair.cuh"
 #include "kernels.cuh"
@@ -149,7 +149,7 @@ __device__ __forceinline__ void plain_part(const PairArgs& p, const CUtensorMap*
 }
 
 // What the convolution has to know of a token: place in its sequence's rows of this call, up to 3, and rows behind it, up to 3.
-constexpr int kTokenPlain = 15, kTokenNone = 16;
+constexpr int kTokenNone = 16;
 __device__ __forceinline__ int sequence_of(const LaConvArgs& a, const int* first_rows, int t) {
     int lo = 0, hi = a.n_seqs - 1;                       // the last sequence that starts at or before row t (empty ones start where the next does)
     while (lo < hi) {
@@ -388,7 +388,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
         tmem_alloc_pair(smem_u32(tmem_slot), 512);
         tmem_relinquish_pair();
     }
-    if (warp == kEpiWarps && lane == 0) { 
+    if (warp == kEpiWarps && lane == 0) {
         tma_prefetch_desc(&maps.a);
         tma_prefetch_desc(&maps.b);
         tma_prefetch_desc(&maps.out[0]);

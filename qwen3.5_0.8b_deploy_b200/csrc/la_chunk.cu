@@ -350,104 +350,102 @@ la_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
     if (warp == 8) {
         // ------------------------------ TMA + MMA issuer: the warp as one, an elected lane at each issue (elect_one) ------------------------------
-        {
-            constexpr uint32_t id64 = umma_idesc(kFmtF16, 128, 64, 0, 0);
-            constexpr uint32_t id64_amn = umma_idesc(kFmtF16, 128, 64, 1, 0);                    // A MN-major (a TMA tile as it came)
-            constexpr uint32_t id64_bmn_neg = umma_idesc(kFmtF16, 128, 64, 0, 1) | (1u << 13);   // B MN-major, negated A
-            constexpr uint32_t id_u = umma_idesc(kFmtF16, 128, 128, 0, 1);                       // B MN-major, N = 128
-            auto load_kq = [&](int c) {
-                const int row = sq.row0 + c * kC;
-                const uint32_t dst = base + ((c & 1) ? kOffY : kOffX);
-                if (!elect_one()) return;
-                mbar_arrive_expect_tx(bar(G_FULL_KQ), 32768);
+        constexpr uint32_t id64 = umma_idesc(kFmtF16, 128, 64, 0, 0);
+        constexpr uint32_t id64_amn = umma_idesc(kFmtF16, 128, 64, 1, 0);                    // A MN-major (a TMA tile as it came)
+        constexpr uint32_t id64_bmn_neg = umma_idesc(kFmtF16, 128, 64, 0, 1) | (1u << 13);   // B MN-major, negated A
+        constexpr uint32_t id_u = umma_idesc(kFmtF16, 128, 128, 0, 1);                       // B MN-major, N = 128
+        auto load_kq = [&](int c) {
+            const int row = sq.row0 + c * kC;
+            const uint32_t dst = base + ((c & 1) ? kOffY : kOffX);
+            if (!elect_one()) return;
+            mbar_arrive_expect_tx(bar(G_FULL_KQ), 32768);
+            for (int blk = 0; blk < 2; ++blk) {
+                tma_load_3d(dst + blk * 16384, &map_k, bar(G_FULL_KQ), blk * 64, h, row);
+                tma_load_3d(dst + blk * 16384 + 8192, &map_q, bar(G_FULL_KQ), blk * 64, h, row);
+            }
+        };
+        auto load_v = [&](int c) {
+            const int row = sq.row0 + c * kC;
+            if (!elect_one()) return;
+            mbar_arrive_expect_tx(bar(G_FULL_V), 16384);
+            for (int blk = 0; blk < 2; ++blk) tma_load_3d(base + kOffV + blk * 8192, &map_v, bar(G_FULL_V), blk * 64, h, row);
+        };
+        auto issue_a = [&](int c) {            // (a) D1 = [K;Q] K^T of chunk c, into the Ut columns
+            const uint64_t kq = umma_smem_desc(base + ((c & 1) ? kOffY : kOffX), 16, 1024);
+            if (!elect_one()) return;
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+                const uint64_t at = kq + desc_step((ks >> 2) * 16384 + (ks & 3) * 32);
+                umma_f16(tm_ut, at, at, id64, ks > 0 ? 1u : 0u);
+            }
+            umma_commit(bar(G_A_DONE));
+        };
+        load_kq(0);
+        load_v(0);
+        bool ok = mbar_wait_warp(bar(G_FULL_KQ), 0, abort_flag);
+        if (ok) { tc_fence_after(); issue_a(0); }
+        for (int c = 0; ok && c < n_chunks; ++c) {
+            const uint32_t par = c & 1;
+            const uint32_t kq = base + (par ? kOffY : kOffX);       // this chunk's K/Q tiles
+            const uint32_t wr = base + (par ? kOffX : kOffY);       // this chunk's T tiles, then its state tile
+            if (c > 0) {                        // V_new of chunk c-1 has been read by its last products: the V tile may land
+                if (!mbar_wait_warp(bar(G_C3), (c - 1) & 1, abort_flag)) break;
+                load_v(c);
+            }
+            if (c + 1 < n_chunks && elect_one()) {             // ask L2 for the next chunk's tiles well ahead of their loads
+                const int row = sq.row0 + (c + 1) * kC;
                 for (int blk = 0; blk < 2; ++blk) {
-                    tma_load_3d(dst + blk * 16384, &map_k, bar(G_FULL_KQ), blk * 64, h, row);
-                    tma_load_3d(dst + blk * 16384 + 8192, &map_q, bar(G_FULL_KQ), blk * 64, h, row);
+                    tma_prefetch_l2_3d(&map_k, blk * 64, h, row);
+                    tma_prefetch_l2_3d(&map_q, blk * 64, h, row);
+                    tma_prefetch_l2_3d(&map_v, blk * 64, h, row);
                 }
-            };
-            auto load_v = [&](int c) {
-                const int row = sq.row0 + c * kC;
-                if (!elect_one()) return;
-                mbar_arrive_expect_tx(bar(G_FULL_V), 16384);
-                for (int blk = 0; blk < 2; ++blk) tma_load_3d(base + kOffV + blk * 8192, &map_v, bar(G_FULL_V), blk * 64, h, row);
-            };
-            auto issue_a = [&](int c) {            // (a) D1 = [K;Q] K^T of chunk c, into the Ut columns
-                const uint64_t kq = umma_smem_desc(base + ((c & 1) ? kOffY : kOffX), 16, 1024);
-                if (!elect_one()) return;
+            }
+            const uint64_t v_mn = umma_smem_desc(base + kOffV, 8192, 1024), v_k = umma_smem_desc(base + kOffV, 16, 1024), mq = umma_smem_desc(base + kOffMQ, 16, 1024);
+            const uint64_t kq_mn = umma_smem_desc(kq, 16384, 1024), q_k = umma_smem_desc(kq + 8192, 16, 1024), wr_k = umma_smem_desc(wr, 16, 1024);
+            if (!mbar_wait_warp(bar(G_B1), par, abort_flag)) break;
+            if (!mbar_wait_warp(bar(G_FULL_V), par, abort_flag)) break;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint64_t at = kq + desc_step((ks >> 2) * 16384 + (ks & 3) * 32);
-                    umma_f16(tm_ut, at, at, id64, ks > 0 ? 1u : 0u);
-                }
-                umma_commit(bar(G_A_DONE));
-            };
-            load_kq(0);
-            load_v(0);
-            bool ok = mbar_wait_warp(bar(G_FULL_KQ), 0, abort_flag);
-            if (ok) { tc_fence_after(); issue_a(0); }
-            for (int c = 0; ok && c < n_chunks; ++c) {
-                const uint32_t par = c & 1;
-                const uint32_t kq = base + (par ? kOffY : kOffX);       // this chunk's K/Q tiles
-                const uint32_t wr = base + (par ? kOffX : kOffY);       // this chunk's T tiles, then its state tile
-                if (c > 0) {                        // V_new of chunk c-1 has been read by its last products: the V tile may land
-                    if (!mbar_wait_warp(bar(G_C3), (c - 1) & 1, abort_flag)) break;
-                    load_v(c);
-                }
-                if (c + 1 < n_chunks && elect_one()) {             // ask L2 for the next chunk's tiles well ahead of their loads
-                    const int row = sq.row0 + (c + 1) * kC;
-                    for (int blk = 0; blk < 2; ++blk) {
-                        tma_prefetch_l2_3d(&map_k, blk * 64, h, row);
-                        tma_prefetch_l2_3d(&map_q, blk * 64, h, row);
-                        tma_prefetch_l2_3d(&map_v, blk * 64, h, row);
+                for (int hl = 0; hl < 2; ++hl)    // (uw): T diag(beta) and T diag(beta e^b) as hi + lo pairs
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) {
+                        const uint32_t acc = (hl > 0 || ks > 0) ? 1u : 0u;
+                        umma_f16(tm_ut, v_mn + desc_step(ks * 2048), wr_k + desc_step(hl * 8192 + ks * 32), id64_amn, acc);
+                        umma_f16(tm_x, kq_mn + desc_step(ks * 2048), wr_k + desc_step(16384 + hl * 8192 + ks * 32), id64_amn, acc);
                     }
+                umma_commit(bar(G_C1));
+            }
+            if (!mbar_wait_warp(bar(G_B2), par, abort_flag)) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks) {   // (ws) Ut -= S0^T W^T ; (o) Ot = S0^T (Q e^b)^T
+                    const uint64_t a = wr_k + desc_step((ks >> 2) * 16384 + (ks & 3) * 32);
+                    umma_f16(tm_ut, a, v_mn + desc_step(ks * 2048), id64_bmn_neg, 1u);
+                    umma_f16(tm_x, a, q_k + desc_step((ks >> 2) * 16384 + (ks & 3) * 32), id64, ks > 0 ? 1u : 0u);
                 }
-                const uint64_t v_mn = umma_smem_desc(base + kOffV, 8192, 1024), v_k = umma_smem_desc(base + kOffV, 16, 1024), mq = umma_smem_desc(base + kOffMQ, 16, 1024);
-                const uint64_t kq_mn = umma_smem_desc(kq, 16384, 1024), q_k = umma_smem_desc(kq + 8192, 16, 1024), wr_k = umma_smem_desc(wr, 16, 1024);
-                if (!mbar_wait_warp(bar(G_B1), par, abort_flag)) break;
-                if (!mbar_wait_warp(bar(G_FULL_V), par, abort_flag)) break;
+                umma_commit(bar(G_C2));
+            }
+            if (c + 1 < n_chunks) {            // the state tile is dead once these products are done: the next K/Q tiles go there
+                if (!mbar_wait_warp(bar(G_C2), par, abort_flag)) break;
+                load_kq(c + 1);
+            }
+            if (!mbar_wait_warp(bar(G_B3), par, abort_flag)) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {   // (o) Ot += V_new^T Mq^T ; (u) D3 += V_new^T (e^{b_C-b} K)
+                    const uint64_t a = v_k + desc_step(ks * 32);
+                    umma_f16(tm_x, a, mq + desc_step(ks * 32), id64, 1u);
+                    umma_f16(tm_d3, a, kq_mn + desc_step(ks * 2048), id_u, 1u);
+                }
+                umma_commit(bar(G_C3));
+            }
+            if (c + 1 < n_chunks) {            // (a) of the next chunk runs right behind; V_new has left the Ut columns
+                if (!mbar_wait_warp(bar(G_FULL_KQ), (c + 1) & 1, abort_flag)) break;
                 tc_fence_after();
-                if (elect_one()) {
-#pragma unroll
-                    for (int hl = 0; hl < 2; ++hl)    // (uw): T diag(beta) and T diag(beta e^b) as hi + lo pairs
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            const uint32_t acc = (hl > 0 || ks > 0) ? 1u : 0u;
-                            umma_f16(tm_ut, v_mn + desc_step(ks * 2048), wr_k + desc_step(hl * 8192 + ks * 32), id64_amn, acc);
-                            umma_f16(tm_x, kq_mn + desc_step(ks * 2048), wr_k + desc_step(16384 + hl * 8192 + ks * 32), id64_amn, acc);
-                        }
-                    umma_commit(bar(G_C1));
-                }
-                if (!mbar_wait_warp(bar(G_B2), par, abort_flag)) break;
-                tc_fence_after();
-                if (elect_one()) {
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {   // (ws) Ut -= S0^T W^T ; (o) Ot = S0^T (Q e^b)^T
-                        const uint64_t a = wr_k + desc_step((ks >> 2) * 16384 + (ks & 3) * 32);
-                        umma_f16(tm_ut, a, v_mn + desc_step(ks * 2048), id64_bmn_neg, 1u);
-                        umma_f16(tm_x, a, q_k + desc_step((ks >> 2) * 16384 + (ks & 3) * 32), id64, ks > 0 ? 1u : 0u);
-                    }
-                    umma_commit(bar(G_C2));
-                }
-                if (c + 1 < n_chunks) {            // the state tile is dead once these products are done: the next K/Q tiles go there
-                    if (!mbar_wait_warp(bar(G_C2), par, abort_flag)) break;
-                    load_kq(c + 1);
-                }
-                if (!mbar_wait_warp(bar(G_B3), par, abort_flag)) break;
-                tc_fence_after();
-                if (elect_one()) {
-#pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) {   // (o) Ot += V_new^T Mq^T ; (u) D3 += V_new^T (e^{b_C-b} K)
-                        const uint64_t a = v_k + desc_step(ks * 32);
-                        umma_f16(tm_x, a, mq + desc_step(ks * 32), id64, 1u);
-                        umma_f16(tm_d3, a, kq_mn + desc_step(ks * 2048), id_u, 1u);
-                    }
-                    umma_commit(bar(G_C3));
-                }
-                if (c + 1 < n_chunks) {            // (a) of the next chunk runs right behind; V_new has left the Ut columns
-                    if (!mbar_wait_warp(bar(G_FULL_KQ), (c + 1) & 1, abort_flag)) break;
-                    tc_fence_after();
-                    issue_a(c + 1);
-                }
+                issue_a(c + 1);
             }
         }
     } else {
@@ -748,7 +746,7 @@ la_chunk_walk_kernel(const unsigned char* __restrict__ images, const float* __re
     pdl_enter();
     const int h = blockIdx.x;
     const LaSeqMeta sq = seqs[blockIdx.y];
-    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), tid = threadIdx.x;
     const int n_chunks = (sq.count + kC - 1) / kC;
     if (n_chunks == 0) return;
     if (*reinterpret_cast<volatile int*>(error_word) != 0) return;
@@ -770,57 +768,55 @@ la_chunk_walk_kernel(const unsigned char* __restrict__ images, const float* __re
     const uint32_t tmem = *tmem_slot, tm_d3 = tmem, tm_ut = tmem + 128, tm_o = tmem + 192;       // O of even and odd chunks: 64 columns each
 
     if (warp == 8) {
-        {
-            constexpr uint32_t id64 = umma_idesc(kFmtF16, 128, 64, 0, 0);
-            constexpr uint32_t id64_bmn_neg = umma_idesc(kFmtF16, 128, 64, 0, 1) | (1u << 13);   // B MN-major, negated A
-            constexpr uint32_t id_u = umma_idesc(kFmtF16, 128, 128, 0, 1);
-            auto load = [&](int c) {
-                const uint32_t dst = base + 1024 + (c & 1) * kImgTiles;
-                const unsigned char* src = images + (unit0 + (size_t)c * kLaHeads) * kImg;
-                if (!elect_one()) return;
-                mbar_arrive_expect_tx(bar(W_FULL0 + (c & 1)), kImgTiles);
-                for (int i = 0; i < 7; ++i) bulk_g2s(dst + i * 8192, src + i * 8192, 8192, bar(W_FULL0 + (c & 1)));
-            };
-            load(0);
-            if (n_chunks > 1) load(1);
-            const uint64_t s_k = umma_smem_desc(base + kWalkS, 16, 1024), v_k = umma_smem_desc(base + kWalkV, 16, 1024);
-            int c = 0;
-            for (; c < n_chunks; ++c) {
-                const uint32_t par = c & 1, kq = base + 1024 + par * kImgTiles, w = kq + 32768, mq = kq + 49152, tm_x = tm_o + par * 64;
-                const uint64_t w_mn = umma_smem_desc(w, 8192, 1024), kq_mn = umma_smem_desc(kq, 16384, 1024), q_k = umma_smem_desc(kq + 8192, 16, 1024);
-                const uint64_t mq_k = umma_smem_desc(mq, 16, 1024);
-                if (!mbar_wait_warp(bar(W_FULL0 + par), (c >> 1) & 1, abort_flag)) break;
-                if (!mbar_wait_warp(bar(W_B2), par, abort_flag)) break;
-                tc_fence_after();
-                if (elect_one()) {
+        constexpr uint32_t id64 = umma_idesc(kFmtF16, 128, 64, 0, 0);
+        constexpr uint32_t id64_bmn_neg = umma_idesc(kFmtF16, 128, 64, 0, 1) | (1u << 13);   // B MN-major, negated A
+        constexpr uint32_t id_u = umma_idesc(kFmtF16, 128, 128, 0, 1);
+        auto load = [&](int c) {
+            const uint32_t dst = base + 1024 + (c & 1) * kImgTiles;
+            const unsigned char* src = images + (unit0 + (size_t)c * kLaHeads) * kImg;
+            if (!elect_one()) return;
+            mbar_arrive_expect_tx(bar(W_FULL0 + (c & 1)), kImgTiles);
+            for (int i = 0; i < 7; ++i) bulk_g2s(dst + i * 8192, src + i * 8192, 8192, bar(W_FULL0 + (c & 1)));
+        };
+        load(0);
+        if (n_chunks > 1) load(1);
+        const uint64_t s_k = umma_smem_desc(base + kWalkS, 16, 1024), v_k = umma_smem_desc(base + kWalkV, 16, 1024);
+        int c = 0;
+        for (; c < n_chunks; ++c) {
+            const uint32_t par = c & 1, kq = base + 1024 + par * kImgTiles, w = kq + 32768, mq = kq + 49152, tm_x = tm_o + par * 64;
+            const uint64_t w_mn = umma_smem_desc(w, 8192, 1024), kq_mn = umma_smem_desc(kq, 16384, 1024), q_k = umma_smem_desc(kq + 8192, 16, 1024);
+            const uint64_t mq_k = umma_smem_desc(mq, 16, 1024);
+            if (!mbar_wait_warp(bar(W_FULL0 + par), (c >> 1) & 1, abort_flag)) break;
+            if (!mbar_wait_warp(bar(W_B2), par, abort_flag)) break;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks)     // (ws) Ut -= S0^T W^T
-                        umma_f16(tm_ut, s_k + desc_step((ks >> 2) * 16384 + (ks & 3) * 32), w_mn + desc_step(ks * 2048), id64_bmn_neg, 1u);
-                    umma_commit(bar(W_C2));
+                for (int ks = 0; ks < 8; ++ks)     // (ws) Ut -= S0^T W^T
+                    umma_f16(tm_ut, s_k + desc_step((ks >> 2) * 16384 + (ks & 3) * 32), w_mn + desc_step(ks * 2048), id64_bmn_neg, 1u);
+                umma_commit(bar(W_C2));
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {   // (o) Ot = S0^T (Q e^b)^T, behind what V_new waits for
-                        const uint32_t off = desc_step((ks >> 2) * 16384 + (ks & 3) * 32);
-                        umma_f16(tm_x, s_k + off, q_k + off, id64, ks > 0 ? 1u : 0u);
-                    }
-                }
-                if (!mbar_wait_warp(bar(W_B3), par, abort_flag)) break;
-                tc_fence_after();
-                if (elect_one()) {
-#pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) {   // (u) D3 += V_new^T (e^{b_C-b} K) ; (o) Ot += V_new^T Mq^T
-                        const uint64_t a = v_k + desc_step(ks * 32);
-                        umma_f16(tm_d3, a, kq_mn + desc_step(ks * 2048), id_u, 1u);
-                        umma_f16(tm_x, a, mq_k + desc_step(ks * 32), id64, 1u);
-                    }
-                    umma_commit(bar(W_C3));
-                }
-                if (c + 2 < n_chunks) {            // this chunk's image is dead once its last products are done
-                    if (!mbar_wait_warp(bar(W_C3), par, abort_flag)) break;
-                    load(c + 2);
+                for (int ks = 0; ks < 8; ++ks) {   // (o) Ot = S0^T (Q e^b)^T, behind what V_new waits for
+                    const uint32_t off = desc_step((ks >> 2) * 16384 + (ks & 3) * 32);
+                    umma_f16(tm_x, s_k + off, q_k + off, id64, ks > 0 ? 1u : 0u);
                 }
             }
-            for (int e = c; e < min(c + 2, n_chunks); ++e) mbar_drain(bar(W_FULL0 + (e & 1)), (e >> 1) & 1);     // after a wait that ran out
+            if (!mbar_wait_warp(bar(W_B3), par, abort_flag)) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {   // (u) D3 += V_new^T (e^{b_C-b} K) ; (o) Ot += V_new^T Mq^T
+                    const uint64_t a = v_k + desc_step(ks * 32);
+                    umma_f16(tm_d3, a, kq_mn + desc_step(ks * 2048), id_u, 1u);
+                    umma_f16(tm_x, a, mq_k + desc_step(ks * 32), id64, 1u);
+                }
+                umma_commit(bar(W_C3));
+            }
+            if (c + 2 < n_chunks) {            // this chunk's image is dead once its last products are done
+                if (!mbar_wait_warp(bar(W_C3), par, abort_flag)) break;
+                load(c + 2);
+            }
         }
+        for (int e = c; e < min(c + 2, n_chunks); ++e) mbar_drain(bar(W_FULL0 + (e & 1)), (e >> 1) & 1);     // after a wait that ran out
     } else {
         const int r = tid & 127, hf = tid >> 7;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;

@@ -128,59 +128,57 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     } else if (warp == 9) {
         // ------------------------------ MMA issuer: the warp as one, an elected lane at each issue (elect_one) ------------------------------
         // Twenty products a key step: a thread on its own took some 80 cycles for each, more than the products themselves (55.7 -> 45.7 us at 5 x 771 tokens).
-        {
-            const uint64_t q_k = umma_smem_desc(base, 16, 1024), k_k = umma_smem_desc(base + L.off_k, 16, 1024), p_k = umma_smem_desc(base + L.off_p, 16, 1024);
-            const uint64_t v_mn = umma_smem_desc(base + L.off_v, kKBlk, 1024);
-            constexpr uint32_t id_s = umma_idesc(kFmtBF16, kLM, kLN, 0, 0);
-            const uint32_t id_pv = umma_idesc(kFmtBF16, kLM, 64 * L.nv, 0, 1);
-            // PV product of global step g; `first` overwrites O (the previous item's epilogue has read it), after `last` O is final
-            auto issue_pv = [&](int g, bool first, bool last, int it) -> bool {
-                const int b = g & 1, s = g % NST;
-                if (!mbar_wait_warp(bar(L_VF + s), (g / NST) & 1, abort_flag)) return false;
-                if (!mbar_wait_warp(bar(L_PF + b), (g >> 1) & 1, abort_flag)) return false;
-                if (first && it > 0 && !mbar_wait_warp(bar(L_OD), (it - 1) & 1, abort_flag)) return false;
-                tc_fence_after();
-                const uint64_t a = p_k + b * desc_step(kPBuf), v = v_mn + s * L.nv * desc_step(kKBlk);
-                if (elect_one()) {
+        const uint64_t q_k = umma_smem_desc(base, 16, 1024), k_k = umma_smem_desc(base + L.off_k, 16, 1024), p_k = umma_smem_desc(base + L.off_p, 16, 1024);
+        const uint64_t v_mn = umma_smem_desc(base + L.off_v, kKBlk, 1024);
+        constexpr uint32_t id_s = umma_idesc(kFmtBF16, kLM, kLN, 0, 0);
+        const uint32_t id_pv = umma_idesc(kFmtBF16, kLM, 64 * L.nv, 0, 1);
+        // PV product of global step g; `first` overwrites O (the previous item's epilogue has read it), after `last` O is final
+        auto issue_pv = [&](int g, bool first, bool last, int it) -> bool {
+            const int b = g & 1, s = g % NST;
+            if (!mbar_wait_warp(bar(L_VF + s), (g / NST) & 1, abort_flag)) return false;
+            if (!mbar_wait_warp(bar(L_PF + b), (g >> 1) & 1, abort_flag)) return false;
+            if (first && it > 0 && !mbar_wait_warp(bar(L_OD), (it - 1) & 1, abort_flag)) return false;
+            tc_fence_after();
+            const uint64_t a = p_k + b * desc_step(kPBuf), v = v_mn + s * L.nv * desc_step(kKBlk);
+            if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) umma_f16(tmem_o, a + desc_step(ks * 32), v + desc_step(ks * 2048), id_pv, (!first || ks > 0) ? 1u : 0u);
-                    umma_commit(bar(L_PV + b));
-                    umma_commit(bar(L_VE + s));
-                    if (last) umma_commit(bar(L_OF));
-                }
-                return true;
-            };
-            bool ok = true, pending = false, pfirst = false, plast = false;
-            int pg = 0, pitem = 0, gs = 0;
-            for (int i = 0; ok && i < n_my; ++i) {
-                const int n_kt = item(i).n_kt;
-                if (pending) {         // the previous item's last PV goes out before the wait for this item's Q tile
-                    if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
-                    pending = false;
-                }
-                if (!mbar_wait_warp(bar(L_Q), i & 1, abort_flag)) { ok = false; break; }
-                for (int j = 0; j < n_kt; ++j, ++gs) {
-                    const int b = gs & 1, s = gs % NST;
-                    if (!mbar_wait_warp(bar(L_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
-                    if (gs >= 2 && !mbar_wait_warp(bar(L_SE + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t k0 = k_k + s * nq * desc_step(kKBlk);
-                    if (elect_one()) {
-                        for (int blk = 0; blk < nq; ++blk)
-#pragma unroll
-                            for (int ks = 0; ks < 4; ++ks)
-                                umma_f16(tmem + b * kLN, q_k + blk * desc_step(kQBlk) + desc_step(ks * 32), k0 + blk * desc_step(kKBlk) + desc_step(ks * 32), id_s,
-                                         (blk > 0 || ks > 0) ? 1u : 0u);
-                        umma_commit(bar(L_SF + b));
-                        umma_commit(bar(L_KE + s));
-                        if (j == n_kt - 1) umma_commit(bar(L_QE));
-                    }
-                    if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
-                    pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
-                }
+                for (int ks = 0; ks < 4; ++ks) umma_f16(tmem_o, a + desc_step(ks * 32), v + desc_step(ks * 2048), id_pv, (!first || ks > 0) ? 1u : 0u);
+                umma_commit(bar(L_PV + b));
+                umma_commit(bar(L_VE + s));
+                if (last) umma_commit(bar(L_OF));
             }
-            if (ok && pending) issue_pv(pg, pfirst, plast, pitem);
+            return true;
+        };
+        bool ok = true, pending = false, pfirst = false, plast = false;
+        int pg = 0, pitem = 0, gs = 0;
+        for (int i = 0; ok && i < n_my; ++i) {
+            const int n_kt = item(i).n_kt;
+            if (pending) {         // the previous item's last PV goes out before the wait for this item's Q tile
+                if (!issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
+                pending = false;
+            }
+            if (!mbar_wait_warp(bar(L_Q), i & 1, abort_flag)) { ok = false; break; }
+            for (int j = 0; j < n_kt; ++j, ++gs) {
+                const int b = gs & 1, s = gs % NST;
+                if (!mbar_wait_warp(bar(L_KF + s), (gs / NST) & 1, abort_flag)) { ok = false; break; }
+                if (gs >= 2 && !mbar_wait_warp(bar(L_SE + b), ((gs >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t k0 = k_k + s * nq * desc_step(kKBlk);
+                if (elect_one()) {
+                    for (int blk = 0; blk < nq; ++blk)
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_f16(tmem + b * kLN, q_k + blk * desc_step(kQBlk) + desc_step(ks * 32), k0 + blk * desc_step(kKBlk) + desc_step(ks * 32), id_s,
+                                     (blk > 0 || ks > 0) ? 1u : 0u);
+                    umma_commit(bar(L_SF + b));
+                    umma_commit(bar(L_KE + s));
+                    if (j == n_kt - 1) umma_commit(bar(L_QE));
+                }
+                if (pending && !issue_pv(pg, pfirst, plast, pitem)) { ok = false; break; }
+                pending = true; pg = gs; pfirst = (j == 0); plast = (j == n_kt - 1); pitem = i;
+            }
         }
+        if (ok && pending) issue_pv(pg, pfirst, plast, pitem);
     } else {
         // ------------------------------ softmax / correction / epilogue ------------------------------
         const int r = threadIdx.x & 127;                 // query row == TMEM lane
