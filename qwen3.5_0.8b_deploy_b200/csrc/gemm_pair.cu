@@ -529,7 +529,9 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const PairArgs p) {
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();                   // neither CTA reads the other's shared memory, arrives on its barriers or works on its TMEM any more
+    // Neither CTA reads the other's shared memory, arrives on its barriers or works on its TMEM any more: each has waited for what it started there.  Nothing
+    // is handed over here, so the arrival need not wait for this CTA's stores (475 us for 3 x 333 tokens through four layers with, 473 without that).
+    cluster_stay();
     if (warp == kEpiWarps + 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem, 512);

@@ -119,6 +119,11 @@ __device__ __forceinline__ void cluster_sync_all() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same where nothing that was written has to be seen: no CTA goes on, and none leaves, before the others have come this far.
+__device__ __forceinline__ void cluster_stay() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 
 // Warp-uniform form for roles whose next instruction is warp-collective (.sync.aligned): either every
 // lane proceeds or every lane gives up.

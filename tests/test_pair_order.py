@@ -25,7 +25,7 @@ def test_every_wait_of_a_pair_is_of_cluster_scope():
     for kernel, body in pairs.items():
         waits = re.findall(r"\bmbar_(?:try_|test_)?wait(?:_warp)?\b\s*(<\w+>)?", body)
         assert waits and set(waits) == {"<kClusterScope>"}, kernel
-        assert not re.search(r"\bcluster_\w*meet\w*\b", body), kernel
+        assert re.findall(r"\bcluster_(\w+)\(\);", body) == ["sync_all", "stay"], kernel        # barriers and TMEM are handed over, the exit is not
         loads = set(re.findall(r"\btma_load_2d\w*\b", body))
         assert loads == {"tma_load_2d_pair"}, kernel
         signal = re.search(r"const uint32_t dst = [^;]*, bar = (\w+) \+ 8u \* s;", body)
