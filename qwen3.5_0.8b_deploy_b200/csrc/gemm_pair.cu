@@ -605,13 +605,14 @@ int gemm_glu(cudaStream_t s, ElemType t, int act_kind, const void* x, const void
     return launch_pair<kPairGlu, __nv_bfloat16, B200ATTN_ACT_GELU_TANH>(m, p, s);
 }
 
-// A tile goes through all its weights whatever its rows, and a start of a sequence costs its chunk of 32 tokens a look-up of the state that nothing hides;
-// the library's product with la_conv_seq_kernel behind it pays for neither.  A prompt pass of three such layers and an attention layer, in parts / fused in
-// us: 1 x 1000 622 / 591; 4 x 100 406 / 413, 4 x 140 460 / 459, 4 x 220 515 / 501; 8 x 60 396 / 417, 8 x 100 491 / 483; 32 x 40 615 / 631, 32 x 50 674 / 668; 64 x 40 952 / 954, 64 x 48 1044 / 1007; 128 x 20 1159 / 1169, 128 x 26 1308 / 1275, 128 x 64 2263 / 2045
-// (around the line, of 3 and 4 tiles of rows in 6 or 8 sequences, up to 2.7 % either way).  The projection and convolution alone with sequences of 16 tokens:
-// 256 x 16 122 / 128, 512 x 16 225 / 243, 1024 x 16 431 / 553; of 32: 256 x 32 213 / 197.  One sequence of 4 to 128 rows takes 19 to 23 us against 15 to 19
-// in parts, but a user who waits for every call is served sooner without the parts' run table (a prompt and two tokens, in parts / fused: 9 tokens 714 /
-// 691 us, 77 786 / 771, 128 770 / 770, 253 804 / 800).
+// A tile goes through all its weights whatever its rows, and a start of a sequence costs its chunk of 32 tokens a look-up of the state that nothing
+// hides; the library's product with la_conv_seq_kernel behind it pays for neither.  A prompt pass of three such layers and an attention layer, in parts
+// / fused in us: 1 x 1000 622 / 591; 4 x 100 406 / 413, 4 x 140 460 / 459, 4 x 220 515 / 501; 8 x 60 396 / 417, 8 x 100 491 / 483; 32 x 40 615 / 631, 32
+// x 50 674 / 668; 64 x 40 952 / 954, 64 x 48 1044 / 1007; 128 x 20 1159 / 1169, 128 x 26 1308 / 1275, 128 x 64 2263 / 2045 (around the line, of 3 and 4
+// tiles of rows in 6 or 8 sequences, up to 2.7 % either way).  The projection and convolution alone with sequences of 16 tokens: 256 x 16 122 / 128, 512
+// x 16 225 / 243, 1024 x 16 431 / 553; of 32: 256 x 32 213 / 197.  One sequence of 4 to 128 rows takes 19 to 23 us against 15 to 19 in parts, but a user
+// who waits for every call is served sooner without the parts' run table (a prompt and two tokens, in parts / fused: 9 tokens 714 / 691 us, 77 786 /
+// 771, 128 770 / 770, 253 804 / 800).
 bool gemm_la_conv_takes(const void* x, const void* w, long long rows, int n_seqs) {
     const bool long_enough = n_seqs == 1 || (rows >= std::min(300 + 36LL * n_seqs, 3000LL) && rows >= 24LL * n_seqs);
     return long_enough && aligned16(x) && aligned16(w);
